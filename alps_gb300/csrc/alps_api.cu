@@ -136,7 +136,6 @@ void alps_destroy(alps_ctx* c) {
     cudaFree(S.d_G);
     cudaFree(S.d_X);
     cudaFree(S.d_mom);
-    cudaFree(S.d_momf);
     cudaFree(S.d_Vh);  // d_Vl points into it
     cudaFree(S.d_Vscale);
     cudaFree(S.d_Bt);
@@ -157,7 +156,6 @@ void alps_destroy(alps_ctx* c) {
   cudaFree(c->d_om);
   cudaFree(c->d_D);
   cudaFree(c->d_part);
-  cudaFree(c->d_low);
   cudaFree(c->d_count);
   cudaFree(c->d_slot_nn);
   cudaFree(c->d_items);

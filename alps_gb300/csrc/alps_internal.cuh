@@ -77,9 +77,6 @@ struct __align__(16) SpecDev {
   const double* bessel;
   const double* V;
   const double* mom;  // Laurent moments [(nmax+1)][ALPS_KFAR][12]
-  const float* momf;  // the same moments rounded to FP32 (for the series tails)
-  const float* momh;  // the moments as float pairs scaled like Vh/Vl (momh + moml)
-  const float* moml;
   // V as pairs of floats (hi + lo, ~48 bits) scaled by 2^-e per order, Vscale
   // = 2^e, and ppar as float pairs: the fast path's node sums run on the
   // FP32 pipes in double-float arithmetic
@@ -190,8 +187,6 @@ struct SpeciesHost {
   double* d_G = nullptr;                  // contraction RHS [2][N-1][M-1]
   double* d_X = nullptr;                  // x_j^k, x_j = (ppar_j - pcen)/prad
   double* d_mom = nullptr;                // Laurent moments
-  float* d_momf = nullptr;                // the same in FP32; the pairs below share its allocation
-  float *d_momh = nullptr, *d_moml = nullptr;  // the moments as float pairs (scale Vscale per order)
   float* d_Bt = nullptr;                  // base tables of the fast pole sums: Bt, mBt, bfac
   size_t Bt_cap = 0;
   double* d_Bd = nullptr;                 // and their FP64 part: Escale[8], Cfull, Pre
@@ -203,7 +198,6 @@ struct SpeciesHost {
   double* d_Vscale = nullptr;             // per-order scale of the pairs
   size_t Vs_cap = 0;
   float *d_pph = nullptr, *d_ppl = nullptr;  // ppar as float pairs
-  size_t momf_cap = 0;
   double* d_fit_aux = nullptr;            // Maxwellian continuation factors
   bool aux_ready = false;                 // d_fit_aux and the Landau row bounds are those of the current fit
   double* d_lmom = nullptr;               // factorised Landau moments
@@ -241,8 +235,6 @@ struct alps_ctx {
   double2* d_D = nullptr;       // [n]
   double2* d_part = nullptr;    // [n][S][nchunk][6]
   size_t part_cap = 0;
-  double2* d_low = nullptr;     // [n][S][nchunk][3][6]
-  size_t low_cap = 0;
   int* d_count = nullptr;       // [n][S]
   size_t count_cap = 0;
   int* d_slot_nn = nullptr;     // [n][S][rcap]

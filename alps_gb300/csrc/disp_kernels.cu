@@ -57,9 +57,13 @@ struct __align__(16) DispArgs {
 // per warp of k_resonant.  It follows from the batch size and the context
 // alone, so a batch sums in the same order wherever it runs.
 struct DispShape {
-  int nchunk;    // order chunks per species
-  int csize;     // orders per chunk
+  int js;        // lanes per frequency of the pole sums (a power of two up to 32)
+  int wt;        // warps of frequencies: ceil(n js / 32)
+  int kmid;      // longest Laurent series that a lane sums alone
+  int nchunk;    // order chunks of the species with the most (the stride of the partial sums)
+  int nch[ALPS_MAX_SPECIES];  // order chunks of each species (0: no pole sums)
   int ipw;       // resonant-item slots per warp of k_resonant (1..256)
+  int fin_warp;  // k_finalize takes a warp per omega (else a thread)
 };
 
 namespace {
@@ -112,9 +116,22 @@ __device__ __forceinline__ void classify_body(const DispArgs& a, const double2* 
 }
 
 // ---------------------------------------------------------------------------
-// Pole sums.  Block = TW omegas x JS slices of j.  grid = (omega tiles,
-// species, order chunks).  Each thread accumulates the six chi entries of its
-// omega over the orders of its chunk (and the n = -1,0,1 parts for chi_low).
+// Pole sums.
+//
+// A warp is 32 / js frequencies by js lanes, js a power of two (32: one
+// frequency over the whole warp, for a few of them; 1: one frequency a
+// lane, for lattices).  Its unit of work is an order chunk of one species:
+// the signed orders nn = -nmax + chunk, + nch, + 2 nch, ...  The stride
+// spreads the orders near resonance, which are neighbours and cost a sum
+// over the p_par nodes each, over the chunks; contiguous chunks left them
+// all in one block, which the others waited for.
+//
+// The js lanes of a frequency take an order each for what an order's set-up
+// needs (the resonance geometry and its FP64 divisions) and for the Laurent
+// series of far poles, whose set-up costs more than its few terms; the
+// orders left, long series and node sums, then go over the lanes one by
+// one, the lanes slicing their terms.  Each lane keeps its own sums and the
+// lanes are added once per chunk.
 // ---------------------------------------------------------------------------
 // Complex double-float helpers of the order-fused pole sums
 __device__ __forceinline__ void df_cmul2(dflt ax, dflt ay, dflt bx, dflt by, dflt& rx, dflt& ry) {
@@ -144,10 +161,101 @@ __device__ __forceinline__ cdf om_combr(cdf o, dflt kap, dflt c1, dflt c2) {
   return {df_add(df_mul(o.x, c1), df_mul(kap, c2)), df_mul(o.y, c1)};
 }
 
+#define FULL_WARP 0xffffffffu
+
+// adds the js adjacent lanes' values by halving: each step hands half of a
+// lane's values to its partner, so 12 values over 32 lanes take 13 additions
+// a lane and not 60.  On return v[0 .. cnt) holds the totals of components
+// first .. first + cnt of the lane's frequency (cnt 0: none).
+struct dbl_val {
+  double v;
+};
+__device__ __forceinline__ dbl_val lane_add(dbl_val a, int off) {
+  return {a.v + __shfl_xor_sync(FULL_WARP, a.v, off)};
+}
+__device__ __forceinline__ dflt lane_add(dflt a, int off) {
+  return df_add(a, {__shfl_xor_sync(FULL_WARP, a.h, off), __shfl_xor_sync(FULL_WARP, a.l, off)});
+}
+// keep + the partner's give
+__device__ __forceinline__ dbl_val lane_swap_add(dbl_val keep, dbl_val give, int off) {
+  return {keep.v + __shfl_xor_sync(FULL_WARP, give.v, off)};
+}
+__device__ __forceinline__ dflt lane_swap_add(dflt keep, dflt give, int off) {
+  return df_add(keep, {__shfl_xor_sync(FULL_WARP, give.h, off), __shfl_xor_sync(FULL_WARP, give.l, off)});
+}
+template <typename T>
+__device__ __forceinline__ void lane_sum12(T v[12], int js, int lane, int& first, int& cnt) {
+  first = 0;
+  cnt = 12;
+  int off = js >> 1;
+  if (off == 0) return;
+  bool hi = lane & off;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) v[q] = lane_swap_add(hi ? v[6 + q] : v[q], hi ? v[q] : v[6 + q], off);
+  first = hi ? 6 : 0;
+  cnt = 6;
+  off >>= 1;
+  if (off == 0) return;
+  hi = lane & off;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) v[q] = lane_swap_add(hi ? v[3 + q] : v[q], hi ? v[q] : v[3 + q], off);
+  first += hi ? 3 : 0;
+  cnt = 3;
+  off >>= 1;
+  if (off == 0) return;
+  // three values: the lower lane keeps two, the upper one (its second is
+  // the lower lane's second added to itself, unused)
+  hi = lane & off;
+  {
+    const T k0 = lane_swap_add(hi ? v[2] : v[0], hi ? v[0] : v[2], off);
+    v[1] = lane_swap_add(v[1], v[1], off);
+    v[0] = k0;
+  }
+  first += hi ? 2 : 0;
+  cnt = hi ? 1 : 2;
+  off >>= 1;
+  if (off == 0) return;
+  const bool two = cnt == 2;  // the same on both partners of the steps below
+  hi = lane & off;
+  {
+    const T s0 = lane_swap_add((hi && two) ? v[1] : v[0], (hi || !two) ? v[0] : v[1], off);
+    v[0] = s0;
+  }
+  if (two) {
+    first += hi ? 1 : 0;
+    cnt = 1;
+  } else {
+    cnt = hi ? 0 : 1;
+  }
+  off >>= 1;
+  if (off == 0) return;
+  v[0] = lane_add(v[0], off);
+  if (lane & off) cnt = 0;
+}
+
+// what the lanes of a frequency need of one signed order
+struct OrderInfo {
+  int nn, K, K32;         // K > kfar: node sum; else the Laurent terms (K32 of them in double-float)
+  int lo1, hi1, lo2, hi2; // summed node ranges
+  int flags;              // 1 resonant, 2 the double-float node sum applies
+};
+__device__ __forceinline__ OrderInfo shfl_info(const OrderInfo& a, int src) {
+  OrderInfo r;
+  r.nn = __shfl_sync(FULL_WARP, a.nn, src);
+  r.K = __shfl_sync(FULL_WARP, a.K, src);
+  r.K32 = __shfl_sync(FULL_WARP, a.K32, src);
+  r.lo1 = __shfl_sync(FULL_WARP, a.lo1, src);
+  r.hi1 = __shfl_sync(FULL_WARP, a.hi1, src);
+  r.lo2 = __shfl_sync(FULL_WARP, a.lo2, src);
+  r.hi2 = __shfl_sync(FULL_WARP, a.hi2, src);
+  r.flags = __shfl_sync(FULL_WARP, a.flags, src);
+  return r;
+}
+
 // ---------------------------------------------------------------------------
-// Fast path of the pole sums (no chi_low), on the base tables: per (omega,
-// signed order) the sums of the three Bessel families against g1 and g2
-// (6 real vectors, complex weights), in double-float on the FP32 pipes:
+// Fast path, on the base tables: per (omega, signed order) the sums of the
+// three Bessel families against g1 and g2 (6 real vectors, complex
+// weights), in double-float on the FP32 pipes:
 //   * node sums Q = sum_j w_j F_j R_j, R_j = 1/(A - k_par p_j + i D), the
 //     p_par-weighted entries from zeta Q - (1/k_par) sum w F (the sums of
 //     the family vectors over the summed ranges: full-range table, or FP64
@@ -161,10 +269,17 @@ __device__ __forceinline__ cdf om_combr(cdf o, dflt kap, dflt c1, dflt c2) {
 // added, times the order factor C0 v_e(n) (sign of -n for xy, xz), to one
 // double-float sum per entry; the phase (i for xy, yz) and the entry scale
 // are applied once per chunk in FP64.
+//
+// Bound by FP32 issue on lattices and by the length of one warp's chain of
+// instructions on a few frequencies.  One loop body serves every order (a
+// lane's own series, then the orders shared by the lanes), which keeps the
+// code in the instruction cache.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, double2 o, int js, int js_count,
-                                           int n_begin, int n_end, double2* acc_out) {
-  const int M = S.M;
+__device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, double2 o, bool active, int js,
+                                           int chunk, int nch, int kmid, double* out) {
+  const int M = S.M, U_ = 2 * S.nmax + 1;
+  const int lane = threadIdx.x & 31, j = lane & (js - 1), gbase = lane - j;
+  const unsigned gmask = (js == 32) ? FULL_WARP : (((1u << js) - 1u) << gbase);
   const double kpar = sys.kpar;
   dflt acc[12];
 #pragma unroll
@@ -178,51 +293,54 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
   const dflt dyd = df_mul(Dd, ikd);  // Im p_res
   const dflt mox = df_mul(msd, oxd);
   const float ikp32 = (float)sys.ikpar;
-  const int k0 = (js >= 2) ? js : js + js_count * ((2 - js + js_count - 1) / js_count);  // first k >= 2
-  for (int n = n_begin; n < n_end; ++n) {
-    const float* __restrict__ Bn = S.Bt + (size_t)n * (M - 1) * 12;
-    const float* __restrict__ mBn = S.mBt + (size_t)n * ALPS_KFAR * 12;
-    for (int sg = 0; sg < (n == 0 ? 1 : 2); ++sg) {
-      const int nn = sg ? -n : n;
+  for (int i0 = 0; chunk + i0 * nch < U_; i0 += js) {
+    // ---- this lane's own order: resonance geometry, series or nodes ----
+    const int u = chunk + (i0 + j) * nch;
+    const bool own = active && u < U_;
+    OrderInfo cur = {0, S.kfar + 1, S.kfar + 1, 1, 0, 1, 0, 0};
+    if (own) {
+      const int nn = u - S.nmax;
       // A = m omega_r - nn q, the pole's real part times k_par
       const dflt Ad = df_add(mox, df_neg(df_mul({(float)nn, 0.0f}, qsd)));
       const float x32 = Ad.h * ikp32;
       const float mg = 9.5367431640625e-7f * fabsf(x32);  // 2^-20 |x|
-      ResGeom g;
+      bool res = false;
       float ddf;  // |p_res - pcen|^2 (in FP32 alone for orders far from resonance)
+      cur.nn = nn;
+      cur.hi1 = M - 1;
       if (x32 < S.qlo - mg || x32 > S.qhi + mg) {
-        g.res = 0;
-        g.lo1 = 1;
-        g.hi1 = M - 1;
-        g.lo2 = 1;
-        g.hi2 = 0;
         const float dx = x32 - S.pcen32;
         ddf = fmaf(dx, dx, dyd.h * dyd.h);
       } else {
-        g = res_geometry(S, sys.M_I, o, nn, kpar);
+        const ResGeom g = res_geometry(S, sys.M_I, o, nn, kpar);
         const double2 dfar = cmk(g.pr - S.pcen, g.pi);
         ddf = (float)(dfar.x * dfar.x + dfar.y * dfar.y);
+        res = g.res;
+        cur.lo1 = g.lo1;
+        cur.hi1 = g.hi1;
+        cur.lo2 = g.lo2;
+        cur.hi2 = g.hi2;
       }
-      int K = S.kfar + 1, K32 = K;
       // the series is used up to rho^2 < 0.58, where its K <= kfar terms
       // (checked below) cost less than the node sum
-      if (!g.res && S.prad32 * S.prad32 < 0.58f * ddf) {
+      if (!res && S.prad32 * S.prad32 < 0.58f * ddf) {
         const float rho = S.prad32 * rsqrtf(ddf);
         const float lr = -__logf(rho), l1 = log1pf(-rho);
-        K = (int)ceilf((36.7368006f - l1) / lr) + 1;    // 53 ln 2
-        K32 = (int)ceilf((22.8738570f - l1) / lr) + 1;  // 33 ln 2
+        cur.K = (int)ceilf((36.7368006f - l1) / lr) + 1;    // 53 ln 2
+        cur.K32 = (int)ceilf((22.8738570f - l1) / lr) + 1;  // 33 ln 2
       }
       // the double-float values stay normal floats: |f| = 1/(k_par |d|) for
       // the series, |A - k_par p_j|^2 + D^2 at the summed ranges' ends for
       // the node sum (zero if the pole lies inside a summed range)
-      if (K <= S.kfar) {
+      if (cur.K <= S.kfar) {
         const float fm = fabsf(ikp32) * rsqrtf(ddf);
-        if (!(fm >= 1e-30f && fm <= 1e30f)) K = K32 = S.kfar + 1;
+        if (!(fm >= 1e-30f && fm <= 1e30f)) cur.K = cur.K32 = S.kfar + 1;
       }
       bool nodes_df = true;
-      if (K > S.kfar) {
+      if (cur.K > S.kfar) {
         float lo = 3.0e38f, hi = 0.0f;
-        const int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
+        const int ends[4] = {cur.lo1, cur.hi1, cur.lo2, cur.hi2};
+#pragma unroll
         for (int r2 = 0; r2 < 2; ++r2) {
           const int j0 = max(1, ends[2 * r2]), j1 = min(M - 1, ends[2 * r2 + 1]);
           if (j0 > j1) continue;
@@ -233,537 +351,376 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
         const float d2 = D2.h;
         nodes_df = d2 + lo * lo >= 1e-30f && d2 + hi * hi <= 1e30f;
       }
-      cdf X[6];  // the order's entries (xx yy zz xy xz yz), scaled by 1/Vscale[n]
-      if (K > S.kfar && !nodes_df) {
-        // FP64 node sum of this order over V, X_e = omega S_e1 + kappa S_e2
-        const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
-        const double Ar = S.ms * o.x - (double)nn * S.qs, Di = S.ms * o.y;
-        double2 Sx[12];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
-        auto nd = [&](int j, double wgt) {
-          const double dr = fma(-kpar, S.ppar[j], Ar);
-          const double rr = wgt / fma(dr, dr, Di * Di);
-          const double* v = Vn + (size_t)(j - 1) * 12;
-#pragma unroll
-          for (int q = 0; q < 12; ++q) {
-            Sx[q].x = fma(v[q], dr * rr, Sx[q].x);
-            Sx[q].y = fma(v[q], -Di * rr, Sx[q].y);
-          }
-        };
-        for (int j = 1 + js; j <= M - 1; j += js_count)
-          if ((j >= g.lo1 && j <= g.hi1) || (j >= g.lo2 && j <= g.hi2)) nd(j, 1.0);
-        const int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
-        for (int r2 = 0; r2 < 2; ++r2) {
-          const int lo = ends[2 * r2], hi = ends[2 * r2 + 1];
-          if (lo >= hi) continue;
-          for (int side = 0; side < 2; ++side) {
-            const int j = side ? hi : lo;
-            if (j >= 1 && j <= M - 1 && ((j - 1) % js_count) == js) nd(j, -0.5);
-          }
-        }
-        const double isc = 1.0 / S.Vscale[n], kapd = S.kappa;
-#pragma unroll
-        for (int e = 0; e < 6; ++e) {
-          const double2 t = cscale(cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kapd)), isc);
-          X[e] = {df_of(t.x), df_of(t.y)};
-        }
-      } else if (K <= S.kfar) {
-        // Laurent series: d = p_res - pcen, t = prad/d, f = 1/(k_par d)
-        const cdf d = {df_add(df_mul(Ad, ikd), df_neg(pcd)), dyd};
-        const dflt r = df_rcp_approx(df_add(df_mul(d.x, d.x), df_mul(d.y, d.y)));
-        const cdf iv = {df_mul(d.x, r), df_neg(df_mul(d.y, r))};
-        const cdf t1 = cdf_rmul(iv, prd), f = cdf_rmul(iv, ikd);
-        // U = f sum_{k >= 2} mom_k t^k over this slice's k: powers from f t^k0,
-        // step t^js_count (both by squaring)
-        cdf tp = f, st = t1;
-        {
-          cdf pw = t1;
-          for (int q = k0; q; q >>= 1) {
-            if (q & 1) tp = cdf_mul(tp, pw);
-            pw = cdf_mul(pw, pw);
-          }
-          for (int q = js_count; q > 1; q >>= 1) st = cdf_mul(st, st);
-        }
-        dflt U[12];
-        float Uf[12];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) {
-          U[q] = {0.0f, 0.0f};
-          Uf[q] = 0.0f;
-        }
-        int k = k0;
-        for (; k < K32; k += js_count) {
-          const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
-          const float4 a0 = __ldg(m4), a1 = __ldg(m4 + 1), a2 = __ldg(m4 + 2);
-          const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
-#pragma unroll
-          for (int b = 0; b < 6; ++b) {
-            df_mac(U[2 * b], hb[b], lb[b], tp.x);
-            df_mac(U[2 * b + 1], hb[b], lb[b], tp.y);
-          }
-          tp = cdf_mul(tp, st);
-        }
-        if (k < K) {
-          // the tail: terms below 2^-33 of the bound, in FP32
-          float fx = tp.x.h + tp.x.l, fy = tp.y.h + tp.y.l;
-          const float gx = st.x.h + st.x.l, gy = st.y.h + st.y.l;
-          for (; k < K; k += js_count) {
-            const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
-            const float4 a0 = __ldg(m4);
-            const float2 a1 = __ldg(reinterpret_cast<const float2*>(m4 + 1));
-            const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
-#pragma unroll
-            for (int b = 0; b < 6; ++b) {
-              Uf[2 * b] = fmaf(hb[b], fx, Uf[2 * b]);
-              Uf[2 * b + 1] = fmaf(hb[b], fy, Uf[2 * b + 1]);
-            }
-            const float nx = fx * gx - fy * gy;
-            fy = fx * gy + fy * gx;
-            fx = nx;
-          }
-        }
-        // per family F1, F2, F3: omega U_{F,g1} + kappa U_{F,g2}
-        cdf Uw[3];
-#pragma unroll
-        for (int fm = 0; fm < 3; ++fm) {
-          const int b1 = 2 * fm, b2 = 2 * fm + 1;
-          const cdf u1 = {df_add(U[2 * b1], {Uf[2 * b1], 0.0f}), df_add(U[2 * b1 + 1], {Uf[2 * b1 + 1], 0.0f})};
-          const cdf u2 = {df_add(U[2 * b2], {Uf[2 * b2], 0.0f}), df_add(U[2 * b2 + 1], {Uf[2 * b2 + 1], 0.0f})};
-          Uw[fm] = om_comb(omd, kap, u1, u2);
-        }
-        // T = f mom_1 t + U, Q = f mom_0 + T on the slices that own k = 1, 0
-        cdf T[3] = {Uw[0], Uw[1], Uw[2]};
-        auto mterm = [&](int kk, cdf w, cdf* out) {
-          const float* m = mBn + (size_t)kk * 12;
-#pragma unroll
-          for (int fm = 0; fm < 3; ++fm) {
-            const cdf mw = om_combr(omd, kap, {m[2 * fm], m[6 + 2 * fm]}, {m[2 * fm + 1], m[6 + 2 * fm + 1]});
-            out[fm] = cdf_add(out[fm], cdf_mul(w, mw));
-          }
-        };
-        if (js == 1 % js_count) mterm(1, cdf_mul(f, t1), T);
-        cdf Q[3] = {T[0], T[1], T[2]};
-        if (js == 0) mterm(0, f, Q);
-        X[0] = Q[0];
-        X[1] = Q[1];
-        X[3] = Q[2];
-        X[4] = cdf_mul(d, T[0]);
-        X[5] = cdf_mul(d, T[2]);
-        if (S.pcen32 != 0.0f) {
-          // sum F p R = pcen Q + d T, sum F p^2 R = pcen (sum F p R) + d (pcen T + d U)
-          X[4] = cdf_add(cdf_rmul(Q[0], pcd), X[4]);
-          X[5] = cdf_add(cdf_rmul(Q[2], pcd), X[5]);
-          X[2] = cdf_add(cdf_rmul(X[4], pcd), cdf_mul(d, cdf_add(cdf_rmul(T[0], pcd), cdf_mul(d, Uw[0]))));
-        } else {
-          X[2] = cdf_mul(d, cdf_mul(d, Uw[0]));
-        }
-      } else {
-        // node sum in double-float: Q_b = sum_j w_j B_b(j) / (A - k_par p_j + i D)
-        dflt Qs[12];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) Qs[q] = {0.0f, 0.0f};
-        // node j's terms; the trapezoid ends enter again at weight -1/2
-        auto node = [&](int j, bool end) {
-          const dflt dr = df_add(Ad, df_neg(df_mul(kd, {S.pph[j], S.ppl[j]})));
-          const dflt r = df_rcp_approx(df_add(df_mul(dr, dr), D2));
-          dflt Rr = df_mul(dr, r), Ri = df_neg(df_mul(Dd, r));
-          if (end) {
-            Rr = df_scale(Rr, -0.5f);
-            Ri = df_scale(Ri, -0.5f);
-          }
-          const float4* b4 = reinterpret_cast<const float4*>(Bn + (size_t)(j - 1) * 12);
-          const float4 a0 = __ldg(b4), a1 = __ldg(b4 + 1), a2 = __ldg(b4 + 2);
-          const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
-#pragma unroll
-          for (int b = 0; b < 6; ++b) {
-            df_mac(Qs[2 * b], hb[b], lb[b], Rr);
-            df_mac(Qs[2 * b + 1], hb[b], lb[b], Ri);
-          }
-        };
-        const int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
-        // the summed ranges (disjoint), each over this slice's nodes
-        // j = 1 + js (mod js_count)
-#pragma unroll
-        for (int r2 = 0; r2 < 2; ++r2) {
-          const int lo = max(1, ends[2 * r2]), hi = min(M - 1, ends[2 * r2 + 1]);
-          const int j0 = lo + (((js - (lo - 1)) % js_count) + js_count) % js_count;
-          for (int j = j0; j <= hi; j += js_count) node(j, false);
-        }
-        // trapezoid end weights
-#pragma unroll
-        for (int r2 = 0; r2 < 2; ++r2) {
-          const int lo = ends[2 * r2], hi = ends[2 * r2 + 1];
-          if (lo >= hi) continue;
-#pragma unroll
-          for (int side = 0; side < 2; ++side) {
-            const int j = side ? hi : lo;
-            if (j >= 1 && j <= M - 1 && ((j - 1) % js_count) == js) node(j, true);
-          }
-        }
-        cdf P[3];
-#pragma unroll
-        for (int fm = 0; fm < 3; ++fm)
-          P[fm] = om_comb(omd, kap, {Qs[4 * fm], Qs[4 * fm + 1]}, {Qs[4 * fm + 2], Qs[4 * fm + 3]});
-        const cdf zeta = {df_mul(Ad, ikd), dyd};
-        X[0] = P[0];
-        X[1] = P[1];
-        X[3] = P[2];
-        cdf xz = cdf_mul(zeta, P[0]), yz = cdf_mul(zeta, P[2]);
-        cdf cp = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-        if (js == 0) {
-          // (1/k_par) times the omega-combined sums of F1, F3 and p_par F1
-          // over the summed ranges (slice 0 adds them once)
-          double C[6];
-          const double* __restrict__ Cf = S.Cfull + (size_t)n * 6;
-          if (!g.res) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) C[c] = Cf[c];
-          } else {
-            const double* __restrict__ P0 = S.Pre + (size_t)n * M * 6;
-            const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
-            const double isc = 1.0 / S.Vscale[n];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) C[c] = 0.0;
-            for (int r2 = 0; r2 < 2; ++r2) {
-              const int lo = max(1, ends[2 * r2]), hi = min(M - 1, ends[2 * r2 + 1]);
-              if (lo > hi) continue;
-              const bool trap = ends[2 * r2] < ends[2 * r2 + 1];
-#pragma unroll
-              for (int c = 0; c < 6; ++c) {
-                const int q = (c < 2) ? c : c + 4;
-                double v = P0[(size_t)hi * 6 + c] - P0[(size_t)(lo - 1) * 6 + c];
-                if (trap) v -= 0.5 * (Vn[(size_t)(lo - 1) * 12 + q] + Vn[(size_t)(hi - 1) * 12 + q]) * isc;
-                C[c] += v;
-              }
-            }
-          }
-          const dflt ik = ikd;
-          const cdf c1 = cdf_rmul(om_combr(omd, kap, df_of(C[0]), df_of(C[1])), ik);
-          const cdf c3 = cdf_rmul(om_combr(omd, kap, df_of(C[2]), df_of(C[3])), ik);
-          cp = cdf_rmul(om_combr(omd, kap, df_of(C[4]), df_of(C[5])), ik);
-          xz = {df_add(xz.x, df_neg(c1.x)), df_add(xz.y, df_neg(c1.y))};
-          yz = {df_add(yz.x, df_neg(c3.x)), df_add(yz.y, df_neg(c3.y))};
-        }
-        const cdf zz = cdf_mul(zeta, xz);
-        X[2] = {df_add(zz.x, df_neg(cp.x)), df_add(zz.y, df_neg(cp.y))};
-        X[4] = xz;
-        X[5] = yz;
-      }
-      // add the order's entries with its factors C0 v_e(n) (xy and xz odd in n)
-      const float* __restrict__ fac = S.bfac + (size_t)n * 12;
-#pragma unroll
-      for (int e = 0; e < 6; ++e) {
-        dflt fe = {fac[2 * e], fac[2 * e + 1]};
-        if (nn < 0 && (e == 3 || e == 4)) fe = df_neg(fe);
-        df_acc(acc[2 * e], df_mul(fe, X[e].x));
-        df_acc(acc[2 * e + 1], df_mul(fe, X[e].y));
-      }
+      cur.flags = (res ? 1 : 0) | (nodes_df ? 2 : 0);
     }
-  }
-  // rescale and apply the phase (i for xy and yz)
+    // a lane sums its own order alone if it is a short series (or if it has
+    // the frequency to itself); the others go over the frequency's lanes
+    const bool solo = own && (js == 1 || cur.K <= kmid);
+    unsigned pend = __ballot_sync(FULL_WARP, own && !solo) & gmask;
+    bool go = solo;
+    int jj = 0, jc = 1;
+    const OrderInfo mine = cur;
+    for (;;) {
+      if (go) {
+        const int nn = cur.nn, n = nn < 0 ? -nn : nn, K = cur.K, K32 = cur.K32;
+        const dflt Ad = df_add(mox, df_neg(df_mul({(float)nn, 0.0f}, qsd)));
+        const float* __restrict__ Bn = S.Bt + (size_t)n * (M - 1) * 12;
+        const float* __restrict__ mBn = S.mBt + (size_t)n * ALPS_KFAR * 12;
+        cdf X[6];  // the order's entries (xx yy zz xy xz yz), scaled by 1/Vscale[n]
+        if (K > S.kfar && !(cur.flags & 2)) {
+          // FP64 node sum of this order over V, X_e = omega S_e1 + kappa S_e2
+          const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
+          const double Ar = S.ms * o.x - (double)nn * S.qs, Di = S.ms * o.y;
+          double2 Sx[12];
 #pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const double sc = S.Escale[e];
-    const double2 t = cmk(df_val(acc[2 * e]) * sc, df_val(acc[2 * e + 1]) * sc);
-    acc_out[e] = (e == 3 || e == 5) ? cmk(-t.y, t.x) : t;
-  }
-}
-
-// The double-float node sum keeps |A - k_par p_j|^2 + D^2 a normal float:
-// its smallest value (at a summed range's end, or zero if the pole lies
-// inside a summed range) at least 1e-30, its largest at most 1e30.
-__device__ __forceinline__ bool df_node_range(const SpecDev& S, const ResGeom& g, double Ar, double kpar,
-                                              double Di) {
-  double lo = 1e300, hi = 0.0;
-  const int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int j0 = max(1, ends[2 * r]), j1 = min(S.M - 1, ends[2 * r + 1]);
-    if (j0 > j1) continue;
-    const double d0 = Ar - kpar * S.ppar[j0], d1 = Ar - kpar * S.ppar[j1];
-    lo = ((d0 < 0.0) != (d1 < 0.0)) ? 0.0 : fmin(lo, fmin(fabs(d0), fabs(d1)));
-    hi = fmax(hi, fmax(fabs(d0), fabs(d1)));
-  }
-  return Di * Di + lo * lo >= 1e-30 && Di * Di + hi * hi <= 1e30;
-}
-
-template <bool LOW>
-__device__ __forceinline__ void pole_body(const SysDev& sys, const SpecDev& S, const DispShape& sh, const double2* __restrict__ om,
-                                          int n_om, int js_count, double2* part, double2* low, int tile, int s,
-                                          int chunk) {
-  const int n_begin = chunk * sh.csize;
-  const int n_end = (S.relat || S.bm) ? n_begin : min(S.nmax + 1, n_begin + sh.csize);
-  // the js_count slices of an omega are adjacent threads, so an omega's
-  // per-order set-up is one warp instruction for all its slices
-  const int TW = blockDim.x / js_count;
-  const int wl = threadIdx.x / js_count, js = threadIdx.x % js_count;
-  const int w = tile * TW + wl;
-  const bool active = (w < n_om);
-  const double2 o = active ? om[w] : cmk(0.0, 0.0);
-  const int M = S.M;
-  const double kpar = sys.kpar;
-  const double kappa = kpar / S.ms;
-  const double C0 = 2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25 * S.qs;
-  const double z = sys.kperp_norm ? sys.kperp / S.qs : 1.0 / S.qs;
-  const double Di = S.ms * o.y;
-  const double Di2 = Di * Di;
-  const double* __restrict__ pp = S.ppar;
-  double2 acc[6];
-  double2 lacc[LOW ? 3 : 1][6];
-#pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    acc[e] = cmk(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < (LOW ? 3 : 1); ++q) lacc[q][e] = cmk(0.0, 0.0);
-  }
-  if (active && !LOW && S.df_sums && S.Bt && n_end > n_begin) {
-    pole_fused(sys, S, o, js, js_count, n_begin, n_end, acc);
-  } else if (active) {
-    for (int n = n_begin; n < n_end; ++n) {
-      const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
-      for (int sg = 0; sg < (n == 0 ? 1 : 2); ++sg) {
-        const int nn = sg ? -n : n;
-        ResGeom g = res_geometry(S, sys.M_I, o, nn, kpar);
-        const double Ar = S.ms * o.x - (double)nn * S.qs;
-        double2 Sx[12];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
-        // Laurent series for a pole far outside the grid: truncation
-        // rho^K <= 2^-53 (1 - rho), rho = prad/|p_res - pcen|.  With
-        // |mom_k| <= sum_j |V_j|, the terms from K32 on (rho^K32 <= 2^-33
-        // (1 - rho)) add at most 2^-33 of that bound, so they are summed in
-        // FP32: their rounding stays below 2^-53 of it.
-        int K = S.kfar + 1, K32 = K;
-        double2 d = cmk(g.pr - S.pcen, g.pi);
-        double dd = d.x * d.x + d.y * d.y;
-        if (!g.res && S.prad * S.prad < 0.5 * dd) {
-          // term counts from FP32 logarithms, one term added to each for
-          // their rounding (rho < 0.71 here, so the counts are below 110)
-          const float rho = (float)(S.prad * rsqrt(dd));
-          const float lr = -__logf(rho), l1 = log1pf(-rho);
-          K = (int)ceilf((36.7368006f - l1) / lr) + 1;    // 53 ln 2
-          K32 = (int)ceilf((22.8738570f - l1) / lr) + 1;  // 33 ln 2
-        }
-        if (K <= S.kfar) {
-          const double* __restrict__ mom = S.mom + (size_t)n * ALPS_KFAR * 12;
-          double idd = 1.0 / dd;
-          double2 inv = cmk(d.x * idd, -d.y * idd);
-          double2 t = cscale(inv, S.prad);
-          double2 tk = cmk(1.0, 0.0), step = t;
-          // tk = t^js, step = t^js_count by squaring (js_count is a power of 2)
-          double2 pw = t;
-          for (int q = js; q; q >>= 1) {
-            if (q & 1) tk = cmul(tk, pw);
-            pw = cmul(pw, pw);
-          }
-          for (int q = js_count; q > 1; q >>= 1) step = cmul(step, step);
-          int k = js;
-          if (S.df_sums) {
-            // fast path: the leading terms in double-float arithmetic on the
-            // FP32 pipes (moments as pairs scaled by 2^-e per order)
-            const float* __restrict__ mh = S.momh + (size_t)n * ALPS_KFAR * 12;
-            const float* __restrict__ ml = S.moml + (size_t)n * ALPS_KFAR * 12;
-            dflt tx = df_of(tk.x), ty = df_of(tk.y);
-            const dflt sx = df_of(step.x), sy = df_of(step.y);
-            dflt sacc[24];
-#pragma unroll
-            for (int q = 0; q < 24; ++q) sacc[q] = {0.0f, 0.0f};
-            for (; k < K32; k += js_count) {
-              const float4* h4 = reinterpret_cast<const float4*>(mh + (size_t)k * 12);
-              const float4* l4 = reinterpret_cast<const float4*>(ml + (size_t)k * 12);
-#pragma unroll
-              for (int q = 0; q < 3; ++q) {
-                const float4 h = __ldg(h4 + q), l = __ldg(l4 + q);
-                df_mac(sacc[8 * q + 0], h.x, l.x, tx);
-                df_mac(sacc[8 * q + 1], h.x, l.x, ty);
-                df_mac(sacc[8 * q + 2], h.y, l.y, tx);
-                df_mac(sacc[8 * q + 3], h.y, l.y, ty);
-                df_mac(sacc[8 * q + 4], h.z, l.z, tx);
-                df_mac(sacc[8 * q + 5], h.z, l.z, ty);
-                df_mac(sacc[8 * q + 6], h.w, l.w, tx);
-                df_mac(sacc[8 * q + 7], h.w, l.w, ty);
-              }
-              const dflt nx = df_add(df_mul(tx, sx), df_neg(df_mul(ty, sy)));
-              ty = df_add(df_mul(tx, sy), df_mul(ty, sx));
-              tx = nx;
-            }
-            const double sc = S.Vscale[n];
-#pragma unroll
-            for (int q = 0; q < 12; ++q) Sx[q] = cmk(df_val(sacc[2 * q]) * sc, df_val(sacc[2 * q + 1]) * sc);
-            tk = cmk(df_val(tx), df_val(ty));
-          }
-          for (; k < K32; k += js_count) {
-            const double2* m2 = reinterpret_cast<const double2*>(mom + (size_t)k * 12);
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-              double2 m = __ldg(m2 + q);
-              Sx[2 * q].x = fma(m.x, tk.x, Sx[2 * q].x);
-              Sx[2 * q].y = fma(m.x, tk.y, Sx[2 * q].y);
-              Sx[2 * q + 1].x = fma(m.y, tk.x, Sx[2 * q + 1].x);
-              Sx[2 * q + 1].y = fma(m.y, tk.y, Sx[2 * q + 1].y);
-            }
-            tk = cmul(tk, step);
-          }
-          if (k < K) {
-            const float* __restrict__ momf = S.momf + (size_t)n * ALPS_KFAR * 12;
-            float2 tf = make_float2((float)tk.x, (float)tk.y);
-            const float2 sf = make_float2((float)step.x, (float)step.y);
-            float2 Sf[12];
-#pragma unroll
-            for (int q = 0; q < 12; ++q) Sf[q] = make_float2(0.0f, 0.0f);
-            for (; k < K; k += js_count) {
-              const float4* m4 = reinterpret_cast<const float4*>(momf + (size_t)k * 12);
-#pragma unroll
-              for (int q = 0; q < 3; ++q) {
-                const float4 m = __ldg(m4 + q);
-                Sf[4 * q].x = fmaf(m.x, tf.x, Sf[4 * q].x);
-                Sf[4 * q].y = fmaf(m.x, tf.y, Sf[4 * q].y);
-                Sf[4 * q + 1].x = fmaf(m.y, tf.x, Sf[4 * q + 1].x);
-                Sf[4 * q + 1].y = fmaf(m.y, tf.y, Sf[4 * q + 1].y);
-                Sf[4 * q + 2].x = fmaf(m.z, tf.x, Sf[4 * q + 2].x);
-                Sf[4 * q + 2].y = fmaf(m.z, tf.y, Sf[4 * q + 2].y);
-                Sf[4 * q + 3].x = fmaf(m.w, tf.x, Sf[4 * q + 3].x);
-                Sf[4 * q + 3].y = fmaf(m.w, tf.y, Sf[4 * q + 3].y);
-              }
-              tf = make_float2(tf.x * sf.x - tf.y * sf.y, tf.x * sf.y + tf.y * sf.x);
-            }
-#pragma unroll
-            for (int q = 0; q < 12; ++q) {
-              Sx[q].x += (double)Sf[q].x;
-              Sx[q].y += (double)Sf[q].y;
-            }
-          }
-          // S = (1/(k_par d)) sum_k mom_k t^k
-          double2 f = cscale(inv, sys.ikpar);
-#pragma unroll
-          for (int q = 0; q < 12; ++q) Sx[q] = cmul(Sx[q], f);
-        } else if (S.df_sums && df_node_range(S, g, Ar, kpar, Di)) {
-          // fast path: the node sum in double-float arithmetic on the FP32
-          // pipes (about 46 bits; V in pairs scaled by 2^-e per order)
-          const float* __restrict__ Vh = S.Vh + (size_t)n * (M - 1) * 12;
-          const float* __restrict__ Vl = S.Vl + (size_t)n * (M - 1) * 12;
-          const dflt Ad = df_of(Ar), kd = df_of(kpar), Dd = df_of(Di);
-          const dflt D2 = df_mul(Dd, Dd);
-          dflt sacc[24];
-#pragma unroll
-          for (int q = 0; q < 24; ++q) sacc[q] = {0.0f, 0.0f};
-          auto node = [&](int j, float wgt) {
-            const dflt dr = df_add(Ad, df_neg(df_mul(kd, {S.pph[j], S.ppl[j]})));
-            const dflt r = df_rcp_approx(df_add(df_mul(dr, dr), D2));
-            const dflt Rr = df_scale(df_mul(dr, r), wgt), Ri = df_scale(df_neg(df_mul(Dd, r)), wgt);
-            const float4* vh4 = reinterpret_cast<const float4*>(Vh + (size_t)(j - 1) * 12);
-            const float4* vl4 = reinterpret_cast<const float4*>(Vl + (size_t)(j - 1) * 12);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-              const float4 h = __ldg(vh4 + q), l = __ldg(vl4 + q);
-              df_mac(sacc[8 * q + 0], h.x, l.x, Rr);
-              df_mac(sacc[8 * q + 1], h.x, l.x, Ri);
-              df_mac(sacc[8 * q + 2], h.y, l.y, Rr);
-              df_mac(sacc[8 * q + 3], h.y, l.y, Ri);
-              df_mac(sacc[8 * q + 4], h.z, l.z, Rr);
-              df_mac(sacc[8 * q + 5], h.z, l.z, Ri);
-              df_mac(sacc[8 * q + 6], h.w, l.w, Rr);
-              df_mac(sacc[8 * q + 7], h.w, l.w, Ri);
-            }
-          };
-          for (int j = 1 + js; j <= M - 1; j += js_count) {
-            bool in = (j >= g.lo1 && j <= g.hi1) || (j >= g.lo2 && j <= g.hi2);
-            if (in) node(j, 1.0f);
-          }
-          // trapezoid end weights, as below
-          int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
-#pragma unroll
+          for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
           for (int r2 = 0; r2 < 2; ++r2) {
-            int lo = ends[2 * r2], hi = ends[2 * r2 + 1];
-            if (lo >= hi) continue;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-              int j = side ? hi : lo;
-              if (((j - 1) % js_count) == js) node(j, -0.5f);
-            }
-          }
-          const double sc = S.Vscale[n];
-#pragma unroll
-          for (int q = 0; q < 12; ++q) Sx[q] = cmk(df_val(sacc[2 * q]) * sc, df_val(sacc[2 * q + 1]) * sc);
-        } else {
-          for (int j = 1 + js; j <= M - 1; j += js_count) {
-            bool in = (j >= g.lo1 && j <= g.hi1) || (j >= g.lo2 && j <= g.hi2);
-            if (!in) continue;
-            double dr = fma(-kpar, pp[j], Ar);
-            double r = rcp_fast(fma(dr, dr, Di2));
-            double Rr = dr * r, Ri = -Di * r;
-            const double2* v2 = reinterpret_cast<const double2*>(Vn + (size_t)(j - 1) * 12);
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-              double2 v = __ldg(v2 + q);
-              Sx[2 * q].x = fma(v.x, Rr, Sx[2 * q].x);
-              Sx[2 * q].y = fma(v.x, Ri, Sx[2 * q].y);
-              Sx[2 * q + 1].x = fma(v.y, Rr, Sx[2 * q + 1].x);
-              Sx[2 * q + 1].y = fma(v.y, Ri, Sx[2 * q + 1].y);
-            }
-          }
-          // trapezoid end weights: the range ends carry half weight unless the
-          // range is a single node (integrate(a,a) weighs it fully)
-          int ends[4] = {g.lo1, g.hi1, g.lo2, g.hi2};
-#pragma unroll
-          for (int r2 = 0; r2 < 2; ++r2) {
-            int lo = ends[2 * r2], hi = ends[2 * r2 + 1];
-            if (lo >= hi) continue;
-#pragma unroll
-            for (int side = 0; side < 2; ++side) {
-              int j = side ? hi : lo;
-              if (((j - 1) % js_count) != js) continue;
-              double dr = fma(-kpar, pp[j], Ar);
-              double r = rcp_fast(fma(dr, dr, Di2));
-              double Rr = -0.5 * dr * r, Ri = 0.5 * Di * r;
-              const double* v = Vn + (size_t)(j - 1) * 12;
+            const int b = r2 ? cur.lo2 : cur.lo1, e = r2 ? cur.hi2 : cur.hi1;
+            const int lo = max(1, b), hi = min(M - 1, e);
+            for (int jn = lo + ((jj - lo + 1) & (jc - 1)); jn <= hi; jn += jc) {
+              const double wgt = (b < e && (jn == b || jn == e)) ? 0.5 : 1.0;
+              const double dr = fma(-kpar, S.ppar[jn], Ar);
+              const double rr = wgt / fma(dr, dr, Di * Di);
+              const double* v = Vn + (size_t)(jn - 1) * 12;
 #pragma unroll
               for (int q = 0; q < 12; ++q) {
-                Sx[q].x = fma(v[q], Rr, Sx[q].x);
-                Sx[q].y = fma(v[q], Ri, Sx[q].y);
+                Sx[q].x = fma(v[q], dr * rr, Sx[q].x);
+                Sx[q].y = fma(v[q], -Di * rr, Sx[q].y);
               }
             }
           }
+          const double isc = 1.0 / S.Vscale[n], kapd = S.kappa;
+#pragma unroll
+          for (int e = 0; e < 6; ++e) {
+            const double2 t = cscale(cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kapd)), isc);
+            X[e] = {df_of(t.x), df_of(t.y)};
+          }
+        } else if (K <= S.kfar) {
+          // Laurent series: d = p_res - pcen, t = prad/d, f = 1/(k_par d)
+          const int k0 = (jj >= 2) ? jj : jj + jc * ((2 - jj + jc - 1) / jc);  // first k >= 2 of this slice
+          const cdf d = {df_add(df_mul(Ad, ikd), df_neg(pcd)), dyd};
+          const dflt r = df_rcp_approx(df_add(df_mul(d.x, d.x), df_mul(d.y, d.y)));
+          const cdf iv = {df_mul(d.x, r), df_neg(df_mul(d.y, r))};
+          const cdf t1 = cdf_rmul(iv, prd), f = cdf_rmul(iv, ikd);
+          // U = f sum_{k >= 2} mom_k t^k over this slice's k: powers from f t^k0,
+          // step t^jc (both by squaring)
+          cdf tp = f, st = t1;
+          {
+            cdf pw = t1;
+            for (int q = k0; q; q >>= 1) {
+              if (q & 1) tp = cdf_mul(tp, pw);
+              pw = cdf_mul(pw, pw);
+            }
+            for (int q = jc; q > 1; q >>= 1) st = cdf_mul(st, st);
+          }
+          dflt U[12];
+          float Uf[12];
+#pragma unroll
+          for (int q = 0; q < 12; ++q) {
+            U[q] = {0.0f, 0.0f};
+            Uf[q] = 0.0f;
+          }
+          int k = k0;
+          for (; k < K32; k += jc) {
+            const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
+            const float4 a0 = __ldg(m4), a1 = __ldg(m4 + 1), a2 = __ldg(m4 + 2);
+            const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+#pragma unroll
+            for (int b = 0; b < 6; ++b) {
+              df_mac(U[2 * b], hb[b], lb[b], tp.x);
+              df_mac(U[2 * b + 1], hb[b], lb[b], tp.y);
+            }
+            tp = cdf_mul(tp, st);
+          }
+          if (k < K) {
+            // the tail: terms below 2^-33 of the bound, in FP32
+            float fx = tp.x.h + tp.x.l, fy = tp.y.h + tp.y.l;
+            const float gx = st.x.h + st.x.l, gy = st.y.h + st.y.l;
+            for (; k < K; k += jc) {
+              const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
+              const float4 a0 = __ldg(m4);
+              const float2 a1 = __ldg(reinterpret_cast<const float2*>(m4 + 1));
+              const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
+#pragma unroll
+              for (int b = 0; b < 6; ++b) {
+                Uf[2 * b] = fmaf(hb[b], fx, Uf[2 * b]);
+                Uf[2 * b + 1] = fmaf(hb[b], fy, Uf[2 * b + 1]);
+              }
+              const float nx = fx * gx - fy * gy;
+              fy = fx * gy + fy * gx;
+              fx = nx;
+            }
+          }
+          // per family F1, F2, F3: omega U_{F,g1} + kappa U_{F,g2}
+          cdf Uw[3];
+#pragma unroll
+          for (int fm = 0; fm < 3; ++fm) {
+            const int b1 = 2 * fm, b2 = 2 * fm + 1;
+            const cdf u1 = {df_add(U[2 * b1], {Uf[2 * b1], 0.0f}), df_add(U[2 * b1 + 1], {Uf[2 * b1 + 1], 0.0f})};
+            const cdf u2 = {df_add(U[2 * b2], {Uf[2 * b2], 0.0f}), df_add(U[2 * b2 + 1], {Uf[2 * b2 + 1], 0.0f})};
+            Uw[fm] = om_comb(omd, kap, u1, u2);
+          }
+          // T = f mom_1 t + U, Q = f mom_0 + T on the slices that own k = 1, 0
+          cdf T[3] = {Uw[0], Uw[1], Uw[2]};
+          auto mterm = [&](int kk, cdf w, cdf* outv) {
+            const float* m = mBn + (size_t)kk * 12;
+#pragma unroll
+            for (int fm = 0; fm < 3; ++fm) {
+              const cdf mw = om_combr(omd, kap, {m[2 * fm], m[6 + 2 * fm]}, {m[2 * fm + 1], m[6 + 2 * fm + 1]});
+              outv[fm] = cdf_add(outv[fm], cdf_mul(w, mw));
+            }
+          };
+          if (jj == (jc > 1 ? 1 : 0)) mterm(1, cdf_mul(f, t1), T);
+          cdf Q[3] = {T[0], T[1], T[2]};
+          if (jj == 0) mterm(0, f, Q);
+          X[0] = Q[0];
+          X[1] = Q[1];
+          X[3] = Q[2];
+          X[4] = cdf_mul(d, T[0]);
+          X[5] = cdf_mul(d, T[2]);
+          if (S.pcen32 != 0.0f) {
+            // sum F p R = pcen Q + d T, sum F p^2 R = pcen (sum F p R) + d (pcen T + d U)
+            X[4] = cdf_add(cdf_rmul(Q[0], pcd), X[4]);
+            X[5] = cdf_add(cdf_rmul(Q[2], pcd), X[5]);
+            X[2] = cdf_add(cdf_rmul(X[4], pcd), cdf_mul(d, cdf_add(cdf_rmul(T[0], pcd), cdf_mul(d, Uw[0]))));
+          } else {
+            X[2] = cdf_mul(d, cdf_mul(d, Uw[0]));
+          }
+        } else {
+          // node sum in double-float: Q_b = sum_j w_j B_b(j) / (A - k_par p_j + i D)
+          dflt Qs[12];
+#pragma unroll
+          for (int q = 0; q < 12; ++q) Qs[q] = {0.0f, 0.0f};
+          // the summed ranges (disjoint), each over this slice's nodes
+          // jn = 1 + jj (mod jc), then their ends again at weight -1/2
+          auto node = [&](int jn, bool end) {
+            const dflt dr = df_add(Ad, df_neg(df_mul(kd, {S.pph[jn], S.ppl[jn]})));
+            const dflt r = df_rcp_approx(df_add(df_mul(dr, dr), D2));
+            dflt Rr = df_mul(dr, r), Ri = df_neg(df_mul(Dd, r));
+            if (end) {
+              Rr = df_scale(Rr, -0.5f);
+              Ri = df_scale(Ri, -0.5f);
+            }
+            const float4* b4 = reinterpret_cast<const float4*>(Bn + (size_t)(jn - 1) * 12);
+            const float4 a0 = __ldg(b4), a1 = __ldg(b4 + 1), a2 = __ldg(b4 + 2);
+            const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+#pragma unroll
+            for (int b2 = 0; b2 < 6; ++b2) {
+              df_mac(Qs[2 * b2], hb[b2], lb[b2], Rr);
+              df_mac(Qs[2 * b2 + 1], hb[b2], lb[b2], Ri);
+            }
+          };
+          for (int r2 = 0; r2 < 2; ++r2) {
+            const int b = r2 ? cur.lo2 : cur.lo1, e = r2 ? cur.hi2 : cur.hi1;
+            const int lo = max(1, b), hi = min(M - 1, e);
+            for (int jn = lo + ((jj - lo + 1) & (jc - 1)); jn <= hi; jn += jc) node(jn, false);
+          }
+          for (int q = 0; q < 4; ++q) {
+            const int b = (q & 2) ? cur.lo2 : cur.lo1, e = (q & 2) ? cur.hi2 : cur.hi1, jn = (q & 1) ? e : b;
+            if (b < e && jn >= 1 && jn <= M - 1 && ((jn - 1 - jj) & (jc - 1)) == 0) node(jn, true);
+          }
+          cdf P[3];
+#pragma unroll
+          for (int fm = 0; fm < 3; ++fm)
+            P[fm] = om_comb(omd, kap, {Qs[4 * fm], Qs[4 * fm + 1]}, {Qs[4 * fm + 2], Qs[4 * fm + 3]});
+          const cdf zeta = {df_mul(Ad, ikd), dyd};
+          // (1/k_par) times the omega-combined sums of F1, F3 and p_par F1
+          // over the summed ranges: six real sums C_c, added once; lane c
+          // of the slices forms C_c where there are eight or more of them,
+          // the first slice all six otherwise
+          auto csum = [&](int c) -> double {
+            if (!(cur.flags & 1)) return S.Cfull[(size_t)n * 6 + c];
+            const double* __restrict__ P0 = S.Pre + (size_t)n * M * 6;
+            const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
+            const int q = (c < 2) ? c : c + 4;
+            const double isc = 1.0 / S.Vscale[n];
+            double C = 0.0;
+            for (int r2 = 0; r2 < 2; ++r2) {
+              const int b = r2 ? cur.lo2 : cur.lo1, e = r2 ? cur.hi2 : cur.hi1;
+              const int lo = max(1, b), hi = min(M - 1, e);
+              if (lo > hi) continue;
+              double v = P0[(size_t)hi * 6 + c] - P0[(size_t)(lo - 1) * 6 + c];
+              if (b < e) v -= 0.5 * (Vn[(size_t)(lo - 1) * 12 + q] + Vn[(size_t)(hi - 1) * 12 + q]) * isc;
+              C += v;
+            }
+            return C;
+          };
+          dflt C[6];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) C[c] = {0.0f, 0.0f};
+          if (jc >= 8) {
+            if (jj < 6) {
+              const dflt v = df_of(csum(jj));
+#pragma unroll
+              for (int c = 0; c < 6; ++c)
+                if (c == jj) C[c] = v;
+            }
+          } else if (jj == 0) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) C[c] = df_of(csum(c));
+          }
+          X[0] = P[0];
+          X[1] = P[1];
+          X[3] = P[2];
+          const cdf c1 = cdf_rmul(om_combr(omd, kap, C[0], C[1]), ikd);
+          const cdf c3 = cdf_rmul(om_combr(omd, kap, C[2], C[3]), ikd);
+          const cdf cp = cdf_rmul(om_combr(omd, kap, C[4], C[5]), ikd);
+          cdf xz = cdf_mul(zeta, P[0]), yz = cdf_mul(zeta, P[2]);
+          xz = {df_add(xz.x, df_neg(c1.x)), df_add(xz.y, df_neg(c1.y))};
+          yz = {df_add(yz.x, df_neg(c3.x)), df_add(yz.y, df_neg(c3.y))};
+          const cdf zz = cdf_mul(zeta, xz);
+          X[2] = {df_add(zz.x, df_neg(cp.x)), df_add(zz.y, df_neg(cp.y))};
+          X[4] = xz;
+          X[5] = yz;
         }
-        double2 pref[6];
-        t_prefactors(nn, z, sys.kperp, sys.kperp_norm, pref);
+        // add the order's entries with its factors C0 v_e(n) (xy and xz odd in n)
+        const float* __restrict__ fac = S.bfac + (size_t)n * 12;
 #pragma unroll
         for (int e = 0; e < 6; ++e) {
-          if (n == 0 && (e == 0 || e == 3 || e == 4)) continue;
-          // integrate = C0 * pref * (omega S_e1 + kappa S_e2)
-          double2 t1 = cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kappa));
-          double2 val = cscale(cmul(pref[e], t1), C0);
-          acc[e] = cadd(acc[e], val);
-          if (LOW && nn >= -1 && nn <= 1) lacc[LOW ? nn + 1 : 0][e] = cadd(lacc[LOW ? nn + 1 : 0][e], val);
+          dflt fe = {fac[2 * e], fac[2 * e + 1]};
+          if (nn < 0 && (e == 3 || e == 4)) fe = df_neg(fe);
+          df_acc(acc[2 * e], df_mul(fe, X[e].x));
+          df_acc(acc[2 * e + 1], df_mul(fe, X[e].y));
         }
+      }
+      if (!__any_sync(FULL_WARP, pend != 0)) break;
+      go = pend != 0;
+      const int t = go ? __ffs(pend) - 1 : lane;
+      pend &= pend - 1;
+      cur = shfl_info(mine, t);
+      jj = j;
+      jc = js;
+    }
+  }
+  // add the lanes, rescale and apply the phase (i for xy and yz)
+  int first, cnt;
+  lane_sum12(acc, js, lane, first, cnt);
+  if (!active) return;
+#pragma unroll
+  for (int q = 0; q < 12; ++q)
+    if (q < cnt) {
+      const int c = first + q, e = c >> 1;
+      const double v = df_val(acc[q]) * S.Escale[e];
+      if (e == 3 || e == 5) out[c ^ 1] = (c & 1) ? -v : v;  // (x, y) -> (-y, x)
+      else out[c] = v;
+    }
+}
+
+// Plain path: the trapezoid node sum of every order in FP64 over the reduced
+// vectors.  Bound by the FP64 pipe (two lanes a clock and SM): 24 FMA of a
+// node's 32 instructions are the twelve real vectors against R_j.
+__device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, double2 o, bool active, int js,
+                                           int chunk, int nch, double* out) {
+  const int M = S.M, U_ = 2 * S.nmax + 1;
+  const int lane = threadIdx.x & 31, j = lane & (js - 1), gbase = lane - j;
+  const unsigned gmask = (js == 32) ? FULL_WARP : (((1u << js) - 1u) << gbase);
+  const double kpar = sys.kpar, kappa = S.kappa;
+  const double C0 = 2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25 * S.qs;
+  const double z = sys.kperp_norm ? sys.kperp / S.qs : 1.0 / S.qs;
+  const double Di = S.ms * o.y, Di2 = Di * Di;
+  const double* __restrict__ pp = S.ppar;
+  const float ikp32 = (float)sys.ikpar;
+  dbl_val acc[12];
+#pragma unroll
+  for (int q = 0; q < 12; ++q) acc[q] = {0.0};
+  for (int i0 = 0; chunk + i0 * nch < U_; i0 += js) {
+    const int u = chunk + (i0 + j) * nch;
+    const bool own = active && u < U_;
+    int nn = 0, lo1 = 1, hi1 = 0, lo2 = 1, hi2 = 0;
+    if (own) {
+      nn = u - S.nmax;
+      hi1 = M - 1;
+      // the FP32 test of k_classify: an order clearly outside the resonance
+      // interval sums every node
+      const float x32 = (float)(S.ms * o.x - (double)nn * S.qs) * ikp32;
+      const float mg = 9.5367431640625e-7f * fabsf(x32);
+      if (!(x32 < S.qlo - mg || x32 > S.qhi + mg)) {
+        const ResGeom g = res_geometry(S, sys.M_I, o, nn, kpar);
+        lo1 = g.lo1;
+        hi1 = g.hi1;
+        lo2 = g.lo2;
+        hi2 = g.hi2;
+      }
+    }
+    unsigned pend = __ballot_sync(FULL_WARP, own) & gmask;
+    while (__any_sync(FULL_WARP, pend != 0)) {
+      const bool go = pend != 0;
+      const int t = go ? __ffs(pend) - 1 : lane;
+      pend &= pend - 1;
+      const int cn = __shfl_sync(FULL_WARP, nn, t);
+      const int b1 = __shfl_sync(FULL_WARP, lo1, t), e1 = __shfl_sync(FULL_WARP, hi1, t);
+      const int b2 = __shfl_sync(FULL_WARP, lo2, t), e2 = __shfl_sync(FULL_WARP, hi2, t);
+      if (!go) continue;
+      const int n = cn < 0 ? -cn : cn;
+      const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
+      const double Ar = S.ms * o.x - (double)cn * S.qs;
+      double2 Sx[12];
+#pragma unroll
+      for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
+      // a range's two ends carry weight 1/2 (a range of a single node none:
+      // integrate(a,a) weighs it fully)
+      for (int r2 = 0; r2 < 2; ++r2) {
+        const int b = r2 ? b2 : b1, e = r2 ? e2 : e1;
+        const int lo = max(1, b), hi = min(M - 1, e);
+        for (int jn = lo + ((j - lo + 1) & (js - 1)); jn <= hi; jn += js) {
+          const double dr = fma(-kpar, pp[jn], Ar);
+          double r = rcp_fast(fma(dr, dr, Di2));
+          if (b < e && (jn == b || jn == e)) r *= 0.5;
+          const double Rr = dr * r, Ri = -Di * r;
+          const double2* v2 = reinterpret_cast<const double2*>(Vn + (size_t)(jn - 1) * 12);
+#pragma unroll
+          for (int q = 0; q < 6; ++q) {
+            const double2 v = __ldg(v2 + q);
+            Sx[2 * q].x = fma(v.x, Rr, Sx[2 * q].x);
+            Sx[2 * q].y = fma(v.x, Ri, Sx[2 * q].y);
+            Sx[2 * q + 1].x = fma(v.y, Rr, Sx[2 * q + 1].x);
+            Sx[2 * q + 1].y = fma(v.y, Ri, Sx[2 * q + 1].y);
+          }
+        }
+      }
+      // integrate = C0 * pref * (omega S_e1 + kappa S_e2); xy and yz carry
+      // the factor i, applied at the end
+      double2 pref[6];
+      t_prefactors(cn, z, sys.kperp, sys.kperp_norm, pref);
+#pragma unroll
+      for (int e = 0; e < 6; ++e) {
+        if (n == 0 && (e == 0 || e == 3 || e == 4)) continue;
+        const double f = C0 * ((e == 3 || e == 5) ? pref[e].y : pref[e].x);
+        const double2 t1 = cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kappa));
+        acc[2 * e].v = fma(f, t1.x, acc[2 * e].v);
+        acc[2 * e + 1].v = fma(f, t1.y, acc[2 * e + 1].v);
       }
     }
   }
-  // reduce over the j slices: they are adjacent lanes of one warp (js_count
-  // divides 32), so a butterfly over the lane offsets below js_count
-  auto slice_sum = [&](double2& v) {
-    for (int off = js_count >> 1; off > 0; off >>= 1) {
-      v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-      v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+  int first, cnt;
+  lane_sum12(acc, js, lane, first, cnt);
+  if (!active) return;
+#pragma unroll
+  for (int q = 0; q < 12; ++q)
+    if (q < cnt) {
+      const int c = first + q, e = c >> 1;
+      const double v = acc[q].v;
+      if (e == 3 || e == 5) out[c ^ 1] = (c & 1) ? -v : v;
+      else out[c] = v;
     }
-  };
-  if (js_count > 1) {
-    for (int e = 0; e < 6; ++e) slice_sum(acc[e]);
-    if (LOW)
-      for (int l = 0; l < 3; ++l)
-        for (int e = 0; e < 6; ++e) slice_sum(lacc[LOW ? l : 0][e]);
-  }
-  if (js == 0 && active) {
-    size_t base = ((size_t)w * sys.nspec + s) * sh.nchunk + chunk;
-    for (int e = 0; e < 6; ++e) part[base * 6 + e] = acc[e];
-    if (LOW)
-      for (int l = 0; l < 3; ++l)
-        for (int e = 0; e < 6; ++e) low[(base * 3 + l) * 6 + e] = lacc[LOW ? l : 0][e];
-  }
 }
 
-
+// one warp's unit: an order chunk of species s for a tile of 32 / js
+// frequencies; its entries go to part[(w S + s) nchunk + chunk]
+__device__ __forceinline__ void pole_body(const SysDev& sys, const SpecDev& S, const DispShape& sh,
+                                          const double2* __restrict__ om, int n_om, double2* part, int s, long unit) {
+  const int chunk = (int)(unit / sh.wt), tile = (int)(unit % sh.wt);
+  const int js = sh.js, lane = threadIdx.x & 31;
+  const int w = tile * (32 / js) + lane / js;
+  const bool active = w < n_om;
+  if (tile * (32 / js) >= n_om) return;
+  const double2 o = active ? om[w] : cmk(0.0, 0.0);
+  double* out = active ? reinterpret_cast<double*>(part + (((size_t)w * sys.nspec + s) * sh.nchunk + chunk) * 6) : nullptr;
+  if (S.df_sums)
+    pole_fused(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, out);
+  else
+    pole_plain(sys, S, o, active, js, chunk, sh.nch[s], out);
+}
 
 // ---------------------------------------------------------------------------
 // Analytic continuation f(pperp_i, complex ppar) (eval_fit,
@@ -2102,145 +2059,20 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
 
 // ---------------------------------------------------------------------------
 // chi, epsilon, wave tensor, det (src/ALPS_fns.f90:500-626)
+//
+// Two forms: a thread per omega for lattices, where the FP64 pipe is the
+// bound, and a warp per omega for everything smaller, where one thread's
+// chain of some 600 FP64 operations was (24 us for 31 frequencies, 87 us for
+// 2999).  There lane c + 12 h holds component c (re, im of xx yy zz xy xz yz)
+// of half h of the sums, and the products of the determinant go side by side.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void finalize_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
-                                              int n_om, const double2* __restrict__ part,
-                                              const double2* __restrict__ low, const int* __restrict__ count,
-                                              const int* __restrict__ slot_nn, const double2* __restrict__ items,
-                                              const double2* __restrict__ rel, const double2* __restrict__ bmres,
-                                              double2* D, double2* ext, int w, bool warp_mode) {
-  if (w >= n_om) return;
-  // warp_mode: the 32 lanes of a warp share one omega; they split the sums
-  // over order chunks and run the rest redundantly, lane 0 writes
-  const int lane = threadIdx.x & 31, lstep = warp_mode ? 32 : 1, l0 = warp_mode ? lane : 0;
-  auto wsum = [&](double2& v) {
-    if (warp_mode)
-      for (int off = 16; off > 0; off >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
-      }
-  };
-  const int S_ = a.sys.nspec;
-  const double2 o = om[w];
-  double2 eps[6];
-  for (int e = 0; e < 6; ++e) eps[e] = cmk(0.0, 0.0);
-  const double kperp = a.sys.kperp, kpar = a.sys.kpar, vA = a.sys.vA;
-  double2 denom = cmul(o, o);
-  denom = a.sys.kperp_norm ? cscale(cscale(denom, vA), vA) : cscale(cscale(cscale(cscale(denom, vA), vA), kperp), kperp);
-  for (int s = 0; s < S_; ++s) {
-    const SpecDev& S = a.sp[s];
-    double2 chi[6], cl[3][6];
-    for (int e = 0; e < 6; ++e) {
-      chi[e] = cmk(0.0, 0.0);
-      for (int l = 0; l < 3; ++l) cl[l][e] = cmk(0.0, 0.0);
-    }
-    size_t base = ((size_t)w * S_ + s) * sh.nchunk;
-    // small batches leave one partial per order: unrolled, so that the
-    // loads of several chunks are in flight at once
-#pragma unroll 4
-    for (int ch = l0; ch < sh.nchunk; ch += lstep)
-      for (int e = 0; e < 6; ++e) chi[e] = cadd(chi[e], part[(base + ch) * 6 + e]);
-    if (ext && low)
-      for (int ch = l0; ch < sh.nchunk; ch += lstep)
-        for (int l = 0; l < 3; ++l)
-          for (int e = 0; e < 6; ++e) cl[l][e] = cadd(cl[l][e], low[((base + ch) * 3 + l) * 6 + e]);
-    int cnt = count[(size_t)w * S_ + s];
-    for (int r = l0; r < cnt; r += lstep) {
-      size_t ib = ((size_t)w * S_ + s) * a.rcap + r;
-      int nn = slot_nn[ib];
-      for (int e = 0; e < 6; ++e) {
-        double2 v = items[ib * 6 + e];
-        chi[e] = cadd(chi[e], v);
-        if (nn == -1) cl[0][e] = cadd(cl[0][e], v);
-        if (nn == 0) cl[1][e] = cadd(cl[1][e], v);
-        if (nn == 1) cl[2][e] = cadd(cl[2][e], v);
-      }
-    }
-    // warp mode: each lane summed its share of the chunks and items
-    for (int e = 0; e < 6; ++e) wsum(chi[e]);
-    if (ext)
-      for (int l = 0; l < 3; ++l)
-        for (int e = 0; e < 6; ++e) wsum(cl[l][e]);
-    if (S.bm) {
-      // NHDS chi, divided by n q before the common normalisation as in disp
-      // (src/ALPS_fns.f90:344-358); no ee term
-      const double2* b = bmres + ((size_t)w * S_ + s) * 24;
-      const double nq = S.ns * S.qs;
-      for (int e = 0; e < 6; ++e) chi[e] = cadd(chi[e], cmk(b[e].x / nq, b[e].y / nq));
-      for (int l = 0; l < 3; ++l)
-        for (int e = 0; e < 6; ++e) cl[l][e] = cmk(b[6 + 6 * l + e].x / nq, b[6 + 6 * l + e].y / nq);
-    } else if (S.relat) {
-      // orders in the reference's order; n = 0 adds yy, zz, yz only, and the
-      // ee term goes into chi alone (src/ALPS_fns.f90:461-497)
-      for (int n = 0; n <= S.nmax; ++n) {
-        // the row blocks' partial sums of +n and -n, added in order
-        const double2* base = rel + ((((size_t)w * S_ + s) * a.relcap + n) * 2 + 0) * REL_RB * 6;
-        double2 pl[6], mi[6];
-        for (int e = 0; e < 6; ++e) {
-          pl[e] = base[e];
-          mi[e] = base[REL_RB * 6 + e];
-          for (int q = 1; q < REL_RB; ++q) {
-            pl[e] = cadd(pl[e], base[q * 6 + e]);
-            mi[e] = cadd(mi[e], base[(REL_RB + q) * 6 + e]);
-          }
-        }
-        if (n == 0) {
-          const int e0[3] = {1, 2, 5};
-          for (int q = 0; q < 3; ++q) {
-            chi[e0[q]] = cadd(chi[e0[q]], pl[e0[q]]);
-            cl[1][e0[q]] = pl[e0[q]];
-          }
-        } else {
-          for (int e = 0; e < 6; ++e) {
-            if (n == 1) {
-              cl[2][e] = pl[e];
-              cl[0][e] = mi[e];
-              chi[e] = cadd(chi[e], cadd(pl[e], mi[e]));
-            } else {
-              chi[e] = cadd(cadd(chi[e], pl[e]), mi[e]);
-            }
-          }
-        }
-      }
-      double ee = a.sys.kperp_norm ? S.int_ee_rel : kperp * kperp * S.int_ee_rel;
-      chi[2] = cadd(chi[2], cmk(ee, 0.0));
-    } else {
-      double ee = a.sys.kperp_norm ? S.int_ee : kperp * kperp * S.int_ee;
-      chi[2] = cadd(chi[2], cmk(ee, 0.0));
-      cl[1][2] = cadd(cl[1][2], cmk(ee, 0.0));
-    }
-    double norm = S.ns * S.qs;
-    for (int e = 0; e < 6; ++e) {
-      chi[e] = cscale(chi[e], norm);
-      for (int l = 0; l < 3; ++l) cl[l][e] = cscale(cl[l][e], norm);
-      eps[e] = cadd(eps[e], chi[e]);
-    }
-    if (ext && l0 == 0) {
-      // chi0 (S x 3 x 3) then chi0_low (S x 3 x 3 x 3), then wave (9)
-      double2* c0 = ext + (size_t)w * (S_ * 36 + 9) + s * 9;
-      const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
-      double2 t[9];
-      for (int e = 0; e < 6; ++e) t[3 * ii[e] + jj[e]] = cdiv(chi[e], denom);
-      t[3] = cneg(t[1]);
-      t[6] = t[2];
-      t[7] = cneg(t[5]);
-      for (int q = 0; q < 9; ++q) c0[q] = t[q];
-      double2* c1 = ext + (size_t)w * (S_ * 36 + 9) + S_ * 9 + s * 27;
-      for (int l = 0; l < 3; ++l) {
-        double2 u[9];
-        for (int e = 0; e < 6; ++e) u[3 * ii[e] + jj[e]] = cdiv(cl[l][e], denom);
-        u[3] = cneg(u[1]);
-        u[6] = u[2];
-        u[7] = cneg(u[5]);
-        for (int q = 0; q < 9; ++q) c1[l * 9 + q] = u[q];
-      }
-    }
-  }
-  // eps entries: xx yy zz xy xz yz
-  double2 unit = a.sys.kperp_norm ? cmul(cscale(o, vA), cscale(o, vA))
-                                  : cmul(cscale(cscale(o, kperp), vA), cscale(cscale(o, kperp), vA));
+// the wave tensor's entries w11 w22 w33 w12 w13 w23 from eps
+__device__ __forceinline__ void wave_entries(const SysDev& sy, double2 o, const double2 eps[6], double2 w[6]) {
+  const double kperp = sy.kperp, kpar = sy.kpar, vA = sy.vA;
+  const double2 ov = sy.kperp_norm ? cscale(o, vA) : cscale(cscale(o, kperp), vA);
+  const double2 unit = cmul(ov, ov);
   double enx2, enz2, enxnz;
-  if (a.sys.kperp_norm) {
+  if (sy.kperp_norm) {
     enx2 = kperp * kperp;
     enz2 = kpar * kpar;
     enxnz = kpar * kperp;
@@ -2249,32 +2081,196 @@ __device__ __forceinline__ void finalize_body(const DispArgs& a, const DispShape
     enz2 = kpar * kpar * kperp * kperp;
     enxnz = kpar * kperp * kperp * kperp;
   }
-  double2 w11 = csub(cadd(eps[0], unit), cmk(enz2, 0.0));
-  double2 w22 = csub(csub(cadd(eps[1], unit), cmk(enz2, 0.0)), cmk(enx2, 0.0));
-  double2 w33 = csub(cadd(eps[2], unit), cmk(enx2, 0.0));
-  double2 w13 = cadd(eps[4], cmk(enxnz, 0.0));
-  double2 w12 = eps[3];
-  double2 w23 = eps[5];
-  double2 det = cadd(cadd(csub(cadd(cmul(w11, cadd(cmul(w22, w33), cmul(w23, w23))),
-                                    cscale(cmul(cmul(w12, w23), w13), 2.0)),
-                               cmul(cmul(w13, w13), w22)),
-                          cmul(cmul(w12, w12), w33)),
-                     cmk(0.0, 0.0));
-  if (l0 == 0) D[w] = det;
-  if (ext && l0 == 0) {
-    double2* wv = ext + (size_t)w * (S_ * 36 + 9) + S_ * 36;
-    wv[0] = w11;
-    wv[1] = w12;
-    wv[2] = w13;
-    wv[3] = cneg(w12);
-    wv[4] = w22;
-    wv[5] = w23;
-    wv[6] = w13;
-    wv[7] = cneg(w23);
-    wv[8] = w33;
-  }
+  w[0] = csub(cadd(eps[0], unit), cmk(enz2, 0.0));
+  w[1] = csub(csub(cadd(eps[1], unit), cmk(enz2, 0.0)), cmk(enx2, 0.0));
+  w[2] = csub(cadd(eps[2], unit), cmk(enx2, 0.0));
+  w[3] = eps[3];
+  w[4] = cadd(eps[4], cmk(enxnz, 0.0));
+  w[5] = eps[5];
 }
 
+// one thread per omega (no tensors, plain species, few chunks)
+__device__ __forceinline__ void finalize_thread(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
+                                                int n_om, const double2* __restrict__ part,
+                                                const int* __restrict__ count, const double2* __restrict__ items,
+                                                double2* D, int w) {
+  if (w >= n_om) return;
+  const int S_ = a.sys.nspec;
+  const double2 o = om[w];
+  const double kperp = a.sys.kperp;
+  double2 eps[6];
+  for (int e = 0; e < 6; ++e) eps[e] = cmk(0.0, 0.0);
+  for (int s = 0; s < S_; ++s) {
+    const SpecDev& S = a.sp[s];
+    double2 chi[6];
+    for (int e = 0; e < 6; ++e) chi[e] = cmk(0.0, 0.0);
+    const size_t ws = (size_t)w * S_ + s, base = ws * sh.nchunk;
+    for (int ch = 0; ch < sh.nch[s]; ++ch)
+      for (int e = 0; e < 6; ++e) chi[e] = cadd(chi[e], part[(base + ch) * 6 + e]);
+    const int cnt = count[ws];
+    for (int r = 0; r < cnt; ++r)
+      for (int e = 0; e < 6; ++e) chi[e] = cadd(chi[e], items[(ws * a.rcap + r) * 6 + e]);
+    chi[2].x += a.sys.kperp_norm ? S.int_ee : kperp * kperp * S.int_ee;
+    const double norm = S.ns * S.qs;
+    for (int e = 0; e < 6; ++e) eps[e] = cmk(fma(norm, chi[e].x, eps[e].x), fma(norm, chi[e].y, eps[e].y));
+  }
+  double2 q[6];
+  wave_entries(a.sys, o, eps, q);
+  // w11 (w22 w33 + w23^2) + 2 w12 w23 w13 - w13^2 w22 + w12^2 w33
+  D[w] = cadd(csub(cadd(cmul(q[0], cadd(cmul(q[1], q[2]), cmul(q[5], q[5]))), cscale(cmul(cmul(q[3], q[5]), q[4]), 2.0)),
+                   cmul(cmul(q[4], q[4]), q[1])),
+              cmul(cmul(q[3], q[3]), q[2]));
+}
+
+// one warp per omega; all lanes take part.  With ext the order chunks are
+// single orders, from which the n = -1, 0, 1 parts follow.
+__device__ __forceinline__ void finalize_warp(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
+                                              int n_om, const double2* __restrict__ part,
+                                              const int* __restrict__ count, const int* __restrict__ slot_nn,
+                                              const double2* __restrict__ items, const double2* __restrict__ rel,
+                                              const double2* __restrict__ bmres, double2* D, double2* ext, long w) {
+  if (w >= n_om) return;
+  const int lane = threadIdx.x & 31, h = lane / 12, c = lane % 12, e = c >> 1;
+  const int S_ = a.sys.nspec;
+  const double2 o = om[w];
+  const double kperp = a.sys.kperp, vA = a.sys.vA;
+  double2 denom = cmk(1.0, 0.0);
+  if (ext) {
+    denom = cmul(o, o);
+    denom = a.sys.kperp_norm ? cscale(cscale(denom, vA), vA)
+                             : cscale(cscale(cscale(cscale(denom, vA), vA), kperp), kperp);
+  }
+  double eps = 0.0;  // component c of the sum over species (lanes 0..11)
+  for (int s = 0; s < S_; ++s) {
+    const SpecDev& S = a.sp[s];
+    const size_t ws = (size_t)w * S_ + s, base = ws * sh.nchunk;
+    double v = 0.0, lw[3] = {0.0, 0.0, 0.0};
+    if (h < 2) {
+      const int nch = sh.nch[s];
+      const double* __restrict__ pt = reinterpret_cast<const double*>(part + base * 6) + c;
+#pragma unroll 4
+      for (int ch = h; ch < nch; ch += 2) {
+        const double x = pt[(size_t)ch * 12];
+        v += x;
+        if (ext)
+          for (int l = 0; l < 3; ++l)
+            if (ch - S.nmax == l - 1) lw[l] += x;
+      }
+      const int cnt = count[ws];
+      const double* __restrict__ it = reinterpret_cast<const double*>(items + ws * a.rcap * 6) + c;
+#pragma unroll 2
+      for (int r = h; r < cnt; r += 2) {
+        const double x = it[(size_t)r * 12];
+        v += x;
+        if (ext) {
+          const int nn = slot_nn[ws * a.rcap + r];
+          for (int l = 0; l < 3; ++l)
+            if (nn == l - 1) lw[l] += x;
+        }
+      }
+      if (S.relat) {
+        // the row blocks' partial sums of +n and -n; n = 0 adds yy, zz, yz only
+        const bool in0 = e == 1 || e == 2 || e == 5;
+        for (int n = h; n <= S.nmax; n += 2) {
+          const double* __restrict__ b = reinterpret_cast<const double*>(rel + (ws * a.relcap + n) * 2 * REL_RB * 6) + c;
+          double pl = 0.0, mi = 0.0;
+#pragma unroll
+          for (int q = 0; q < REL_RB; ++q) {
+            pl += b[q * 12];
+            if (n > 0) mi += b[(REL_RB + q) * 12];
+          }
+          if (n == 0) {
+            if (in0) {
+              v += pl;
+              lw[1] += pl;
+            }
+          } else {
+            v += pl + mi;
+            if (n == 1) {
+              lw[2] += pl;
+              lw[0] += mi;
+            }
+          }
+        }
+      }
+    }
+    const double ov = __shfl_down_sync(FULL_WARP, v, 12);
+    v += ov;
+    if (ext)
+      for (int l = 0; l < 3; ++l) lw[l] += __shfl_down_sync(FULL_WARP, lw[l], 12);
+    if (S.bm) {
+      // NHDS chi, divided by n q before the common normalisation as in disp
+      // (src/ALPS_fns.f90:344-358); no ee term
+      const double* b = reinterpret_cast<const double*>(bmres + ws * 24);
+      const double nq = S.ns * S.qs;
+      v += b[c] / nq;
+      if (ext)
+        for (int l = 0; l < 3; ++l) lw[l] = b[12 + 12 * l + c] / nq;
+    } else {
+      // the ee term; a relativistic species' goes into chi alone
+      // (src/ALPS_fns.f90:461-497)
+      double ee = S.relat ? S.int_ee_rel : S.int_ee;
+      if (!a.sys.kperp_norm) ee *= kperp * kperp;
+      if (c == 4) {
+        v += ee;
+        if (!S.relat) lw[1] += ee;
+      }
+    }
+    const double norm = S.ns * S.qs;
+    v *= norm;
+    eps += v;
+    if (ext) {
+      // chi0 (S x 3 x 3) and chi0_low (S x 3 x 3 x 3): lane 6 q + entry takes
+      // one division, q = 0 chi, q = 1..3 the n = -1, 0, 1 parts
+      for (int l = 0; l < 3; ++l) lw[l] *= norm;
+      const int q = lane / 6, en = lane % 6;
+      double x = __shfl_sync(FULL_WARP, v, 2 * en), y = __shfl_sync(FULL_WARP, v, 2 * en + 1);
+      for (int l = 0; l < 3; ++l) {
+        const double lx = __shfl_sync(FULL_WARP, lw[l], 2 * en), ly = __shfl_sync(FULL_WARP, lw[l], 2 * en + 1);
+        if (q == l + 1) {
+          x = lx;
+          y = ly;
+        }
+      }
+      if (q < 4) {
+        const double2 t = cdiv(cmk(x, y), denom);
+        double2* dst = ext + (size_t)w * (S_ * 36 + 9) + (q == 0 ? s * 9 : S_ * 9 + s * 27 + (q - 1) * 9);
+        const int ii[6] = {0, 1, 2, 0, 0, 1}, jj[6] = {0, 1, 2, 1, 2, 2};
+        dst[3 * ii[en] + jj[en]] = t;
+        if (en >= 3) dst[3 * jj[en] + ii[en]] = (en == 4) ? t : cneg(t);
+      }
+    }
+  }
+  double2 ep[6], q[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    ep[k].x = __shfl_sync(FULL_WARP, eps, 2 * k);
+    ep[k].y = __shfl_sync(FULL_WARP, eps, 2 * k + 1);
+  }
+  wave_entries(a.sys, o, ep, q);  // w11 w22 w33 w12 w13 w23
+  // det = w11 (w22 w33 + w23^2) + 2 w12 w23 w13 - w13^2 w22 + w12^2 w33: first
+  // the pair products on lanes 0..4, then the four terms on lanes 0..3
+  auto from = [&](double2 v, int src) {
+    return cmk(__shfl_sync(FULL_WARP, v.x, src), __shfl_sync(FULL_WARP, v.y, src));
+  };
+  const double2 p = cmul(lane == 0 ? q[1] : (lane == 1 ? q[5] : (lane == 3 ? q[4] : q[3])),
+                         lane == 0 ? q[2] : (lane == 1 || lane == 2 ? q[5] : (lane == 3 ? q[4] : q[3])));
+  const double2 p1 = from(p, 1), pn = from(p, lane + 1);
+  double2 t = cmul(lane == 0 ? cadd(p, p1) : pn, lane == 0 ? q[0] : (lane == 1 ? q[4] : (lane == 2 ? q[1] : q[2])));
+  if (lane == 1) t = cscale(t, 2.0);
+  const double2 t1 = from(t, 1), t2 = from(t, 2), t3 = from(t, 3);
+  if (lane == 0) D[w] = cadd(csub(cadd(t, t1), t2), t3);
+  if (ext && lane < 9) {
+    // the wave tensor: w12, w13, w23 above the diagonal
+    const int m[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+    double2 x = q[0];
+#pragma unroll
+    for (int k = 1; k < 6; ++k)
+      if (m[lane] == k) x = q[k];
+    if (lane == 3 || lane == 7) x = cneg(x);
+    ext[(size_t)w * (S_ * 36 + 9) + S_ * 36 + lane] = x;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Jobs.  Every batch, of one context or fused over many, runs the same four
@@ -2288,7 +2284,7 @@ __device__ __forceinline__ void finalize_body(const DispArgs& a, const DispShape
 struct DispJob {
   const DispArgs* a;  // the context's arguments (device copy)
   DispShape sh;
-  int n, js, tiles, S;
+  int n, S;
   long blk[4];        // first block of the job in classify, pole sums, resonant, finalize
   const double2* om;
   double2* D;
@@ -2297,11 +2293,12 @@ struct DispJob {
   int* slot_nn;
   double2* items;
   int* flags;
-  double2* low;       // chi_low partials (calc_eigen) or null
   double2* ext;       // chi0, chi0_low, wave per omega, or null
   const double2* rel; // relativistic orders, or null
   const double2* bm;  // closed-form species, or null
 };
+
+#define DISP_JOB_BYTES sizeof(DispJob)
 
 // stores a lone batch's arguments and job where its kernels read them
 __global__ void k_stage(DispArgs a, DispJob j, DispArgs* da, DispJob* dj) {
@@ -2324,11 +2321,18 @@ __device__ __forceinline__ const DispJob& job_of(const DispJob* jobs, int nj, lo
   return jobs[lo];
 }
 
-// k_finalize: one warp per omega when a batch leaves many order chunks
-// (small batches), one thread per omega otherwise
-__host__ __device__ inline bool fin_warp_mode(const DispShape& sh) { return sh.nchunk >= 8; }
+// blocks of k_pole_sums_multi: four warps a block, whole blocks per species
+__host__ __device__ inline long pole_blocks(const DispShape& sh, int s) { return ((long)sh.nch[s] * sh.wt + 3) / 4; }
+inline long pole_blocks_all(const DispShape& sh, int S_) {
+  long b = 0;
+  for (int s = 0; s < S_; ++s) b += pole_blocks(sh, s);
+  return b;
+}
+
+// k_finalize: one warp per omega up to FIN_WARP_MAX of them, where its
+// blocks still fill the chip a few times over; one thread per omega beyond
 __host__ __device__ inline long fin_blocks(const DispShape& sh, int n) {
-  return fin_warp_mode(sh) ? (n + 3) / 4 : (n + 127) / 128;
+  return sh.fin_warp ? (n + 3) / 4 : (n + 127) / 128;
 }
 
 // A block's job is one context: its arguments go to shared memory once, and
@@ -2366,17 +2370,22 @@ __device__ __forceinline__ void stage_bytes(const void* src, void* dst, int n) {
 // A pole-sums block works on one species: it stages the system constants
 // and that species' constants only (an eighth of DispArgs), which matters
 // when a fused round has many small jobs, each of many small blocks.
-template <bool LOW>
 __global__ void __launch_bounds__(128, 3) k_pole_sums_multi(const DispJob* __restrict__ jobs, int nj) {
   __shared__ __align__(16) SysDev ssys;
   __shared__ __align__(16) SpecDev sspec;
   const DispJob& J = job_of(jobs, nj, blockIdx.x, 1);
-  const long lb = (long)blockIdx.x - J.blk[1];
-  const int tile = (int)(lb % J.tiles), s = (int)((lb / J.tiles) % J.S), chunk = (int)(lb / ((long)J.tiles * J.S));
+  long lb = (long)blockIdx.x - J.blk[1];
+  int s = 0;
+  for (; s + 1 < J.S; ++s) {
+    const long nb = pole_blocks(J.sh, s);
+    if (lb < nb) break;
+    lb -= nb;
+  }
   stage_bytes(&J.a->sys, &ssys, sizeof(SysDev));
   stage_bytes(&J.a->sp[s], &sspec, sizeof(SpecDev));
   __syncthreads();
-  pole_body<LOW>(ssys, sspec, J.sh, J.om, J.n, J.js, J.part, J.low, tile, s, chunk);
+  const long unit = lb * 4 + (threadIdx.x >> 5);
+  if (unit < (long)J.sh.nch[s] * J.sh.wt) pole_body(ssys, sspec, J.sh, J.om, J.n, J.part, s, unit);
 }
 
 __global__ void __launch_bounds__(RES_WARPS * 32, 3) k_resonant_multi(const DispJob* __restrict__ jobs, int nj) {
@@ -2391,10 +2400,11 @@ __global__ void k_finalize_multi(const DispJob* __restrict__ jobs, int nj) {
   const DispJob& J = job_of(jobs, nj, blockIdx.x, 3);
   const DispArgs& a = stage_args(J.a, sa);
   const long lb = (long)blockIdx.x - J.blk[3];
-  const bool wm = fin_warp_mode(J.sh);
-  const long w = wm ? lb * (blockDim.x / 32) + threadIdx.x / 32 : lb * blockDim.x + threadIdx.x;
-  finalize_body(a, J.sh, J.om, J.n, J.part, J.low, J.count, J.slot_nn, J.items, J.rel, J.bm, J.D, J.ext, (int)w,
-                wm);
+  if (J.sh.fin_warp)
+    finalize_warp(a, J.sh, J.om, J.n, J.part, J.count, J.slot_nn, J.items, J.rel, J.bm, J.D, J.ext,
+                  lb * (blockDim.x / 32) + threadIdx.x / 32);
+  else
+    finalize_thread(a, J.sh, J.om, J.n, J.part, J.count, J.items, J.D, (int)(lb * blockDim.x + threadIdx.x));
 }
 
 template <typename T>
@@ -2459,9 +2469,6 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->bessel = S.d_bessel;
   o->V = S.d_V;
   o->mom = S.d_mom;
-  o->momf = S.d_momf;
-  o->momh = S.d_momh;
-  o->moml = S.d_moml;
   o->Vh = S.d_Vh;
   o->Vl = S.d_Vl;
   o->Vscale = S.d_Vscale;
@@ -2625,47 +2632,127 @@ TuneShape tune_lookup(const alps_ctx* c, int n, int maxn) {
 
 uint64_t tune_epoch() { return g_tune_epoch.load(); }
 
-// launch shape of a batch of n omegas on a context: j slices and order
-// chunks give small batches more pole-sum blocks, up to about four per SM
-// (default rule), or the autotuner's shape for the batch's bucket.  The
-// shape depends on n, the context and the table only: the slices and
-// chunks fix the summation order.
+// The default lanes per frequency and signed orders per chunk of a batch of
+// u = n orders / 32 warps of single orders at one lane each: more lanes where
+// one lane's sum over the nodes would be the longest chain, fewer where the
+// lanes' own set-up counts.  Within a class the shape is the same for every
+// n, and so are a frequency's sums (csize 0: as many orders as leave twice 32
+// warps per SM, where a batch has warps to spare).  The lines lie where the
+// next form measured faster (us of the pole sums, 128x256 grid, 73 signed
+// orders).  Mixed path: n = 64: 27 with 32 lanes, 30 with 16; 128: 34 with
+// 16, 41 with 32 or 8; 512: 59 with 8, 72 with 16, 80 with 4; 2048: 150 with
+// 8 or 4, 167 with 2; 4096: 256 with 1, 262 with 2, 269 with 4.  FP64 path:
+// 64: 97 with 32, 102 with 16; 512: 622 with 8, 636 with 4; 2867: 3301 with
+// 4, 3452 with 2; 16384: 17760 with 1, 17960 with 2.  At a given number of
+// lanes about one order per lane is best (512 frequencies, 8 lanes: 59 with 8
+// orders, 64 with 4, 81 with 2).
+void default_shape(long u, bool mixed, int* lanes, long* csize) {
+  *lanes = u < 220 ? 32 : (u < 440 ? 16 : (u < 3000 ? 8 : (u < 7700 ? 4 : 1)));
+  if (mixed) *csize = u < 75 ? 8 : (u < 440 ? 4 : (u < 3000 ? 8 : (u < 7700 ? 4 : 0)));
+  else *csize = u < 440 ? 1 : (u < 3000 ? 2 : (u < 7700 ? 4 : 0));
+}
+
+// launch shape of a batch of n omegas on a context (default rule, or the
+// autotuner's shape for the batch's bucket).  The shape depends on n, the
+// context and the table only: the lanes and chunks fix the summation order.
+// tensors: the batch writes chi_low, so every order is a chunk of its own.
+#define FIN_WARP_MAX 4096
+#define ALPS_NOALLOC_SCRATCH_BYTES (16u << 20)
+
+// 256-byte aligned carve-out of n bytes from a scratch array
+inline size_t carve(size_t& off, size_t bytes) {
+  size_t at = (off + 255) & ~(size_t)255;
+  off = at + bytes;
+  return at;
+}
+
+// the scratch of a batch in one array: error word, counts, slots, items,
+// relativistic and closed-form results, arguments, job, and last the
+// partial sums (part_bytes of them); off[] receives the offsets
+enum { SC_FLAGS, SC_COUNT, SC_SLOTS, SC_ITEMS, SC_REL, SC_BM, SC_ARGS, SC_JOB, SC_PART, SC_N };
+size_t scratch_layout(const alps_ctx* c, size_t n, size_t nslots, size_t part_bytes, size_t* off) {
+  const size_t S_ = c->sys.nspec;
+  size_t end = 0;
+  off[SC_FLAGS] = carve(end, sizeof(int));
+  off[SC_COUNT] = carve(end, n * S_ * sizeof(int));
+  off[SC_SLOTS] = carve(end, nslots * sizeof(int));
+  off[SC_ITEMS] = carve(end, nslots * 6 * sizeof(double2));
+  off[SC_REL] = carve(end, n * S_ * rel_capacity(c) * 2 * REL_RB * 6 * sizeof(double2));
+  off[SC_BM] = carve(end, n * S_ * (any_bm(c) ? 24 : 0) * sizeof(double2));
+  off[SC_ARGS] = carve(end, sizeof(DispArgs));
+  off[SC_JOB] = carve(end, DISP_JOB_BYTES);
+  off[SC_PART] = carve(end, part_bytes);
+  return end;
+}
+
+// The order chunks that alps_disp_batch_noalloc has always had room for: one
+// for about every four warps per SM of 128-frequency tiles.  A batch that
+// fits its static array with so many chunks has to fit it with the shape
+// chosen here, which is the same for every entry point.
+long noalloc_chunks(int n, int S_, int maxn) {
+  const int js = n < 32 ? 32 : (n < 64 ? 4 : (n < 128 ? 2 : 1)), tw = 128 / js;
+  const long tiles = (long)((n + tw - 1) / tw) * S_;
+  const long nchunk = std::max(1L, std::min(maxn + 1L, (152L * 4 + tiles - 1) / tiles));
+  long csize = (maxn + nchunk) / nchunk;
+  if (n < 32) csize = std::max(csize, (long)std::min(maxn + 1, 16 / std::max(1, n)));
+  return (maxn + csize) / csize;
+}
+
 struct BatchGeom {
-  int js, tiles;
   size_t nslots;
   DispShape sh;
 };
-BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap) {
+BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool tensors) {
   BatchGeom b;
   const TuneShape ts = tune_lookup(c, n, maxn);
-  b.js = ts.js ? ts.js : ((n < 32) ? 32 : ((n < 64) ? 4 : ((n < 128) ? 2 : 1)));
-  const int TW = 128 / b.js;
-  b.tiles = (n + TW - 1) / TW;
-  const int want_blocks = 152 * (ts.blocks_per_sm ? ts.blocks_per_sm : 4);
-  const int nchunk = std::max(1, std::min(maxn + 1, (want_blocks + b.tiles * S_ - 1) / (b.tiles * S_)));
-  b.sh.csize = (maxn + 1 + nchunk - 1) / nchunk;
-  // a batch of a few frequencies gives each block at least about 16
-  // (frequency, order) pairs: alone it still spreads over enough blocks, and
-  // in a fused round of thousands of such batches (the uneven batch, the
-  // server) the blocks stay worth their set-up
-  if (n < 32) b.sh.csize = std::max(b.sh.csize, std::min(maxn + 1, 16 / std::max(1, n)));
-  b.sh.nchunk = (maxn + 1 + b.sh.csize - 1) / b.sh.csize;
+  const bool mixed = c->precision != ALPS_PREC_FP64;
+  DispShape& sh = b.sh;
+  long orders = 0;
+  for (int s = 0; s < S_; ++s)
+    if (!c->spec[s].sp.relat && !c->spec[s].sp.use_bM) orders += 2 * c->spec[s].nmax + 1;
+  long csize = 0;
+  default_shape((long)n * orders / 32, mixed, &sh.js, &csize);
+  if (tensors) sh.js = 32;
+  else if (ts.js) sh.js = ts.js;
+  sh.wt = (int)(((long)n * sh.js + 31) / 32);
+  if (ts.blocks_per_sm || csize == 0) {
+    const long want = ts.blocks_per_sm ? 152L * 4 * ts.blocks_per_sm : 152L * 64;
+    csize = (orders * sh.wt + want - 1) / want;
+  }
+  if (tensors) csize = 1;
+  csize = std::max(csize, 1L);
   b.nslots = (size_t)n * S_ * rcap;
-  b.sh.ipw = res_items_per_warp((long)b.nslots, ts.warps_per_sm ? ts.warps_per_sm : 12);
+  if (!tensors) {
+    size_t off[SC_N];
+    const size_t row = (size_t)n * S_ * 6 * sizeof(double2);
+    if (scratch_layout(c, n, b.nslots, row * noalloc_chunks(n, S_, maxn), off) <= ALPS_NOALLOC_SCRATCH_BYTES) {
+      const long room = (long)((ALPS_NOALLOC_SCRATCH_BYTES - off[SC_PART]) / row);
+      csize = std::max(csize, (2L * maxn + room) / room);
+    }
+  }
+  sh.nchunk = 1;
+  for (int s = 0; s < ALPS_MAX_SPECIES; ++s) {
+    const bool has = s < S_ && !c->spec[s].sp.relat && !c->spec[s].sp.use_bM;
+    sh.nch[s] = has ? (int)((2 * c->spec[s].nmax + 1 + csize - 1) / csize) : 0;
+    sh.nchunk = std::max(sh.nchunk, sh.nch[s]);
+  }
+  // a lane sums a series alone while its terms cost less than the slices of
+  // a node sum
+  sh.kmid = (int)(0.8 * (c->sys.npar - 1) / sh.js) + 16;
+  sh.ipw = res_items_per_warp((long)b.nslots, ts.warps_per_sm ? ts.warps_per_sm : 12);
+  sh.fin_warp = (n <= FIN_WARP_MAX || tensors || rel_capacity(c) || any_bm(c)) ? 1 : 0;
   return b;
 }
 
 namespace {
 
 // the job of a lone batch (first blocks at 0)
-DispJob lone_job(const DispShape& sh, int n, int js, int tiles, int S_, const double2* om, double2* D, double2* part,
+DispJob lone_job(const DispShape& sh, int n, int S_, const double2* om, double2* D, double2* part,
                  int* count, int* slots, double2* items, int* flags) {
   DispJob j;
   j.a = nullptr;
   j.sh = sh;
   j.n = n;
-  j.js = js;
-  j.tiles = tiles;
   j.S = S_;
   for (int k = 0; k < 4; ++k) j.blk[k] = 0;
   j.om = om;
@@ -2675,7 +2762,6 @@ DispJob lone_job(const DispShape& sh, int n, int js, int tiles, int S_, const do
   j.slot_nn = slots;
   j.items = items;
   j.flags = flags;
-  j.low = nullptr;
   j.ext = nullptr;
   j.rel = nullptr;
   j.bm = nullptr;
@@ -2707,12 +2793,11 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   DispArgs a;
   int maxn = 0;
   build_disp_args(c, &a, &maxn);
-  const BatchGeom bg = batch_geom(c, n, S_, maxn, a.rcap);
+  const BatchGeom bg = batch_geom(c, n, S_, maxn, a.rcap, d_ext != nullptr);
   const DispShape sh = bg.sh;
-  const int js = bg.js, tiles = bg.tiles;
   const size_t nslots = bg.nslots;
   int rcode;
-  const void* before[8] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_low, c->d_rel, c->d_bm, c->d_flags};
+  const void* before[7] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_rel, c->d_bm, c->d_flags};
   if ((rcode = ensure_buf(c->d_part, c->part_cap, (size_t)n * S_ * sh.nchunk * 6))) return rcode;
   if ((rcode = ensure_buf(c->d_count, c->count_cap, (size_t)n * S_))) return rcode;
   if (nslots * 6 > c->items_cap || !c->d_slot_nn) {
@@ -2722,16 +2807,13 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     c->d_slot_nn = nullptr;
     ALPS_CUDA_TRY(cudaMalloc(&c->d_slot_nn, (c->items_cap / 6) * sizeof(int)));
   }
-  bool want_low = d_ext != nullptr;
-  if (want_low)
-    if ((rcode = ensure_buf(c->d_low, c->low_cap, (size_t)n * S_ * sh.nchunk * 18))) return rcode;
   if (a.relcap)
     if ((rcode = ensure_buf(c->d_rel, c->rel_cap, (size_t)n * S_ * a.relcap * 2 * REL_RB * 6))) return rcode;
   if (a.has_bm)
     if ((rcode = ensure_buf(c->d_bm, c->bm_cap, (size_t)n * S_ * 24))) return rcode;
   if (!c->d_flags) ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, sizeof(int)));
-  const void* after[8] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_low, c->d_rel, c->d_bm, c->d_flags};
-  for (int q = 0; q < 8; ++q)
+  const void* after[7] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_rel, c->d_bm, c->d_flags};
+  for (int q = 0; q < 7; ++q)
     if (before[q] != after[q]) c->gen++;  // buffer addresses changed: cached graphs are stale
   ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, sizeof(int), st));
 
@@ -2754,8 +2836,7 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     ALPS_CUDA_TRY(cudaMallocHost(&c->h_args, sizeof(DispArgs)));
   }
   if (!c->d_job) ALPS_CUDA_TRY(cudaMalloc(&c->d_job, sizeof(DispJob)));
-  DispJob job = lone_job(sh, n, js, tiles, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_flags);
-  job.low = want_low ? c->d_low : nullptr;
+  DispJob job = lone_job(sh, n, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_flags);
   job.ext = d_ext;
   job.rel = a.relcap ? c->d_rel : nullptr;
   job.bm = a.has_bm ? c->d_bm : nullptr;
@@ -2768,14 +2849,11 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   k_classify_multi<<<(unsigned)cls_blocks(n, S_), 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (c->profiling) ALPS_CUDA_TRY(cudaEventRecord(ev[1], st));
-  const unsigned g2 = (unsigned)((long)tiles * S_ * sh.nchunk);
+  const long g2 = pole_blocks_all(sh, S_);
   const size_t smem = res_smem(c);
   if ((rcode = res_smem_optin(smem))) return rcode;
   long blocks = ((long)nslots + RES_WARPS * sh.ipw - 1) / (RES_WARPS * sh.ipw);
-  if (want_low)
-    k_pole_sums_multi<true><<<g2, 128, 0, st>>>(dj, 1);
-  else
-    k_pole_sums_multi<false><<<g2, 128, 0, st>>>(dj, 1);
+  if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (c->profiling) ALPS_CUDA_TRY(cudaEventRecord(ev[2], st));
   k_resonant_multi<<<(unsigned)blocks, RES_WARPS * 32, smem, st>>>(dj, 1);
@@ -2882,18 +2960,16 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     int rcode = ctx_device_args(c, st, &da);
     if (rcode) return rcode;
     const int S_ = c->sys.nspec;
-    const BatchGeom bg = batch_geom(c, n[j], S_, c->args_maxn, c->args_rcap);
+    const BatchGeom bg = batch_geom(c, n[j], S_, c->args_maxn, c->args_rcap, false);
     DispJob& J = m->h_jobs[j];
     J.a = da;
     J.sh = bg.sh;
     J.n = n[j];
-    J.js = bg.js;
-    J.tiles = bg.tiles;
     J.S = S_;
     J.blk[0] = blk[0];
     blk[0] += cls_blocks(n[j], S_);
     J.blk[1] = blk[1];
-    blk[1] += (long)bg.tiles * S_ * bg.sh.nchunk;
+    blk[1] += pole_blocks_all(bg.sh, S_);
     J.blk[2] = blk[2];
     blk[2] += ((long)bg.nslots + RES_WARPS * bg.sh.ipw - 1) / (RES_WARPS * bg.sh.ipw);
     J.blk[3] = blk[3];
@@ -2901,7 +2977,6 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     J.om = d_om + om_off;
     J.D = d_D + om_off;
     J.flags = d_flags + j;
-    J.low = nullptr;
     J.ext = nullptr;
     J.rel = nullptr;
     J.bm = nullptr;
@@ -2962,7 +3037,7 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
   ALPS_CUDA_TRY(cudaMemsetAsync(ml.flags, 0, (size_t)ml.nj * sizeof(int), st));
   k_classify_multi<<<(unsigned)ml.blocks[0], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
-  k_pole_sums_multi<false><<<(unsigned)ml.blocks[1], 128, 0, st>>>(jobs, ml.nj);
+  k_pole_sums_multi<<<(unsigned)ml.blocks[1], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
   k_resonant_multi<<<(unsigned)ml.blocks[2], RES_WARPS * 32, ml.smem, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
@@ -2996,7 +3071,6 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 // alps_batch_status reports the call's device errors (read it before the
 // next call on the device clears the word).
 // ===========================================================================
-#define ALPS_NOALLOC_SCRATCH_BYTES (16u << 20)
 #define ALPS_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[ALPS_NOALLOC_SCRATCH_BYTES];
@@ -3004,13 +3078,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[ALPS_NOALLOC_SC
 namespace {
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[ALPS_NOALLOC_MAX_DEVICES] = {nullptr};
-
-// 256-byte aligned carve-out of n bytes from the scratch array
-inline size_t carve(size_t& off, size_t bytes) {
-  size_t at = (off + 255) & ~(size_t)255;
-  off = at + bytes;
-  return at;
-}
 }  // namespace
 
 extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d_om, alps_complex* d_D,
@@ -3040,44 +3107,35 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   DispArgs a;
   int maxn = 0;
   build_disp_args(c, &a, &maxn);
-  const BatchGeom bg = batch_geom(c, n, S_, maxn, a.rcap);
+  const BatchGeom bg = batch_geom(c, n, S_, maxn, a.rcap, false);
   const DispShape sh = bg.sh;
-  const int js = bg.js, tiles = bg.tiles;
-  // scratch layout: flags | count | slot_nn | part | items | relativistic orders | NHDS
-  size_t off = 0;
-  size_t o_flags = carve(off, sizeof(int));
-  size_t o_count = carve(off, (size_t)n * S_ * sizeof(int));
-  size_t nslots = bg.nslots;
-  size_t o_slots = carve(off, nslots * sizeof(int));
-  size_t o_part = carve(off, (size_t)n * S_ * sh.nchunk * 6 * sizeof(double2));
-  size_t o_items = carve(off, nslots * 6 * sizeof(double2));
-  size_t o_rel = carve(off, (size_t)n * S_ * a.relcap * 2 * REL_RB * 6 * sizeof(double2));
-  size_t o_bm = carve(off, (size_t)n * S_ * (a.has_bm ? 24 : 0) * sizeof(double2));
-  size_t o_args = carve(off, sizeof(DispArgs));
-  size_t o_job = carve(off, sizeof(DispJob));
-  if (scratch_bytes) *scratch_bytes = off;
-  if (off > ALPS_NOALLOC_SCRATCH_BYTES) return ALPS_E_INVALID;  // batch too large for the static scratch
+  size_t off[SC_N];
+  const size_t nslots = bg.nslots;
+  const size_t total = scratch_layout(c, n, nslots, (size_t)n * S_ * sh.nchunk * 6 * sizeof(double2), off);
+  if (scratch_bytes) *scratch_bytes = total;
+  if (total > ALPS_NOALLOC_SCRATCH_BYTES) return ALPS_E_INVALID;  // batch too large for the static scratch
   unsigned char* b = static_cast<unsigned char*>(base);
-  int* flags = reinterpret_cast<int*>(b + o_flags);
-  int* count = reinterpret_cast<int*>(b + o_count);
-  int* slots = reinterpret_cast<int*>(b + o_slots);
-  double2* part = reinterpret_cast<double2*>(b + o_part);
-  double2* items = reinterpret_cast<double2*>(b + o_items);
-  double2* relb = reinterpret_cast<double2*>(b + o_rel);
-  double2* bmb = reinterpret_cast<double2*>(b + o_bm);
+  int* flags = reinterpret_cast<int*>(b + off[SC_FLAGS]);
+  int* count = reinterpret_cast<int*>(b + off[SC_COUNT]);
+  int* slots = reinterpret_cast<int*>(b + off[SC_SLOTS]);
+  double2* part = reinterpret_cast<double2*>(b + off[SC_PART]);
+  double2* items = reinterpret_cast<double2*>(b + off[SC_ITEMS]);
+  double2* relb = reinterpret_cast<double2*>(b + off[SC_REL]);
+  double2* bmb = reinterpret_cast<double2*>(b + off[SC_BM]);
   const double2* om = reinterpret_cast<const double2*>(d_om);
   double2* D = reinterpret_cast<double2*>(d_D);
   ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
-  DispJob job = lone_job(sh, n, js, tiles, S_, om, D, part, count, slots, items, flags);
+  DispJob job = lone_job(sh, n, S_, om, D, part, count, slots, items, flags);
   job.rel = a.relcap ? relb : nullptr;
   job.bm = a.has_bm ? bmb : nullptr;
-  DispArgs* da = reinterpret_cast<DispArgs*>(b + o_args);
-  DispJob* dj = reinterpret_cast<DispJob*>(b + o_job);
+  DispArgs* da = reinterpret_cast<DispArgs*>(b + off[SC_ARGS]);
+  DispJob* dj = reinterpret_cast<DispJob*>(b + off[SC_JOB]);
   k_stage<<<1, 128, 0, st>>>(a, job, da, dj);
   ALPS_CUDA_TRY(cudaGetLastError());
   k_classify_multi<<<(unsigned)cls_blocks(n, S_), 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
-  k_pole_sums_multi<false><<<(unsigned)((long)tiles * S_ * sh.nchunk), 128, 0, st>>>(dj, 1);
+  const long g2 = pole_blocks_all(sh, S_);
+  if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   const size_t smem = res_smem(c);
   int rcode0 = res_smem_optin(smem);
@@ -3188,8 +3246,8 @@ extern "C" int alps_autotune(alps_ctx* c, int n, const alps_complex* d_om_in, al
       g_tune[tune_key(c, n, maxn)] = best;
     }
     g_tune_epoch++;
-    const BatchGeom bg = batch_geom(c, n, c->sys.nspec, maxn, a.rcap);
-    out->js = bg.js;
+    const BatchGeom bg = batch_geom(c, n, c->sys.nspec, maxn, a.rcap, false);
+    out->js = bg.sh.js;
     out->blocks_per_sm = best.blocks_per_sm ? best.blocks_per_sm : 4;
     out->warps_per_sm = best.warps_per_sm ? best.warps_per_sm : 12;
     out->tuned = best.js != 0;

@@ -128,7 +128,7 @@ size_t ctx_device_bytes(const alps_ctx* c) {
     }
   }
   b += c->batch_cap * 2 * sizeof(double2) + c->ext_cap * sizeof(double2);
-  b += (c->part_cap + c->low_cap + c->items_cap + c->rel_cap + c->bm_cap) * sizeof(double2);
+  b += (c->part_cap + c->items_cap + c->rel_cap + c->bm_cap) * sizeof(double2);
   return b;
 }
 
