@@ -63,10 +63,10 @@ __global__ void k_int_ee(const double* __restrict__ g2, const double* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// Levenberg-Marquardt fit of the analytic continuation.  One warp walks the
+// Levenberg-Marquardt fit of the analytic continuation.  One block walks the
 // iperp rows of one species in order (each row starts from the previous
-// result, src/ALPS_analyt.f90:518); within a row the lanes share the points
-// and the entries of J^T J, and every sum keeps the reference's order.
+// result, src/ALPS_analyt.f90:518); within a row the threads share the
+// points, the warps the entries of J^T J, and one warp solves.
 // ---------------------------------------------------------------------------
 struct FitArgs {
   int N, M, nf, log_fit;
@@ -187,206 +187,322 @@ __device__ void fit_jacobian(const FitArgs& a, const double* params, int iperp, 
 #define FIT_MAXP (5 * ALPS_MAX_FITS)
 
 // One species' fit: fit[(i*5+ip)*nf + ifit] holds the seeds at row 0 on
-// entry and the fitted rows on exit.  scratch: (M+1)*(FIT_MAXP+1), with M
-// the largest row length.  Rows are the iperp rows of the f0 table, or for a
-// relativistic species the Gamma rows of f0_rel restricted to the subluminal
-// cone (src/ALPS_analyt.f90:546-607).
-// One species' fit, run by one warp: the points of a row are spread over
-// the lanes; the scalar control flow (LM step, LU, parameter update) runs
-// identically in every lane, and every sum over points runs in the
-// reference's order.  Am_sh / jr_sh: the warp's shared scratch.
+// entry and the fitted rows on exit.  Rows are the iperp rows of the f0
+// table, or for a relativistic species the Gamma rows of f0_rel restricted to
+// the subluminal cone (src/ALPS_analyt.f90:546-607).
+//
+// Bound by the FP64 pipe of one SM (two lanes a clock) and by the chain of
+// its iterations: the rows follow one another, so a fit cannot take more than
+// one.  Hence few FP64 operations per point and iteration:
+//   * the logarithms of a row's table are taken once, for the next row while
+//     one warp solves;
+//   * an accepted step's residuals are the next iteration's (the reference
+//     forms them twice);
+//   * one Maxwellian in log space (the usual fit) needs no exponential: its
+//     log is linear in (log p0, p1) and its Jacobian over the value is
+//     (1/p0, -d^2, 2 p1 d).  Where the value itself would leave the normal
+//     numbers the exponentials decide as the reference's do.
+// Sums over points are trees (32 lanes), more exact than the reference's
+// running sums; the step solves (J^T J + lambda diag) delta = J^T r by the
+// same partial-pivot elimination without forming the inverse.
+// On a 192x384 grid, two species: 35.7 ms as one warp with the sums in
+// series, 3.7 ms so.
+#define FIT_THREADS 256
+struct FitShared {
+  double a[FIT_MAXP * (FIT_MAXP + 1)];  // normal matrix, right-hand side in the last column
+  double params[FIT_MAXP], delta[FIT_MAXP];
+  double red[FIT_THREADS / 32];
+  int lower, upper, singular;
+};
+// doubles of point storage per point: two rows of table values, residual,
+// value, Jacobian
+__host__ __device__ inline int fit_point_words(int n_params) { return 4 + n_params; }
+
+__device__ __forceinline__ double fit_block_sum(double v, FitShared& sh) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh.red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = sh.red[0];
+  for (int k = 1; k < FIT_THREADS / 32; ++k) t += sh.red[k];
+  __syncthreads();
+  return t;
+}
+
 __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, const double* __restrict__ pperp,
-                            const double* __restrict__ ppar, double* fit, double* scratch, int* status,
-                            double* Am_sh, double* jr_sh) {
-  const int lane = threadIdx.x & 31;
-  int nf = a.nf, N = a.rel ? a.ng : a.N;
+                            const double* __restrict__ ppar, double* fit, double* pts, int* status,
+                            FitShared& sh) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nf = a.nf, N = a.rel ? a.ng : a.N;
+  const int maxpts = a.rel ? a.np : a.M, P = maxpts + 1;
   int n_params = 0;
   for (int f = 0; f < nf; ++f) n_params += fit_nparams(a, a.fit_type[f]);
-  double params[FIT_MAXP];
-  bool mask[FIT_MAXP];
-  double* JT = scratch;                         // [(npts)][FIT_MAXP]
-  int maxpts = a.rel ? a.np : a.M;
-  double* resid = scratch + (size_t)(maxpts + 1) * FIT_MAXP;
   if (!a.rel && (1 + a.M) < n_params) {
-    if (lane == 0) *status = ALPS_E_FIT_POINTS;
+    if (tid == 0) *status = ALPS_E_FIT_POINTS;
     return;
   }
-  for (int iperp = 0; iperp <= N; ++iperp) {
-    if (iperp != 0 && lane == 0)
-      for (int ip = 0; ip < 5; ++ip)
-        for (int f = 0; f < nf; ++f) fit[(iperp * 5 + ip) * nf + f] = fit[((iperp - 1) * 5 + ip) * nf + f];
-    __syncwarp();
-    int par_ind = 0, nJT = 0;
-    for (int k = 0; k < n_params; ++k) mask[k] = true;
+  double *resid = pts + 2 * (size_t)P, *fval = pts + 3 * (size_t)P, *JT = pts + 4 * (size_t)P;
+  const bool maxw = nf == 1 && a.fit_type[0] == 1 && a.log_fit && !a.rel;
+  // the seeds
+  {
+    int par_ind = 0;
     for (int ifit = 1; ifit <= nf; ++ifit) {
-      int t = a.fit_type[ifit - 1];
-      int np = fit_nparams(a, t);
-      for (int k = 0; k < np; ++k) params[ifit + par_ind + k - 1] = fit[(iperp * 5 + k) * nf + ifit - 1];
-      if (t == 2 && iperp == 0) { nJT -= 1; mask[ifit + par_ind + 4 - 1] = false; }
-      if (t == 6 && iperp == 0) { nJT -= 1; mask[ifit + par_ind + 3 - 1] = false; }
+      const int np = fit_nparams(a, a.fit_type[ifit - 1]);
+      if (tid < np) sh.params[ifit + par_ind + tid - 1] = fit[tid * nf + ifit - 1];
       par_ind += np - 1;
     }
-    nJT += n_params;
+  }
+  // the table values of a row (log f0 in log space) to buffer row & 1
+  auto load_row = [&](int row, int off, int npts, int t0, int nt) {
+    double* g = pts + (size_t)(row & 1) * P;
+    for (int j = t0; j <= npts; j += nt) {
+      const double v = a.rel ? a.f0rel[(size_t)row * (a.np + 1) + off + j] : f0[row * (a.M + 1) + j];
+      g[j] = a.log_fit ? log(v) : v;
+    }
+  };
+  if (!a.rel) load_row(0, 0, a.M, tid, FIT_THREADS);
+  __syncthreads();
+  for (int iperp = 0; iperp <= N; ++iperp) {
+    if (iperp != 0)
+      for (int t = tid; t < 5 * nf; t += FIT_THREADS) fit[(iperp * 5) * nf + t] = fit[((iperp - 1) * 5) * nf + t];
+    int nJT = n_params;
+    unsigned mask = 0xffffffffu;  // parameters that are fitted
+    {
+      int par_ind = 0;
+      for (int ifit = 1; ifit <= nf; ++ifit) {
+        const int t = a.fit_type[ifit - 1];
+        if (t == 2 && iperp == 0) { nJT -= 1; mask &= ~(1u << (ifit + par_ind + 4 - 1)); }
+        if (t == 6 && iperp == 0) { nJT -= 1; mask &= ~(1u << (ifit + par_ind + 3 - 1)); }
+        par_ind += fit_nparams(a, t) - 1;
+      }
+    }
     // points of this row: coordinates and fitted values
-    int npts, off = 0;
+    int npts = a.M, off = 0;
     double xperp;
     if (a.rel) {
       const double* fr = a.f0rel + (size_t)iperp * (a.np + 1);
-      bool fl = false, fu = false;
-      int lower = 1, upper = a.np - 1;
-      for (int ip = 1; ip <= a.np - 1; ++ip) {
-        if (!fl && fr[ip - 1] <= -1.0 && fr[ip] > -1.0) { lower = ip; fl = true; }
-        if (!fu && fr[ip] > -1.0 && fr[ip + 1] <= -1.0) { upper = ip; fu = true; }
+      if (tid == 0) sh.lower = sh.upper = a.np;
+      __syncthreads();
+      // the cone's ends: the first rise above -1 and the first fall below it
+      for (int ip = 1 + tid; ip <= a.np - 1; ip += FIT_THREADS) {
+        if (fr[ip - 1] <= -1.0 && fr[ip] > -1.0) atomicMin(&sh.lower, ip);
+        if (fr[ip] > -1.0 && fr[ip + 1] <= -1.0) atomicMin(&sh.upper, ip);
       }
+      __syncthreads();
+      const int lower = sh.lower < a.np ? sh.lower : 1, upper = sh.upper < a.np ? sh.upper : a.np - 1;
+      __syncthreads();
       xperp = a.grel[iperp];
       if ((upper - lower) <= 2) {
-        int pi2 = 0;
-        for (int ifit = 1; ifit <= nf; ++ifit) {
-          params[ifit + pi2 - 1] = fr[(upper + lower) / 2] / exp(-a.pc[ifit - 1] * a.grel[iperp]);
-          if (a.fit_type[ifit - 1] == 5) {
-            params[ifit + pi2] = 1.0e-12;
-            params[ifit + pi2 + 1] = 0.0;
-            pi2 += 2;
+        if (tid == 0) {
+          int pi2 = 0;
+          for (int ifit = 1; ifit <= nf; ++ifit) {
+            sh.params[ifit + pi2 - 1] = fr[(upper + lower) / 2] / exp(-a.pc[ifit - 1] * a.grel[iperp]);
+            if (a.fit_type[ifit - 1] == 5) {
+              sh.params[ifit + pi2] = 1.0e-12;
+              sh.params[ifit + pi2 + 1] = 0.0;
+              pi2 += 2;
+            }
           }
         }
         npts = -1;
       } else {
         npts = upper - lower;
         off = lower;
+        load_row(iperp, off, npts, tid, FIT_THREADS);
       }
+      __syncthreads();
     } else {
-      npts = a.M;
       xperp = pperp[iperp];
     }
-    auto xpar = [&](int j) { return a.rel ? a.prel[off + j] : ppar[j]; };
-    auto gval = [&](int j) {
-      double v = a.rel ? a.f0rel[(size_t)iperp * (a.np + 1) + off + j] : f0[iperp * (a.M + 1) + j];
-      return a.log_fit ? log(v) : v;
-    };
+    const double* g = pts + (size_t)(iperp & 1) * P;
+    const double* xp = a.rel ? a.prel + off : ppar;
+    bool ahead = a.rel || iperp == N;  // the next row's table values are there (or are not wanted)
     if (npts >= 0) {
-      double lambda_fit = a.lambda0, LSQ = 0.0, LSQnew;
+      // residuals (and values) at the current parameters; returns their sum
+      // of squares.  maxw without exponentials, where the value is a normal
+      // number on the whole row.
+      auto residuals = [&](bool& plain) {
+        double s = 0.0;
+        plain = false;
+        double lp = 0.0;
+        const double p0 = sh.params[0], p1 = sh.params[1], p2 = sh.params[2];
+        if (maxw && p0 > 0.0) {
+          lp = log(p0) - a.pc[0] * (xperp * xperp);
+          const double d0 = xp[0] - p2, d1 = xp[npts] - p2, dm = fmax(d0 * d0, d1 * d1);
+          plain = p1 >= 0.0 && fabs(lp) < 600.0 && lp - p1 * dm > -690.0;
+        }
+        if (plain) {
+          for (int j = tid; j <= npts; j += FIT_THREADS) {
+            const double d = xp[j] - p2, r = (g[j] - lp) + p1 * (d * d);
+            resid[j] = r;
+            s = fma(r, r, s);
+          }
+        } else {
+          for (int j = tid; j <= npts; j += FIT_THREADS) {
+            const double fv = fit_value_real(a, sh.params, xperp, xp[j]);
+            const double r = a.log_fit ? g[j] - log(fv) : g[j] - fv;
+            fval[j] = fv;
+            resid[j] = r;
+            s = fma(r, r, s);
+          }
+        }
+        return fit_block_sum(s, sh);
+      };
+      double lambda_fit = a.lambda0;
       int counter = 0;
-      bool converged = false;
+      bool converged = false, plain;
+      double LSQ = residuals(plain);
       while (!converged) {
         counter++;
-        for (int j = lane; j <= npts; j += 32) {
-          double* Jc = JT + (size_t)j * FIT_MAXP;
-          fit_jacobian(a, params, iperp, xperp, xpar(j), Jc);
-          double fv = fit_value_real(a, params, xperp, xpar(j));
-          if (a.log_fit) {
-            for (int k = 0; k < nJT; ++k) Jc[k] = Jc[k] / fv;
-            resid[j] = gval(j) - log(fv);
-          } else {
-            resid[j] = gval(j) - fv;
+        if (plain) {
+          const double ip0 = 1.0 / sh.params[0], p1 = sh.params[1], p2 = sh.params[2];
+          for (int j = tid; j <= npts; j += FIT_THREADS) {
+            const double d = xp[j] - p2;
+            JT[j] = ip0;
+            JT[P + j] = -(d * d);
+            JT[2 * P + j] = 2.0 * p1 * d;
+          }
+        } else {
+          for (int j = tid; j <= npts; j += FIT_THREADS) {
+            double J[FIT_MAXP];
+            fit_jacobian(a, sh.params, iperp, xperp, xp[j], J);
+            const double iv = a.log_fit ? 1.0 / fval[j] : 1.0;
+            for (int k = 0; k < nJT; ++k) JT[(size_t)k * P + j] = J[k] * iv;
           }
         }
-        __syncwarp();
-        LSQ = 0.0;
-        for (int j = 0; j <= npts; ++j) LSQ = LSQ + resid[j] * resid[j];
-        double Am[FIT_MAXP * FIT_MAXP], jr[FIT_MAXP];
-        for (int t = lane; t < nJT * nJT + nJT; t += 32) {
+        __syncthreads();
+        // J^T J (upper triangle) and J^T r: a warp per entry
+        const int nq = nJT * (nJT + 1) / 2 + nJT, ld = nJT + 1;
+        for (int t = warp; t < nq; t += FIT_THREADS / 32) {
+          int k, l;
+          if (t < nJT) {
+            k = t;
+            l = nJT;
+          } else {
+            int u = t - nJT;
+            for (k = 0; u >= nJT - k; ++k) u -= nJT - k;
+            l = k + u;
+          }
+          const double *x = JT + (size_t)k * P, *y = l == nJT ? resid : JT + (size_t)l * P;
           double acc = 0.0;
-          if (t < nJT * nJT) {
-            int k = t % nJT, l = t / nJT;
-            for (int j = 0; j <= npts; ++j) acc += JT[(size_t)j * FIT_MAXP + k] * JT[(size_t)j * FIT_MAXP + l];
-            Am_sh[t] = acc;
-          } else {
-            int k = t - nJT * nJT;
-            for (int j = 0; j <= npts; ++j) acc += JT[(size_t)j * FIT_MAXP + k] * resid[j];
-            jr_sh[k] = acc;
+          for (int j = lane; j <= npts; j += 32) acc = fma(x[j], y[j], acc);
+          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          if (lane == 0) {
+            if (l == k) acc = acc + lambda_fit * acc;
+            sh.a[k * ld + l] = acc;
+            if (l < nJT) sh.a[l * ld + k] = acc;
           }
         }
-        __syncwarp();
-        for (int t = 0; t < nJT * nJT; ++t) Am[t] = Am_sh[t];
-        for (int k = 0; k < nJT; ++k) jr[k] = jr_sh[k];
-        __syncwarp();
-        for (int k = 0; k < nJT; ++k) Am[k + nJT * k] = Am[k + nJT * k] + lambda_fit * Am[k + nJT * k];
-        // LU with partial pivoting (dgetrf), then inverse (dgetri) times JT*r
-        int piv[FIT_MAXP];
-        bool singular = false;
-        for (int k = 0; k < nJT && !singular; ++k) {
-          int p = k;
-          double mx = fabs(Am[k + nJT * k]);
-          for (int i = k + 1; i < nJT; ++i)
-            if (fabs(Am[i + nJT * k]) > mx) { mx = fabs(Am[i + nJT * k]); p = i; }
-          piv[k] = p;
-          if (Am[p + nJT * k] == 0.0) { singular = true; break; }
-          if (p != k)
-            for (int jj = 0; jj < nJT; ++jj) {
-              double tmp = Am[k + nJT * jj];
-              Am[k + nJT * jj] = Am[p + nJT * jj];
-              Am[p + nJT * jj] = tmp;
+        __syncthreads();
+        if (warp == 0) {
+          // elimination with partial pivoting on the augmented matrix
+          bool singular = false;
+          for (int k = 0; k < nJT; ++k) {
+            int p = k;
+            double mx = fabs(sh.a[k * ld + k]);
+            for (int i = k + 1; i < nJT; ++i)
+              if (fabs(sh.a[i * ld + k]) > mx) { mx = fabs(sh.a[i * ld + k]); p = i; }
+            if (sh.a[p * ld + k] == 0.0) { singular = true; break; }
+            __syncwarp();
+            if (p != k && lane >= k && lane <= nJT) {
+              const double tmp = sh.a[k * ld + lane];
+              sh.a[k * ld + lane] = sh.a[p * ld + lane];
+              sh.a[p * ld + lane] = tmp;
             }
-          for (int i = k + 1; i < nJT; ++i) {
-            Am[i + nJT * k] /= Am[k + nJT * k];
-            for (int jj = k + 1; jj < nJT; ++jj) Am[i + nJT * jj] -= Am[i + nJT * k] * Am[k + nJT * jj];
+            __syncwarp();
+            const int i = k + 1 + lane;
+            double f = 0.0;
+            if (i < nJT) f = sh.a[i * ld + k] / sh.a[k * ld + k];
+            __syncwarp();
+            if (i < nJT) sh.a[i * ld + k] = f;
+            __syncwarp();
+            const int m = nJT - k;  // columns k + 1 .. nJT
+            for (int t = lane; t < (nJT - k - 1) * m; t += 32) {
+              const int r = k + 1 + t / m, c = k + 1 + t % m;
+              sh.a[r * ld + c] -= sh.a[r * ld + k] * sh.a[k * ld + c];
+            }
+            __syncwarp();
           }
+          if (!singular)
+            for (int i = nJT - 1; i >= 0; --i) {
+              const double x = sh.a[i * ld + nJT] / sh.a[i * ld + i];
+              __syncwarp();
+              if (lane < i) sh.a[lane * ld + nJT] -= sh.a[lane * ld + i] * x;
+              if (lane == 0) sh.delta[i] = x;
+              __syncwarp();
+            }
+          if (lane == 0) {
+            sh.singular = singular;
+            if (!singular)
+              for (int k = 0, l = 0; k < n_params; ++k)
+                if ((mask >> k) & 1u) sh.params[k] = sh.params[k] + sh.delta[l++];
+          }
+        } else if (!ahead) {
+          load_row(iperp + 1, 0, a.M, tid - 32, FIT_THREADS - 32);
         }
-        if (singular) {
-          if (lane == 0) *status = ALPS_E_SINGULAR;
+        ahead = true;
+        __syncthreads();
+        if (sh.singular) {
+          if (tid == 0) *status = ALPS_E_SINGULAR;
           return;
         }
-        double inv[FIT_MAXP * FIT_MAXP];
-        for (int cc = 0; cc < nJT; ++cc) {
-          double x[FIT_MAXP];
-          for (int i = 0; i < nJT; ++i) x[i] = (i == cc) ? 1.0 : 0.0;
-          for (int k = 0; k < nJT; ++k) {
-            double tmp = x[k];
-            x[k] = x[piv[k]];
-            x[piv[k]] = tmp;
-          }
-          for (int i = 0; i < nJT; ++i)
-            for (int k = 0; k < i; ++k) x[i] -= Am[i + nJT * k] * x[k];
-          for (int i = nJT - 1; i >= 0; --i) {
-            for (int k = i + 1; k < nJT; ++k) x[i] -= Am[i + nJT * k] * x[k];
-            x[i] /= Am[i + nJT * i];
-          }
-          for (int i = 0; i < nJT; ++i) inv[i + nJT * cc] = x[i];
-        }
-        double delta[FIT_MAXP];
-        for (int k = 0; k < nJT; ++k) {
-          double acc = 0.0;
-          for (int l = 0; l < nJT; ++l) acc += inv[k + nJT * l] * jr[l];
-          delta[k] = acc;
-        }
-        int l = 0;
-        for (int k = 0; k < n_params; ++k)
-          if (mask[k]) params[k] = params[k] + delta[l++];
-        for (int j = lane; j <= npts; j += 32) {
-          double fv = fit_value_real(a, params, xperp, xpar(j));
-          resid[j] = a.log_fit ? gval(j) - log(fv) : gval(j) - fv;
-        }
-        __syncwarp();
-        LSQnew = 0.0;
-        for (int j = 0; j <= npts; ++j) LSQnew = LSQnew + resid[j] * resid[j];
-        __syncwarp();
+        const double LSQnew = residuals(plain);
+        const double diff = fabs(LSQnew - LSQ);
         if (LSQnew > LSQ) {
-          l = 0;
-          for (int k = 0; k < n_params; ++k)
-            if (mask[k]) params[k] = params[k] - delta[l++];
+          if (tid == 0)
+            for (int k = 0, l = 0; k < n_params; ++k)
+              if ((mask >> k) & 1u) sh.params[k] = sh.params[k] - sh.delta[l++];
+          __syncthreads();
           lambda_fit = lambda_fit * a.lambdafac;
         } else {
           lambda_fit = lambda_fit / a.lambdafac;
         }
-        if (fabs(LSQnew - LSQ) < a.eps) converged = true;
+        if (diff < a.eps) converged = true;
         if (counter == a.maxsteps) converged = true;
+        // the residuals at the parameters the next iteration starts from
+        if (!converged) LSQ = (LSQnew > LSQ) ? residuals(plain) : LSQnew;
       }
     }
-    par_ind = 0;
-    for (int ifit = 1; ifit <= nf && lane == 0; ++ifit) {
-      int np = fit_nparams(a, a.fit_type[ifit - 1]);
-      for (int k = 0; k < np; ++k) fit[(iperp * 5 + k) * nf + ifit - 1] = params[ifit + par_ind + k - 1];
-      par_ind += np - 1;
+    if (!ahead) load_row(iperp + 1, 0, a.M, tid, FIT_THREADS);
+    {
+      int par_ind = 0;
+      for (int ifit = 1; ifit <= nf; ++ifit) {
+        const int np = fit_nparams(a, a.fit_type[ifit - 1]);
+        if (tid < np) fit[(iperp * 5 + tid) * nf + ifit - 1] = sh.params[ifit + par_ind + tid - 1];
+        par_ind += np - 1;
+      }
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
-__global__ void k_lm_fit(FitArgs a, const double* __restrict__ f0, const double* __restrict__ pperp,
-                         const double* __restrict__ ppar, double* fit, double* scratch, int* status) {
+// the fit's point storage: shared memory where it fits, else the global
+// scratch (maxpts + 1) fit_point_words(FIT_MAXP) of the species
+__device__ __forceinline__ double* fit_points(const FitArgs& a, double* scratch, double* smem, int smem_words) {
+  int n_params = 0;
+  for (int f = 0; f < a.nf; ++f) n_params += fit_nparams(a, a.fit_type[f]);
+  const int P = (a.rel ? a.np : a.M) + 1;
+  return (long)P * fit_point_words(n_params) <= smem_words ? smem : scratch;
+}
+
+__global__ void __launch_bounds__(FIT_THREADS) k_lm_fit(FitArgs a, const double* __restrict__ f0,
+                                                        const double* __restrict__ pperp,
+                                                        const double* __restrict__ ppar, double* fit, double* scratch,
+                                                        int* status, int smem_words) {
+  extern __shared__ double fit_smem[];
+  __shared__ FitShared sh;
   if (blockIdx.x != 0) return;
-  __shared__ double Am_sh[FIT_MAXP * FIT_MAXP], jr_sh[FIT_MAXP];
-  lm_fit_body(a, f0, pperp, ppar, fit, scratch, status, Am_sh, jr_sh);
+  lm_fit_body(a, f0, pperp, ppar, fit, fit_points(a, scratch, fit_smem, smem_words), status, sh);
+}
+
+// Dynamic shared memory (in doubles) that a fit wants, at most FIT_SMEM_WORDS;
+// a larger one uses its global scratch
+#define FIT_SMEM_WORDS 12288
+inline int fit_smem_words(const FitArgs& a) {
+  static const int np[7] = {1, 3, 5, 3, 1, 3, 4};  // parameters by fit type
+  int n_params = 0;
+  for (int f = 0; f < a.nf; ++f) n_params += np[a.fit_type[f] >= 1 && a.fit_type[f] <= 6 ? a.fit_type[f] : 0];
+  const long w = (long)((a.rel ? a.np : a.M) + 1) * fit_point_words(n_params);
+  return w <= FIT_SMEM_WORDS ? (int)w : 0;
 }
 
 }  // namespace
@@ -401,14 +517,25 @@ struct FitJob {
 
 namespace {
 
-// every job of the batch, one warp each: fits of different plasmas are
+// every job of the batch, one block each: fits of different plasmas are
 // independent; within a fit the reference's warm start orders the rows
-__global__ void k_lm_fit_many(const FitJob* __restrict__ jobs, int n) {
+__global__ void __launch_bounds__(FIT_THREADS) k_lm_fit_many(const FitJob* __restrict__ jobs, int n, int smem_words) {
+  extern __shared__ double fit_smem[];
+  __shared__ FitShared sh;
+  __shared__ FitJob J;
   const int j = blockIdx.x;
   if (j >= n) return;
-  __shared__ double Am_sh[FIT_MAXP * FIT_MAXP], jr_sh[FIT_MAXP];
-  const FitJob& J = jobs[j];
-  lm_fit_body(J.a, J.f0, J.pperp, J.ppar, J.fit, J.scratch, J.status, Am_sh, jr_sh);
+  if (threadIdx.x == 0) J = jobs[j];
+  __syncthreads();
+  lm_fit_body(J.a, J.f0, J.pperp, J.ppar, J.fit, fit_points(J.a, J.scratch, fit_smem, smem_words), J.status, sh);
+}
+
+// both fit kernels may take FIT_SMEM_WORDS doubles
+int fit_smem_optin() {
+  const int bytes = FIT_SMEM_WORDS * (int)sizeof(double);
+  ALPS_CUDA_TRY(cudaFuncSetAttribute(k_lm_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  ALPS_CUDA_TRY(cudaFuncSetAttribute(k_lm_fit_many, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  return ALPS_OK;
 }
 
 // determine_nmax for one species: the smallest n >= 1 with
@@ -1004,9 +1131,13 @@ int launch_prepare_species(alps_ctx* c, int is) {
     a.prel = S.d_prel;
     int maxpts = a.rel ? a.np : M;
     int rc;
-    if ((rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(maxpts + 1) * (FIT_MAXP + 1)))) return rc;
+    if ((rc = fit_smem_optin())) return rc;
+    const int words = fit_smem_words(a);
+    if (!words && (rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(maxpts + 1) * fit_point_words(FIT_MAXP))))
+      return rc;
     ALPS_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));
-    k_lm_fit<<<1, 32, 0, st>>>(a, S.d_f0, S.d_pperp, S.d_ppar, S.d_fit, S.d_fit_scratch, d_status);
+    k_lm_fit<<<1, FIT_THREADS, words * sizeof(double), st>>>(a, S.d_f0, S.d_pperp, S.d_ppar, S.d_fit, S.d_fit_scratch,
+                                                             d_status, words);
     ALPS_CUDA_TRY(cudaGetLastError());
     ALPS_CUDA_TRY(cudaMemcpyAsync(&st_fit, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ALPS_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1022,7 +1153,7 @@ int launch_prepare_species(alps_ctx* c, int is) {
 // Batched preparation of many contexts (alps_prepare_many): the derivative
 // and ee kernels of every context on a few streams, then the
 // Levenberg-Marquardt fits of every (context, species) in one launch, one
-// warp each, then one synchronisation.  Relativistic species and the
+// block each, then one synchronisation.  Relativistic species and the
 // Chebyshev continuation take the per-context path.
 // ---------------------------------------------------------------------------
 static FitArgs fit_args_of(const alps_ctx* c, const SpeciesHost& S) {
@@ -1062,7 +1193,7 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
   for (int q = 0; q < NS; ++q) ALPS_CUDA_TRY(cudaStreamCreateWithFlags(&st[q], cudaStreamNonBlocking));
   std::vector<FitJob> jobs;
   std::vector<std::pair<int, int>> who;  // (context, species) of each job
-  int rc = ALPS_OK;
+  int rc = fit_smem_optin(), fit_words = 0;
   for (int i = 0; i < n && !rc; ++i) {
     alps_ctx* c = ctx[i];
     cudaStream_t s = st[i % NS];
@@ -1079,8 +1210,13 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
       if (!S.d_g2 && !rc) fail(cudaMalloc(&S.d_g2, nn * sizeof(double)));
       if (!S.d_G && !rc) fail(cudaMalloc(&S.d_G, (size_t)(N - 1) * 2 * (M - 1) * sizeof(double)));
       if (!S.d_words && !rc) fail(cudaMalloc(&S.d_words, 2 * sizeof(double)));
-      if (!rc && (rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(M + 1) * (FIT_MAXP + 1)))) break;
       if (rc) break;
+      const FitArgs fa = fit_args_of(c, S);
+      const int words = fit_smem_words(fa);
+      fit_words = std::max(fit_words, words);
+      if (!words &&
+          (rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(M + 1) * fit_point_words(FIT_MAXP))))
+        break;
       fail(cudaMemsetAsync(S.d_g1, 0, nn * sizeof(double), s));
       fail(cudaMemsetAsync(S.d_g2, 0, nn * sizeof(double), s));
       fail(cudaMemsetAsync(S.d_words + 1, 0, sizeof(double), s));
@@ -1091,7 +1227,7 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
       k_int_ee<<<1, 256, 0, s>>>(S.d_g2, S.d_ppar, N, M, scale, S.d_words);
       fail(cudaGetLastError());
       FitJob j;
-      j.a = fit_args_of(c, S);
+      j.a = fa;
       j.f0 = S.d_f0;
       j.pperp = S.d_pperp;
       j.ppar = S.d_ppar;
@@ -1111,7 +1247,8 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
                    cudaSuccess)
       rc = ALPS_E_CUDA;
     if (!rc) {
-      k_lm_fit_many<<<(unsigned)jobs.size(), 32, 0, st[0]>>>(d_jobs, (int)jobs.size());
+      k_lm_fit_many<<<(unsigned)jobs.size(), FIT_THREADS, fit_words * sizeof(double), st[0]>>>(
+          d_jobs, (int)jobs.size(), fit_words);
       if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st[0]) != cudaSuccess) rc = ALPS_E_CUDA;
     }
   }
