@@ -149,7 +149,8 @@ void alps_destroy(alps_ctx* c) {
     cudaFree(S.d_f0rel);
     cudaFree(S.d_dfr1);
     cudaFree(S.d_dfr2);
-    cudaFree(S.d_jrel);
+    cudaFree(S.d_jrel);  // d_relfam and d_relcoef point into it
+    cudaFree(S.d_relgam);
     cudaFree(S.d_cone);
     cudaFree(S.d_bmI);
   }

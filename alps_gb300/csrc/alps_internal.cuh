@@ -137,7 +137,12 @@ struct __align__(16) SpecDev {
   const double* f0rel;  // [(ng+1)*(np+1)], -1 outside the subluminal cone
   const double* dfr1;   // d f0_rel / d Gamma
   const double* dfr2;   // d f0_rel / d pparbar
-  const double* jrel;   // [(n)*(ng+1)*(np+1)], n = 0..nmax+1: J_n at each node
+  const double* relfam;  // [(n*3 + F)*(ng+1)*(np+1)]: the Bessel products of each node
+  const double* relcoef; // [(nu)*21], nu = 0..nmax+1: CBESSJ's series coefficients
+  const double* relgam;  // [(N+1)(M+1)] gamma on the (pperp, ppar) grid
+  const double* relg2g;  // g2 / gamma
+  const float* relgf;    // gamma in FP32
+  const double* Rw;      // [(F*(nmax+1) + n)*(N-1) + i-1] weighted Bessel rows
   const int2* cone;     // [ng+1] first and last pparbar index inside the cone
   double int_ee_rel;
   // Chebyshev continuation (ACmethod 2): order, log10 cut, p_par end points
@@ -207,7 +212,9 @@ struct SpeciesHost {
   // relativistic species
   std::vector<double> grel, prel;         // host copies of the grid vectors
   double *d_grel = nullptr, *d_prel = nullptr, *d_f0rel = nullptr, *d_dfr1 = nullptr, *d_dfr2 = nullptr;
-  double* d_jrel = nullptr;
+  double* d_jrel = nullptr;               // J_n planes; the two below share its allocation
+  double *d_relfam = nullptr, *d_relcoef = nullptr;
+  double* d_relgam = nullptr;             // gamma, g2/gamma and gamma in FP32 on the (pperp, ppar) grid
   int2* d_cone = nullptr;
   // NHDS species: exp(-z) I_n(z) table of the current k_perp
   double* d_bmI = nullptr;

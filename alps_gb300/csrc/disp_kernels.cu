@@ -2539,7 +2539,15 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->f0rel = S.d_f0rel;
   o->dfr1 = S.d_dfr1;
   o->dfr2 = S.d_dfr2;
-  o->jrel = S.d_jrel;
+  o->relfam = S.d_relfam;
+  o->relcoef = S.d_relcoef;
+  {
+    const size_t nn = (size_t)(c->sys.nperp + 1) * (c->sys.npar + 1);
+    o->relgam = S.d_relgam;
+    o->relg2g = S.d_relgam ? S.d_relgam + nn : nullptr;
+    o->relgf = S.d_relgam ? reinterpret_cast<const float*>(S.d_relgam + 2 * nn) : nullptr;
+  }
+  o->Rw = S.d_Rw;
   o->cone = S.d_cone;
   o->int_ee_rel = S.int_ee_rel;
   o->poly_order = S.sp.poly_order;

@@ -6,10 +6,10 @@
 // mask (f0_rel = -1 outside), normalisation, and the one-sided derivatives at
 // the cone edge (derivative_f0_rel, :36-289; polyharmonic_spline, :293-426),
 // then the ee term (int_ee_rel, :1097-1215).
-// Per k (launch_rel_bessel): J_n at every (Gamma, pparbar) node; the
-// reference calls BESSJ there once per point and mode (int_T_rel, :1297-1298),
-// with omega-independent arguments, so a table holds the same values.
-// Per omega batch (launch_rel_orders): one block per (omega, species, n):
+// Per k (launch_rel_bessel): the Bessel products of int_T_rel (:1256-1369) at
+// every (Gamma, pparbar) node, whose arguments do not depend on omega, and the
+// coefficients of CBESSJ's power series.
+// Per omega batch (launch_rel_orders): REL_RB blocks per (omega, species, n):
 // the resonance test over the whole (pperp, ppar) grid (determine_resonances,
 // src/ALPS_fns.f90:680-702), then either the regular-grid trapezoid sum with
 // the Lorentz factor in resU (src/ALPS_fns.f90:799-864, 1560-1596) or the
@@ -261,6 +261,39 @@ __global__ void k_rel_jtab(const double* __restrict__ grel, const double* __rest
   jrel[t] = (z == z) ? alps_bessj(n, z) : z;
 }
 
+// The Bessel products of int_T_rel at every node, planes fam[(n*3 + F)] of
+// (ng+1)(np+1): F = 0: J_n^2, 1: J_n'^2 pperpbar^2, 2: J_n J_n' pperpbar, from
+// the planes J_0 .. J_nmax+1.  They are the same for orders n and -n.
+__global__ void k_rel_families(const double* __restrict__ jrel, const double* __restrict__ grel,
+                               const double* __restrict__ prel, int ng, int np, int nmax, double* fam) {
+  const long tot = (long)(ng + 1) * (np + 1);
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= tot * (nmax + 1)) return;
+  const int n = (int)(t / tot);
+  const long pt = t % tot;
+  const double g = grel[pt / (np + 1)], pb = prel[pt % (np + 1)];
+  const double pp = sqrt(g * g - 1.0 - pb * pb);
+  const double b = jrel[n * tot + pt];
+  const double bp = n == 0 ? -jrel[tot + pt] : 0.5 * (jrel[(n - 1) * tot + pt] - jrel[(n + 1) * tot + pt]);
+  fam[(n * 3L + 0) * tot + pt] = b * b;
+  fam[(n * 3L + 1) * tot + pt] = bp * bp * pp * pp;
+  fam[(n * 3L + 2) * tot + pt] = b * bp * pp;
+}
+
+// gamma on the (pperp, ppar) grid, g2/gamma, and gamma in FP32 (the resonance
+// test's estimate)
+__global__ void k_rel_gamma(const double* __restrict__ pperp, const double* __restrict__ ppar,
+                            const double* __restrict__ g2, int N, int M, double vA, double ms, double* gam,
+                            double* g2g, float* gf) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long)(N + 1) * (M + 1)) return;
+  const double p1 = pperp[t / (M + 1)], p2 = ppar[t % (M + 1)];
+  const double g = sqrt((p1 * p1 + p2 * p2) * (vA * vA) / (ms * ms) + 1.0);
+  gam[t] = g;
+  g2g[t] = g2[t] / g;
+  gf[t] = (float)g;
+}
+
 // first and last pparbar index inside the cone of each Gamma row
 // (integrate_resU_rel, src/ALPS_fns_rel.f90:603-617)
 __global__ void k_rel_cone(const double* __restrict__ f0rel, int ng, int np, int2* cone) {
@@ -482,6 +515,14 @@ int launch_rel_prepare(alps_ctx* c, int is) {
   if (!S.d_dfr1) ALPS_CUDA_TRY(cudaMalloc(&S.d_dfr1, nf * sizeof(double)));
   if (!S.d_dfr2) ALPS_CUDA_TRY(cudaMalloc(&S.d_dfr2, nf * sizeof(double)));
   if (!S.d_cone) ALPS_CUDA_TRY(cudaMalloc(&S.d_cone, (ng + 1) * sizeof(int2)));
+  if (!S.d_relgam) ALPS_CUDA_TRY(cudaMalloc(&S.d_relgam, (size_t)(N + 1) * (M + 1) * 20));
+  {
+    const size_t nn = (size_t)(N + 1) * (M + 1);
+    k_rel_gamma<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(S.d_pperp, S.d_ppar, S.d_g2, N, M, vA, ms, S.d_relgam,
+                                                               S.d_relgam + nn,
+                                                               reinterpret_cast<float*>(S.d_relgam + 2 * nn));
+    ALPS_CUDA_TRY(cudaGetLastError());
+  }
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_grel, S.grel.data(), (ng + 1) * sizeof(double), cudaMemcpyHostToDevice, st));
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_prel, S.prel.data(), (np + 1) * sizeof(double), cudaMemcpyHostToDevice, st));
   // dense thin-plate-spline system (the reference sets its smoothing to 0
@@ -591,23 +632,6 @@ extern "C" int alps_interpolate(const double* pperp_c, const double* ppar_c, con
   return status;
 }
 
-int launch_rel_bessel(alps_ctx* c, int is, double kperp) {
-  SpeciesHost& S = c->spec[is];
-  int ng = c->sys.ngamma, np = c->sys.npparbar, nrows = S.nmax + 2;
-  size_t need = (size_t)nrows * (ng + 1) * (np + 1);
-  if (need > S.jrel_cap || !S.d_jrel) {
-    if (S.d_jrel) cudaFree(S.d_jrel);
-    S.d_jrel = nullptr;
-    ALPS_CUDA_TRY(cudaMalloc(&S.d_jrel, need * sizeof(double)));
-    S.jrel_cap = need;
-  }
-  double zfac = kperp * S.sp.ms / (c->sys.vA * S.sp.qs);
-  k_rel_jtab<<<(unsigned)((need + 127) / 128), 128, 0, c->stream>>>(S.d_grel, S.d_prel, ng, np, nrows, zfac,
-                                                                     S.d_jrel);
-  ALPS_CUDA_TRY(cudaGetLastError());
-  return ALPS_OK;
-}
-
 // ===========================================================================
 // omega batch
 // ===========================================================================
@@ -618,61 +642,6 @@ struct RelArgs {
   SpecDev sp[ALPS_MAX_SPECIES];
   int relcap;
 };
-
-// six int_T entries with the factors i (entry 4) and -i (entry 6) left out;
-// they are applied once to the finished sums (multiplying by i is exact)
-struct C6 {
-  double2 v[6];
-};
-
-__device__ inline void c6_zero(C6& a) {
-#pragma unroll
-  for (int e = 0; e < 6; ++e) a.v[e] = cmk(0.0, 0.0);
-}
-
-// sum over the 32 lanes of a warp, the same butterfly on every lane (the
-// result, on all lanes, does not depend on timing)
-__device__ inline void c6_warp_sum(C6& a) {
-#pragma unroll
-  for (int e = 0; e < 6; ++e)
-    for (int o = 16; o > 0; o >>= 1) {
-      a.v[e].x += __shfl_xor_sync(0xffffffffu, a.v[e].x, o);
-      a.v[e].y += __shfl_xor_sync(0xffffffffu, a.v[e].y, o);
-    }
-}
-
-// Bessel pair of signed order m from J(k), k >= 0 (int_T_rel :1297-1329)
-template <typename T, typename F>
-__device__ inline void bessel_pair_m(int m, F J, T& b, T& bp) {
-  auto sgn = [](int k) { return (k % 2 == 0) ? 1.0 : -1.0; };
-  if (m < 0) b = J(-m) * sgn(m);
-  else b = J(m);
-  if (m >= 1) bp = (J(m - 1) - J(m + 1)) * 0.5;
-  else if (m < -1) bp = (J(-(m - 1)) * sgn(m - 1) - J(-(m + 1)) * sgn(m + 1)) * 0.5;
-  else if (m == 0) bp = J(1) * -1.0;
-  else bp = (J(2) - J(0)) * 0.5;
-}
-
-// int_T_rel entries at node (ig, ip) (src/ALPS_fns_rel.f90:1256-1369)
-__device__ inline void t_node_rel(const SpecDev& S, const SysDev& sy, int m, int ig, int ip, double t[6]) {
-  const double ms = S.ms, qs = S.qs, vA = sy.vA, kperp = sy.kperp;
-  const bool kn = sy.kperp_norm != 0;
-  const double g = S.grel[ig], pb = S.prel[ip];
-  const double pperpbar = sqrt(g * g - 1.0 - pb * pb);
-  const double zbar = kn ? kperp * ms / (vA * qs) : ms / (vA * qs);
-  const size_t plane = (size_t)(S.ng + 1) * (S.np + 1);
-  const double* J0 = S.jrel + (size_t)ig * (S.np + 1) + ip;
-  auto J = [&](int k) { return J0[(size_t)k * plane]; };
-  double b, bp;
-  bessel_pair_m(m, J, b, bp);
-  const double kf = kn ? 1.0 : kperp, kf2 = kn ? 1.0 : kperp * kperp;
-  t[0] = 1.0 * (m * m) * b * b / (zbar * zbar);
-  t[1] = kf2 * bp * bp * pperpbar * pperpbar;
-  t[2] = kf2 * b * b * (pb * pb);
-  t[3] = (1.0 * m) * kf * b * bp * pperpbar / zbar;
-  t[4] = (1.0 * m) * kf * b * b * pb / zbar;
-  t[5] = kf2 * b * bp * pb * pperpbar;
-}
 
 // fit_function for the Gamma rows, fit types 4 and 5 (src/ALPS_analyt.f90:244-258)
 __device__ inline double2 eval_fit_rel(const SpecDev& S, int ig, double2 p) {
@@ -707,60 +676,55 @@ __device__ inline double gamma_lanczos(double xx) {
   return exp(tmp + log(2.50662827465 * ser));
 }
 
+// coefficients of CBESSJ's power series (src/ALPS_fns_rel.f90:1502-1553):
+// coef[nu*21 + k] = 1 / (k! Gamma(nu + k + 1)), nu = 0 .. nmax + 1
+__global__ void k_rel_coef(int nmax, double* coef) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (nmax + 2) * 21) return;
+  const int nu = t / 21, k = t % 21;
+  double fk = 1.0;
+  for (int q = 2; q <= k; ++q) fk = fk * (1.0 * q);
+  coef[t] = 1.0 / (fk * gamma_lanczos(1.0 * (nu + k + 1)));
+}
+
+// CBESSJ over (z/2)^nu: sum_k coef[k] q^k, q = -z^2/4
+__device__ inline double2 cbessj_series(const double* coef, double2 q) {
+  double2 s = cmk(coef[20], 0.0);
+  for (int k = 19; k >= 0; --k) s = cmk(fma(s.x, q.x, fma(-s.y, q.y, coef[k])), fma(s.x, q.y, s.y * q.x));
+  return s;
+}
+
+// x^n, n >= 0
 __device__ inline double2 cpowi_d(double2 x, int n) {
   double2 pw = cmk(1.0, 0.0);
-  if (n == 0) return pw;
-  unsigned u = (unsigned)(n < 0 ? -n : n);
-  for (;;) {
+  for (unsigned u = (unsigned)n; u; u >>= 1) {
     if (u & 1) pw = cmul(pw, x);
-    u >>= 1;
-    if (u) x = cmul(x, x);
-    else break;
+    x = cmul(x, x);
   }
-  if (n < 0) pw = cdiv(cmk(1.0, 0.0), pw);
   return pw;
 }
 
-// CBESSJ (src/ALPS_fns_rel.f90:1502-1553): 21-term power series
-__device__ double2 cbessj_d(double2 z, int nu) {
-  double2 sum = cmk(0.0, 0.0);
-  double2 q = cscale(cmul(cneg(z), z), 0.25);
-  double fk = 1.0;
-  for (int k = 0; k <= 20; ++k) {
-    if (k >= 2) fk = fk * (1.0 * k);
-    double2 t = cpowi_d(q, k);
-    t = cmk(t.x / fk, t.y / fk);
-    double gm = gamma_lanczos(1.0 * (nu + k + 1));
-    t = cmk(t.x / gm, t.y / gm);
-    sum = cadd(sum, t);
+// The three Bessel products of int_T_res_rel (src/ALPS_fns_rel.f90:1374-1495)
+// at complex momentum p: J^2, J'^2 pperpbar^2, J J' pperpbar of order n >= 0.
+__device__ inline void res_products(const SpecDev& S, double zfac, int n, double g, double2 p, double2 F[3]) {
+  const double2 pp = csqrt_d(csub(cmk(g * g - 1.0, 0.0), cmul(p, p)));
+  const double2 z = cscale(pp, zfac), hz = cscale(z, 0.5);
+  const double2 q = cscale(cmul(cneg(z), z), 0.25);
+  double2 J, Jp;
+  if (n == 0) {
+    J = cbessj_series(S.relcoef, q);
+    Jp = cneg(cmul(hz, cbessj_series(S.relcoef + 21, q)));
+  } else {
+    const double2 lo = cpowi_d(hz, n - 1), mid = cmul(lo, hz), up = cmul(mid, hz);
+    J = cmul(mid, cbessj_series(S.relcoef + n * 21, q));
+    Jp = cscale(csub(cmul(lo, cbessj_series(S.relcoef + (n - 1) * 21, q)),
+                     cmul(up, cbessj_series(S.relcoef + (n + 1) * 21, q))),
+                0.5);
   }
-  return cmul(cpowi_d(cscale(z, 0.5), nu), sum);
-}
-
-struct cwrap {  // complex value with the arithmetic bessel_pair_m needs
-  double2 v;
-  __device__ cwrap operator*(double s) const { return cwrap{cscale(v, s)}; }
-  __device__ cwrap operator-(const cwrap& o) const { return cwrap{csub(v, o.v)}; }
-};
-
-// int_T_res_rel entries (src/ALPS_fns_rel.f90:1374-1495)
-__device__ void t_res_rel(const SpecDev& S, const SysDev& sy, int m, int ig, double2 pr, double2 t[6]) {
-  const double ms = S.ms, qs = S.qs, vA = sy.vA, kperp = sy.kperp;
-  const bool kn = sy.kperp_norm != 0;
-  const double g = S.grel[ig];
-  double2 pperpbar = csqrt_d(csub(cmk(g * g - 1.0, 0.0), cmul(pr, pr)));
-  double2 z = cscale(pperpbar, kperp * ms / (vA * qs));
-  const double zbar = kn ? kperp * ms / (vA * qs) : ms / (vA * qs);
-  cwrap b, bp;
-  bessel_pair_m(m, [&](int k) { return cwrap{cbessj_d(z, k)}; }, b, bp);
-  const double kf = kn ? 1.0 : kperp, kf2 = kn ? 1.0 : kperp * kperp;
-  double2 bb = cmul(b.v, b.v), bbp = cmul(b.v, bp.v);
-  t[0] = cscale(bb, 1.0 * (m * m) / (zbar * zbar));
-  t[1] = cscale(cmul(cmul(bp.v, bp.v), cmul(pperpbar, pperpbar)), kf2);
-  t[2] = cscale(cmul(bb, cmul(pr, pr)), kf2);
-  t[3] = cscale(cmul(bbp, pperpbar), (1.0 * m) * kf / zbar);
-  t[4] = cscale(cmul(bb, pr), (1.0 * m) * kf / zbar);
-  t[5] = cscale(cmul(bbp, cmul(pr, pperpbar)), kf2);
+  const double2 b = cmul(Jp, pp);
+  F[0] = cmul(J, J);
+  F[1] = cmul(b, b);
+  F[2] = cmul(J, b);
 }
 
 __device__ inline double fr_at(const SpecDev& S, int ig, int ip) {
@@ -768,173 +732,59 @@ __device__ inline double fr_at(const SpecDev& S, int ig, int ip) {
   return S.f0rel[(size_t)ig * (S.np + 1) + ip];
 }
 
-struct RowCtx {
-  const SpecDev& S;
-  const SysDev& sy;
-  double2 om;
-  int m, ig;
-  double Kc;  // -2 pi (ms/vA)^3 q vA / (k_par m)
-};
-
-// integrand of funct_g_rel at a node, six entries
-__device__ inline void h_node_rel(const RowCtx& r, int ip, double2 h[6]) {
-  const SpecDev& S = r.S;
-  size_t k = (size_t)r.ig * (S.np + 1) + ip;
-  double2 A = cadd(cscale(r.om, S.dfr1[k]), cmk((r.sy.kpar / r.sy.vA) * S.dfr2[k], 0.0));
-  A = cscale(A, r.Kc);
-  double t[6];
-  t_node_rel(S, r.sy, r.m, r.ig, ip, t);
-#pragma unroll
-  for (int e = 0; e < 6; ++e) h[e] = cscale(A, t[e]);
-}
-
-// funct_g_rel (src/ALPS_fns_rel.f90:918-999)
-__device__ void funct_g_rel_d(const RowCtx& r, double pp, double2 G[6]) {
-  const SpecDev& S = r.S;
+// funct_g_rel's node for a momentum (src/ALPS_fns_rel.f90:918-960): the last
+// node k in 0..np-1 with pb[k] <= pp (-2 outside the grid) ...
+__device__ inline int rel_piece(const SpecDev& S, double pp) {
   const int np = S.np;
   const double* pb = S.prel;
-  const double dpb = pb[2] - pb[1];
-  int close = -2;
-  if (pp >= pb[0] && pp < pb[np]) {
-    // the last k in 0..np-1 with pb[k] <= pp: the uniform grid's index,
-    // moved by the grid values themselves where rounding put it one off
-    int k = (int)floor((pp - pb[0]) * ((double)np / (pb[np] - pb[0])));
-    k = max(0, min(np - 1, k));
-    while (k > 0 && pb[k] > pp) --k;
-    while (k < np - 1 && pb[k + 1] <= pp) ++k;
-    close = k;
-  }
-  if (fr_at(S, r.ig, close + 1) <= -1.0) close = close - 1;
-  if (fr_at(S, r.ig, close - 1) <= -1.0) close = close + 1;
-  if (pp == pb[np]) close = np - 2;
+  if (!(pp >= pb[0] && pp < pb[np])) return -2;
+  int k = (int)floor((pp - pb[0]) * ((double)np / (pb[np] - pb[0])));
+  k = max(0, min(np - 1, k));
+  while (k > 0 && pb[k] > pp) --k;
+  while (k < np - 1 && pb[k + 1] <= pp) ++k;
+  return k;
+}
+// ... moved inwards at the subluminal cone's edge and off the grid's ends
+__device__ inline int rel_node(const SpecDev& S, int ig, int close, bool at_end) {
+  const int np = S.np;
+  if (fr_at(S, ig, close + 1) <= -1.0) close = close - 1;
+  if (fr_at(S, ig, close - 1) <= -1.0) close = close + 1;
+  if (at_end) close = np - 2;
   if (close >= (np - 1)) close = np - 2;
   if (close <= 1) close = 2;
-  double2 hp[6], hm[6];
-  h_node_rel(r, close + 1, hp);
-  h_node_rel(r, close - 1, hm);
-  h_node_rel(r, close, G);
-  double dx = pp - pb[close];
-#pragma unroll
-  for (int e = 0; e < 6; ++e) G[e] = cadd(G[e], cscale(cscale(csub(hp[e], hm[e]), 1.0 / dpb), 0.5 * dx));
+  return close;
 }
 
-// principal_integral_rel (src/ALPS_fns_rel.f90:724-913), by the 32 lanes of
-// a warp: the sample points are spread over the lanes and the lanes' sums
-// are added by a warp reduction; out (on every lane) receives the window's
-// contribution
-__device__ void principal_rel_d(const RowCtx& r, int ipres, int upperlimit, C6& out, int lane) {
-  const SpecDev& S = r.S;
-  const SysDev& sy = r.sy;
-  const double ms = S.ms, qs = S.qs, vA = sy.vA, kpar = sy.kpar;
-  const int M_I = sy.M_I, M_P = sy.M_P;
-  const double* pb = S.prel;
-  const double dpb = pb[2] - pb[1];
-  const double g = S.grel[r.ig];
-  double2 t1 = cscale(cscale(r.om, g), vA);
-  t1 = cmk(t1.x / kpar, t1.y / kpar);
-  const double denomR = t1.x - (1.0 * r.m) * (qs / ms) * vA / kpar;
-  const double denomI = t1.y;
-  const double capDelta = denomR - pb[ipres - M_I];
-  const double smdelta = capDelta / (1.0 * M_P);
-  C6 pi;
-  c6_zero(pi);
-  double2 Ga[6], Gb[6];
-  const double2 dIp = cmk(0.0, -denomI), dIm = cmk(0.0, denomI);
-  // sum += w*(G(pp)/(pp-dR-i dI) - G(2dR-pp)/(pp-dR+i dI))
-  auto pair = [&](double pp, double w) {
-    funct_g_rel_d(r, pp, Ga);
-    funct_g_rel_d(r, 2.0 * denomR - pp, Gb);
-    double2 da = cadd(cmk(pp - denomR, 0.0), dIp), db = cadd(cmk(pp - denomR, 0.0), dIm);
-#pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      pi.v[e] = cadd(pi.v[e], cdiv(cscale(Ga[e], w), da));
-      pi.v[e] = csub(pi.v[e], cdiv(cscale(Gb[e], w), db));
-    }
-  };
-  if (fabs(denomI) > sy.Tlim) {
-    if (lane == 0) pair(denomR, 1.0);
-    if (lane == 1) pair(denomR + capDelta, 1.0);
-    // sample points rounded as the reference writes them (no FMA): a point
-    // can fall on a node, where funct_g_rel's choice of node depends on it
-    for (int ip = 1 + lane; ip <= M_P - 1; ip += 32) pair(__dadd_rn(denomR, __dmul_rn(smdelta, (double)ip)), 2.0);
-  } else {
-    funct_g_rel_d(r, denomR + dpb, Ga);
-    funct_g_rel_d(r, denomR - dpb, Gb);
-    double2 gp[6];
-#pragma unroll
-    for (int e = 0; e < 6; ++e) {
-      gp[e] = csub(Ga[e], Gb[e]);
-      gp[e] = cmk(gp[e].x / (2.0 * dpb), gp[e].y / (2.0 * dpb));
-    }
-    auto lor = [&](double pp, double w) {
-      double d = pp - denomR;
-      double f = (d * d) / ((d * d) + denomI * denomI);
-#pragma unroll
-      for (int e = 0; e < 6; ++e) pi.v[e] = cadd(pi.v[e], cscale(cscale(gp[e], w), f));
-    };
-    if (lane == 0) lor(denomR + capDelta, 2.0);
-    for (int ip = 1 + lane; ip <= M_P - 1; ip += 32) lor(__dadd_rn(denomR, __dmul_rn(smdelta, (double)ip)), 4.0);
-    if (denomI != 0.0 && lane == 0) {
-      funct_g_rel_d(r, denomR, Ga);
-      double sgn = denomI > 0.0 ? 1.0 : -1.0;
-#pragma unroll
-      for (int e = 0; e < 6; ++e) {
-        double2 q = cscale(Ga[e], 2.0 * ALPS_PI / smdelta);
-        pi.v[e] = cadd(pi.v[e], cmk(-sgn * q.y, sgn * q.x));  // +- i q
-      }
-    }
-  }
-  int ntiny = (int)((pb[upperlimit] - denomR - capDelta) / smdelta);
-  if (ntiny > 0) {
-    double correction = ((pb[upperlimit] - denomR - capDelta) / (1.0 * ntiny)) / smdelta;
-    auto tail = [&](double pp, double w) {
-      funct_g_rel_d(r, pp, Ga);
-      double2 da = cmk(pp - denomR, -denomI);
-#pragma unroll
-      for (int e = 0; e < 6; ++e) pi.v[e] = cadd(pi.v[e], cscale(cdiv(Ga[e], da), w * correction));
-    };
-    if (lane == 0) tail(denomR + capDelta, 1.0);
-    auto tp = [&](int ip) {
-      return __dadd_rn(__dadd_rn(denomR, capDelta), __dmul_rn(__dmul_rn(correction, smdelta), (double)ip));
-    };
-    if (lane == 1) tail(tp(ntiny), 1.0);
-    for (int ip = 1 + lane; ip <= ntiny - 1; ip += 32) tail(tp(ip), 2.0);
-  }
-  c6_warp_sum(pi);
-#pragma unroll
-  for (int e = 0; e < 6; ++e) out.v[e] = cadd(out.v[e], cscale(pi.v[e], smdelta));
-}
+// one Gamma row's integration limits and resonance (integrate_resU_rel,
+// src/ALPS_fns_rel.f90:516-660)
+struct RelRow {
+  double dR, dI;   // the pole
+  double sm;       // spacing of the principal-value samples
+  int i0, lo, up, i1;  // trapezoid over i0..lo and up..i1
+  int ipres;
+  int pv;          // the row has a principal-value window
+};
 
-// integrate_resU_rel for one Gamma row (src/ALPS_fns_rel.f90:516-719), by
-// the 32 lanes of a warp: the window decisions on every lane, the nodes and
-// the principal-value samples spread over the lanes; out (on every lane)
-// receives the row's integral
-__device__ void row_rel_d(const RowCtx& r, C6& out, bool& err, int lane) {
-  const SpecDev& S = r.S;
-  const SysDev& sy = r.sy;
+__device__ RelRow rel_row(const SpecDev& S, const SysDev& sy, double2 om, int m, int ig, bool& err) {
+  RelRow r;
   const double ms = S.ms, qs = S.qs, vA = sy.vA, kpar = sy.kpar;
   const int M_I = sy.M_I, np = S.np;
   const double* pb = S.prel;
   const double dpb = pb[2] - pb[1];
-  const double g = S.grel[r.ig];
-  c6_zero(out);
+  const double g = S.grel[ig];
   // the resonance and its window decided as the reference rounds them (no FMA)
-  const double x = __ddiv_rn(__dmul_rn(__dsub_rn(__dmul_rn(g, r.om.x), __ddiv_rn(__dmul_rn(1.0 * r.m, qs), ms)), vA), kpar);
+  const double x = __ddiv_rn(__dmul_rn(__dsub_rn(__dmul_rn(g, om.x), __ddiv_rn(__dmul_rn(1.0 * m, qs), ms)), vA), kpar);
   int ipres = 0;
   bool found = false;
   if (__dmul_rn(x, x) <= __dsub_rn(__dmul_rn(g, g), 1.0)) {
     // the ip in 1..np-2 with pb[ip] <= x < pb[ip+1]
-    int lo = 1, hi = np - 2;
-    if (np - 2 >= 1 && pb[1] <= x) {
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (pb[mid] <= x) lo = mid;
-        else hi = mid - 1;
-      }
-      if (pb[lo + 1] > x) {
-        ipres = lo;
-        found = true;
-      }
+    if (np - 2 >= 1 && pb[1] <= x && x < pb[np - 1]) {
+      int k = 1 + (int)floor((x - pb[1]) / dpb);
+      k = max(1, min(np - 2, k));
+      while (k > 1 && pb[k] > x) --k;
+      while (k < np - 2 && pb[k + 1] <= x) ++k;
+      ipres = k;
+      found = true;
     }
   }
   for (int ip = 0; ip <= M_I; ++ip) {
@@ -948,113 +798,333 @@ __device__ void row_rel_d(const RowCtx& r, C6& out, bool& err, int lane) {
       found = true;
     }
   }
-  const int2 cn = S.cone[r.ig];
+  const int2 cn = S.cone[ig];
   const int lowerC = cn.x, upperC = cn.y;
-  int int_start, int_end, lowerlimit, upperlimit;
+  r.i0 = lowerC;
   if (found) {
-    int_start = lowerC;
-    int_end = upperC;
-    lowerlimit = ipres - M_I;
-    upperlimit = ipres + M_I + 1;
+    r.i1 = upperC;
+    r.lo = ipres - M_I;
+    r.up = ipres + M_I + 1;
     if ((ipres >= 0) && (ipres <= np))
-      if (fabs(x - pb[ipres]) > (0.5 * dpb)) upperlimit = upperlimit + 1;
-    if ((lowerlimit < lowerC) && (upperlimit > upperC)) {
+      if (fabs(x - pb[ipres]) > (0.5 * dpb)) r.up = r.up + 1;
+    if ((r.lo < lowerC) && (r.up > upperC)) {
       err = true;
-      return;
-    } else if (lowerlimit <= lowerC) {
-      int_start = 1;
-      lowerlimit = 0;
-      upperlimit = lowerC;
-    } else if (upperlimit >= upperC) {
-      lowerlimit = upperC;
-      upperlimit = np;
-      int_end = np - 1;
+      r.i0 = 1;  // nothing is summed
+      r.lo = 0;
+      r.up = 1;
+      r.i1 = 0;
+      found = false;
+    } else if (r.lo <= lowerC) {
+      r.i0 = 1;
+      r.lo = 0;
+      r.up = lowerC;
+    } else if (r.up >= upperC) {
+      r.lo = upperC;
+      r.up = np;
+      r.i1 = np - 1;
     }
   } else {
-    int_start = lowerC;
-    lowerlimit = upperC;
-    int_end = np - 1;
-    upperlimit = np;
+    r.lo = upperC;
+    r.i1 = np - 1;
+    r.up = np;
   }
-  // trapezoid over the nodes away from the pole
-  double2 gom = cscale(cscale(r.om, g), vA);
-  gom = cmk(gom.x / kpar, gom.y / kpar);
-  const double nq = (1.0 * r.m) * qs * vA / (kpar * ms);
-  auto term = [&](int ip, double w) {
-    double2 h[6];
-    h_node_rel(r, ip, h);
-    double2 den = cadd(csub(cmk(pb[ip], 0.0), gom), cmk(nq, 0.0));
-#pragma unroll
-    for (int e = 0; e < 6; ++e) out.v[e] = cadd(out.v[e], cscale(cdiv(h[e], den), w));
-  };
-  if (lane == 0 && int_start <= lowerlimit) term(int_start, 1.0);
-  for (int ip = int_start + 1 + lane; ip <= lowerlimit - 1; ip += 32) term(ip, 2.0);
-  if (lane == 1 && int_start < lowerlimit) term(lowerlimit, 1.0);
-  if (lane == 2 && upperlimit <= int_end) term(upperlimit, 1.0);
-  for (int ip = upperlimit + 1 + lane; ip <= int_end - 1; ip += 32) term(ip, 2.0);
-  if (lane == 3 && upperlimit < int_end) term(int_end, 1.0);
-  c6_warp_sum(out);
-#pragma unroll
-  for (int e = 0; e < 6; ++e) out.v[e] = cscale(out.v[e], dpb);
-  if (found && (lowerlimit >= int_start) && (upperlimit <= int_end)) principal_rel_d(r, ipres, upperlimit, out, lane);
+  const double gx = ((om.x * g) * vA) / kpar;
+  r.dI = ((om.y * g) * vA) / kpar;
+  r.dR = gx - (1.0 * m) * (qs / ms) * vA / kpar;
+  r.ipres = ipres;
+  r.pv = (found && r.lo >= r.i0 && r.up <= r.i1) ? 1 : 0;
+  r.sm = r.pv ? (r.dR - pb[ipres - M_I]) / (1.0 * sy.M_P) : 0.0;
+  return r;
 }
 
-// one Landau row of landau_integrate_rel (src/ALPS_fns_rel.f90:1005-1092)
-__device__ void landau_row_rel_d(const RowCtx& r, C6& acc) {
-  const SpecDev& S = r.S;
-  const SysDev& sy = r.sy;
-  const double ms = S.ms, qs = S.qs, vA = sy.vA, kpar = sy.kpar;
-  const int ig = r.ig;
-  const double g = S.grel[ig];
-  const double dg = S.grel[2] - S.grel[1], dpb = S.prel[2] - S.prel[1];
-  double2 pr = cscale(cscale(r.om, g), vA);
-  pr = cmk(pr.x / kpar - (1.0 * r.m) * qs * vA / (kpar * ms), pr.y / kpar);
-  // inside the subluminal cone, decided as the reference rounds it (no FMA)
-  if (!(__dmul_rn(pr.x, pr.x) <= __dsub_rn(__dmul_rn(g, g), 1.0))) return;
-  double h = (ig == S.ng - 1) ? 0.5 : 1.0;
-  double2 dfg;
-  if (ig == 1) {
-    dfg = csub(eval_fit_rel(S, ig + 1, pr), eval_fit_rel(S, ig, pr));
-    dfg = cmk(dfg.x / dg, dfg.y / dg);
+// A principal-value piece: the samples whose interpolant is that of node a
+// (close), their weights' sum A and first moment B about the node
+struct RelPiece {
+  double2 A, B;
+  int a;
+};
+
+#define REL_WARPS (REL_THREADS / 32)
+#define REL_CHUNK 128  // samples a warp sums between two looks at the pieces' ends
+
+#define REL_PRE_WORDS (3 * (REL_CHUNK + 1) + 1)  // even: the pieces after them are 16-byte aligned
+
+// pieces of a row at most: both sides of the window, the tiny rest
+__host__ __device__ inline int rel_max_pieces(int M_I) { return 2 * (M_I + 4) + 8; }
+// shared memory per warp in doubles: prefix sums of a chunk of samples, pieces
+__host__ __device__ inline size_t rel_warp_words(int M_I) {
+  return REL_PRE_WORDS + (size_t)rel_max_pieces(M_I) * (sizeof(RelPiece) / sizeof(double));
+}
+
+// sum of the 32 lanes before this one
+__device__ inline double lanes_before(double v, int lane) {
+  double s = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double t = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += t;
+  }
+  return s - v;
+}
+
+// Samples p_k, k = 0 .. K, of the principal-value sums, with the weights
+// w_k / (dx - i dI), dx = p_k - dR, cut at given k's: for the lane's cut kc
+// (first k beyond its piece) returns the sums over k < kc of w r dx, w r and
+// w r dx^2, r = 1/(dx^2 + dI^2).  tiny: the rest beyond the symmetric window.
+struct RelSums {
+  double s1, s2, s3;
+};
+struct RelSamples {
+  double dR, cap, sm, corr;
+  int K;
+  bool tiny;
+  __device__ double at(int k) const {
+    if (!tiny) return k == 0 ? dR : (k == K ? dR + cap : __dadd_rn(dR, __dmul_rn(sm, (double)k)));
+    return k == 0 ? dR + cap : __dadd_rn(__dadd_rn(dR, cap), __dmul_rn(__dmul_rn(corr, sm), (double)k));
+  }
+};
+__device__ RelSums rel_cut_sums(const RelSamples& q, double dI2, bool from0, int kc, double* pre, int lane) {
+  RelSums out = {0.0, 0.0, 0.0}, carry = {0.0, 0.0, 0.0};
+  for (int k0 = 0; k0 <= q.K; k0 += REL_CHUNK) {
+    const int n = min(REL_CHUNK, q.K + 1 - k0), per = (n + 31) / 32;
+    const int b = min(n, lane * per), e = min(n, b + per);
+    RelSums loc = {0.0, 0.0, 0.0};
+    for (int j = b; j < e; ++j) {
+      const int k = k0 + j;
+      pre[3 * j] = loc.s1;
+      pre[3 * j + 1] = loc.s2;
+      pre[3 * j + 2] = loc.s3;
+      if (k == 0 && !from0) continue;
+      const double dx = q.at(k) - q.dR;
+      double r = rcp_fast(fma(dx, dx, dI2));
+      r *= (k == 0 || k == q.K) ? 1.0 : 2.0;
+      const double t = dx * r;
+      loc.s1 += t;
+      loc.s2 += r;
+      loc.s3 = fma(dx, t, loc.s3);
+    }
+    const RelSums bef = {carry.s1 + lanes_before(loc.s1, lane), carry.s2 + lanes_before(loc.s2, lane),
+                         carry.s3 + lanes_before(loc.s3, lane)};
+    for (int j = b; j < e; ++j) {
+      pre[3 * j] += bef.s1;
+      pre[3 * j + 1] += bef.s2;
+      pre[3 * j + 2] += bef.s3;
+    }
+    carry.s1 = __shfl_sync(0xffffffffu, bef.s1 + loc.s1, 31);
+    carry.s2 = __shfl_sync(0xffffffffu, bef.s2 + loc.s2, 31);
+    carry.s3 = __shfl_sync(0xffffffffu, bef.s3 + loc.s3, 31);
+    __syncwarp();
+    const int at = kc - k0;
+    if (at >= 0 && at < n) out = {pre[3 * at], pre[3 * at + 1], pre[3 * at + 2]};
+    __syncwarp();
+  }
+  if (kc > q.K) out = carry;
+  return out;
+}
+
+// The pieces of one row's principal-value sum (principal_integral_rel,
+// src/ALPS_fns_rel.f90:724-913), by a warp.  A sample's interpolant is that
+// of one node and linear in p, so each piece needs only the sums of its
+// samples' weights and of their first moments; the samples are summed once,
+// as prefix sums, for both sides of the window, and each lane cuts them at
+// the ends of its piece.  Returns the number of pieces left in rec.
+__device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, int ig, double* pre, RelPiece* rec,
+                          int lane) {
+  const double* pb = S.prel;
+  const int np = S.np, M_P = sy.M_P;
+  const double dpb = pb[2] - pb[1];
+  const double dR = r.dR, dI = r.dI, dI2 = dI * dI;
+  const double cap = dR - pb[r.ipres - sy.M_I], sm = r.sm;
+  const bool sym = fabs(dI) > sy.Tlim;
+  const int cap_rec = rel_max_pieces(sy.M_I);
+  int nrec = 0;
+  RelSamples q = {dR, cap, sm, 1.0, M_P, false};
+  if (sym) {
+    const int jc = rel_piece(S, dR);  // the pole's own interval (the window lies inside the grid)
+    const int nu = max(0, rel_piece(S, dR + cap) - jc) + 1, nd = max(0, jc - rel_piece(S, 2.0 * dR - (dR + cap))) + 1;
+    for (int t0 = 0; t0 < nu + nd; t0 += 32) {
+      const int t = t0 + lane;
+      const bool has = t < nu + nd && t < cap_rec, down = t >= nu;
+      const int i = down ? t - nu : t, j = down ? jc - i : jc + i;
+      // first sample beyond the piece: up p_k >= pb[j+1], down 2 dR - p_k < pb[j]
+      int kc = M_P + 1;
+      if (has && i + 1 < (down ? nd : nu)) {
+        const double edge = down ? pb[j] : pb[j + 1];
+        auto beyond = [&](int k) { return down ? 2.0 * dR - q.at(k) < edge : q.at(k) >= edge; };
+        int k = (int)ceil((down ? dR - edge : edge - dR) / sm);
+        k = max(0, min(M_P + 1, k));
+        while (k > 0 && beyond(k - 1)) --k;
+        while (k <= M_P && !beyond(k)) ++k;
+        kc = k;
+      }
+      const RelSums end = rel_cut_sums(q, dI2, true, kc, pre, lane);
+      // less the sums of the piece before (the lane before; a later round of
+      // 32 pieces starts from its own cut)
+      RelSums beg;
+      beg.s1 = __shfl_up_sync(0xffffffffu, end.s1, 1);
+      beg.s2 = __shfl_up_sync(0xffffffffu, end.s2, 1);
+      beg.s3 = __shfl_up_sync(0xffffffffu, end.s3, 1);
+      if (i == 0) beg = {0.0, 0.0, 0.0};
+      if (t0 > 0 && __any_sync(0xffffffffu, has && lane == 0 && i > 0)) {
+        // the cut at this lane's piece's beginning
+        int kb = 0;
+        if (lane == 0) {
+          const double edge = down ? pb[j + 1] : pb[j];
+          auto beyond = [&](int k) { return down ? 2.0 * dR - q.at(k) < edge : q.at(k) >= edge; };
+          int k = (int)ceil((down ? dR - edge : edge - dR) / sm);
+          k = max(0, min(M_P + 1, k));
+          while (k > 0 && beyond(k - 1)) --k;
+          while (k <= M_P && !beyond(k)) ++k;
+          kb = k;
+        }
+        const RelSums b0 = rel_cut_sums(q, dI2, true, kb, pre, lane);
+        if (lane == 0) beg = b0;
+      }
+      if (has) {
+        const double s1 = end.s1 - beg.s1, s2 = (end.s2 - beg.s2) * dI, s3 = end.s3 - beg.s3;
+        const int a = rel_node(S, ig, j, false);
+        const double del = dR - pb[a];
+        RelPiece pc;
+        pc.a = a;
+        // up: w/(dx - i dI) = w r (dx + i dI); down: -w/(dx + i dI) at -dx
+        pc.A = down ? cmk(-s1, s2) : cmk(s1, s2);
+        pc.B = cmk(fma(del, pc.A.x, s3), fma(del, pc.A.y, down ? -dI * s1 : dI * s1));
+        rec[t] = pc;
+      }
+    }
+    nrec = min(nu + nd, cap_rec);
   } else {
-    dfg = csub(eval_fit_rel(S, ig + 1, pr), eval_fit_rel(S, ig - 1, pr));
-    dfg = cmk(dfg.x / (2.0 * dg), dfg.y / (2.0 * dg));
+    // g' sum_k w_k dx^2/(dx^2 + dI^2), and +- i pi G(p_res)/smdelta
+    const RelSums s = rel_cut_sums(q, dI2, false, M_P + 1, pre, lane);
+    if (lane < 3) {
+      const double p = lane == 0 ? dR + dpb : (lane == 1 ? dR - dpb : dR);
+      const int a = rel_node(S, ig, rel_piece(S, p), p == pb[np]);
+      RelPiece pc;
+      pc.a = a;
+      const double c = s.s3 / dpb;
+      if (lane < 2) pc.A = cmk(lane == 0 ? c : -c, 0.0);
+      else pc.A = cmk(0.0, dI > 0.0 ? 2.0 * ALPS_PI / sm : (dI < 0.0 ? -2.0 * ALPS_PI / sm : 0.0));
+      pc.B = cscale(pc.A, p - pb[a]);
+      rec[lane] = pc;
+    }
+    nrec = 3;
   }
-  double2 dfp = csub(eval_fit_rel(S, ig, cadd(pr, cmk(dpb, 0.0))), eval_fit_rel(S, ig, csub(pr, cmk(dpb, 0.0))));
-  dfp = cmk(dfp.x / (2.0 * dpb), dfp.y / (2.0 * dpb));
-  double2 coef = cscale(cadd(cmul(r.om, dfg), cscale(dfp, kpar / vA)), h);
-  double2 t[6];
-  t_res_rel(S, sy, r.m, ig, pr, t);
-#pragma unroll
-  for (int e = 0; e < 6; ++e) acc.v[e] = csub(acc.v[e], cmul(coef, t[e]));
+  // the tiny rest between dR + capDelta and the upper limit
+  // (bounded: a window of no width, possible only with no principal positions, would ask for 2^31)
+  const double rest = (pb[r.up] - dR - cap) / sm;
+  const int ntiny = rest < 4194304.0 ? (int)rest : (rest >= 4194304.0 ? 4194304 : 0);
+  if (ntiny > 0) {
+    q.corr = ((pb[r.up] - dR - cap) / (1.0 * ntiny)) / sm;
+    q.K = ntiny;
+    q.tiny = true;
+    const int jc = rel_piece(S, q.at(0)), nu = min(4, max(0, rel_piece(S, q.at(ntiny)) - jc) + 1);
+    int kc = ntiny + 1;
+    if (lane + 1 < nu) {
+      const double edge = pb[jc + lane + 1];
+      int k = (int)ceil((edge - q.at(0)) / (q.corr * sm));
+      k = max(0, min(ntiny + 1, k));
+      while (k > 0 && q.at(k - 1) >= edge) --k;
+      while (k <= ntiny && q.at(k) < edge) ++k;
+      kc = k;
+    }
+    const RelSums end = rel_cut_sums(q, dI2, true, kc, pre, lane);
+    RelSums beg;
+    beg.s1 = __shfl_up_sync(0xffffffffu, end.s1, 1);
+    beg.s2 = __shfl_up_sync(0xffffffffu, end.s2, 1);
+    beg.s3 = __shfl_up_sync(0xffffffffu, end.s3, 1);
+    if (lane == 0) beg = {0.0, 0.0, 0.0};
+    if (lane < nu && nrec + lane < cap_rec) {
+      const double s1 = (end.s1 - beg.s1) * q.corr, s2 = (end.s2 - beg.s2) * q.corr * dI, s3 = (end.s3 - beg.s3) * q.corr;
+      const int j = jc + lane, a = rel_node(S, ig, j, q.at(ntiny) == pb[np] && lane == nu - 1);
+      const double del = dR - pb[a];
+      RelPiece pc;
+      pc.a = a;
+      pc.A = cmk(s1, s2);
+      pc.B = cmk(fma(del, s1, s3), fma(del, s2, dI * s1));
+      rec[nrec + lane] = pc;
+    }
+    nrec = min(nrec + nu, cap_rec);
+  }
+  __syncwarp();
+  return nrec;
 }
 
-// deterministic block sum of 12 doubles per thread (blockDim.x = 128)
-// sum over the block's threads (REL_THREADS), in warp order
-__device__ void block_sum12(double v[12], double* sh /* [REL_THREADS/32][12] */) {
+// sum of 12 doubles per thread over the block's threads, in warp order; the
+// total on thread q < 12
+__device__ double block_sum12(double v[12], double* sh /* [REL_WARPS][12] */) {
 #pragma unroll
   for (int q = 0; q < 12; ++q)
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], o);
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
-    for (int q = 0; q < 12; ++q) sh[warp * 12 + q] = v[q];
+    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int q = 0; q < 12; ++q) {
-      double t = sh[q];
-      for (int k = 1; k < REL_THREADS / 32; ++k) t += sh[k * 12 + q];
-      v[q] = t;
-    }
+#pragma unroll
+  for (int q = 0; q < 12; ++q)
+    if (lane == q) sh[warp * 12 + q] = v[q];
   __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 12)
+    for (int k = 0; k < REL_WARPS; ++k) t += sh[k * 12 + threadIdx.x];
+  return t;
 }
 
-// One block per (omega, species, signed order, row block): the REL_RB row
-// blocks of an order each take every REL_RB-th group of Gamma rows (a warp
-// per row) or every REL_RB-th stretch of the regular grid, and write their
-// partial sums to their own slot; k_finalize adds the slots in order.
+// determine_resonances, relativistic branch (src/ALPS_fns.f90:680-702): is
+// there a node (i, j) with ppar_j <= p_res(gamma_ij) < ppar_j+1?  An FP32
+// estimate (error below eps) settles all nodes but those near an interval's
+// ends, where the reference's own rounding decides.
+__device__ bool rel_resonant(const SpecDev& S, const SysDev& sy, double2 om, int m) {
+  const double ms = S.ms, qs = S.qs, vA = sy.vA, kpar = sy.kpar;
+  const int N = S.N, M = S.M;
+  const float a1 = (float)(ms * om.x / kpar), a2 = (float)((1.0 * m) * qs / kpar);
+  const float dp = (float)(S.ppar[2] - S.ppar[1]);
+  const float pmax = fmaxf(fabsf((float)S.ppar[0]), fabsf((float)S.ppar[M]));
+  const int tcols = min(M, (int)blockDim.x), rows = max(1, (int)blockDim.x / tcols);
+  const int c0 = (int)threadIdx.x % tcols, r0 = (int)threadIdx.x / tcols;
+  bool res = false;
+  if (r0 < rows)
+    for (int j = c0; j < M && !res; j += tcols) {
+      const float pj = (float)S.ppar[j];
+      for (int i = r0; i <= N; i += rows) {
+        const float ga = S.relgf[(size_t)i * (M + 1) + j] * a1;
+        const float d = (ga - a2) - pj;
+        const float eps = 1.0e-6f * (fabsf(ga) + fabsf(a2) + pmax);
+        if (d < -eps || d > dp + eps) continue;
+        if (d > eps && d < dp - eps) {
+          res = true;
+          break;
+        }
+        const double p1 = S.pperp[i], p2 = S.ppar[j];
+        const double gamma = __dsqrt_rn(__dadd_rn(
+            __ddiv_rn(__dmul_rn(__dadd_rn(__dmul_rn(p1, p1), __dmul_rn(p2, p2)), __dmul_rn(vA, vA)), __dmul_rn(ms, ms)),
+            1.0));
+        const double pr = __ddiv_rn(__dsub_rn(__dmul_rn(__dmul_rn(gamma, ms), om.x), __dmul_rn(1.0 * m, qs)), kpar);
+        if ((S.ppar[j] <= pr) && (S.ppar[j + 1] > pr)) {
+          res = true;
+          break;
+        }
+      }
+    }
+  return __syncthreads_or(res) != 0;
+}
+
+// REL_RB blocks per (omega, species, signed order): each takes every
+// REL_RB-th Gamma row, or every REL_RB-th row of the regular grid, and writes
+// its partial sums to its own slot; k_finalize adds the slots in order.
+//
+// Bound by the FP64 pipe (two lanes a clock and SM), so the work is laid out
+// to spend few operations per node.  The T-tensor's Bessel products come from
+// tables (k_rel_families; both signs of an order share them), its constant
+// factors, Kc and the derivative's omega are applied once, and a node costs
+// one real reciprocal and 30 operations where six complex divisions took 330.
+// A principal-value sample costs 10 (see rel_pieces) where two interpolants
+// of six entries over three nodes took 1500, and the window then is a few
+// more nodes with complex weights.  Rows' decisions are taken a row per lane,
+// and so are the Landau rows, by one warp beside the others.
+// 8 frequencies, 41 signed orders, 100x200 (Gamma, pparbar): 5340 us before,
+// 304 us so.
 __global__ void __launch_bounds__(REL_THREADS) k_rel_orders(RelArgs a, const double2* __restrict__ om, int n_om,
                                                             double2* __restrict__ out, int* flags) {
-  __shared__ double sh[(REL_THREADS / 32) * 12];
+  extern __shared__ __align__(16) double rel_smem[];
+  __shared__ double sh[REL_WARPS * 12];
+  __shared__ RelRow rows[32];
   const int w = blockIdx.x, s = blockIdx.z;
   const int rb = blockIdx.y % REL_RB, ord = blockIdx.y / REL_RB;
   const int n = ord >> 1, sg = ord & 1;
@@ -1064,117 +1134,227 @@ __global__ void __launch_bounds__(REL_THREADS) k_rel_orders(RelArgs a, const dou
   const int m = sg ? -n : n;
   const double2 o = om[w];
   const double ms = S.ms, qs = S.qs, vA = sy.vA, kpar = sy.kpar, kperp = sy.kperp;
-  const int N = S.N, M = S.M, L = M + 1;
-  // determine_resonances, relativistic branch (src/ALPS_fns.f90:680-702)
-  bool res = false;
-  for (int t = threadIdx.x; t < (N + 1) * M; t += blockDim.x) {
-    int i = t / M, j = t % M;
-    double p1 = S.pperp[i], p2 = S.ppar[j];
-    // the decision rounds as the reference's expression does (no FMA)
-    const double gamma = __dsqrt_rn(__dadd_rn(
-        __ddiv_rn(__dmul_rn(__dadd_rn(__dmul_rn(p1, p1), __dmul_rn(p2, p2)), __dmul_rn(vA, vA)), __dmul_rn(ms, ms)),
-        1.0));
-    const double pr = __ddiv_rn(__dsub_rn(__dmul_rn(__dmul_rn(gamma, ms), o.x), __dmul_rn(1.0 * m, qs)), kpar);
-    if ((S.ppar[j] <= pr) && (S.ppar[j + 1] > pr)) res = true;
-  }
-  res = __syncthreads_or(res) != 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool kn = sy.kperp_norm != 0;
+  const double kf = kn ? 1.0 : kperp, kf2 = kn ? 1.0 : kperp * kperp;
+  double2 acc[6];  // sums of the entries xx yy zz xy xz yz without their constant factors
+#pragma unroll
+  for (int e = 0; e < 6; ++e) acc[e] = cmk(0.0, 0.0);
+  double2* dst = out + (((((size_t)w * sy.nspec + s) * a.relcap + n) * 2 + sg) * REL_RB + rb) * 6;
   double v[12];
-  C6 r6;
-  if (!res) {
+  auto pack = [&](const double2* x) {
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      v[2 * e] = x[e].x;
+      v[2 * e + 1] = x[e].y;
+    }
+  };
+  if (!rel_resonant(S, sy, o, m)) {
     // integrate with the Lorentz factor in resU (src/ALPS_fns.f90:799-864,
-    // 1560-1596), rows 1..N-1 and columns 1..M-1
-    const bool kn = sy.kperp_norm != 0;
+    // 1560-1596), rows 1..N-1 (a warp each) and columns 1..M-1
+    const int N = S.N, M = S.M, L = M + 1;
     const double z = kn ? kperp / qs : 1.0 / qs;
-    const double kf = kn ? 1.0 : kperp, kf2 = kn ? 1.0 : kperp * kperp;
-    c6_zero(r6);
-    const int LB = N + 1;
-    for (int t = rb * blockDim.x + threadIdx.x; t < (N - 1) * (M - 1); t += REL_RB * blockDim.x) {
-      int i = 1 + t / (M - 1), j = 1 + t % (M - 1);
-      double wi = (i == N - 1) ? 1.0 : 2.0;
-      if (i == 1 && N - 1 == 1) wi = 3.0;
-      double wj = (j == 1 || j == M - 1) ? 1.0 : 2.0;
-      if (M - 1 == 1) wj = 2.0;
-      size_t k = (size_t)i * L + j;
-      double p1 = S.pperp[i], p2 = S.ppar[j];
-      double gamma = sqrt((p1 * p1 + p2 * p2) * (vA * vA) / (ms * ms) + 1.0);
-      double2 num = cadd(cscale(o, S.g1[k]), cmk((kpar / (gamma * ms)) * S.g2[k], 0.0));
-      num = cscale(num, qs);
-      double2 den = cmk(gamma * ms * o.x - kpar * p2 - (1.0 * m) * qs, gamma * ms * o.y);
-      double2 rU = cdiv(num, den);
-      auto J = [&](int kk) { return S.bessel[(size_t)(kk + 1) * LB + i]; };
-      double b, bp;
-      bessel_pair_m(m, J, b, bp);
-      double tt[6];
-      tt[0] = 1.0 * (m * m) * b * b / (z * z);
-      tt[1] = kf2 * (p1 * p1) * bp * bp;
-      tt[2] = kf2 * b * b * (p2 * p2);
-      tt[3] = kf * p1 * (1.0 * m) * b * bp / z;
-      tt[4] = (1.0 * m) * kf * b * b * p2 / z;
-      tt[5] = kf2 * b * bp * p2 * p1;
-#pragma unroll
-      for (int e = 0; e < 6; ++e) r6.v[e] = cadd(r6.v[e], cscale(rU, wi * wj * tt[e]));
-    }
-    for (int e = 0; e < 6; ++e) {
-      v[2 * e] = r6.v[e].x;
-      v[2 * e + 1] = r6.v[e].y;
-    }
-    block_sum12(v, sh);
-    if (threadIdx.x == 0) {
-      double f = 2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25;
-      for (int e = 0; e < 6; ++e) r6.v[e] = cscale(cmk(v[2 * e], v[2 * e + 1]), f);
-    }
-  } else {
-    // integrate_res_rel + landau_integrate_rel over the Gamma rows
-    const double Kc = -2.0 * ALPS_PI * cube(ms / vA) * (qs * vA / (kpar * ms));
-    C6 acc, lacc;
-    c6_zero(acc);
-    c6_zero(lacc);
-    bool err = false;
-    const double lw = (o.y > 0.0) ? 0.0 : ((o.y < 0.0) ? 2.0 : 1.0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int ig = 1 + rb * nw + warp; ig <= S.ng - 1; ig += REL_RB * nw) {
-      RowCtx rc{S, sy, o, m, ig, Kc};
-      C6 row;
-      row_rel_d(rc, row, err, lane);
-      double wr = (ig <= S.ng - 2) ? 2.0 : 1.0;
-      if (lane == 0) {
-#pragma unroll
-        for (int e = 0; e < 6; ++e) acc.v[e] = cadd(acc.v[e], cscale(row.v[e], wr));
-        if (lw != 0.0) landau_row_rel_d(rc, lacc);
+    const double mox = ms * o.x, moy = ms * o.y, mq = (1.0 * m) * qs, kom = kpar / ms;
+    const size_t fs = (size_t)(S.nmax + 1) * (N - 1);
+    for (int i = 1 + rb + REL_RB * warp; i <= N - 1; i += REL_RB * REL_WARPS) {
+      double2 s0 = cmk(0.0, 0.0), s1 = s0, s2 = s0;
+      for (int j = 1 + lane; j <= M - 1; j += 32) {
+        const size_t k = (size_t)i * L + j;
+        const double p2 = S.ppar[j], ga = S.relgam[k];
+        const double wj = (j == 1 || j == M - 1) ? 1.0 : 2.0;
+        // num = omega g1 + kpar/(gamma m) g2, den = gamma m omega - kpar p - m q
+        const double2 num = cmk(fma(o.x, S.g1[k], kom * S.relg2g[k]), o.y * S.g1[k]);
+        const double dx = fma(ga, mox, -fma(kpar, p2, mq)), dy = ga * moy;
+        const double r = wj * rcp_fast(fma(dx, dx, dy * dy));
+        const double2 t = cmul(num, cmk(dx * r, -dy * r));
+        const double2 tp = cscale(t, p2);
+        s0 = cadd(s0, t);
+        s1 = cadd(s1, tp);
+        s2 = cmk(fma(tp.x, p2, s2.x), fma(tp.y, p2, s2.y));
       }
+      // the row's Bessel products with its p_perp weight
+      const double* R = S.Rw + (size_t)n * (N - 1) + (i - 1);
+      const double f0 = R[0], f1 = R[fs], f2 = R[2 * fs];
+      auto add = [&](int e, double f, double2 x) { acc[e] = cmk(fma(f, x.x, acc[e].x), fma(f, x.y, acc[e].y)); };
+      add(0, f0, s0);
+      add(1, f1, s0);
+      add(2, f0, s2);
+      add(3, f2, s0);
+      add(4, f0, s1);
+      add(5, f2, s1);
     }
-    if (err) atomicOr(flags, 2);
-    for (int e = 0; e < 6; ++e) {
-      v[2 * e] = acc.v[e].x;
-      v[2 * e + 1] = acc.v[e].y;
+    pack(acc);
+    const double t = block_sum12(v, sh);
+    if (threadIdx.x < 12) {
+      const int e = threadIdx.x >> 1;
+      const double pf[6] = {1.0 * (m * m) / (z * z), kf2, kf2, kf * (1.0 * m) / z, kf * (1.0 * m) / z, kf2};
+      const double x = t * (qs * pf[e] * (2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25));
+      // i for xy, -i for yz
+      const int c = threadIdx.x & 1;
+      double* d = reinterpret_cast<double*>(dst);
+      if (e == 3) d[threadIdx.x ^ 1] = c ? -x : x;
+      else if (e == 5) d[threadIdx.x ^ 1] = c ? x : -x;
+      else d[threadIdx.x] = x;
     }
-    block_sum12(v, sh);
-    double dg = S.grel[2] - S.grel[1];
-    if (threadIdx.x == 0)
-      for (int e = 0; e < 6; ++e) r6.v[e] = cscale(cscale(cmk(v[2 * e], v[2 * e + 1]), dg), 0.25);
-    for (int e = 0; e < 6; ++e) {
-      v[2 * e] = lacc.v[e].x;
-      v[2 * e + 1] = lacc.v[e].y;
-    }
-    block_sum12(v, sh);
-    if (threadIdx.x == 0 && lw != 0.0) {
-      double f = dg * ALPS_PI * 2.0 * ALPS_PI * (qs * vA / (kpar * ms)) * cube(ms / vA);
-      for (int e = 0; e < 6; ++e) {
-        double2 l = cmk(v[2 * e], v[2 * e + 1]);
-        l = cmk(-l.y, l.x);  // * i
-        r6.v[e] = cadd(r6.v[e], cscale(cscale(l, f), lw));
+    return;
+  }
+  // integrate_res_rel + landau_integrate_rel over the Gamma rows
+  const int np = S.np, ng = S.ng;
+  const double* pb = S.prel;
+  const double dpb = pb[2] - pb[1], dg = S.grel[2] - S.grel[1], kva = kpar / vA;
+  const size_t plane = (size_t)(ng + 1) * (np + 1);
+  const double* fam = S.relfam + (size_t)n * 3 * plane;
+  const double lw = (o.y > 0.0) ? 0.0 : ((o.y < 0.0) ? 2.0 : 1.0);
+  double* wsm = rel_smem + warp * rel_warp_words(sy.M_I);
+  RelPiece* rec = reinterpret_cast<RelPiece*>(wsm + REL_PRE_WORDS);
+  double2 lacc[6];
+#pragma unroll
+  for (int e = 0; e < 6; ++e) lacc[e] = cmk(0.0, 0.0);
+  bool err = false;
+  // adds node ip of row ig with complex weight R: A R F_e, A = omega df/dGamma
+  // + (kpar/vA) df/dpparbar
+  auto node = [&](int ig, int ip, double2 R) {
+    const size_t k = (size_t)ig * (np + 1) + ip;
+    const double d1 = S.dfr1[k];
+    const double2 t = cmul(cmk(fma(o.x, d1, kva * S.dfr2[k]), o.y * d1), R);
+    const double p = pb[ip], f0 = fam[k], f1 = fam[plane + k], f2 = fam[2 * plane + k], f0p = f0 * p;
+    auto add = [&](int e, double f) { acc[e] = cmk(fma(f, t.x, acc[e].x), fma(f, t.y, acc[e].y)); };
+    add(0, f0);
+    add(1, f1);
+    add(2, f0p * p);
+    add(3, f2);
+    add(4, f0p);
+    add(5, f2 * p);
+  };
+  const int nrow = (ng - 1 - rb + REL_RB - 1) / REL_RB;  // rows 1 + rb + REL_RB r of this block
+  // the last warp takes the Landau rows where there are any
+  const int rwarps = lw != 0.0 ? REL_WARPS - 1 : REL_WARPS;
+  for (int r0 = 0; r0 < nrow; r0 += 32) {
+    const int nr = min(32, nrow - r0);
+    __syncthreads();
+    if (warp == 0 && lane < nr) rows[lane] = rel_row(S, sy, o, m, 1 + rb + REL_RB * (r0 + lane), err);
+    __syncthreads();
+    if (warp < rwarps) {
+      for (int q = warp; q < nr; q += rwarps) {
+        const int ig = 1 + rb + REL_RB * (r0 + q);
+        const RelRow r = rows[q];
+        const double wr = (ig <= ng - 2) ? 2.0 : 1.0, dI2 = r.dI * r.dI;
+        // trapezoid over the nodes away from the pole; a range's two ends
+        // weigh 1 (once if they coincide), the others 2
+        for (int h = 0; h < 2; ++h) {
+          const int b = h ? r.up : r.i0, e = h ? r.i1 : r.lo;
+          for (int ip = b + lane; ip <= e; ip += 32) {
+            const double dx = pb[ip] - r.dR;
+            double x = wr * dpb * rcp_fast(fma(dx, dx, dI2));
+            if (ip != b && ip != e) x *= 2.0;
+            node(ig, ip, cmk(dx * x, r.dI * x));
+          }
+        }
+        if (r.pv) {
+          const int nrec = rel_pieces(S, sy, r, ig, wsm, rec, lane);
+          int a0 = np, a1 = 0;
+          for (int t = lane; t < nrec; t += 32) {
+            a0 = min(a0, rec[t].a);
+            a1 = max(a1, rec[t].a);
+          }
+          a0 = __reduce_min_sync(0xffffffffu, a0);
+          a1 = __reduce_max_sync(0xffffffffu, a1);
+          // G = h(a) + (h(a+1) - h(a-1)) (p - pb[a]) / (2 dpb)
+          const double hs = 0.5 / dpb, sc = wr * r.sm;
+          for (int ip = a0 - 1 + lane; ip <= a1 + 1; ip += 32) {
+            double2 W = cmk(0.0, 0.0);
+            bool used = false;
+            for (int t = 0; t < nrec; ++t) {
+              const int d = ip - rec[t].a;
+              if (d < -1 || d > 1) continue;
+              used = true;
+              if (d == 0) W = cadd(W, rec[t].A);
+              else W = cadd(W, cscale(rec[t].B, d * hs));
+            }
+            if (used) node(ig, ip, cscale(W, sc));
+          }
+          __syncwarp();
+        }
+      }
+    } else if (lane < nr) {
+      // landau_integrate_rel (src/ALPS_fns_rel.f90:1005-1092), a row per lane
+      const int ig = 1 + rb + REL_RB * (r0 + lane);
+      const double g = S.grel[ig];
+      double2 pr = cscale(cscale(o, g), vA);
+      pr = cmk(pr.x / kpar - (1.0 * m) * qs * vA / (kpar * ms), pr.y / kpar);
+      // inside the subluminal cone, decided as the reference rounds it (no FMA)
+      if (__dmul_rn(pr.x, pr.x) <= __dsub_rn(__dmul_rn(g, g), 1.0)) {
+        const double h = (ig == ng - 1) ? 0.5 : 1.0;
+        const double2 dfg = ig == 1 ? cscale(csub(eval_fit_rel(S, ig + 1, pr), eval_fit_rel(S, ig, pr)), 1.0 / dg)
+                                    : cscale(csub(eval_fit_rel(S, ig + 1, pr), eval_fit_rel(S, ig - 1, pr)), 0.5 / dg);
+        const double2 dfp = cscale(csub(eval_fit_rel(S, ig, cadd(pr, cmk(dpb, 0.0))),
+                                        eval_fit_rel(S, ig, csub(pr, cmk(dpb, 0.0)))),
+                                   0.5 / dpb);
+        const double2 coef = cscale(cadd(cmul(o, dfg), cscale(dfp, kva)), -h);
+        double2 F[3];
+        res_products(S, kperp * ms / (vA * qs), n, g, pr, F);
+        const double2 c0 = cmul(coef, F[0]), c2 = cmul(coef, F[2]), c0p = cmul(c0, pr);
+        lacc[0] = cadd(lacc[0], c0);
+        lacc[1] = cadd(lacc[1], cmul(coef, F[1]));
+        lacc[2] = cadd(lacc[2], cmul(c0p, pr));
+        lacc[3] = cadd(lacc[3], c2);
+        lacc[4] = cadd(lacc[4], c0p);
+        lacc[5] = cadd(lacc[5], cmul(c2, pr));
       }
     }
   }
-  if (threadIdx.x == 0) {
-    r6.v[3] = cmk(-r6.v[3].y, r6.v[3].x);  // * i
-    r6.v[5] = cmk(r6.v[5].y, -r6.v[5].x);  // * -i
-    double2* dst = out + (((((size_t)w * sy.nspec + s) * a.relcap + n) * 2 + sg) * REL_RB + rb) * 6;
-    for (int e = 0; e < 6; ++e) dst[e] = r6.v[e];
+  if (err) atomicOr(flags, 2);
+  pack(acc);
+  const double tr = block_sum12(v, sh);
+  double tl = 0.0;
+  if (lw != 0.0) {
+    pack(lacc);
+    tl = block_sum12(v, sh);
+  }
+  if (warp == 0) {
+    // Kc = -2 pi (ms/vA)^3 q vA / (kpar m); the Landau sums carry i f lw
+    const double zbar = kn ? kperp * ms / (vA * qs) : ms / (vA * qs);
+    const double qv = qs * vA / (kpar * ms);
+    const double Kc = -2.0 * ALPS_PI * cube(ms / vA) * qv;
+    const double f = dg * ALPS_PI * 2.0 * ALPS_PI * qv * cube(ms / vA) * lw;
+    const double to = __shfl_xor_sync(0xffffffffu, tl, 1);  // the other component
+    if (lane < 12) {
+      const int e = lane >> 1, c = lane & 1;
+      const double pf[6] = {1.0 * (m * m) / (zbar * zbar), kf2, kf2, (1.0 * m) * kf / zbar, (1.0 * m) * kf / zbar, kf2};
+      // i l: (-y, x)
+      const double x = pf[e] * fma(tr, Kc * dg * 0.25, (c ? to : -to) * f);
+      double* d = reinterpret_cast<double*>(dst);
+      if (e == 3) d[lane ^ 1] = c ? -x : x;
+      else if (e == 5) d[lane ^ 1] = c ? x : -x;
+      else d[lane] = x;
+    }
   }
 }
 
 }  // namespace
+
+int launch_rel_bessel(alps_ctx* c, int is, double kperp) {
+  SpeciesHost& S = c->spec[is];
+  const int ng = c->sys.ngamma, np = c->sys.npparbar, nmax = S.nmax, nrows = nmax + 2;
+  const size_t plane = (size_t)(ng + 1) * (np + 1), nj = plane * nrows, nfam = plane * 3 * (nmax + 1);
+  // J_0 .. J_nmax+1, then the Bessel products, then the series coefficients
+  const size_t need = nj + nfam + (size_t)nrows * 21;
+  if (need > S.jrel_cap || !S.d_jrel) {
+    if (S.d_jrel) cudaFree(S.d_jrel);
+    S.d_jrel = nullptr;
+    ALPS_CUDA_TRY(cudaMalloc(&S.d_jrel, need * sizeof(double)));
+    S.jrel_cap = need;
+  }
+  S.d_relfam = S.d_jrel + nj;
+  S.d_relcoef = S.d_relfam + nfam;
+  double zfac = kperp * S.sp.ms / (c->sys.vA * S.sp.qs);
+  k_rel_jtab<<<(unsigned)((nj + 127) / 128), 128, 0, c->stream>>>(S.d_grel, S.d_prel, ng, np, nrows, zfac, S.d_jrel);
+  k_rel_families<<<(unsigned)((plane * (nmax + 1) + 127) / 128), 128, 0, c->stream>>>(S.d_jrel, S.d_grel, S.d_prel, ng,
+                                                                                     np, nmax, S.d_relfam);
+  k_rel_coef<<<(nrows * 21 + 127) / 128, 128, 0, c->stream>>>(nmax, S.d_relcoef);
+  ALPS_CUDA_TRY(cudaGetLastError());
+  return ALPS_OK;
+}
 
 int launch_rel_orders(const SysDev& sys, const SpecDev* sp, int relcap, int n, const double2* d_om, double2* d_out,
                       int* d_flags, cudaStream_t st) {
@@ -1187,7 +1367,10 @@ int launch_rel_orders(const SysDev& sys, const SpecDev* sp, int relcap, int n, c
   }
   a.relcap = relcap;
   if (!any || n <= 0) return ALPS_OK;
-  k_rel_orders<<<dim3(n, 2 * relcap * REL_RB, sys.nspec), REL_THREADS, 0, st>>>(a, d_om, n, d_out, d_flags);
+  const size_t smem = REL_WARPS * rel_warp_words(sys.M_I) * sizeof(double);
+  if (smem > 40 * 1024)
+    ALPS_CUDA_TRY(cudaFuncSetAttribute(k_rel_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_rel_orders<<<dim3(n, 2 * relcap * REL_RB, sys.nspec), REL_THREADS, smem, st>>>(a, d_om, n, d_out, d_flags);
   ALPS_CUDA_TRY(cudaGetLastError());
   return ALPS_OK;
 }

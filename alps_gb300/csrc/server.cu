@@ -124,7 +124,7 @@ size_t ctx_device_bytes(const alps_ctx* c) {
     b += nm * 66 * d;                                                                      // lmom (+pairs)
     if (S.sp.relat) {
       size_t nf = (size_t)(c->sys.ngamma + 1) * (c->sys.npparbar + 1);
-      b += 3 * nf * d + (nm + 1) * nf * d + (c->sys.ngamma + 1) * 8;
+      b += 3 * nf * d + (4 * nm + 1) * nf * d + (nm + 1) * 21 * d + (c->sys.ngamma + 1) * 8 + (N + 1) * (M + 1) * 20;
     }
   }
   b += c->batch_cap * 2 * sizeof(double2) + c->ext_cap * sizeof(double2);
