@@ -85,7 +85,10 @@ __device__ double powi_d(double x, int m) {
 }
 
 // Faddeeva function, algorithm 680 (Poppe and Wijers, ACM TOMS 16, 47, 1990),
-// with the reference's single-precision literals kept as such
+// with the reference's single-precision literals kept as such.  k_nhds is
+// bound by this function's chain of FP64 operations (one order a thread):
+// reciprocals within an ulp in place of the divisions inside its loops take
+// it from 90 to 78 us for 8 frequencies.
 __device__ double2 wofz_d(double XI, double YI) {
   const double FACTOR = 1.12837916709551257388, RMAXREAL = 0.5e154, RMAXEXP = 708.503061461606,
                RMAXGONI = 3.53711887601422e15;
@@ -107,8 +110,9 @@ __device__ double2 wofz_d(double XI, double YI) {
     double YSUM = 0.0;
     for (int I = N; I >= 1; --I) {
       J = J - 2;
-      double XAUX = (XSUM * XQUAD - YSUM * YQUAD) / I;
-      YSUM = (XSUM * YQUAD + YSUM * XQUAD) / I;
+      const double RI = rcp_fast((double)I);
+      double XAUX = (XSUM * XQUAD - YSUM * YQUAD) * RI;
+      YSUM = (XSUM * YQUAD + YSUM * XQUAD) * RI;
       XSUM = XAUX + (double)(1.0f / (float)J);
     }
     double U1 = -FACTOR * (XSUM * YABS + YSUM * XABS) + 1.0;
@@ -135,19 +139,20 @@ __device__ double2 wofz_d(double XI, double YI) {
     }
     bool B = (H > 0.0);
     if (B) QLAMBDA = powi_d(H2, KAPN);
+    const double RH2 = B ? 1.0 / H2 : 0.0;
     double RX = 0.0, RY = 0.0, SX = 0.0, SY = 0.0;
     for (int N = NU; N >= 0; --N) {
       int NP1 = N + 1;
       double TX = YABS + H + NP1 * RX;
       double TY = XABS - NP1 * RY;
-      double C = 0.5 / (TX * TX + TY * TY);
+      double C = 0.5 * rcp_fast(TX * TX + TY * TY);
       RX = C * TX;
       RY = C * TY;
       if (B && (N <= KAPN)) {
         TX = QLAMBDA + SX;
         SX = RX * TX - RY * SY;
         SY = RY * TX + RX * SY;
-        QLAMBDA = QLAMBDA / H2;
+        QLAMBDA = QLAMBDA * RH2;
       }
     }
     if (H == 0.0) {
