@@ -107,6 +107,11 @@ struct __align__(16) SpecDev {
   float dpph, dppl;   // dppar (signed) as a float pair
   float idph, idpl;   // 1/dppar as a float pair
   float tpmh, tpml;   // 2 pi M_P as a float pair
+  float pdh, pdl;     // |dppar|, q/|k_par|, -dpperp 2 pi^2 and 1/z as float pairs,
+  float qlh, qll;     // z = k_perp/q (1/q without kperp_norm)
+  float lih, lil;
+  float izh, izl;
+  double iz;
   double kappa;       // k_par / m_s
   double pvc;         // 2 pi dpperp/4 (-q/(2 k_par)): the principal-value scale over smdelta
   double pcen, prad;  // centre and half-width of ppar[1..M-1]
@@ -159,9 +164,11 @@ struct __align__(16) SysDev {
   int nspec;
   int kperp_norm;
   int M_I, M_P;
+  double iM_P;   // 1 / M_P
   double Tlim, vA;
   double kperp, kpar;
   double ikpar;  // 1 / kpar
+  float k1h, k1l, k2h, k2l;  // k_perp and k_perp^2 (1 with kperp_norm) as float pairs
 };
 
 // ---------------------------------------------------------------------------
@@ -351,8 +358,9 @@ void multi_scratch_free(MultiScratch* m);
 struct MultiLaunch {
   const void* jobs;  // device job table
   int nj;
-  long blocks[4];    // grids of classify, pole sums, resonant, finalize
+  long blocks[5];    // grids of classify, pole sums, resonant, finalize, resonant lanes
   size_t smem;       // dynamic shared memory of k_resonant_multi
+  size_t lanes_smem; // and of k_resonant_lanes
   int* flags;        // error words, one per job
 };
 int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2* d_om, double2* d_D, int* d_flags,

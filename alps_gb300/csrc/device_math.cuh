@@ -341,6 +341,65 @@ __device__ inline ResGeom res_geometry(const SpecDev& S, int M_I, double2 om, in
   return g;
 }
 
+// The same geometry without the reference's roundings where they cannot
+// matter: the resonance momentum's place in node units, to some 1e-13, settles
+// every index unless it lies within 1e-5 of a node or of a half-way point
+// (nodes are within 1e-6 of a spacing of their uniform positions).  Returns
+// false where res_geometry has to decide.  About 10 FP64 operations for some
+// 150, on a part with two FP64 lanes per SM and clock.
+__device__ __forceinline__ bool res_geometry_fast(const SpecDev& S, int M_I, double2 om, int nn, double ikpar,
+                                                  ResGeom& g) {
+  const int M = S.M;
+  const double x = fma(-(double)nn, S.qs, S.ms * om.x) * ikpar, v = (x - S.ppar[0]) * S.idppar;
+  g.pr = x;
+  g.pi = S.ms * om.y * ikpar;
+  if (!(v > -(double)M_I && v < (double)(M + M_I + 1))) return false;
+  const double fv = floor(v);
+  const int i = (int)fv;
+  const float fr = (float)(v - fv);
+  if (!(fr > 1e-5f && fr < 0.99999f && fabsf(fr - 0.5f) > 1e-5f)) return false;
+  g.res = i >= 1 - M_I && i < M - 1 + (M_I > 1 ? M_I : 1);
+  g.ipar_res = i;
+  g.lower = g.upper = 0;
+  g.lo1 = 1;
+  g.hi1 = M - 1;
+  g.lo2 = 1;
+  g.hi2 = 0;
+  g.kind = 0;
+  if (!g.res) {
+    g.ipar_res = 0;
+  } else if (i - M_I <= 2) {
+    g.kind = 1;
+    g.lo1 = i + M_I;
+  } else if (i + M_I >= M - 2) {
+    g.kind = 2;
+    g.hi1 = i - M_I;
+  } else {
+    g.kind = 3;
+    g.lower = i - M_I;
+    g.upper = i + M_I + (fr < 0.5f ? 1 : 2);
+    g.hi1 = g.lower;
+    g.lo2 = g.upper;
+    g.hi2 = M - 1;
+  }
+  return true;
+}
+
+// the fast form, and the exact one (out of line: it is seldom needed) where
+// it does not settle the geometry
+static __device__ __noinline__ void res_geometry_exact(const SpecDev& S, int M_I, double2 om, int nn, double kpar, ResGeom& g) {
+  g = res_geometry(S, M_I, om, nn, kpar);
+}
+__device__ __forceinline__ ResGeom res_geometry_of(const SpecDev& S, const SysDev& sys, double2 om, int nn) {
+  ResGeom g;
+  if (!res_geometry_fast(S, sys.M_I, om, nn, sys.ikpar, g)) {
+    ResGeom x;
+    res_geometry_exact(S, sys.M_I, om, nn, sys.kpar, x);
+    g = x;
+  }
+  return g;
+}
+
 // Prefactors of the T-tensor entries (int_T, src/ALPS_fns.f90:1601-1707)
 // after the Bessel and momentum factors have been moved into the reduced
 // vectors.  Entry order: xx, yy, zz, xy, xz, yz.

@@ -19,10 +19,13 @@
 //                       tiles x node slices.  Plain path in FP64; fast path
 //                       (pole_fused) in double-float on the FP32 pipes, all
 //                       orders of a chunk in one set of sums
-//   k_resonant_multi    principal value + Landau per resonant (omega,
-//                       species, n): occupied slots gathered into batches
-//                       of 32; scalar work one item per lane, vector work
-//                       one item per warp (fast path: pv_fast, double-float)
+//   k_resonant_lanes    (mixed batches of 2560 and more) principal value +
+//                       Landau per resonant (omega, species, n), an item per
+//                       lane; marks the few items it leaves
+//   k_resonant_multi    the same for all others: occupied slots gathered into
+//                       batches of 32; scalar work one item per lane, the
+//                       principal value one item per warp as weights of the
+//                       window's nodes (FP64 or double-float)
 //   k_finalize_multi    chi, epsilon, wave tensor and det, one thread (or
 //                       warp) per omega; sums in a fixed order, so results
 //                       do not depend on timing or on the other jobs.
@@ -64,6 +67,8 @@ struct DispShape {
   int nch[ALPS_MAX_SPECIES];  // order chunks of each species (0: no pole sums)
   int ipw;       // resonant-item slots per warp of k_resonant (1..256)
   int fin_warp;  // k_finalize takes a warp per omega (else a thread)
+  int lanes;     // slots per warp of k_resonant_lanes, which takes the items, k_resonant_multi
+                 // what it leaves (0: k_resonant_multi takes all)
 };
 
 namespace {
@@ -312,9 +317,9 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
         const float dx = x32 - S.pcen32;
         ddf = fmaf(dx, dx, dyd.h * dyd.h);
       } else {
-        const ResGeom g = res_geometry(S, sys.M_I, o, nn, kpar);
-        const double2 dfar = cmk(g.pr - S.pcen, g.pi);
-        ddf = (float)(dfar.x * dfar.x + dfar.y * dfar.y);
+        const ResGeom g = res_geometry_of(S, sys, o, nn);
+        const float dx = (float)(g.pr - S.pcen);
+        ddf = fmaf(dx, dx, dyd.h * dyd.h);
         res = g.res;
         cur.lo1 = g.lo1;
         cur.hi1 = g.hi1;
@@ -635,7 +640,7 @@ __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, 
       const float x32 = (float)(S.ms * o.x - (double)nn * S.qs) * ikp32;
       const float mg = 9.5367431640625e-7f * fabsf(x32);
       if (!(x32 < S.qlo - mg || x32 > S.qhi + mg)) {
-        const ResGeom g = res_geometry(S, sys.M_I, o, nn, kpar);
+        const ResGeom g = res_geometry_of(S, sys, o, nn);
         lo1 = g.lo1;
         hi1 = g.hi1;
         lo2 = g.lo2;
@@ -794,126 +799,813 @@ __device__ double2 eval_fit_d(const SpecDev& S, double vA, int iperp, double2 p)
   return ff;
 }
 
-// h_e(j) = omega V_{e,1}(j) + kappa V_{e,2}(j)
-__device__ inline double2 h_node(const double* Vn, int j, int e, double2 o, double kappa) {
-  const double* v = Vn + (size_t)(j - 1) * 12 + 2 * e;
-  return cmk(o.x * v[0] + kappa * v[1], o.y * v[0]);
-}
-
 // ---------------------------------------------------------------------------
 // Resonant items: the principal-value part of integrate_res
 // (src/ALPS_fns.f90:1000-1236) and landau_integrate (:1327-1452) for one
-// (omega, species, n).  One warp per item.
+// (omega, species, n).
 //
-// Principal value: summed over iperp, funct_g (:1243-1321) is the linear
+// Principal value.  Summed over iperp, funct_g (:1243-1321) is the linear
 // interpolation H_e(p) = h_e(jc) + s_e(jc) (p - ppar_jc) on the node values
 // h_e(j) = omega V_{e,1}(j) + kappa V_{e,2}(j) with the centred slope
-// s_e(j) = (h_e(j+1) - h_e(j-1)) / (2 dppar); both are staged per window node
-// in shared memory.  Landau: for Maxwellian fit terms the three continuation
-// values a row needs share one Gaussian, exp(-p2 (d +- D)^2) =
-// exp(-p2 d^2) exp(-+2 p2 D d) exp(-p2 D^2), so a row costs two complex
-// exponentials; the omega-independent factors come from k_fit_aux.
+// s_e(j) = (h_e(j+1) - h_e(j-1)) / (2 dppar).  The sum over samples
+//   T_e = sum_k w_k [ H_e(p_k) / (dx_k - i y) - H_e(2 p_res - p_k) / (dx_k + i y) ],
+// dx_k = p_k - p_res, y = Im p_res, therefore needs of each piece jc only the
+// sums over its samples of w r dx, w r and w r dx^2, r = 1/(dx^2 + y^2): they
+// give the weights' sum A and first moment B, and with them T_e is a weighted
+// sum over a few nodes, W_j = A_j + (B_{j-1} - B_{j+1}) / (2 dppar),
+//   T_e = sum_j (omega V_{e,1}(j) + kappa V_{e,2}(j)) W_j.
+// Both sides of the window share the sums: they are running (prefix) sums
+// over k, cut where a side moves to its next piece.
+//
+// The cuts are the reference's decisions.  An FP32 estimate in units of a
+// spacing, measured from the node next to p_res, settles each to 5e-6 of a
+// spacing; nearer, the search over the reference's own sample points does.
+// Exactly half-way its rounded distances may exceed half a spacing to both
+// nodes: funct_g then falls back to the grid's second node, and such an item
+// is summed sample by sample (pv_direct).
+//
+// Landau: for Maxwellian fit terms the three continuation values a row needs
+// share one Gaussian, exp(-p2 (d +- D)^2) = exp(-p2 d^2) exp(-+2 p2 D d)
+// exp(-p2 D^2), so a row costs two complex exponentials; the omega-independent
+// factors come from k_fit_aux.
+//
+// Two kernels:
+//   k_resonant_lanes  an item per lane: lattices on the mixed path.  No
+//     exchange between lanes; items that need the FP64 sums or the Landau
+//     rows are left to the other kernel.
+//   k_resonant_multi  an item per warp (the per-item set-up still one per
+//     lane): everything else.
 // ---------------------------------------------------------------------------
 #define RES_WARPS 4
-#define RES_WIN 32  // largest node window staged in shared memory
-// principal-value piece records per warp, in double2: (group, lane, slot)
-// sums A, B; run sums A, B; then the int tables (group, lane, slot) piece
-// and run start lane, slot, group, piece
-#define PV_GROUPS 3
-#define PV_RECV (PV_GROUPS * 32 * 2 * 2)
-#define PV_RUNV (32 * 2)
-#define PV_INTS (PV_GROUPS * 64 + 4 * 32)
-#define PV_SMEM (PV_RECV + PV_RUNV + (PV_INTS + 3) / 4)
-// record planes: sum ab (0 A, 1 B) of slot sl of (group gi, lane L); lanes
-// are adjacent within a plane, so a warp's record stores and loads touch
-// consecutive 16-byte words (no bank conflicts)
-__host__ __device__ inline int rec_at(int gi, int L, int sl, int ab) { return ((sl * 2 + ab) * PV_GROUPS + gi) * 32 + L; }
-__host__ __device__ inline int recj_at(int gi, int L, int sl) { return (sl * PV_GROUPS + gi) * 32 + L; }
+#define PV_CHUNK 128   // samples a warp sums between two looks at the cuts
+#define PV_TOL 5e-6f   // a cut nearer than this (in spacings) to a sample is decided by the search
 
-// node window of the principal-value sum: nodes lower-2 .. upper+2
-__host__ __device__ inline int res_win(int M_I) { return (2 * M_I + 8 < RES_WIN) ? 2 * M_I + 8 : RES_WIN; }
+// scalar arithmetic of the principal-value sums: FP64 or double-float
+__device__ __forceinline__ double sc_add(double a, double b) { return a + b; }
+__device__ __forceinline__ dflt sc_add(dflt a, dflt b) { return df_add(a, b); }
+__device__ __forceinline__ double sc_neg(double a) { return -a; }
+__device__ __forceinline__ dflt sc_neg(dflt a) { return df_neg(a); }
+__device__ __forceinline__ double sc_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ dflt sc_mul(dflt a, dflt b) { return df_mul(a, b); }
+__device__ __forceinline__ double sc_rcp(double a) { return rcp_fast(a); }
+__device__ __forceinline__ dflt sc_rcp(dflt a) { return df_rcp_approx(a); }
+__device__ __forceinline__ double sc_scale(double a, float s) { return a * (double)s; }  // s a power of 2
+__device__ __forceinline__ dflt sc_scale(dflt a, float s) { return df_scale(a, s); }
+__device__ __forceinline__ void sc_acc(double& a, double c) { a += c; }
+__device__ __forceinline__ void sc_acc(dflt& a, dflt c) { df_acc(a, c); }
+__device__ __forceinline__ void sc_mac(double& a, double v, double r) { a = fma(v, r, a); }
+__device__ __forceinline__ void sc_mac(dflt& a, dflt v, dflt r) { df_mac(a, v.h, v.l, r); }
+__device__ __forceinline__ double sc_val(double a) { return a; }
+__device__ __forceinline__ double sc_val(dflt a) { return df_val(a); }
+__device__ __forceinline__ double sc_shfl(double a, int src) { return __shfl_sync(FULL_WARP, a, src); }
+__device__ __forceinline__ dflt sc_shfl(dflt a, int src) {
+  return {__shfl_sync(FULL_WARP, a.h, src), __shfl_sync(FULL_WARP, a.l, src)};
+}
+__device__ __forceinline__ double sc_up(double a, int o) { return __shfl_up_sync(FULL_WARP, a, o); }
+__device__ __forceinline__ dflt sc_up(dflt a, int o) {
+  return {__shfl_up_sync(FULL_WARP, a.h, o), __shfl_up_sync(FULL_WARP, a.l, o)};
+}
+__device__ __forceinline__ bool sc_is_df(double) { return false; }
+__device__ __forceinline__ bool sc_is_df(dflt) { return true; }
+template <typename T>
+__device__ __forceinline__ T sc_of(double x);
+template <>
+__device__ __forceinline__ double sc_of<double>(double x) { return x; }
+template <>
+__device__ __forceinline__ dflt sc_of<dflt>(double x) { return df_of(x); }
 
-// what the warp phase of k_resonant needs of one item
+// a species' constants and nodes in either arithmetic (the float pairs are
+// formed once on the host: a conversion is FP64 work for the whole warp)
+template <typename T>
+struct ScSpec;
+template <>
+struct ScSpec<double> {
+  static __device__ __forceinline__ double kap(const SpecDev& S) { return S.kappa; }
+  static __device__ __forceinline__ double hid(const SpecDev& S) { return S.hidpa; }
+  static __device__ __forceinline__ double dpp(const SpecDev& S) { return S.dppar; }
+  static __device__ __forceinline__ double idp(const SpecDev& S) { return S.idppar; }
+  static __device__ __forceinline__ double node(const SpecDev& S, int j) { return S.ppar[j]; }
+  static __device__ __forceinline__ double v(const SpecDev& S, size_t at) { return S.V[at]; }
+  static __device__ __forceinline__ double half_turn(const SysDev& y, const SpecDev&, double cap) {
+    return 2.0 * ALPS_PI * (double)y.M_P * rcp_fast(cap);
+  }
+};
+template <>
+struct ScSpec<dflt> {
+  static __device__ __forceinline__ dflt kap(const SpecDev& S) { return {S.kaph, S.kapl}; }
+  static __device__ __forceinline__ dflt hid(const SpecDev& S) { return {S.hidh, S.hidl}; }
+  static __device__ __forceinline__ dflt dpp(const SpecDev& S) { return {S.dpph, S.dppl}; }
+  static __device__ __forceinline__ dflt idp(const SpecDev& S) { return {S.idph, S.idpl}; }
+  static __device__ __forceinline__ dflt node(const SpecDev& S, int j) { return {S.pph[j], S.ppl[j]}; }
+  static __device__ __forceinline__ dflt v(const SpecDev& S, size_t at) { return {S.Vh[at], S.Vl[at]}; }
+  static __device__ __forceinline__ dflt half_turn(const SysDev&, const SpecDev& S, dflt cap) {
+    return df_mul({S.tpmh, S.tpml}, df_rcp_approx(cap));
+  }
+};
+
+// sums over samples of w r dx, w r, w r dx^2
+template <typename T>
+struct PvSums {
+  T s1, s2, s3;
+};
+template <typename T>
+__device__ __forceinline__ PvSums<T> pv_diff(PvSums<T> a, PvSums<T> b) {
+  return {sc_add(a.s1, sc_neg(b.s1)), sc_add(a.s2, sc_neg(b.s2)), sc_add(a.s3, sc_neg(b.s3))};
+}
+
+// the principal-value constants of an item (integrate_res,
+// src/ALPS_fns.f90:1000-1040): capDelta, smdelta, the tiny rest's count and
+// spacing, and the samples' places in spacings from node j0, next to p_res
+// (jt0: next to the first sample of the tiny rest)
+struct PvItem {
+  double pr, pim;
+  double cap, sm, cor;   // capDelta, smdelta, the tiny rest's correction
+  dflt capd, smd, cord, pimd, oxd, oyd;  // and the double-float path's pairs
+  float f0, du, ft0, dut;
+  int j0, jt0, ntiny;
+  int lower, upper, nn;
+  int direct;            // some sample lies half-way between nodes and funct_g's search may find neither
+};
+
+// the reference's own sample points, for the search near half-way points
+struct PvExact {
+  double pr, cap, sm, cor;
+  int M_P;
+  __device__ double sym(int k) const {
+    return k == 0 ? pr : (k == M_P ? __dadd_rn(pr, cap) : __dadd_rn(pr, __dmul_rn(sm, (double)k)));
+  }
+  __device__ double tiny(int k) const {
+    return k == 0 ? __dadd_rn(pr, cap) : __dadd_rn(__dadd_rn(pr, cap), __dmul_rn(__dmul_rn(cor, sm), (double)k));
+  }
+};
+__device__ __noinline__ PvExact pv_exact(const SpecDev& S, const SysDev& sys, const PvItem& it, double omr) {
+  PvExact x;
+  x.M_P = sys.M_P;
+  x.pr = pres_real(S, omr, it.nn, sys.kpar);
+  x.cap = x.pr - S.ppar[it.lower];
+  x.sm = x.cap / (1.0 * sys.M_P);
+  x.cor = it.ntiny > 0 ? ((S.ppar[it.upper] - x.pr - x.cap) / (1.0 * it.ntiny)) / x.sm : 0.0;
+  return x;
+}
+// funct_g's search: the last node in 1..M-1 within half a spacing of p, 0 if none
+__device__ __noinline__ int pv_search(const SpecDev& S, double p) {
+  const int M = S.M;
+  const double jd = floor((p - S.ppar[0]) * fabs(S.idppar) + 0.5), half = 0.5 * S.dppar_abs;
+  if (jd > -10.0 && jd < (double)M + 10.0) {
+    const int j = (int)jd;
+    for (int jj = min(j + 2, M - 1); jj >= max(j - 2, 1); --jj)
+      if (fabs(S.ppar[jj] - p) <= half) return jj;
+  }
+  return 0;
+}
+
+__device__ __forceinline__ void pv_setup(const SpecDev& S, const SysDev& sys, const ResGeom& g, int nn, double omr,
+                                         PvItem& it) {
+  it.pr = g.pr;
+  it.pim = g.pi;
+  it.lower = g.lower;
+  it.upper = g.upper;
+  it.nn = nn;
+  const double cap = g.pr - S.ppar[g.lower];
+  it.cap = cap;
+  it.sm = cap * sys.iM_P;
+  // ntiny = floor(rest / smdelta); the reference's own quotient near integers
+  const double rest = S.ppar[g.upper] - g.pr - cap, q = rest * rcp_fast(it.sm);
+  int nt = (int)q;
+  if (!(fabs(q - rint(q)) > 1e-6)) {
+    it.ntiny = 0;
+    const PvExact x = pv_exact(S, sys, it, omr);
+    nt = (int)((S.ppar[g.upper] - x.pr - x.cap) / x.sm);
+  }
+  it.ntiny = nt;
+  it.cor = nt > 0 ? q * rcp_fast((double)nt) : 0.0;
+  const double u = 1.0 + (g.pr - S.ppar[1]) * S.idppar;
+  it.j0 = (int)rint(u);
+  it.f0 = (float)(u - (double)it.j0);
+  it.du = (float)(it.sm * S.idppar);
+  const double ut = u + cap * S.idppar;
+  it.jt0 = (int)rint(ut);
+  it.ft0 = (float)(ut - (double)it.jt0);
+  it.dut = it.du * (float)it.cor;
+  it.direct = 0;
+  if (fabsf(it.f0) > 0.5f - PV_TOL || (nt > 0 && fabsf(it.ft0) > 0.5f - PV_TOL)) {
+    // the sample at p_res (or the tiny rest's first) half-way between nodes
+    const PvExact x = pv_exact(S, sys, it, omr);
+    const int j = pv_search(S, x.sym(0)), jt = pv_search(S, x.tiny(0));
+    if (j == 0 || (nt > 0 && jt == 0) || fabs(it.pim) <= sys.Tlim) it.direct = 1;
+    if (j > 0 && j != it.j0) {
+      it.f0 += (float)(it.j0 - j);
+      it.j0 = j;
+    }
+    if (jt > 0 && jt != it.jt0) {
+      it.ft0 += (float)(it.jt0 - jt);
+      it.jt0 = jt;
+    }
+  }
+}
+
+// First sample k beyond piece i of a side (0: p_k upwards from p_res, 1: the
+// mirrored points downwards, 2: the tiny rest upwards): i + 1/2 spacings from
+// the side's first node.  A point half-way belongs to the upper node; lost: to
+// none.
+__device__ __forceinline__ int pv_cut(const SpecDev& S, const SysDev& sys, const PvItem& it, double omr, int side,
+                                      int i, bool& lost) {
+  const int K = side == 2 ? it.ntiny : sys.M_P;
+  const float f = side == 2 ? it.ft0 : it.f0, du = side == 2 ? it.dut : it.du;
+  const float dist = (float)i + (side == 1 ? 0.5f + f : 0.5f - f);
+  const float t = dist / du;
+  if (!(t < (float)K + 1.0f)) return K + 1;
+  const float tr = rintf(t);
+  int k = (side == 1) ? (int)floorf(t) + 1 : (int)ceilf(t);
+  if (fabsf(t - tr) * du < PV_TOL) {
+    k = (int)tr;
+    const PvExact x = pv_exact(S, sys, it, omr);
+    const int j = pv_search(S, side == 0 ? x.sym(k) : (side == 1 ? 2.0 * x.pr - x.sym(k) : x.tiny(k)));
+    if (j == 0 && k <= K) lost = true;
+    const bool beyond = side == 0 ? j >= it.j0 + i + 1 : (side == 1 ? j <= it.j0 - i - 1 : j >= it.jt0 + i + 1);
+    if (!beyond) ++k;
+  }
+  return max(0, min(K + 1, k));
+}
+
+// what the sums need of an item, in their arithmetic
+template <typename T>
+struct PvScal {
+  T sm, cap, csd, cor, y, y2;
+};
+template <typename T>
+__device__ __forceinline__ PvScal<T> pv_scal(const PvItem& it);
+template <>
+__device__ __forceinline__ PvScal<double> pv_scal<double>(const PvItem& it) {
+  return {it.sm, it.cap, it.cor * it.sm, it.cor, it.pim, it.pim * it.pim};
+}
+template <>
+__device__ __forceinline__ PvScal<dflt> pv_scal<dflt>(const PvItem& it) {
+  return {it.smd, it.capd, df_mul(it.cord, it.smd), it.cord, it.pimd, df_mul(it.pimd, it.pimd)};
+}
+__device__ __forceinline__ double sc_times(double a, int k) { return a * (double)k; }
+__device__ __forceinline__ dflt sc_times(dflt a, int k) { return df_mul(a, {(float)k, 0.0f}); }
+
+// adds sample k of the symmetric window (tiny: of the tiny rest, without its
+// correction); sym: the first sample counts
+template <typename T>
+__device__ __forceinline__ void pv_sample(PvSums<T>& s, const PvScal<T>& c, int k, int K, bool tiny, bool sym) {
+  T dx = sc_times(tiny ? c.csd : c.sm, k);
+  if (tiny) dx = sc_add(c.cap, dx);
+  else if (k == K) dx = c.cap;
+  T r = sc_scale(sc_rcp(sc_add(sc_mul(dx, dx), c.y2)), (k == 0 || k == K) ? 1.0f : 2.0f);
+  if (k == 0 && !sym) r = sc_of<T>(0.0);
+  const T t = sc_mul(dx, r);
+  sc_acc(s.s1, t);
+  sc_acc(s.s2, r);
+  sc_mac(s.s3, dx, t);
+}
+
+// a piece's A and first moment about p_res from its sums (side as pv_cut)
+template <typename T>
+__device__ __forceinline__ void pv_moment(const PvSums<T>& s, const PvScal<T>& c, int side, T& Ax, T& Ay, T& Cx, T& Cy) {
+  Ax = side == 1 ? sc_neg(s.s1) : s.s1;
+  Ay = sc_mul(c.y, s.s2);
+  Cx = s.s3;
+  Cy = sc_mul(c.y, s.s1);
+  if (side == 1) Cy = sc_neg(Cy);
+  if (side == 2) {
+    Ax = sc_mul(Ax, c.cor);
+    Ay = sc_mul(Ay, c.cor);
+    Cx = sc_mul(Cx, c.cor);
+    Cy = sc_mul(Cy, c.cor);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// One item's principal-value sum by a warp
+// ---------------------------------------------------------------------------
+template <typename T>
+struct __align__(16) PvPiece {
+  T Ax, Ay, Bx, By;
+  int a, pad[3];
+};
+// pieces at most: both sides of the window, the tiny rest
+__host__ __device__ inline int pv_max_pieces(int M_I) { return 2 * (M_I + 4) + 8; }
+// double2 words per warp: prefix sums of a chunk, pieces, node weights
+__host__ __device__ inline size_t pv_warp_words(int M_I) {
+  const size_t np = (size_t)pv_max_pieces(M_I);
+  return (PV_CHUNK * 24 + 15) / 16 + np * (sizeof(PvPiece<double>) / 16) + (2 * (M_I + 4) + 8);
+}
+
+// prefix sums at the lane's cut kc (see pv_sample); pre: PV_CHUNK PvSums
+template <typename T>
+__device__ __forceinline__ PvSums<T> pv_cut_sums(const PvScal<T>& c, int K, bool tiny, bool sym, int kc,
+                                                 PvSums<T>* pre, int lane) {
+  const T z = sc_of<T>(0.0);
+  PvSums<T> out = {z, z, z}, carry = {z, z, z};
+  for (int k0 = 0; k0 <= K; k0 += PV_CHUNK) {
+    const int n = min(PV_CHUNK, K + 1 - k0), per = (n + 31) / 32;
+    const int b = min(n, lane * per), e = min(n, b + per);
+    PvSums<T> loc = {z, z, z};
+    for (int j = b; j < e; ++j) {
+      pre[j] = loc;
+      pv_sample(loc, c, k0 + j, K, tiny, sym);
+    }
+    PvSums<T> inc = loc;
+    for (int o = 1; o < 32; o <<= 1) {
+      const T a = sc_up(inc.s1, o), d = sc_up(inc.s2, o), f = sc_up(inc.s3, o);
+      if (lane >= o) {
+        inc.s1 = sc_add(inc.s1, a);
+        inc.s2 = sc_add(inc.s2, d);
+        inc.s3 = sc_add(inc.s3, f);
+      }
+    }
+    PvSums<T> bef;
+    bef.s1 = sc_up(inc.s1, 1);
+    bef.s2 = sc_up(inc.s2, 1);
+    bef.s3 = sc_up(inc.s3, 1);
+    if (lane == 0) bef = {z, z, z};
+    bef = {sc_add(carry.s1, bef.s1), sc_add(carry.s2, bef.s2), sc_add(carry.s3, bef.s3)};
+    for (int j = b; j < e; ++j)
+      pre[j] = {sc_add(pre[j].s1, bef.s1), sc_add(pre[j].s2, bef.s2), sc_add(pre[j].s3, bef.s3)};
+    carry = {sc_add(carry.s1, sc_shfl(inc.s1, 31)), sc_add(carry.s2, sc_shfl(inc.s2, 31)),
+             sc_add(carry.s3, sc_shfl(inc.s3, 31))};
+    __syncwarp();
+    if (kc >= k0 && kc < k0 + n) out = pre[kc - k0];
+    __syncwarp();
+  }
+  if (kc > K) out = carry;
+  return out;
+}
+
+// The weights W of the nodes a0 .. a0 + cnt - 1 in wts (FP64 or double-float
+// pairs of 16 bytes); false if the item has to be summed directly
+template <typename T>
+__device__ bool pv_warp_weights(const SpecDev& S, const SysDev& sys, const PvItem& it, double omr, PvSums<T>* pre,
+                                PvPiece<T>* rec, T* wts, int lane, int& a0, int& cnt) {
+  const int M = S.M, M_P = sys.M_P, cap_rec = pv_max_pieces(sys.M_I);
+  const PvScal<T> c = pv_scal<T>(it);
+  typedef ScSpec<T> SS;
+  const T z = sc_of<T>(0.0), plo = SS::node(S, it.lower);
+  const bool sym = fabs(it.pim) > sys.Tlim;
+  auto clampj = [&](int j) { return (j >= M - 1) ? M - 2 : ((j <= 1) ? 2 : j); };
+  auto put = [&](int slot, int j, T Ax, T Ay, T Cx, T Cy) {
+    PvPiece<T> p;
+    p.a = clampj(j);
+    // p_res - p_a = capDelta + (p_lower - p_a)
+    const T del = sc_add(c.cap, sc_add(plo, sc_neg(SS::node(S, p.a))));
+    p.Ax = Ax;
+    p.Ay = Ay;
+    p.Bx = sc_add(Cx, sc_mul(del, Ax));
+    p.By = sc_add(Cy, sc_mul(del, Ay));
+    rec[slot] = p;
+  };
+  int nrec = 0;
+  bool lost = it.direct;
+  if (sym) {
+    // pieces of both sides, side by side over the lanes: even slots up, odd down
+    const int most = 2 * (sys.M_I + 4);
+    for (int t0 = 0; t0 < most; t0 += 32) {
+      const int t = t0 + lane, side = t & 1, i = t >> 1;
+      const int kb = i == 0 ? 0 : pv_cut(S, sys, it, omr, side, i - 1, lost);
+      const int ke = pv_cut(S, sys, it, omr, side, i, lost);
+      const bool has = t < most && kb <= M_P;
+      const PvSums<T> se = pv_cut_sums(c, M_P, false, true, has ? ke : 0, pre, lane);
+      PvSums<T> sb;
+      sb.s1 = sc_up(se.s1, 2);
+      sb.s2 = sc_up(se.s2, 2);
+      sb.s3 = sc_up(se.s3, 2);
+      if (t0 > 0 && __any_sync(FULL_WARP, has && lane < 2)) {
+        const PvSums<T> s0 = pv_cut_sums(c, M_P, false, true, kb, pre, lane);
+        if (lane < 2) sb = s0;
+      }
+      if (i == 0) sb = {z, z, z};
+      const unsigned m = __ballot_sync(FULL_WARP, has);
+      if (has) {
+        T Ax, Ay, Cx, Cy;
+        pv_moment(pv_diff(se, sb), c, side, Ax, Ay, Cx, Cy);
+        const int slot = nrec + __popc(m & ((1u << lane) - 1u));
+        if (slot < cap_rec) put(slot, side ? it.j0 - i : it.j0 + i, Ax, Ay, Cx, Cy);
+      }
+      nrec += __popc(m);
+      if (!m) break;
+    }
+  } else {
+    // Tlim branch: g' sum_k w_k dx^2/(dx^2 + y^2) + sign(y) i pi G(p_res)/smdelta
+    const PvSums<T> s = pv_cut_sums(c, M_P, false, false, M_P + 1, pre, lane);
+    if (lane < 3) {
+      // H at p_res + dppar, p_res - dppar and p_res
+      const int d = lane == 0 ? 1 : (lane == 1 ? -1 : 0), j = it.j0 + d;
+      T Ax = z, Ay = z;
+      if (d != 0) {
+        // g' 2 sum = (H1 - H2) sum / dppar
+        Ax = sc_mul(s.s3, SS::idp(S));
+        if (d < 0) Ax = sc_neg(Ax);
+      } else {
+        Ay = sc_scale(SS::half_turn(sys, S, c.cap), it.pim > 0.0 ? 1.0f : (it.pim < 0.0 ? -1.0f : 0.0f));
+      }
+      const T off = sc_scale(SS::dpp(S), (float)d);
+      put(lane, j, Ax, Ay, sc_mul(off, Ax), sc_mul(off, Ay));
+    }
+    nrec = 3;
+  }
+  if (it.ntiny > 0) {
+    const int i = lane;
+    const int ke = pv_cut(S, sys, it, omr, 2, i, lost), kb = i == 0 ? 0 : pv_cut(S, sys, it, omr, 2, i - 1, lost);
+    const bool has = i < 6 && kb <= it.ntiny;
+    const PvSums<T> se = pv_cut_sums(c, it.ntiny, true, true, has ? ke : 0, pre, lane);
+    PvSums<T> sb;
+    sb.s1 = sc_up(se.s1, 1);
+    sb.s2 = sc_up(se.s2, 1);
+    sb.s3 = sc_up(se.s3, 1);
+    if (i == 0) sb = {z, z, z};
+    const unsigned m = __ballot_sync(FULL_WARP, has);
+    if (has && nrec + i < cap_rec) {
+      T Ax, Ay, Cx, Cy;
+      pv_moment(pv_diff(se, sb), c, 2, Ax, Ay, Cx, Cy);
+      put(nrec + i, it.jt0 + i, Ax, Ay, Cx, Cy);
+    }
+    nrec += __popc(m);
+  }
+  if (__any_sync(FULL_WARP, lost)) return false;
+  nrec = min(nrec, cap_rec);
+  __syncwarp();
+  int lo = M, hi = 0;
+  for (int t = lane; t < nrec; t += 32) {
+    lo = min(lo, rec[t].a);
+    hi = max(hi, rec[t].a);
+  }
+  a0 = __reduce_min_sync(FULL_WARP, lo) - 1;
+  cnt = min(__reduce_max_sync(FULL_WARP, hi) + 1 - a0 + 1, 2 * (sys.M_I + 4) + 8);
+  const T hid = SS::hid(S);
+  for (int t = lane; t < cnt; t += 32) {
+    T Wx = z, Wy = z, Dx = z, Dy = z;
+    for (int q = 0; q < nrec; ++q) {
+      const int d = a0 + t - rec[q].a;
+      if (d == 0) {
+        Wx = sc_add(Wx, rec[q].Ax);
+        Wy = sc_add(Wy, rec[q].Ay);
+      } else if (d == 1 || d == -1) {
+        Dx = sc_add(Dx, d > 0 ? rec[q].Bx : sc_neg(rec[q].Bx));
+        Dy = sc_add(Dy, d > 0 ? rec[q].By : sc_neg(rec[q].By));
+      }
+    }
+    wts[2 * t] = sc_add(Wx, sc_mul(hid, Dx));
+    wts[2 * t + 1] = sc_add(Wy, sc_mul(hid, Dy));
+  }
+  __syncwarp();
+  return true;
+}
+
+// adds component c of T_e times the window's scale to the output row; xy and
+// yz have imaginary prefactors: (x, y) -> pe (-y, x)
+__device__ __forceinline__ void pv_add_out(double2* out, const double* pref, int n, int e, int c, double v) {
+  if (n == 0 && (e == 0 || e == 3 || e == 4)) return;
+  double* d = reinterpret_cast<double*>(out + e);
+  v *= pref[e];
+  if (e == 3 || e == 5) d[c ^ 1] += c ? -v : v;
+  else d[c] += v;
+}
+
+// The same sum sample by sample over the reference's own points, in FP64: for
+// items with a sample that funct_g's search finds no node for.
+__device__ __noinline__ void pv_direct(const SpecDev& S, const SysDev& sys, const PvItem& it, double2 o,
+                                       const double* pref, double2* out) {
+  const int lane = threadIdx.x & 31, M = S.M, M_P = sys.M_P, n = it.nn < 0 ? -it.nn : it.nn;
+  const PvExact x = pv_exact(S, sys, it, o.x);
+  const double y = it.pim, y2 = y * y;
+  dbl_val T[12];
+  for (int q = 0; q < 12; ++q) T[q].v = 0.0;
+  // T += f H(p)
+  auto add = [&](double p, double2 f) {
+    int j = pv_search(S, p);
+    j = (j >= M - 1) ? M - 2 : ((j <= 1) ? 2 : j);
+    const double* v = S.V + ((size_t)n * (M - 1) + (j - 1)) * 12;
+    const double dx = (p - S.ppar[j]) * S.hidpa;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      const double v1 = fma(v[12 + 2 * e] - v[2 * e - 12], dx, v[2 * e]);
+      const double v2 = fma(v[13 + 2 * e] - v[2 * e - 11], dx, v[2 * e + 1]);
+      const double2 t = cmul(cmk(fma(o.x, v1, S.kappa * v2), o.y * v1), f);
+      T[2 * e].v += t.x;
+      T[2 * e + 1].v += t.y;
+    }
+  };
+  if (fabs(y) > sys.Tlim) {
+    for (int k = lane; k <= M_P; k += 32) {
+      const double p = x.sym(k), dx = p - x.pr;
+      const double r = ((k == 0 || k == M_P) ? 1.0 : 2.0) * rcp_fast(fma(dx, dx, y2));
+      add(p, cmk(dx * r, y * r));
+      add(2.0 * x.pr - p, cmk(-dx * r, y * r));
+    }
+  } else {
+    double fr = 0.0;
+    for (int k = 1 + lane; k <= M_P; k += 32) {
+      const double d = x.sym(k) - x.pr;
+      fr += (k == M_P ? 1.0 : 2.0) * ((d * d) / (d * d + y2));
+    }
+    for (int off = 16; off > 0; off >>= 1) fr += __shfl_xor_sync(FULL_WARP, fr, off);
+    const double c = fr * S.idppar;
+    if (lane == 0) add(x.pr + S.dppar, cmk(c, 0.0));
+    if (lane == 1) add(x.pr - S.dppar, cmk(-c, 0.0));
+    if (lane == 2 && y != 0.0) add(x.pr, cmk(0.0, (y > 0.0 ? 2.0 : -2.0) * ALPS_PI / x.sm));
+  }
+  for (int k = lane; k <= it.ntiny && it.ntiny > 0; k += 32) {
+    const double p = x.tiny(k), dx = p - x.pr;
+    const double r = ((k == 0 || k == it.ntiny) ? 1.0 : 2.0) * x.cor * rcp_fast(fma(dx, dx, y2));
+    add(p, cmk(dx * r, y * r));
+  }
+  int first, cnt;
+  lane_sum12(T, 32, lane, first, cnt);
+  if (cnt) pv_add_out(out, pref, n, first >> 1, first & 1, T[0].v * (x.sm * S.pvc));
+  __syncwarp();
+}
+
+__device__ __forceinline__ void pv_omega(const PvItem&, double2 o, double& x, double& y) {
+  x = o.x;
+  y = o.y;
+}
+__device__ __forceinline__ void pv_omega(const PvItem& it, double2, dflt& x, dflt& y) {
+  x = it.oxd;
+  y = it.oyd;
+}
+
+// adds an item's principal-value part to its output row; pv_scal<dflt> needs
+// values that stay normal floats (df_ok of the item)
+template <typename T>
+__device__ __noinline__ void pv_warp(const SpecDev& S, const SysDev& sys, const PvItem& it, double2 o,
+                                     const double* pref, double2* wk, double2* out) {
+  const int lane = threadIdx.x & 31, M = S.M, n = it.nn < 0 ? -it.nn : it.nn;
+  PvSums<T>* pre = reinterpret_cast<PvSums<T>*>(wk);
+  PvPiece<T>* rec = reinterpret_cast<PvPiece<T>*>(wk + (PV_CHUNK * 24 + 15) / 16);
+  T* wts = reinterpret_cast<T*>(wk + (PV_CHUNK * 24 + 15) / 16 + pv_max_pieces(sys.M_I) * (sizeof(PvPiece<double>) / 16));
+  int a0, cnt;
+  if (!pv_warp_weights<T>(S, sys, it, o.x, pre, rec, wts, lane, a0, cnt)) {
+    pv_direct(S, sys, it, o, pref, out);
+    return;
+  }
+  // lane 4 e + 2 g + c: component c of sum_j V_{e,g}(j) W_j
+  T s = sc_of<T>(0.0);
+  if (lane < 24) {
+    const size_t base = ((size_t)n * (M - 1) + (a0 - 1)) * 12 + (lane >> 1);
+    for (int t = 0; t < cnt; ++t) {
+      const int j = a0 + t;
+      if (j < 1 || j > M - 1) continue;
+      sc_mac(s, ScSpec<T>::v(S, base + (size_t)t * 12), wts[2 * t + (lane & 1)]);
+    }
+  }
+  s = sc_add(s, sc_of<T>(0.0));  // (normalises a double-float accumulator)
+  const T other = sc_shfl(s, lane ^ 1), g2 = sc_shfl(s, (lane + 2) & 31);
+  T ox, oy;
+  pv_omega(it, o, ox, oy);
+  const T kap = ScSpec<T>::kap(S);
+  const bool im = lane & 1;
+  const T x = sc_add(sc_add(sc_mul(ox, s), im ? sc_mul(oy, other) : sc_neg(sc_mul(oy, other))), sc_mul(kap, g2));
+  // G = K_e H with K_e = -(q/kpar) pref_e / 2; result 2 pi T smdelta dpperp/4
+  if (lane < 24 && !(lane & 2))
+    pv_add_out(out, pref, n, lane >> 2, im ? 1 : 0, sc_val(x) * (it.sm * S.pvc * (sc_is_df(s) ? S.Vscale[n] : 1.0)));
+  __syncwarp();
+}
+
+// ---------------------------------------------------------------------------
+// The factorised Landau term of one item on one lane: res_e for entries
+// xx yy zz xy xz yz.  Valid when the rows' deviation |delta_i(p')| <= 1e-5 for
+// p' = p, p +- dppar (second-order remainder <= 1.7e-16); the bound in FP32
+// with a margin (an item just inside it takes the rows).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool landau_factorises(const SpecDev& S, double2 p) {
+  if (!S.lmom) return false;
+  const float ap = sqrtf(fmaf((float)p.x, (float)p.x, (float)p.y * (float)p.y)) * 1.00001f + (float)S.dppar_abs;
+  return fmaf(fmaf(S.la32, ap, S.lb32), ap, S.lc32) <= 0.999e-5f;
+}
+// m 2^e as a double: m's exponent moved in its bits where the result stays a
+// normal number (no FP64 operation), two products otherwise
+__device__ __forceinline__ double scale_exp(double m, int e) {
+  const int hi = __double2hiint(m), x = (hi >> 20) & 0x7ff, y = x + e;
+  if (x != 0 && x != 0x7ff && y > 0 && y < 0x7ff) return __hiloint2double(hi + (e << 20), __double2loint(m));
+  const int e1 = max(-1000, min(1000, e / 2)), e2 = max(-1000, min(1000, e - e1));
+  return m * __hiloint2double((1023 + e1) << 20, 0) * __hiloint2double((1023 + e2) << 20, 0);
+}
+__device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p, int lf, int n, const dflt* prefd,
+                                            double2* res) {
+  // Row Gaussian G(x) = exp(-p2r (x - p3r)^2) at x = p, p +- dppar:
+  // G(p +- pd) = lgc G(p) X^{+-1}, X = exp(-2 p2r pd (p - p3r)).  In
+  // double-float with powers of two kept apart: G(p) = 2^k0 g0,
+  // X = 2^kx xm.  With P_F, Q_F the moment polynomials of family F,
+  //   Spar  = (G(p+pd) P_F(p+pd) - G(p-pd) P_F(p-pd)) / (2 pd)
+  //         = lgc/(2 pd) G(p) (X P_F(p+pd) - X^-1 P_F(p-pd)),
+  //   Sperp = G(p) Q_F(p),
+  //   sum_F = (q/|k_par|) (kappa Spar + (omega - kappa p) Sperp).
+  const double dx = p.x - S.p3r, dy = p.y;
+  int k0 = 0, kx = 0;
+  cdf g0, xm, xi;
+#pragma unroll 1
+  for (int u = 0; u < 2; ++u) {
+    int e;
+    dflt cs, sn;
+    const dflt m = df_exp_scaled(u ? S.lcx * dx : -S.p2r * ((dx - dy) * (dx + dy)), e);
+    df_cis(u ? S.lcx * dy : -2.0 * S.p2r * dx * dy, cs, sn);
+    const cdf v = {df_mul(m, cs), df_mul(m, sn)};
+    if (u) {
+      const dflt im = df_rcp_approx(m);
+      xm = v;
+      xi = {df_mul(im, cs), df_neg(df_mul(im, sn))};
+      kx = e;
+    } else {
+      g0 = v;
+      k0 = e;
+    }
+  }
+  // an underflowing Gaussian (|G| min_a0 below the FP64 range at any of the
+  // three points) leaves the term zero, as in FP64
+  const int akx = kx < 0 ? -kx : kx;
+  if ((k0 + S.lze < -1072) || (k0 - akx + S.lge + S.lze < -1072)) return;
+  // X P+ - X^-1 P- = 2^|kx| (a P+ - b P-): (a, b) = (xm, 2^-2kx xi) for
+  // kx >= 0, (2^2kx xm, xi) otherwise (a term below 2^-126 of the other is
+  // dropped); Sperp enters with 2^-|kx| of it
+  const float sc = akx <= 63 ? ldexpf(1.0f, -2 * akx) : 0.0f, sp = akx <= 126 ? ldexpf(1.0f, -akx) : 0.0f;
+  if (kx >= 0) xi = {df_scale(xi.x, sc), df_scale(xi.y, sc)};
+  else xm = {df_scale(xm.x, sc), df_scale(xm.y, sc)};
+  const cdf pz = {df_of(p.x), df_of(p.y)};
+  const dflt pdd = {S.pdh, S.pdl}, kapd = {S.kaph, S.kapl};
+  const dflt lk = df_mul({S.lgch, S.lgcl}, df_mul(kapd, df_rcp_approx(df_scale(pdd, 2.0f))));  // kappa lgc / (2 pd)
+  const float* lm0 = S.lmomf + (size_t)n * 72;
+  const dflt z = {0.0f, 0.0f};
+  cdf sum[3] = {{z, z}, {z, z}, {z, z}};  // per family: kappa Spar + (omega - kappa p) Sperp over G
+#pragma unroll 1
+  for (int u = 0; u < 3; ++u) {
+    // the moment polynomials at p + pd, p - pd (P_F) and p (Q_F), each times
+    // its factor
+    cdf zu = pz, f;
+    if (u == 0) {
+      zu.x = df_add(pz.x, pdd);
+      f = cdf_rmul(xm, lk);
+    } else if (u == 1) {
+      zu.x = df_add(pz.x, df_neg(pdd));
+      f = cdf_rmul(xi, df_neg(lk));
+    } else {
+      f = {df_scale(df_add(omd.x, df_neg(df_mul(kapd, pz.x))), sp),
+           df_scale(df_add(omd.y, df_neg(df_mul(kapd, pz.y))), sp)};
+    }
+    const cdf z2 = cdf_mul(zu, zu), z3 = cdf_mul(z2, zu), z4 = cdf_mul(z2, z2);
+#pragma unroll
+    for (int F = 0; F < 3; ++F) {
+      const float* cf = lm0 + F * 24 + (u == 2 ? 5 : 0);
+      cdf q = {{cf[0], cf[10]}, z};
+      q = cdf_add(q, cdf_rmul(zu, {cf[1], cf[11]}));
+      q = cdf_add(q, cdf_rmul(z2, {cf[2], cf[12]}));
+      q = cdf_add(q, cdf_rmul(z3, {cf[3], cf[13]}));
+      q = cdf_add(q, cdf_rmul(z4, {cf[4], cf[14]}));
+      sum[F] = cdf_add(sum[F], cdf_mul(f, q));
+    }
+  }
+  // res_e = pref_e c_e sum_F(e) ifac, c_e = 1, p or p^2; ifac =
+  // -i dpperp 2 pi^2 lf, pref_e real (imaginary for xy, yz); with q / |k_par|
+  const cdf gq = cdf_rmul(g0, df_mul({S.qlh, S.qll}, df_scale({S.lih, S.lil}, (float)lf)));
+  cdf v[6];
+  v[0] = cdf_mul(gq, sum[0]);
+  v[1] = cdf_mul(gq, sum[1]);
+  v[3] = cdf_mul(gq, sum[2]);
+  v[4] = cdf_mul(v[0], pz);
+  v[2] = cdf_mul(v[4], pz);
+  v[5] = cdf_mul(v[3], pz);
+#pragma unroll
+  for (int e = 0; e < 6; ++e) {
+    const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0), ex = k0 + akx + (int)lm0[fam * 24 + 20];
+    // pref ifac: real pref -> i pref fi; imaginary i pref -> -(pref fi)
+    const bool im = (e == 3 || e == 5);
+    const double vx = scale_exp(df_val(df_mul(v[e].x, prefd[e])), ex), vy = scale_exp(df_val(df_mul(v[e].y, prefd[e])), ex);
+    res[e] = im ? cmk(-vx, -vy) : cmk(-vy, vx);
+  }
+}
+
+// what the warp phase of k_resonant_multi needs of one item
 struct __align__(16) ResItem {
-  double pr, pim;     // complex resonance momentum
-  double smdelta;     // principal-value sample spacing (integrate_res's smdelta)
-  int lower, upper;   // principal-value window
-  int nn, work;       // signed order; bit 0 principal value, bit 1 Landau rows, lf << 2
-  int w, s;           // omega, species
-  long long slot;     // the item's slot (its output row)
-  // the fast path's principal-value constants, formed one item per lane:
-  int ntiny, pvdf;    // sample points of the tiny rest; pv_fast applies
-  float u0, du, ut0, dut;  // FP32 piece estimates of the sample points
-  float smd[2], capd[2], pimd[2], pim2[2], csd[2], cord[2];  // double-float pairs
+  PvItem pv;
   double pref[6];     // T-tensor prefactors: imaginary for xy and yz, else real
+  int work;           // 1 principal value, 2 Landau rows, 4 the sums in double-float; lf << 3
+  int w, s, pad;      // omega, species
+  long long slot;     // the item's slot (its output row)
 };
 // prefactor e of an item as the complex number t_prefactors gives
 __device__ __forceinline__ double2 item_pref(const ResItem& it, int e) {
   return (e == 3 || e == 5) ? cmk(0.0, it.pref[e]) : cmk(it.pref[e], 0.0);
 }
 
-// The principal-value constants of a resonant item (integrate_res,
-// src/ALPS_fns.f90:1000-1040: capDelta, smdelta, the tiny rest's ntiny and
-// corr), and for the fast path their double-float pairs and FP32 piece
-// estimates, formed in the one-item-per-lane phase so that the warp phase
-// starts from them.  pvdf = 0 leaves the item to the FP64 code: a spacing,
-// window or |p_im| outside 1e-12 .. 1e12 would leave the normal floats.
-__device__ __forceinline__ void pv_constants(const DispArgs& a, const SpecDev& S, const ResGeom& g, ResItem& it) {
-  it.smdelta = 0.0;
-  it.ntiny = 0;
-  it.pvdf = 0;
-  if (g.kind != 3) return;
-  const double pr = g.pr, pim = g.pi;
-  const double capDelta = pr - S.ppar[g.lower];
-  const double smdelta = capDelta / (1.0 * a.sys.M_P);
-  const int ntiny = (int)((S.ppar[g.upper] - pr - capDelta) / smdelta);
-  const double corr = (ntiny > 0) ? ((S.ppar[g.upper] - pr - capDelta) / (1.0 * ntiny)) / smdelta : 0.0;
-  it.smdelta = smdelta;
-  it.ntiny = ntiny;
-  if (!S.df_sums) return;
-  const bool sym = fabs(pim) > a.sys.Tlim;
-  auto inr = [](double x) { return x >= 1e-12 && x <= 1e12; };
-  if (!(inr(smdelta) && inr(capDelta) && fabs(pim) <= 1e12 && (!sym || inr(fabs(pim))) &&
-        (ntiny <= 0 || inr(corr * smdelta))))
-    return;
-  it.pvdf = 1;
-  it.u0 = (float)(1.0 + (pr - S.ppar[1]) * S.idppar);
-  it.du = (float)(smdelta * S.idppar);
-  it.ut0 = (float)(1.0 + (pr + capDelta - S.ppar[1]) * S.idppar);
-  it.dut = (float)(corr * smdelta * S.idppar);
-  auto put2 = [](float* d, double x) {
-    const dflt v = df_of(x);
-    d[0] = v.h;
-    d[1] = v.l;
-  };
-  put2(it.smd, smdelta);
-  put2(it.capd, capDelta);
-  put2(it.pimd, pim);
-  put2(it.pim2, pim * pim);
-  put2(it.csd, __dmul_rn(corr, smdelta));
-  put2(it.cord, corr);
+// An item's per-lane part: geometry, prefactors, principal-value constants,
+// Landau term where it factorises (in res).  Returns the work left (ResItem).
+__device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, double2 o, int nn, PvItem& pv,
+                                        double pref[6], double2 res[6], int& lf) {
+  const int n = nn < 0 ? -nn : nn;
+  {
+    // t_prefactors' nonzero parts, with 1/z
+    const double dz = (double)nn * S.iz;
+    const double k2 = a.sys.kperp_norm ? 1.0 : a.sys.kperp * a.sys.kperp, k1 = a.sys.kperp_norm ? 1.0 : a.sys.kperp;
+    pref[0] = dz * dz;
+    pref[1] = pref[2] = k2;
+    pref[3] = pref[4] = k1 * dz;
+    pref[5] = -k2;
+  }
+#pragma unroll
+  for (int e = 0; e < 6; ++e) res[e] = cmk(0.0, 0.0);
+  const ResGeom g = res_geometry_of(S, a.sys, o, nn);
+  lf = (o.y < 0.0) ? 2 : ((o.y == 0.0) ? 1 : 0);
+  int work = 0;
+  pv.pr = g.pr;
+  pv.pim = g.pi;
+  pv.nn = nn;
+  if (g.kind == 3) {
+    pv_setup(S, a.sys, g, nn, o.x, pv);
+    work = 1;
+    if (S.df_sums) {
+      // a spacing, window or |p_im| outside 1e-12 .. 1e12 would leave the
+      // normal floats: those items take the FP64 sums
+      auto inr = [](float x) { return x >= 1e-12f && x <= 1e12f; };
+      const float sm = (float)pv.sm, pim = fabsf((float)pv.pim);
+      if (inr(sm) && inr((float)pv.cap) && pim <= 1e12f && (pim <= (float)a.sys.Tlim || inr(pim)) &&
+          (pv.ntiny <= 0 || inr((float)pv.cor * sm)))
+        work |= 4;
+      pv.capd = df_of(pv.cap);
+      pv.smd = df_of(pv.sm);
+      pv.cord = df_of(pv.cor);
+      pv.pimd = df_of(pv.pim);
+    }
+  }
+  if (S.df_sums) {
+    pv.oxd = df_of(o.x);
+    pv.oyd = df_of(o.y);
+  }
+  if (lf > 0) {
+    const double2 p = cmk(g.pr, g.pi);
+    if (landau_factorises(S, p)) {
+      const dflt izd = {S.izh, S.izl}, dzd = df_mul({(float)nn, 0.0f}, izd);
+      const dflt k2d = {a.sys.k2h, a.sys.k2l}, xyd = df_mul({a.sys.k1h, a.sys.k1l}, dzd);
+      const dflt prefd[6] = {df_mul(dzd, dzd), k2d, k2d, xyd, xyd, df_neg(k2d)};
+      landau_lane(S, {pv.oxd, pv.oyd}, p, lf, n, prefd, res);
+      if (n == 0) res[0] = res[3] = res[4] = cmk(0.0, 0.0);
+    } else {
+      work |= 2;
+    }
+  }
+  return work;
 }
 
-// the region used first by the principal-value records, then by the Landau
-// rows, in double2
-__host__ __device__ inline size_t res_region(int N) {
-  const size_t rows = 3 * (size_t)(N + 1);
-  return rows > PV_SMEM ? rows : (size_t)PV_SMEM;
+// a slot's order in k_resonant_multi's list mode: the order and the work that
+// k_resonant_lanes left
+#define FLAG_TODO 256  // bit of a job's error word while such work is left
+__device__ __forceinline__ int todo_slot(int nn, int work) { return (nn & 0xffff) | (work << 16); }
+
+// Walks a warp's slots slot0 .. slot0 + ipw - 1.  Most slots of a large batch
+// are empty (an (omega, species) fills count of its rcap slots), so the
+// occupied ones are gathered, in slot order, into batches of up to 32 items;
+// body(nb, item, mine) runs with the batch's items one per lane.  Which batch
+// or lane an item lands on does not change its result.
+template <typename F, typename G>
+__device__ __forceinline__ void res_batches(const DispArgs& a, int ipw, int n_om, const int* __restrict__ count,
+                                            long slot0, int* queue, F want, G body) {
+  const int lane = threadIdx.x & 31, S_ = a.sys.nspec;
+  const long total = (long)n_om * S_ * a.rcap;
+  const unsigned lt = (1u << lane) - 1u;
+  int qn = 0;
+  for (int c0 = 0; c0 < ipw; c0 += 32) {
+    {
+      const long sl = slot0 + c0 + lane;
+      bool occ = false;
+      if (c0 + lane < ipw && sl < total) {
+        const unsigned u = (unsigned)(sl / a.rcap), r = (unsigned)(sl - (long)u * a.rcap);  // u = w S + s
+        occ = (int)r < count[u] && want(sl);
+      }
+      const unsigned m = __ballot_sync(FULL_WARP, occ);
+      if (occ) queue[qn + __popc(m & lt)] = c0 + lane;
+      qn += __popc(m);
+      __syncwarp();
+    }
+    const bool last = c0 + 32 >= ipw;
+    while (qn >= 32 || (last && qn > 0)) {
+      const int nb = qn < 32 ? qn : 32;
+      const long item = (lane < nb) ? slot0 + queue[lane] : -1;
+      body(nb, item);
+      // the items beyond this batch move to the front of the queue
+      const int rest = qn - nb;
+      const int keep = (lane < rest) ? queue[nb + lane] : 0;
+      __syncwarp();
+      if (lane < rest) queue[lane] = keep;
+      __syncwarp();
+      qn = rest;
+    }
+  }
 }
 
-// per-warp shared memory in double2: the window (h, s), the records / rows
-// region, the warp's 32 items, 6 values handed to lanes 0-5 and the queue of
-// occupied slots (64 ints)
-__host__ __device__ inline size_t res_warp_smem(int N, int W) {
-  return (size_t)W * 12 + res_region(N) + 32 * (sizeof(ResItem) / sizeof(double2)) + 6 + 16;
+// the warp's region for principal-value work, then for the Landau rows, in double2
+__host__ __device__ inline size_t res_region(int N, int M_I) {
+  const size_t rows = 3 * (size_t)(N + 1), pv = pv_warp_words(M_I);
+  return rows > pv ? rows : pv;
+}
+// per-warp shared memory in double2: the region, the warp's 32 items, 3
+// values handed to lanes 0-5 and the queue of occupied slots (64 ints)
+__host__ __device__ inline size_t res_warp_smem(int N, int M_I) {
+  return res_region(N, M_I) + 32 * (sizeof(ResItem) / sizeof(double2)) + 3 + 16;
 }
 
-// Slots per warp: a warp gathers the occupied slots of its range into
-// batches of up to 32 items, does the per-item scalar work one item per
-// lane, then the vector work of the batch's items one after another.  Large
-// batches take up to 256 slots per warp (about 7 waves of resident warps on
-// the map lattice); small ones spread their items over more warps (a single
-// omega's few resonant orders run side by side, as latency wants).
+// Slots per warp: small batches spread their items over many warps (a single
+// omega's few resonant orders run side by side, as latency wants), large ones
+// take up to 256 slots per warp.
 inline int res_items_per_warp(long nslots, int warps_per_sm = 12) {
   const long warps_wanted = 152L * warps_per_sm;  // SMs x resident warps of k_resonant
   long ipw = nslots / warps_wanted;
@@ -925,361 +1617,6 @@ __device__ inline double2 crcp(double2 z) {
   return cmk(z.x * r, -z.y * r);
 }
 
-// ---------------------------------------------------------------------------
-// Fast path of one item's principal-value window: the same sums as the FP64
-// code in resonant_body (sample points, pieces, per-piece sums A and C, the
-// merge in lane order, h A + s B per (run, entry), the Tlim branch), all in
-// double-float arithmetic on the FP32 pipes, on the reduced vectors' float
-// pairs (scaled by 2^-e for order n; the result is rescaled at the end).
-// The pieces are still chosen from the FP64 sample points wherever the FP32
-// estimate lies within its error bound of a half-way point.  Returns false,
-// with nothing written to out, when the item's constants were not formed
-// (a range would leave the normal floats) or the merge does not apply (the
-// caller then runs the FP64 code); otherwise adds the item's
-// principal-value part to out (entry e: pref_e T_e times the window scale).
-// ---------------------------------------------------------------------------
-struct PvSlotF {
-  int jd, jc;  // finished piece (-1: none), current piece
-  dflt Adx, Ady, Bdx, Bdy, Acx, Acy, Bcx, Bcy;
-};
-
-__device__ __forceinline__ float4 f4_of(dflt x, dflt y) { return make_float4(x.h, x.l, y.h, y.l); }
-__device__ __forceinline__ dflt f4x(float4 v) { return {v.x, v.y}; }
-__device__ __forceinline__ dflt f4y(float4 v) { return {v.z, v.w}; }
-// (ax + i ay)(bx + i by), real and imaginary parts
-__device__ __forceinline__ void df_cmul(dflt ax, dflt ay, dflt bx, dflt by, dflt& rx, dflt& ry) {
-  rx = df_add(df_mul(ax, bx), df_neg(df_mul(ay, by)));
-  ry = df_add(df_mul(ax, by), df_mul(ay, bx));
-}
-
-__device__ __noinline__ bool pv_fast(const DispArgs& a, const SpecDev& S, const ResItem& it, double2 o, int n,
-                                     int W, float4* win, double2* pvv, double2* out) {
-  if (!it.pvdf) return false;
-  const int lane = threadIdx.x & 31;
-  const int M = S.M;
-  const double pr = it.pr, pim = it.pim;
-  const double smdelta = it.smdelta;
-  const bool sym = fabs(pim) > a.sys.Tlim;
-  const int NP = a.sys.M_P + 1;
-  const int ntiny = it.ntiny;
-  const int jw0 = max(1, it.lower - 2), jw1 = min(M - 1, it.upper + 2);
-  const int nw = jw1 - jw0 + 1;
-  const float* __restrict__ Vh = S.Vh + (size_t)n * (M - 1) * 12;
-  const float* __restrict__ Vl = S.Vl + (size_t)n * (M - 1) * 12;
-  const dflt oxd = df_of(o.x), oyd = df_of(o.y), kad = {S.kaph, S.kapl}, hid = {S.hidh, S.hidl};
-  // node value h_e(j) = omega V_{e,1}(j) + kappa V_{e,2}(j), scaled
-  auto hnode = [&](int j, int e, dflt& hx, dflt& hy) {
-    const size_t b = (size_t)(j - 1) * 12 + 2 * e;
-    const dflt v1 = {Vh[b], Vl[b]}, v2 = {Vh[b + 1], Vl[b + 1]};
-    hx = df_add(df_mul(oxd, v1), df_mul(kad, v2));
-    hy = df_mul(oyd, v1);
-  };
-  float4* wh = win;           // h at window nodes
-  float4* ws = win + W * 6;   // centred slopes
-  for (int t = lane; t < nw * 6; t += 32) {
-    const int jj = t / 6, e = t % 6;
-    dflt hx, hy;
-    hnode(jw0 + jj, e, hx, hy);
-    wh[jj * 6 + e] = f4_of(hx, hy);
-  }
-  __syncwarp();
-  for (int t = lane; t < nw * 6; t += 32) {
-    const int jj = t / 6, e = t % 6;
-    if (jj >= 1 && jj + 1 < nw) {
-      const float4 u = wh[(jj + 1) * 6 + e], d = wh[(jj - 1) * 6 + e];
-      ws[jj * 6 + e] = f4_of(df_mul(df_add(f4x(u), df_neg(f4x(d))), hid), df_mul(df_add(f4y(u), df_neg(f4y(d))), hid));
-    }
-  }
-  __syncwarp();
-  // node value and slope of entry e at piece jc (window, or from the pairs)
-  auto node1 = [&](int jc, int e, dflt& hx, dflt& hy, dflt& sx, dflt& sy) {
-    if (jc - 1 >= jw0 && jc + 1 <= jw1) {
-      const float4 h = wh[(jc - jw0) * 6 + e], s = ws[(jc - jw0) * 6 + e];
-      hx = f4x(h);
-      hy = f4y(h);
-      sx = f4x(s);
-      sy = f4y(s);
-    } else {
-      dflt ux, uy, dx, dy;
-      hnode(jc, e, hx, hy);
-      hnode(jc + 1, e, ux, uy);
-      hnode(jc - 1, e, dx, dy);
-      sx = df_mul(df_add(ux, df_neg(dx)), hid);
-      sy = df_mul(df_add(uy, df_neg(dy)), hid);
-    }
-  };
-  // pieces, as in resonant_body: the last node in 1..M-1 within half a
-  // spacing of p (funct_g's search), clamped to 2..M-2
-  const double idpa = fabs(S.idppar), half = 0.5 * S.dppar_abs;
-  auto piece_raw = [&](double p) {
-    int jr = 0;
-    double jd = floor((p - S.ppar[0]) * idpa + 0.5);
-    if (jd > -10.0 && jd < (double)M + 10.0) {
-      int j0 = (int)jd;
-      int hi = min(j0 + 2, M - 1), lo = max(j0 - 2, 1);
-      for (int jj = hi; jj >= lo; --jj)
-        if (fabs(S.ppar[jj] - p) <= half) {
-          jr = jj;
-          break;
-        }
-    }
-    return jr;
-  };
-  auto clampj = [&](int jr) { return (jr >= M - 1) ? M - 2 : ((jr <= 1) ? 2 : jr); };
-  // the FP32 estimates u (node j at u = j) are within 2^-23 (M + 20) of a
-  // spacing (two roundings of numbers below M + 10) and the nodes within
-  // 1e-6 of a spacing of their uniform positions: farther than four times
-  // that from a half-way point, the nearest node is the search's answer
-  const float hthr = 0.5f - (4.0f * 1.1920929e-7f * (float)(M + 20) + 4.0e-6f);
-  auto off_half = [&](float u) { return fabsf(u - rintf(u)) < hthr; };
-  auto node_of = [&](float u) {
-    const int j = (int)rintf(u);
-    return (j >= 1 && j <= M - 1) ? j : 0;
-  };
-  const dflt prd = df_of(pr);
-  auto ppd = [&](int j) { return dflt{S.pph[j], S.ppl[j]}; };
-  // the FP64 sample points as integrate_res writes them (for the search
-  // near half-way points only)
-  auto sym_p = [&](int k) {
-    const double capDelta = pr - S.ppar[it.lower];
-    return (k == 0) ? pr : ((k == a.sys.M_P) ? __dadd_rn(pr, capDelta) : __dadd_rn(pr, __dmul_rn(smdelta, (double)k)));
-  };
-  auto tiny_p = [&](int k) {
-    const double capDelta = pr - S.ppar[it.lower];
-    const double corr = ((S.ppar[it.upper] - pr - capDelta) / (1.0 * ntiny)) / smdelta;
-    return (k == 0) ? __dadd_rn(pr, capDelta)
-                    : __dadd_rn(__dadd_rn(pr, capDelta), __dmul_rn(__dmul_rn(corr, smdelta), (double)k));
-  };
-  bool bad = false;
-  const dflt z0 = {0.0f, 0.0f};
-  auto putf = [&](PvSlotF& q, int j, dflt dx, dflt cx, dflt cy, int dir) {
-    if (j != q.jc) {
-      if (q.jc >= 0) {
-        if (q.jd >= 0 || (dir > 0 ? j < q.jc : j > q.jc)) bad = true;
-        q.jd = q.jc;
-        q.Adx = q.Acx;
-        q.Ady = q.Acy;
-        q.Bdx = q.Bcx;
-        q.Bdy = q.Bcy;
-      }
-      q.jc = j;
-      q.Acx = q.Acy = q.Bcx = q.Bcy = z0;
-    }
-    df_acc(q.Acx, cx);
-    df_acc(q.Acy, cy);
-    df_mac(q.Bcx, cx.h, cx.l, dx);
-    df_mac(q.Bcy, cy.h, cy.l, dx);
-  };
-  // records: (group, lane, slot) sums A, B as float4 pairs; run tables as in
-  // resonant_body
-  float4* recv = reinterpret_cast<float4*>(pvv);
-  float4* runv = reinterpret_cast<float4*>(pvv + PV_RECV);
-  int* recj = reinterpret_cast<int*>(pvv + PV_RECV + PV_RUNV);
-  int* runL = recj + PV_GROUPS * 64;
-  int* runS = runL + 32;
-  int* runG = runS + 32;
-  int* runJ = runG + 32;
-  int nruns = 0, nl[PV_GROUPS] = {0, 0, 0};
-  const unsigned lt = (1u << lane) - 1u;
-  auto records = [&](int gi, const PvSlotF& q, int dir) {
-    const bool two = q.jd >= 0;
-    const int j0 = two ? q.jd : q.jc, j1 = two ? q.jc : -1;
-    recj[recj_at(gi, lane, 0)] = j0;
-    recj[recj_at(gi, lane, 1)] = j1;
-    recv[rec_at(gi, lane, 0, 0)] = two ? f4_of(q.Adx, q.Ady) : f4_of(q.Acx, q.Acy);
-    recv[rec_at(gi, lane, 0, 1)] = two ? f4_of(q.Bdx, q.Bdy) : f4_of(q.Bcx, q.Bcy);
-    recv[rec_at(gi, lane, 1, 0)] = two ? f4_of(q.Acx, q.Acy) : f4_of(z0, z0);
-    recv[rec_at(gi, lane, 1, 1)] = two ? f4_of(q.Bcx, q.Bcy) : f4_of(z0, z0);
-    const int last = (j1 >= 0) ? j1 : j0;
-    const int prev = __shfl_up_sync(0xffffffffu, last, 1);
-    const bool st0 = (j0 >= 0) && (lane == 0 || j0 != prev);
-    const bool st1 = (j1 >= 0);
-    if (j0 >= 0 && lane > 0 && (prev < 0 || (dir > 0 ? j0 < prev : j0 > prev))) bad = true;
-    const unsigned m0 = __ballot_sync(0xffffffffu, st0), m1 = __ballot_sync(0xffffffffu, st1);
-    const int nr = __popc(m0) + __popc(m1);
-    if (nruns + nr <= 32) {
-      const int id0 = nruns + __popc(m0 & lt) + __popc(m1 & lt), id1 = id0 + (st0 ? 1 : 0);
-      if (st0) {
-        runL[id0] = lane;
-        runS[id0] = 0;
-        runG[id0] = gi;
-      }
-      if (st1) {
-        runL[id1] = lane;
-        runS[id1] = 1;
-        runG[id1] = gi;
-      }
-    }
-    nruns += nr;
-    nl[gi] = __popc(__ballot_sync(0xffffffffu, j0 >= 0));
-  };
-  const dflt pimd = {it.pimd[0], it.pimd[1]}, pim2 = {it.pim2[0], it.pim2[1]};
-  const dflt smd = {it.smd[0], it.smd[1]}, capd = {it.capd[0], it.capd[1]};
-  dflt Tlx = z0, Tly = z0;  // the Tlim part of entry e on lane e
-  if (sym) {
-    const int per = (NP + 31) / 32;
-    const int k0 = lane * per, k1 = min(NP, k0 + per);
-    PvSlotF su{-1, -1, z0, z0, z0, z0, z0, z0, z0, z0}, sd = su;
-    const float u0 = it.u0, du = it.du;
-    for (int k = k0; k < k1; ++k) {
-      // K = w (dx, p_im) / (dx^2 + p_im^2), dx = p_k - p_res
-      const dflt dx = (k == a.sys.M_P) ? capd : df_mul(smd, {(float)k, 0.0f});
-      const dflt r = df_scale(df_rcp_approx(df_add(df_mul(dx, dx), pim2)), (k == 0 || k == a.sys.M_P) ? 1.0f : 2.0f);
-      const dflt Kx = df_mul(dx, r), Ky = df_mul(pimd, r);
-      const float uu = fmaf((float)k, du, u0), ud = fmaf(-(float)k, du, u0);
-      int cu, cd;
-      if (off_half(uu)) cu = node_of(uu);
-      else cu = piece_raw(sym_p(k));
-      if (off_half(ud)) cd = node_of(ud);
-      else cd = piece_raw(2.0 * pr - sym_p(k));
-      putf(su, clampj(cu), dx, Kx, Ky, 1);
-      putf(sd, clampj(cd), df_neg(dx), Kx, df_neg(Ky), -1);
-    }
-    records(0, su, 1);
-    records(1, sd, -1);
-  } else {
-    // Tlim branch: g' sum_k w_k dx^2/(dx^2 + p_im^2) + sign(p_im) i pi G(p_res)/smdelta
-    dflt frd = z0;
-    for (int k = 1 + lane; k <= a.sys.M_P; k += 32) {
-      const dflt dx = (k == a.sys.M_P) ? capd : df_mul(smd, {(float)k, 0.0f});
-      const dflt d2 = df_mul(dx, dx);
-      const dflt q = df_mul(d2, df_rcp_approx(df_add(d2, pim2)));
-      df_acc(frd, df_scale(q, (k == a.sys.M_P) ? 1.0f : 2.0f));
-    }
-    for (int off = 16; off > 0; off >>= 1)
-      frd = df_add(frd, {__shfl_xor_sync(0xffffffffu, frd.h, off), __shfl_xor_sync(0xffffffffu, frd.l, off)});
-    if (lane < 6) {
-      const int e = lane;
-      const double dps = S.dppar;
-      // H at p_res + side dppar: u = u0 + side, dx = p - pp(jc) in double-float
-      auto Hc1 = [&](int side, dflt& Hx, dflt& Hy) {
-        const float u = it.u0 + (float)side;
-        int jc;
-        if (off_half(u)) jc = node_of(u);
-        else jc = piece_raw(side > 0 ? pr + dps : (side < 0 ? pr - dps : pr));
-        jc = clampj(jc);
-        dflt hx, hy, sx, sy;
-        node1(jc, e, hx, hy, sx, sy);
-        const dflt dx = df_add(df_add(prd, df_scale({S.dpph, S.dppl}, (float)side)), df_neg(ppd(jc)));
-        Hx = df_add(hx, df_mul(sx, dx));
-        Hy = df_add(hy, df_mul(sy, dx));
-      };
-      dflt H1x, H1y, H2x, H2y, H0x, H0y;
-      Hc1(1, H1x, H1y);
-      Hc1(-1, H2x, H2y);
-      Hc1(0, H0x, H0y);
-      // g' 2 fr = (H1 - H2) fr / dppar;  i sign(p_im) 2 pi / smdelta, smdelta = capDelta / M_P
-      const float sgn = (pim > 0.0) ? 1.0f : ((pim < 0.0) ? -1.0f : 0.0f);
-      const dflt c1 = df_mul(frd, {S.idph, S.idpl});
-      const dflt c2 = df_scale(df_mul({S.tpmh, S.tpml}, df_rcp_approx(capd)), sgn);
-      Tlx = df_add(df_mul(df_add(H1x, df_neg(H2x)), c1), df_neg(df_mul(c2, H0y)));
-      Tly = df_add(df_mul(df_add(H1y, df_neg(H2y)), c1), df_mul(c2, H0x));
-    }
-  }
-  if (ntiny > 0) {
-    const int per = (ntiny + 1 + 31) / 32;
-    const int k0 = lane * per, k1 = min(ntiny + 1, k0 + per);
-    PvSlotF sq{-1, -1, z0, z0, z0, z0, z0, z0, z0, z0};
-    const float ut0 = it.ut0, dut = it.dut;
-    const dflt csd = {it.csd[0], it.csd[1]}, cord = {it.cord[0], it.cord[1]};
-    for (int k = k0; k < k1; ++k) {
-      // K = w corr (dx, p_im) / (dx^2 + p_im^2)
-      const dflt dx = (k == 0) ? capd : df_add(capd, df_mul(csd, {(float)k, 0.0f}));
-      const dflt r = df_scale(df_mul(df_rcp_approx(df_add(df_mul(dx, dx), pim2)), cord),
-                              (k == 0 || k == ntiny) ? 1.0f : 2.0f);
-      const dflt Kx = df_mul(dx, r), Ky = df_mul(pimd, r);
-      const float ut = fmaf((float)k, dut, ut0);
-      int ct;
-      if (off_half(ut)) ct = node_of(ut);
-      else ct = piece_raw(tiny_p(k));
-      putf(sq, clampj(ct), dx, Kx, Ky, 1);
-    }
-    records(2, sq, 1);
-  }
-  if (__any_sync(0xffffffffu, bad) || nruns > 32) return false;
-  dflt accd = z0;  // component c = lane (< 12) of T: xx.re, xx.im, yy.re, ...
-  if (nruns > 0) {
-    __syncwarp();
-    // run totals in (lane, slot) order
-    if (lane < nruns) {
-      const int L = runL[lane], sl = runS[lane], gi = runG[lane];
-      int Ln = nl[gi], sn = 0;
-      if (lane + 1 < nruns && runG[lane + 1] == gi) {
-        Ln = runL[lane + 1];
-        sn = runS[lane + 1];
-      }
-      float4 A4 = recv[rec_at(gi, L, sl, 0)], B4 = recv[rec_at(gi, L, sl, 1)];
-      dflt Ax = f4x(A4), Ay = f4y(A4), Bx = f4x(B4), By = f4y(B4);
-      for (int L2 = L + 1; L2 < Ln || (L2 == Ln && sn == 1); ++L2) {
-        const float4 a2 = recv[rec_at(gi, L2, 0, 0)], b2 = recv[rec_at(gi, L2, 0, 1)];
-        Ax = df_add(Ax, f4x(a2));
-        Ay = df_add(Ay, f4y(a2));
-        Bx = df_add(Bx, f4x(b2));
-        By = df_add(By, f4y(b2));
-      }
-      runJ[lane] = recj[recj_at(gi, L, sl)];
-      runv[lane * 2] = f4_of(Ax, Ay);
-      runv[lane * 2 + 1] = f4_of(Bx, By);
-    }
-    __syncwarp();
-    // (run, entry) pairs: h A + s B with B = C + (p_res - pp(jc)) A,
-    // mirrored runs with the minus sign
-    float4* contrib = recv;
-    for (int q = lane; q < nruns * 6; q += 32) {
-      const int rho = q / 6, e = q % 6;
-      const int jc = runJ[rho];
-      dflt hx, hy, sx, sy;
-      node1(jc, e, hx, hy, sx, sy);
-      const float4 A4 = runv[rho * 2], C4 = runv[rho * 2 + 1];
-      const dflt Ax = f4x(A4), Ay = f4y(A4);
-      const dflt del = df_add(prd, df_neg(ppd(jc)));
-      const dflt Bx = df_add(f4x(C4), df_mul(Ax, del)), By = df_add(f4y(C4), df_mul(Ay, del));
-      dflt t1x, t1y, t2x, t2y;
-      df_cmul(hx, hy, Ax, Ay, t1x, t1y);
-      df_cmul(sx, sy, Bx, By, t2x, t2y);
-      dflt tx = df_add(t1x, t2x), ty = df_add(t1y, t2y);
-      if (runG[rho] == 1) {
-        tx = df_neg(tx);
-        ty = df_neg(ty);
-      }
-      contrib[q] = f4_of(tx, ty);
-    }
-    __syncwarp();
-    // component c of T: the runs in order
-    if (lane < 12) {
-      const int e = lane >> 1;
-      dflt s = z0;
-      for (int rho = 0; rho < nruns; ++rho) {
-        const float4 c = contrib[rho * 6 + e];
-        s = df_add(s, (lane & 1) ? f4y(c) : f4x(c));
-      }
-      accd = s;
-    }
-  }
-  {
-    // plus the Tlim part of component c (entry c/2 sits on lane c/2)
-    const int src = (lane < 12) ? (lane >> 1) : 0;
-    const float xh = __shfl_sync(0xffffffffu, Tlx.h, src), xl = __shfl_sync(0xffffffffu, Tlx.l, src);
-    const float yh = __shfl_sync(0xffffffffu, Tly.h, src), yl = __shfl_sync(0xffffffffu, Tly.l, src);
-    accd = df_add(accd, (lane & 1) ? dflt{yh, yl} : dflt{xh, xl});
-  }
-  // out_e += pref_e T_e scale: scale = 2 pi smdelta dpperp/4 (-q/(2 k_par))
-  // and the pairs' 2^e; an imaginary prefactor (xy, yz) maps (x, y) to
-  // pe (-y, x)
-  const double v = df_val(accd) * (S.Vscale[n] * it.smdelta * S.pvc);
-  const double w = __shfl_xor_sync(0xffffffffu, v, 1);
-  if (lane < 12) {
-    const int e = lane >> 1;
-    if (!(n == 0 && (e == 0 || e == 3 || e == 4))) {
-      const double pe = it.pref[e];
-      double* o2 = reinterpret_cast<double*>(out + e);
-      o2[lane & 1] += (e == 3 || e == 5) ? ((lane & 1) ? pe * w : -pe * w) : pe * v;
-    }
-  }
-  __syncwarp();
-  return true;
-}
-
 __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
                                               int n_om, const int* __restrict__ count,
                                               const int* __restrict__ slot_nn, double2* items, long block) {
@@ -1287,670 +1624,67 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int S_ = a.sys.nspec;
   const int N = a.sp[0].N;  // every species has the same p_perp grid
-  const int W = res_win(a.sys.M_I);
-  double2* wh = sm + (size_t)warp * res_warp_smem(N, W);  // node values h
-  double2* ws = wh + W * 6;                                // node slopes s
-  double2* pvv = ws + W * 6;                               // principal-value records
-  double2* frow = pvv;                                     // f(i, p_res), after them
+  double2* wk = sm + (size_t)warp * res_warp_smem(N, a.sys.M_I);
+  double2* frow = wk;                                      // f(i, p_res)
   double2* fpr = frow + (N + 1);                           // f(i, p_res + dppar)
   double2* fmr = fpr + (N + 1);                            // f(i, p_res - dppar)
-  ResItem* ri = reinterpret_cast<ResItem*>(pvv + res_region(N));
+  ResItem* ri = reinterpret_cast<ResItem*>(wk + res_region(N, a.sys.M_I));
   double2* tb = reinterpret_cast<double2*>(ri + 32);      // values handed to lanes 0-5
-  int* queue = reinterpret_cast<int*>(tb + 6);            // occupied slots, offsets from slot0
-  const long total = (long)n_om * S_ * a.rcap;
-  // this warp's slots: slot0 .. slot0 + sh.ipw - 1.  Most slots of a large
-  // batch are empty (an (omega, species) fills count of its rcap slots), so
-  // the occupied ones are gathered, in slot order, into batches of up to 32
-  // items; each batch runs the per-item phase one item per lane and then
-  // the per-warp phase.  Which batch or lane an item lands on does not
-  // change its result.
+  int* queue = reinterpret_cast<int*>(tb + 3);            // occupied slots, offsets from slot0
   const long slot0 = (block * RES_WARPS + warp) * (long)sh.ipw;
-  if (slot0 >= total) return;
-  const unsigned lt = (1u << lane) - 1u;
-  int qn = 0;
-  for (int c0 = 0; c0 < sh.ipw; c0 += 32) {
-    {
-      const long sl = slot0 + c0 + lane;
-      bool occ = false;
-      if (c0 + lane < sh.ipw && sl < total) {
-        const int r = (int)(sl % a.rcap);
-        const int s = (int)((sl / a.rcap) % S_);
-        const int w = (int)(sl / ((long)a.rcap * S_));
-        occ = r < count[(size_t)w * S_ + s];
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, occ);
-      if (occ) queue[qn + __popc(m & lt)] = c0 + lane;
-      qn += __popc(m);
-      __syncwarp();
-    }
-    const bool last = c0 + 32 >= sh.ipw;
-    while (qn >= 32 || (last && qn > 0)) {
-  const int nb = qn < 32 ? qn : 32;
-  const long item = (lane < nb) ? slot0 + queue[lane] : total;
-
-  // ---- one item per thread: geometry, prefactors, factorised Landau rows ----
+  if (slot0 >= (long)n_om * S_ * a.rcap) return;
+  const bool list = sh.lanes;  // only what k_resonant_lanes left
+  res_batches(
+      a, sh.ipw, n_om, count, slot0, queue,
+      [&](long sl) { return !list || (slot_nn[sl] >> 16) != 0; },
+      [&](int nb, long item) {
+  // ---- one item per lane ----
   int work = 0;
-  if (item < total) {
-    const int r = (int)(item % a.rcap);
-    const int s = (int)((item / a.rcap) % S_);
-    const int w = (int)(item / ((long)a.rcap * S_));
-    {
-      const SpecDev& S = a.sp[s];
-      const int nn = slot_nn[((size_t)w * S_ + s) * a.rcap + r];
-      const int n = nn < 0 ? -nn : nn;
-      const double2 o = om[w];
-      const double kpar = a.sys.kpar;
-      const double z = a.sys.kperp_norm ? a.sys.kperp / S.qs : 1.0 / S.qs;
-      double2 pref[6];
-      t_prefactors(nn, z, a.sys.kperp, a.sys.kperp_norm, pref);
-      const ResGeom g = res_geometry(S, a.sys.M_I, o, nn, kpar);
-      double2 res[6];
-      for (int e = 0; e < 6; ++e) res[e] = cmk(0.0, 0.0);
-      const int lf = (o.y < 0.0) ? 2 : ((o.y == 0.0) ? 1 : 0);
-      bool rows = lf > 0;
-      if (lf > 0 && S.lmom) {
-        // factorised rows: valid when the row deviation |delta_i(p')| <= 1e-5
-        // for p' = p, p +- dppar (second-order remainder <= 1.7e-16); the
-        // bound in FP32 with a margin (an item just inside it takes the rows)
-        const double2 p = cmk(g.pr, g.pi);
-        const float ap = sqrtf(fmaf((float)p.x, (float)p.x, (float)p.y * (float)p.y)) * 1.00001f + (float)S.dppar_abs;
-        const float bound = fmaf(fmaf(S.la32, ap, S.lb32), ap, S.lc32);
-        if (bound <= 0.999e-5f) {
-          rows = false;
-          // Row Gaussian G(x) = exp(-p2r (x - p3r)^2) at x = p, p +- dppar:
-          // G(p +- pd) = lgc G(p) X^{+-1}, X = exp(-2 p2r pd (p - p3r)).  In
-          // double-float with powers of two kept apart: G(p) = 2^k0 g0,
-          // X = 2^kx xm.  With P_F, Q_F the moment polynomials of family F,
-          //   Spar  = (G(p+pd) P_F(p+pd) - G(p-pd) P_F(p-pd)) / (2 pd)
-          //         = lgc/(2 pd) G(p) (X P_F(p+pd) - X^-1 P_F(p-pd)),
-          //   Sperp = G(p) Q_F(p),
-          //   sum_F = (q/|k_par|) (kappa Spar + (omega - kappa p) Sperp).
-          const double dx = p.x - S.p3r, dy = p.y;
-          int k0, kx;
-          dflt c0, s0, cx, sx;
-          const dflt m0 = df_exp_scaled(-S.p2r * ((dx - dy) * (dx + dy)), k0);
-          df_cis(-2.0 * S.p2r * dx * dy, c0, s0);
-          const dflt mx = df_exp_scaled(S.lcx * dx, kx);
-          df_cis(S.lcx * dy, cx, sx);
-          // an underflowing Gaussian (|G| min_a0 below the FP64 range at any
-          // of the three points) leaves the term zero, as in FP64
-          const int akx = kx < 0 ? -kx : kx;
-          const bool zero = (k0 + S.lze < -1072) || (k0 - akx + S.lge + S.lze < -1072);
-          if (!zero) {
-            const cdf g0 = {df_mul(m0, c0), df_mul(m0, s0)};
-            const cdf xm = {df_mul(mx, cx), df_mul(mx, sx)};
-            const dflt ixm = df_rcp_approx(mx);
-            const cdf xi = {df_mul(ixm, cx), df_neg(df_mul(ixm, sx))};
-            // X P+ - X^-1 P- = 2^|kx| (a P+ - b P-): (a, b) = (xm, 2^-2kx xi)
-            // for kx >= 0, (2^2kx xm, xi) otherwise (a term below 2^-126 of
-            // the other is dropped)
-            const int sh = 2 * akx;
-            const float sc = sh <= 126 ? ldexpf(1.0f, -sh) : 0.0f;
-            const cdf fa = kx >= 0 ? xm : cdf{df_scale(xm.x, sc), df_scale(xm.y, sc)};
-            const cdf fb = kx >= 0 ? cdf{df_scale(xi.x, sc), df_scale(xi.y, sc)} : xi;
-            const cdf pz = {df_of(p.x), df_of(p.y)};
-            const dflt pdd = df_of(S.dppar_abs);
-            // powers 1..4 of p + pd, p - pd and p
-            cdf zp[3][5];
-            zp[0][1] = {df_add(pz.x, pdd), pz.y};
-            zp[1][1] = {df_add(pz.x, df_neg(pdd)), pz.y};
-            zp[2][1] = pz;
-#pragma unroll
-            for (int u = 0; u < 3; ++u) {
-              zp[u][2] = cdf_mul(zp[u][1], zp[u][1]);
-              zp[u][3] = cdf_mul(zp[u][2], zp[u][1]);
-              zp[u][4] = cdf_mul(zp[u][2], zp[u][2]);
-            }
-            // sum_m c_m z^m, c real (float pairs at c[m], c[10 + m])
-            auto poly = [&](const float* c, int u) {
-              cdf acc = {{c[0], c[10]}, {0.0f, 0.0f}};
-#pragma unroll
-              for (int m = 1; m < 5; ++m) {
-                const dflt cm = {c[m], c[10 + m]};
-                acc = cdf_add(acc, cdf_rmul(zp[u][m], cm));
-              }
-              return acc;
-            };
-            const cdf omd = {df_of(o.x), df_of(o.y)};
-            // q / |k_par| (the sign of the charge stays)
-            const dflt kapd = df_of(S.kappa), qld = df_of(kpar < 0.0 ? -S.qk : S.qk);
-            const cdf wk = {df_add(omd.x, df_neg(df_mul(kapd, pz.x))), df_add(omd.y, df_neg(df_mul(kapd, pz.y)))};
-            // lgc / (2 pd) and the factor 2^-|kx| of Sperp against Spar
-            const dflt lgd = df_mul({S.lgch, S.lgcl}, df_rcp_approx(df_scale(pdd, 2.0f)));
-            const float sp = akx <= 126 ? ldexpf(1.0f, -akx) : 0.0f;
-            cdf sumF[3];
-            int eF[3];
-#pragma unroll
-            for (int F = 0; F < 3; ++F) {
-              const float* lm = S.lmomf + ((size_t)n * 3 + F) * 24;
-              const cdf Pp = poly(lm, 0), Pm = poly(lm, 1);
-              const cdf Qp = poly(lm + 5, 2);
-              const cdf br = {df_add(cdf_mul(fa, Pp).x, df_neg(cdf_mul(fb, Pm).x)),
-                              df_add(cdf_mul(fa, Pp).y, df_neg(cdf_mul(fb, Pm).y))};
-              const cdf spar = cdf_rmul(cdf_mul(g0, br), lgd);
-              const cdf sperp = cdf_mul(cdf_mul(g0, Qp), wk);
-              const cdf t = {df_add(df_mul(spar.x, kapd), df_scale(sperp.x, sp)),
-                             df_add(df_mul(spar.y, kapd), df_scale(sperp.y, sp))};
-              sumF[F] = cdf_rmul(t, qld);
-              eF[F] = k0 + akx + (int)lm[20];
-            }
-            // res_e = pref_e c_e sum_F(e) ifac, c_e = 1, p or p^2; ifac =
-            // -i dpperp 2 pi^2 lf, pref_e real (imaginary for xy, yz)
-            const cdf p2 = cdf_mul(pz, pz);
-            const double fi = -S.dpperp * ALPS_PI * 2.0 * ALPS_PI * (double)lf;
-#pragma unroll
-            for (int e = 0; e < 6; ++e) {
-              const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
-              cdf v = sumF[fam];
-              if (e == 2) v = cdf_mul(v, p2);
-              else if (e == 4 || e == 5) v = cdf_mul(v, pz);
-              // pref ifac: real pref -> i (pref fi); imaginary i pref.y -> -(pref.y fi)
-              const bool im = (e == 3 || e == 5);
-              const dflt f = df_of(im ? -pref[e].y * fi : pref[e].x * fi);
-              const double vx = df_val(df_mul(v.x, f)), vy = df_val(df_mul(v.y, f));
-              // multiply by i for a real prefactor: (x, y) -> (-y, x)
-              res[e] = im ? cmk(ldexp(vx, eF[fam]), ldexp(vy, eF[fam])) : cmk(ldexp(-vy, eF[fam]), ldexp(vx, eF[fam]));
-            }
-          }
-        }
-      }
-      work = ((g.kind == 3) ? 1 : 0) | (rows ? 2 : 0);
-      double2* out = items + item * 6;
-      for (int e = 0; e < 6; ++e) {
-        const bool skip = (n == 0 && (e == 0 || e == 3 || e == 4));
-        out[e] = skip ? cmk(0.0, 0.0) : res[e];
-      }
-      ResItem& it = ri[lane];
-      it.pr = g.pr;
-      it.pim = g.pi;
-      it.lower = g.lower;
-      it.upper = g.upper;
-      it.nn = nn;
-      it.work = work | (lf << 2);
-      it.w = w;
-      it.s = s;
-      it.slot = item;
-      for (int e = 0; e < 6; ++e) it.pref[e] = (e == 3 || e == 5) ? pref[e].y : pref[e].x;
-      pv_constants(a, S, g, it);
-    }
+  if (item >= 0) {
+    const int u = (int)(item / a.rcap), s = u % S_, w = u / S_;
+    const SpecDev& S = a.sp[s];
+    const int sv = slot_nn[item], nn = list ? (int)(short)(sv & 0xffff) : sv;
+    const double2 o = om[w];
+    ResItem& it = ri[lane];
+    double2 res[6];
+    double pref[6];
+    PvItem pv;
+    int lf;
+    work = res_item(a, S, o, nn, pv, pref, res, lf);
+    double2* out = items + item * 6;
+    if (list) work &= (sv >> 16) & 3;  // the FP64 sums and the rows (never the double-float sums)
+    else
+      for (int e = 0; e < 6; ++e) out[e] = res[e];
+    it.pv = pv;
+    it.work = work | (lf << 3);
+    it.w = w;
+    it.s = s;
+    it.slot = item;
+    for (int e = 0; e < 6; ++e) it.pref[e] = pref[e];
   }
   __syncwarp();
 
   // ---- one item per warp: the principal-value sums and the Landau rows ----
-  unsigned pend = __ballot_sync(0xffffffffu, work != 0);
+  unsigned pend = __ballot_sync(FULL_WARP, (work & 3) != 0);
   while (pend) {
     const int il = __ffs(pend) - 1;
     pend &= pend - 1;
     const ResItem& it = ri[il];
-    const int s = it.s, w = it.w, nn = it.nn;
+    const int s = it.s, w = it.w, nn = it.pv.nn;
     const int n = nn < 0 ? -nn : nn;
-    const int wk = it.work & 3, lf = it.work >> 2;
+    const int wkk = it.work & 7, lf = it.work >> 3;
     const SpecDev& S = a.sp[s];
     const double2 o = om[w];
-    const int M = S.M;
-    const double kpar = a.sys.kpar, kappa = S.kappa;
-    const double* Vn = S.V + (size_t)n * (M - 1) * 12;
+    const double kpar = a.sys.kpar;
     double2* out = items + it.slot * 6;
 
-    // ---- principal value window (case 3) ----
-    if (wk & 1) {
-      const double pr = it.pr, pim = it.pim;
-      const double dpa = S.dppar_abs, dps = S.dppar;
-      const int jw0 = max(1, it.lower - 2), jw1 = min(M - 1, it.upper + 2);
-      const int nw = jw1 - jw0 + 1;
-      const bool winok = nw <= W;
-      double2 T[6];
-      for (int e = 0; e < 6; ++e) T[e] = cmk(0.0, 0.0);
-      // the fast path's double-float sums; the FP64 code below otherwise
-      const bool fast = S.df_sums && winok && pv_fast(a, S, it, o, n, W, reinterpret_cast<float4*>(wh), pvv, out);
-      if (!fast) {
-      if (winok) {
-        for (int t = lane; t < nw * 6; t += 32) {
-          int jj = t / 6, e = t % 6;
-          wh[jj * 6 + e] = h_node(Vn, jw0 + jj, e, o, kappa);
-        }
-        __syncwarp();
-        for (int t = lane; t < nw * 6; t += 32) {
-          int jj = t / 6, e = t % 6;
-          if (jj >= 1 && jj + 1 < nw) ws[jj * 6 + e] = cscale(csub(wh[(jj + 1) * 6 + e], wh[(jj - 1) * 6 + e]), S.hidpa);
-        }
-      }
-      __syncwarp();
-      // funct_g summed over iperp (src/ALPS_fns.f90:1243-1321): the node whose
-      // interpolant serves p is "the last ipar in 1..npar-1 with
-      // |pp(ipar) - p| <= dppar/2", clamped to 2..npar-2
-      const double idpa = fabs(S.idppar), half = 0.5 * dpa;
-      // last node in 1..M-1 within half a spacing of p, or 0 (the search of
-      // funct_g before its clamp); the candidates bracket the nearest node
-      auto piece_raw = [&](double p) {
-        int jr = 0;
-        double jd = floor((p - S.ppar[0]) * idpa + 0.5);
-        if (jd > -10.0 && jd < (double)M + 10.0) {
-          int j0 = (int)jd;
-          int hi = min(j0 + 2, M - 1), lo = max(j0 - 2, 1);
-          for (int jj = hi; jj >= lo; --jj)
-            if (fabs(S.ppar[jj] - p) <= half) { jr = jj; break; }
-        }
-        return jr;
-      };
-      auto clampj = [&](int jr) { return (jr >= M - 1) ? M - 2 : ((jr <= 1) ? 2 : jr); };
-      // the same search from u, an FP32 estimate of p in node units (node j
-      // at u = j).  Away from the half-way points between nodes by more than
-      // 1e-3 of a spacing, the nearest node is the search's answer: u's
-      // rounding is below 1e-4 of a spacing, and alps_set_species admits
-      // only grids whose steps agree to 1e-9, so a node is within 1e-6 of a
-      // spacing of its uniform position.  Nearer the half-way points the
-      // FP64 search decides.
-      auto off_half = [&](float u) { return fabsf(u - rintf(u)) < 0.499f; };
-      auto node_of = [&](float u) {
-        const int j = (int)rintf(u);
-        return (j >= 1 && j <= M - 1) ? j : 0;
-      };
-      auto piece = [&](double p) { return clampj(piece_raw(p)); };
-      // the same index for p increasing (up) or decreasing (down) from a known
-      // raw index: |pp(j) - p| is monotone in p, so the last valid node moves
-      // by single steps
-      auto piece_up = [&](int jr, double p) {
-        if (jr == 0) return piece_raw(p);
-        while (jr < M - 1 && fabs(S.ppar[jr + 1] - p) <= half) ++jr;
-        return (fabs(S.ppar[jr] - p) <= half) ? jr : piece_raw(p);
-      };
-      auto piece_down = [&](int jr, double p) {
-        if (jr == 0) return piece_raw(p);
-        while (jr >= 1 && !(fabs(S.ppar[jr] - p) <= half)) --jr;
-        return (jr >= 1) ? jr : piece_raw(p);
-      };
-      // node value h and centred slope s of entry e at node jc
-      auto node1 = [&](int jc, int e, double2& h, double2& sl) {
-        if (winok && jc - 1 >= jw0 && jc + 1 <= jw1) {
-          h = wh[(jc - jw0) * 6 + e];
-          sl = ws[(jc - jw0) * 6 + e];
-        } else {
-          h = h_node(Vn, jc, e, o, kappa);
-          sl = cscale(csub(h_node(Vn, jc + 1, e, o, kappa), h_node(Vn, jc - 1, e, o, kappa)), S.hidpa);
-        }
-      };
-      auto node = [&](int jc, double2* h, double2* sl) {
-  #pragma unroll
-        for (int e = 0; e < 6; ++e) node1(jc, e, h[e], sl[e]);
-      };
-      const double capDelta = pr - S.ppar[it.lower];
-      const double smdelta = capDelta / (1.0 * a.sys.M_P);
-      const bool sym = fabs(pim) > a.sys.Tlim;
-      const int NP = a.sys.M_P + 1;
-      // tiny rest between pr + capDelta and ppar[upper]
-      const int ntiny = (int)((S.ppar[it.upper] - pr - capDelta) / smdelta);
-      const double corr = (ntiny > 0) ? ((S.ppar[it.upper] - pr - capDelta) / (1.0 * ntiny)) / smdelta : 0.0;
-      // the sample points: k in 0..M_P of the symmetric sum (group 0 direct,
-      // group 1 mirrored), k in 0..ntiny of the tiny rest (group 2).  Their
-      // coordinates are rounded as integrate_res writes them, without fused
-      // multiply-adds: a point can sit exactly on a piece boundary
-      // pp(j) + dppar/2, and its piece must be the reference's.
-      auto sym_point = [&](int k, double& p, double& dx, double2& K) {
-        p = (k == 0) ? pr
-                     : ((k == a.sys.M_P) ? __dadd_rn(pr, capDelta) : __dadd_rn(pr, __dmul_rn(smdelta, (double)k)));
-        double wk = (k == 0 || k == a.sys.M_P) ? 1.0 : 2.0;
-        dx = p - pr;
-        double rr = wk * rcp_fast(fma(dx, dx, pim * pim));
-        K = cmk(dx * rr, pim * rr);
-      };
-      auto tiny_point = [&](int k, double& p, double& dx, double2& K) {
-        p = (k == 0) ? __dadd_rn(pr, capDelta)
-                     : __dadd_rn(__dadd_rn(pr, capDelta), __dmul_rn(__dmul_rn(corr, smdelta), (double)k));
-        double wk = (k == 0 || k == ntiny) ? 1.0 : 2.0;
-        dx = p - pr;
-        double rr = wk * corr * rcp_fast(fma(dx, dx, pim * pim));
-        K = cmk(dx * rr, pim * rr);
-      };
-
-      // Sum_k c_k H(p_k) with H linear on each piece jc needs, per piece, only
-      // A = Sum c_k and B = Sum c_k (p_k - pp(jc)) = C + (p_res - pp(jc)) A,
-      // C = Sum c_k (p_k - p_res); the piece adds h A + s B.
-      // Each lane walks a run of consecutive k and keeps the sums of at most
-      // two pieces (pieces are M_P/(M_I+1) or more points wide, far wider
-      // than a lane's run); the lanes' piece sums are merged per piece in
-      // shared memory in lane order, and each (piece, entry) pair is then one
-      // thread's h A + s B.  A lane that meets a third piece, or indices that
-      // are not monotone in k, send the item to the per-lane flush below.
-      struct PvSlot {
-        int jd, jc;          // finished piece (-1: none), current piece
-        double2 Ad, Bd, Ac, Bc;  // A and C of each
-      };
-      bool bad = false;
-      auto put = [&](PvSlot& q, int j, double dx, double2 c, int dir) {
-        if (j != q.jc) {
-          if (q.jc >= 0) {
-            if (q.jd >= 0 || (dir > 0 ? j < q.jc : j > q.jc)) bad = true;
-            q.jd = q.jc;
-            q.Ad = q.Ac;
-            q.Bd = q.Bc;
-          }
-          q.jc = j;
-          q.Ac = q.Bc = cmk(0.0, 0.0);
-        }
-        q.Ac = cadd(q.Ac, c);
-        q.Bc = cmk(fma(c.x, dx, q.Bc.x), fma(c.y, dx, q.Bc.y));
-      };
-      int* recj = reinterpret_cast<int*>(pvv + PV_RECV + PV_RUNV);  // (group, lane, slot) piece
-      int* runL = recj + PV_GROUPS * 64;                               // run start lane
-      int* runS = runL + 32;                                           // run start slot
-      int* runG = runS + 32;                                           // run group
-      int* runJ = runG + 32;                                           // run piece
-      double2* recv = pvv;                                             // (group, lane, slot) A, B
-      double2* runv = pvv + PV_RECV;                                   // run A, B
-      int nruns = 0, nl[PV_GROUPS] = {0, 0, 0};
-      // a lane's two pieces to shared memory; run starts get ids in
-      // (lane, slot) order after the runs of the earlier groups
-      auto records = [&](int gi, const PvSlot& q, int dir) {
-        const int j0 = (q.jd >= 0) ? q.jd : q.jc, j1 = (q.jd >= 0) ? q.jc : -1;
-        recj[recj_at(gi, lane, 0)] = j0;
-        recj[recj_at(gi, lane, 1)] = j1;
-        recv[rec_at(gi, lane, 0, 0)] = (q.jd >= 0) ? q.Ad : q.Ac;
-        recv[rec_at(gi, lane, 0, 1)] = (q.jd >= 0) ? q.Bd : q.Bc;
-        recv[rec_at(gi, lane, 1, 0)] = (q.jd >= 0) ? q.Ac : cmk(0.0, 0.0);
-        recv[rec_at(gi, lane, 1, 1)] = (q.jd >= 0) ? q.Bc : cmk(0.0, 0.0);
-        const int last = (j1 >= 0) ? j1 : j0;
-        const int prev = __shfl_up_sync(0xffffffffu, last, 1);
-        const bool st0 = (j0 >= 0) && (lane == 0 || j0 != prev);
-        const bool st1 = (j1 >= 0);
-        if (j0 >= 0 && lane > 0 && (prev < 0 || (dir > 0 ? j0 < prev : j0 > prev))) bad = true;
-        const unsigned m0 = __ballot_sync(0xffffffffu, st0), m1 = __ballot_sync(0xffffffffu, st1);
-        const unsigned lt = (1u << lane) - 1u;
-        const int nr = __popc(m0) + __popc(m1);
-        if (nruns + nr <= 32) {
-          const int id0 = nruns + __popc(m0 & lt) + __popc(m1 & lt), id1 = id0 + (st0 ? 1 : 0);
-          if (st0) {
-            runL[id0] = lane;
-            runS[id0] = 0;
-            runG[id0] = gi;
-          }
-          if (st1) {
-            runL[id1] = lane;
-            runS[id1] = 1;
-            runG[id1] = gi;
-          }
-        }
-        nruns += nr;
-        nl[gi] = __popc(__ballot_sync(0xffffffffu, j0 >= 0));
-      };
-      // Fast path: the sample sums in double-float arithmetic on the FP32
-      // pipes (about 46 bits; the pieces are still found from the FP64
-      // sample points).  Used where every pair stays a normal float: spacing,
-      // window and |p_im| within 1e-12 .. 1e12.
-      auto inr = [](double x) { return x >= 1e-12 && x <= 1e12; };
-      const bool dfsym = S.df_sums && inr(smdelta) && inr(capDelta) && inr(fabs(pim));
-      const bool dftiny = S.df_sums && inr(capDelta) && inr(corr * smdelta) && fabs(pim) <= 1e12;
-      struct PvSlotF {
-        int jd, jc;
-        dflt Adx, Ady, Bdx, Bdy, Acx, Acy, Bcx, Bcy;
-      };
-      const dflt z0 = {0.0f, 0.0f};
-      auto putf = [&](PvSlotF& q, int j, dflt dx, dflt cx, dflt cy, int dir) {
-        if (j != q.jc) {
-          if (q.jc >= 0) {
-            if (q.jd >= 0 || (dir > 0 ? j < q.jc : j > q.jc)) bad = true;
-            q.jd = q.jc;
-            q.Adx = q.Acx;
-            q.Ady = q.Acy;
-            q.Bdx = q.Bcx;
-            q.Bdy = q.Bcy;
-          }
-          q.jc = j;
-          q.Acx = q.Acy = q.Bcx = q.Bcy = z0;
-        }
-        df_acc(q.Acx, cx);
-        df_acc(q.Acy, cy);
-        df_mac(q.Bcx, cx.h, cx.l, dx);
-        df_mac(q.Bcy, cy.h, cy.l, dx);
-      };
-      auto to64 = [&](const PvSlotF& q) {
-        PvSlot r;
-        r.jd = q.jd;
-        r.jc = q.jc;
-        r.Ad = cmk(df_val(q.Adx), df_val(q.Ady));
-        r.Bd = cmk(df_val(q.Bdx), df_val(q.Bdy));
-        r.Ac = cmk(df_val(q.Acx), df_val(q.Acy));
-        r.Bc = cmk(df_val(q.Bcx), df_val(q.Bcy));
-        return r;
-      };
-      // the sample points as integrate_res writes them (for the FP64 search)
-      auto sym_p = [&](int k) {
-        return (k == 0) ? pr
-                        : ((k == a.sys.M_P) ? __dadd_rn(pr, capDelta) : __dadd_rn(pr, __dmul_rn(smdelta, (double)k)));
-      };
-      auto tiny_p = [&](int k) {
-        return (k == 0) ? __dadd_rn(pr, capDelta)
-                        : __dadd_rn(__dadd_rn(pr, capDelta), __dmul_rn(__dmul_rn(corr, smdelta), (double)k));
-      };
-      if (sym && dfsym) {
-        const int per = (NP + 31) / 32;
-        const int k0 = lane * per, k1 = min(NP, k0 + per);
-        PvSlotF su{-1, -1, z0, z0, z0, z0, z0, z0, z0, z0}, sd = su;
-        const float u0 = (float)(1.0 + (pr - S.ppar[1]) * S.idppar), du = (float)(smdelta * S.idppar);
-        const dflt smd = df_of(smdelta), capd = df_of(capDelta), pimd = df_of(pim), pim2 = df_of(pim * pim);
-        for (int k = k0; k < k1; ++k) {
-          // K = w (dx, p_im) / (dx^2 + p_im^2), dx = p_k - p_res
-          const dflt dx = (k == a.sys.M_P) ? capd : df_mul(smd, {(float)k, 0.0f});
-          const dflt r = df_scale(df_rcp_approx(df_add(df_mul(dx, dx), pim2)),
-                                  (k == 0 || k == a.sys.M_P) ? 1.0f : 2.0f);
-          const dflt Kx = df_mul(dx, r), Ky = df_mul(pimd, r);
-          const float uu = fmaf((float)k, du, u0), ud = fmaf(-(float)k, du, u0);
-          const int cu = clampj(off_half(uu) ? node_of(uu) : piece_raw(sym_p(k)));
-          const int cd = clampj(off_half(ud) ? node_of(ud) : piece_raw(2.0 * pr - sym_p(k)));
-          putf(su, cu, dx, Kx, Ky, 1);
-          putf(sd, cd, df_neg(dx), Kx, df_neg(Ky), -1);
-        }
-        records(0, to64(su), 1);
-        records(1, to64(sd), -1);
-      } else if (sym) {
-        const int per = (NP + 31) / 32;
-        const int k0 = lane * per, k1 = min(NP, k0 + per);
-        PvSlot su{-1, -1, cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)}, sd = su;
-        const float u0 = (float)(1.0 + (pr - S.ppar[1]) * S.idppar), du = (float)(smdelta * S.idppar);
-        for (int k = k0; k < k1; ++k) {
-          double p, dx;
-          double2 K;
-          sym_point(k, p, dx, K);
-          const float uu = fmaf((float)k, du, u0), ud = fmaf(-(float)k, du, u0);
-          const int cu = clampj(off_half(uu) ? node_of(uu) : piece_raw(p));
-          const int cd = clampj(off_half(ud) ? node_of(ud) : piece_raw(2.0 * pr - p));
-          put(su, cu, dx, K, 1);
-          put(sd, cd, -dx, cmk(K.x, -K.y), -1);
-        }
-        records(0, su, 1);
-        records(1, sd, -1);
-      } else {
-        // Tlim branch: g' * sum_k w_k (p-pr)^2/((p-pr)^2+pim^2) + sign(pim) i pi G(pr)/smdelta
-        double fr = 0.0;
-        for (int k = 1 + lane; k <= a.sys.M_P; k += 32) {
-          double p = (k == a.sys.M_P) ? __dadd_rn(pr, capDelta) : __dadd_rn(pr, __dmul_rn(smdelta, (double)k));
-          double wk = (k == a.sys.M_P) ? 1.0 : 2.0;
-          double d = p - pr;
-          fr += wk * ((d * d) / (d * d + pim * pim));
-        }
-        for (int off = 16; off > 0; off >>= 1) fr += __shfl_xor_sync(0xffffffffu, fr, off);
-        // entry e on lane e, then T (on lane 0, as the other branches leave it)
-        double2 Te = cmk(0.0, 0.0);
-        if (lane < 6) {
-          const int e = lane;
-          auto Hc1 = [&](double p) {
-            const int jc = piece(p);
-            double2 h, sl;
-            node1(jc, e, h, sl);
-            const double dx = p - S.ppar[jc];
-            return cmk(fma(sl.x, dx, h.x), fma(sl.y, dx, h.y));
-          };
-          const double2 H1 = Hc1(pr + dps), H2 = Hc1(pr - dps), H0 = Hc1(pr);
-          double sgn = (pim > 0.0) ? 1.0 : ((pim < 0.0) ? -1.0 : 0.0);
-          double2 gp = cscale(csub(H1, H2), 1.0 / (2.0 * dps));
-          Te = cadd(cscale(gp, 2.0 * fr), cmul(cmk(0.0, sgn * 2.0 * ALPS_PI / smdelta), H0));
-        }
-  #pragma unroll
-        for (int e = 0; e < 6; ++e) {
-          const double tx = __shfl_sync(0xffffffffu, Te.x, e), ty = __shfl_sync(0xffffffffu, Te.y, e);
-          if (lane == 0) T[e] = cmk(tx, ty);
-        }
-      }
-      if (ntiny > 0 && dftiny) {
-        const int per = (ntiny + 1 + 31) / 32;
-        const int k0 = lane * per, k1 = min(ntiny + 1, k0 + per);
-        PvSlotF sq{-1, -1, z0, z0, z0, z0, z0, z0, z0, z0};
-        const float ut0 = (float)(1.0 + (pr + capDelta - S.ppar[1]) * S.idppar), dut = (float)(corr * smdelta * S.idppar);
-        const dflt capd = df_of(capDelta), csd = df_of(__dmul_rn(corr, smdelta)), cord = df_of(corr),
-                   pimd = df_of(pim), pim2 = df_of(pim * pim);
-        for (int k = k0; k < k1; ++k) {
-          // K = w corr (dx, p_im) / (dx^2 + p_im^2)
-          const dflt dx = (k == 0) ? capd : df_add(capd, df_mul(csd, {(float)k, 0.0f}));
-          const dflt r = df_scale(df_mul(df_rcp_approx(df_add(df_mul(dx, dx), pim2)), cord),
-                                  (k == 0 || k == ntiny) ? 1.0f : 2.0f);
-          const dflt Kx = df_mul(dx, r), Ky = df_mul(pimd, r);
-          const float ut = fmaf((float)k, dut, ut0);
-          const int ct = clampj(off_half(ut) ? node_of(ut) : piece_raw(tiny_p(k)));
-          putf(sq, ct, dx, Kx, Ky, 1);
-        }
-        records(2, to64(sq), 1);
-      } else if (ntiny > 0) {
-        const int per = (ntiny + 1 + 31) / 32;
-        const int k0 = lane * per, k1 = min(ntiny + 1, k0 + per);
-        PvSlot sq{-1, -1, cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-        const float ut0 = (float)(1.0 + (pr + capDelta - S.ppar[1]) * S.idppar), dut = (float)(corr * smdelta * S.idppar);
-        for (int k = k0; k < k1; ++k) {
-          double p, dx;
-          double2 K;
-          tiny_point(k, p, dx, K);
-          const float ut = fmaf((float)k, dut, ut0);
-          const int ct = clampj(off_half(ut) ? node_of(ut) : piece_raw(p));
-          put(sq, ct, dx, K, 1);
-        }
-        records(2, sq, 1);
-      }
-      const bool merged = !__any_sync(0xffffffffu, bad) && nruns <= 32;
-      if (merged && nruns > 0) {
-        __syncwarp();
-        // run totals in (lane, slot) order: the run's first slot, then slot 0
-        // of the following lanes up to the next run start of its group
-        if (lane < nruns) {
-          const int L = runL[lane], sl = runS[lane], gi = runG[lane];
-          int Ln = nl[0], sn = 0;
-          if (gi == 1) Ln = nl[1];
-          if (gi == 2) Ln = nl[2];
-          if (lane + 1 < nruns && runG[lane + 1] == gi) {
-            Ln = runL[lane + 1];
-            sn = runS[lane + 1];
-          }
-          double2 A = recv[rec_at(gi, L, sl, 0)], B = recv[rec_at(gi, L, sl, 1)];
-          for (int L2 = L + 1; L2 < Ln || (L2 == Ln && sn == 1); ++L2) {
-            A = cadd(A, recv[rec_at(gi, L2, 0, 0)]);
-            B = cadd(B, recv[rec_at(gi, L2, 0, 1)]);
-          }
-          runJ[lane] = recj[recj_at(gi, L, sl)];
-          runv[lane * 2] = A;
-          runv[lane * 2 + 1] = B;
-        }
-        __syncwarp();
-        // (run, entry) pairs: h A + s B, mirrored runs with the minus sign;
-        // the products overwrite the lane records
-        double2* contrib = recv;
-        for (int q = lane; q < nruns * 6; q += 32) {
-          const int rho = q / 6, e = q % 6;
-          const int jc = runJ[rho];
-          double2 h, sl;
-          node1(jc, e, h, sl);
-          const double2 A = runv[rho * 2];
-          const double2 B = cadd(runv[rho * 2 + 1], cscale(A, pr - S.ppar[jc]));
-          double2 t = cadd(cmul(h, A), cmul(sl, B));
-          contrib[q] = (runG[rho] == 1) ? cmk(-t.x, -t.y) : t;
-        }
-        __syncwarp();
-        // component c of T: the runs in order
-        double acc = 0.0;
-        if (lane < 12) {
-          const int e = lane >> 1;
-          for (int rho = 0; rho < nruns; ++rho) acc += (lane & 1) ? contrib[rho * 6 + e].y : contrib[rho * 6 + e].x;
-        }
-  #pragma unroll
-        for (int e = 0; e < 6; ++e) {
-          const double tx = __shfl_sync(0xffffffffu, acc, 2 * e), ty = __shfl_sync(0xffffffffu, acc, 2 * e + 1);
-          T[e] = cadd(T[e], cmk(tx, ty));
-        }
-      } else if (!merged) {
-        // per-lane piece sums flushed as the piece changes, then a warp sum
-        struct Acc {
-          int jc;
-          double2 A, B;
-        };
-        auto flush = [&](Acc& q, double sign) {
-          if (q.jc < 0) return;
-          double2 h[6], sl[6];
-          node(q.jc, h, sl);
-  #pragma unroll
-          for (int e = 0; e < 6; ++e) {
-            double2 t = cadd(cmul(h[e], q.A), cmul(sl[e], q.B));
-            T[e] = cmk(fma(sign, t.x, T[e].x), fma(sign, t.y, T[e].y));
-          }
-          q.A = q.B = cmk(0.0, 0.0);
-        };
-        auto add = [&](Acc& q, int jc, double p, double2 c, double sign) {
-          if (jc != q.jc) {
-            flush(q, sign);
-            q.jc = jc;
-          }
-          double dx = p - S.ppar[jc];
-          q.A = cadd(q.A, c);
-          q.B = cmk(fma(c.x, dx, q.B.x), fma(c.y, dx, q.B.y));
-        };
-        if (sym) {
-          const int per = (NP + 31) / 32;
-          const int k0 = lane * per, k1 = min(NP, k0 + per);
-          Acc up{-1, cmk(0, 0), cmk(0, 0)}, dn{-1, cmk(0, 0), cmk(0, 0)};
-          int ju = -1, jd = -1;
-          for (int k = k0; k < k1; ++k) {
-            double p, dx;
-            double2 K;
-            sym_point(k, p, dx, K);
-            const double pm = 2.0 * pr - p;
-            ju = (ju < 0) ? piece_raw(p) : piece_up(ju, p);
-            jd = (jd < 0) ? piece_raw(pm) : piece_down(jd, pm);
-            add(up, clampj(ju), p, K, 1.0);
-            add(dn, clampj(jd), pm, cmk(K.x, -K.y), -1.0);
-          }
-          flush(up, 1.0);
-          flush(dn, -1.0);
-        }
-        if (ntiny > 0) {
-          const int per = (ntiny + 1 + 31) / 32;
-          const int k0 = lane * per, k1 = min(ntiny + 1, k0 + per);
-          Acc q{-1, cmk(0, 0), cmk(0, 0)};
-          int jt = -1;
-          for (int k = k0; k < k1; ++k) {
-            double p, dx;
-            double2 K;
-            tiny_point(k, p, dx, K);
-            jt = (jt < 0) ? piece_raw(p) : piece_up(jt, p);
-            add(q, clampj(jt), p, K, 1.0);
-          }
-          flush(q, 1.0);
-        }
-        for (int e = 0; e < 6; ++e)
-          for (int off = 16; off > 0; off >>= 1) {
-            T[e].x += __shfl_xor_sync(0xffffffffu, T[e].x, off);
-            T[e].y += __shfl_xor_sync(0xffffffffu, T[e].y, off);
-          }
-      }
-      // G = K_e H with K_e = -(q/kpar) pref_e / 2; result 2 pi T smdelta dpperp/4
-      double scale = 2.0 * ALPS_PI * smdelta * S.dpperp * 0.25 * (-S.qk * 0.5);
-      // lane 0 holds the whole T; lanes 0-5 add entry e
-      if (lane == 0)
-        for (int e = 0; e < 6; ++e) tb[e] = T[e];
-      __syncwarp();
-      if (lane < 6 && !(n == 0 && (lane == 0 || lane == 3 || lane == 4)))
-        out[lane] = cadd(out[lane], cscale(cmul(item_pref(it, lane), tb[lane]), scale));
-      __syncwarp();
-      }  // FP64 code
+    if (wkk & 1) {
+      if (wkk & 4) pv_warp<dflt>(S, a.sys, it.pv, o, it.pref, wk, out);
+      else pv_warp<double>(S, a.sys, it.pv, o, it.pref, wk, out);
     }
 
-    if (wk & 2) {
-      const double2 p = cmk(it.pr, it.pim);
+    if (wkk & 2) {
+      const double2 p = cmk(it.pv.pr, it.pv.pim);
       const double pd = S.dppar_abs, dpp = S.dpperp;
       const double vA = a.sys.vA;
       if (S.fit_aux) {
@@ -2006,7 +1740,9 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
           dfperp = cscale(csub(frow[N], frow[N - 1]), 1.0 / dpp);
           h = 0.5;
         } else {
-          if (cabs_(fpi) == 0.0 || cabs_(fpf) == 0.0 || cabs_(frow[i + 1]) == 0.0) zero = true;
+          // |f| = 0 exactly when both parts are
+          auto nil = [](double2 x) { return x.x == 0.0 && x.y == 0.0; };
+          if (nil(fpi) || nil(fpf) || nil(frow[i + 1])) zero = true;
           dfperp = cscale(csub(frow[i + 1], frow[i - 1]), 1.0 / (2.0 * dpp));
           h = (i == N - 1) ? 0.5 : 1.0;
         }
@@ -2044,17 +1780,271 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
         __syncwarp();
       }
     }
-    __syncwarp();  // the next item reuses the window and the records
+    __syncwarp();  // the next item reuses the region
   }
-      // the items beyond this batch move to the front of the queue
-      const int rest = qn - nb;
-      const int keep = (lane < rest) ? queue[nb + lane] : 0;
-      __syncwarp();
-      if (lane < rest) queue[lane] = keep;
-      __syncwarp();
-      qn = rest;
+      });
+}
+
+// ---------------------------------------------------------------------------
+// One item per lane (mixed path, lattices).  A lane sums its item's samples
+// in turn and leaves the running sums at the cuts in its column of shared
+// memory; the cuts are the bytes of a word per side.  Then it walks the
+// window's nodes, forming each node's weight from the pieces beside it and
+// adding the node's base vectors.  Bound by issue (some 800 warp instructions
+// an item, against 3300 when a warp shared an item's samples and merged its
+// lanes' pieces) and by the instruction cache: the loops over cuts, sample
+// runs, sides and the Landau term's points are kept rolled, which took the
+// kernel from 1847 to 1539 us.  512x512 map, 1.2 M items: 7330 us by warps,
+// 1539 us so; 8192 frequencies 384 and 119 us.
+// ---------------------------------------------------------------------------
+#define PVL_TINY 4  // cuts of the tiny rest at most
+__host__ __device__ inline int pvl_side(int M_I) { return M_I + 3; }  // cuts of a side at most (eight)
+__host__ __device__ inline int pvl_slots(int M_I) { return 2 * pvl_side(M_I) + PVL_TINY; }
+// bytes per block: two float pairs and a weight per cut and lane, the warps' queues
+__host__ __device__ inline size_t pvl_smem(int M_I) {
+  return (size_t)pvl_slots(M_I) * 20 * (RES_WARPS * 32) + RES_WARPS * 64 * sizeof(int);
+}
+// running sums of w r dx, w r and w, half the weights of PvSums
+struct PvRun {
+  dflt s1, s2;
+  float w;
+};
+struct PvCols {
+  float4* a;   // s1, s2 at [slot * 128 + thread]
+  float* b;    // w
+  __device__ __forceinline__ void put(int slot, const PvRun& s) const {
+    a[slot * (RES_WARPS * 32) + threadIdx.x] = make_float4(s.s1.h, s.s1.l, s.s2.h, s.s2.l);
+    b[slot * (RES_WARPS * 32) + threadIdx.x] = s.w;
+  }
+  __device__ __forceinline__ PvRun get(int slot) const {
+    const float4 x = a[slot * (RES_WARPS * 32) + threadIdx.x];
+    return {{x.x, x.y}, {x.z, x.w}, b[slot * (RES_WARPS * 32) + threadIdx.x]};
+  }
+};
+// adds a sample at dx with half its weight, w = 1 or 1/2: r = w / (dx^2 + y2).
+// The pairs stay unnormalised between the steps (low parts below 2^-21 of the
+// high ones), which the sums' error-free additions take: 44 operations.
+__device__ __forceinline__ void pvl_add(PvRun& s, dflt dx, dflt y2, float w) {
+  const float p = __fmul_rn(dx.h, dx.h);
+  const float pl = __fmaf_rn(__fadd_rn(dx.h, dx.h), dx.l, __fmaf_rn(dx.h, dx.h, -p));
+  const dflt d = df_two_sum(p, y2.h);
+  dflt r = df_rcp_approx({d.h, __fadd_rn(d.l, __fadd_rn(pl, y2.l))});
+  if (w != 1.0f) r = df_scale(r, w);
+  const float t = __fmul_rn(dx.h, r.h);
+  const float tl = __fmaf_rn(dx.h, r.l, __fmaf_rn(dx.l, r.h, __fmaf_rn(dx.h, r.h, -t)));
+  df_acc(s.s1, {t, tl});
+  df_acc(s.s2, r);
+  s.w += w;
+}
+__device__ __forceinline__ dflt pvl_times(dflt a, float k) {
+  const float p = __fmul_rn(a.h, k);
+  return df_quick(p, __fmaf_rn(a.l, k, __fmaf_rn(a.h, k, -p)));
+}
+
+// T_e times scale into X (xx yy zz xy xz yz, divided by Vscale[n]); false if
+// the item's shape is not one of the fast form's
+__device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, const PvItem& it, double2 o, PvCols col,
+                                        cdf X[6]) {
+  const int M = S.M, M_P = sys.M_P, n = it.nn < 0 ? -it.nn : it.nn;
+  const int side_max = pvl_side(sys.M_I);
+  const bool sym = fabs(it.pim) > sys.Tlim;
+  // the cuts of the three runs of samples (up, down, tiny rest), a byte each
+  unsigned long long cu = ~0ull, cd = ~0ull, ct = ~0ull;
+  bool ok = M_P < 128 && it.ntiny < 128, lost = it.direct;
+  int nu = 2, nd = 2, nt = 0;  // pieces (without sym: H at p_res and a spacing to either side)
+#pragma unroll 1
+  for (int sd = 0; sd < 3; ++sd) {
+    if (sd == 2 ? it.ntiny <= 0 : !sym) continue;
+    const int K = sd == 2 ? it.ntiny : M_P, most = sd == 2 ? PVL_TINY : side_max;
+    int np = 1, last = 0;
+    unsigned long long pk = ~0ull;
+#pragma unroll 1
+    for (int i = 0; i <= most; ++i) {
+      const int k = pv_cut(S, sys, it, o.x, sd, i, lost);
+      if (k > K) break;
+      ok = ok && k > last && i < most;
+      last = k;
+      np = i + 2;
+      if (i < 8) pk ^= (unsigned long long)(0xff ^ (k & 0xff)) << (8 * i);
+    }
+    if (sd == 0) {
+      cu = pk;
+      nu = np;
+    } else if (sd == 1) {
+      cd = pk;
+      nd = np;
+    } else {
+      ct = pk;
+      nt = np;
     }
   }
+  // (a piece M - 1 takes node M - 2's interpolant)
+  const int jlo = it.j0 - (nd - 1), jtop = max(it.j0 + nu - 1, nt ? it.jt0 + nt - 1 : 0), jhi = min(jtop, M - 2);
+  ok = ok && !lost && jlo >= 2 && jtop <= M - 1;
+  if (!ok) return false;
+  const PvScal<dflt> c = pv_scal<dflt>(it);
+  const dflt z = {0.0f, 0.0f};
+  PvRun end = {z, z, 0.0f}, endt = end;
+#pragma unroll 1
+  for (int rep = 0; rep < (nt ? 2 : 1); ++rep) {  // the window, the tiny rest
+    const int K = rep ? it.ntiny : M_P;
+    const dflt step = rep ? c.csd : c.sm;
+    unsigned long long pa = rep ? ct : cu, pb = rep ? ~0ull : cd;
+    int ia = rep ? 2 * side_max : 0, ib = side_max;
+    PvRun s = {z, z, 0.0f};
+#pragma unroll 1
+    for (int k = (rep || sym) ? 0 : 1; k <= K; ++k) {
+      if ((int)(pa & 0xff) == k && k) {
+        col.put(ia++, s);
+        pa >>= 8;
+      }
+      if ((int)(pb & 0xff) == k && k) {
+        col.put(ib++, s);
+        pb >>= 8;
+      }
+      dflt dx = pvl_times(step, (float)k);
+      if (rep) dx = df_add(c.cap, dx);
+      else if (k == K) dx = c.cap;
+      pvl_add(s, dx, c.y2, (k == 0 || k == K) ? 0.5f : 1.0f);
+    }
+    if (rep) endt = s;
+    else end = s;
+  }
+  // piece j's A and moment B about node j; sums of side sd, run of cuts at
+  // slot b0, piece i of ni, total tot
+  const dflt plo = {S.pph[it.lower], S.ppl[it.lower]};
+  auto part = [&](int sd, int b0, int i, int ni, const PvRun& tot, cdf& A, cdf& C) {
+    PvRun e = (i + 1 < ni) ? col.get(b0 + i) : tot;
+    if (i > 0) {
+      const PvRun b = col.get(b0 + i - 1);
+      e = {df_add(e.s1, df_neg(b.s1)), df_add(e.s2, df_neg(b.s2)), e.w - b.w};
+    } else {
+      e = {df_add(e.s1, z), df_add(e.s2, z), e.w};
+    }
+    // sum of w r dx^2 = sum of w - y^2 sum of w r
+    PvSums<dflt> s = {df_scale(e.s1, 2.0f), df_scale(e.s2, 2.0f), z};
+    s.s3 = df_add({2.0f * e.w, 0.0f}, df_neg(df_mul(c.y2, s.s2)));
+    dflt Ax, Ay, Cx, Cy;
+    pv_moment(s, c, sd, Ax, Ay, Cx, Cy);
+    A = cdf_add(A, {Ax, Ay});
+    C = cdf_add(C, {Cx, Cy});
+  };
+  auto piece = [&](int j, cdf& A, cdf& B) {
+    A = {z, z};
+    cdf C = {z, z};
+#pragma unroll 1
+    for (int jj = j; jj <= (j == jhi ? jtop : j); ++jj) {
+      const int i = jj - it.j0;
+#pragma unroll 1
+      for (int sd = sym ? 0 : 2; sd < 3; ++sd) {
+        const int q = sd == 0 ? i : (sd == 1 ? -i : jj - it.jt0), nq = sd == 0 ? nu : (sd == 1 ? nd : nt);
+        if (q >= 0 && q < nq) part(sd, sd * side_max, q, nq, sd == 2 ? endt : end, A, C);
+      }
+      if (!sym && i >= -1 && i <= 1) {
+        if (i != 0) {
+          // g' sum_k w_k dx^2/(dx^2 + y^2)
+          const dflt s3 = df_add({2.0f * end.w, 0.0f}, df_neg(df_mul(c.y2, df_scale(df_add(end.s2, z), 2.0f))));
+          dflt x = df_mul(s3, {S.idph, S.idpl});
+          if (i < 0) x = df_neg(x);
+          A.x = df_add(A.x, x);
+          C.x = df_add(C.x, df_mul(df_scale({S.dpph, S.dppl}, (float)i), x));
+        } else {
+          const float sgn = (it.pim > 0.0) ? 1.0f : ((it.pim < 0.0) ? -1.0f : 0.0f);
+          A.y = df_add(A.y, df_scale(df_mul({S.tpmh, S.tpml}, df_rcp_approx(c.cap)), sgn));
+        }
+      }
+    }
+    // p_res - p_j = capDelta + (p_lower - p_j)
+    const dflt del = df_add(c.cap, df_add(plo, df_neg({S.pph[j], S.ppl[j]})));
+    B = cdf_add(C, cdf_rmul(A, del));
+  };
+  dflt Sx[24];
+#pragma unroll
+  for (int q = 0; q < 24; ++q) Sx[q] = z;
+  const dflt hid = {S.hidh, S.hidl};
+  cdf Aj = {z, z}, Bp = {z, z}, Bj = {z, z};
+#pragma unroll 1
+  for (int j = jlo - 1; j <= jhi + 1; ++j) {
+    cdf An = {z, z}, Bn = {z, z};
+    if (j + 1 <= jhi) piece(j + 1, An, Bn);
+    // W_j = A_j + (B_{j-1} - B_{j+1}) / (2 dppar)
+    const cdf W = cdf_add(Aj, cdf_rmul({df_add(Bp.x, df_neg(Bn.x)), df_add(Bp.y, df_neg(Bn.y))}, hid));
+    const dflt pj = {S.pph[j], S.ppl[j]};
+    const cdf Wp = cdf_rmul(W, pj), Wpp = cdf_rmul(Wp, pj);
+    const float4* b4 = reinterpret_cast<const float4*>(S.Bt + ((size_t)n * (M - 1) + (j - 1)) * 12);
+    const float4 a0 = __ldg(b4), a1 = __ldg(b4 + 1), a2 = __ldg(b4 + 2);
+    const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+    // entries xx yy zz xy xz yz: vectors (F1, F2, F1 p^2, F3, F1 p, F3 p)
+    auto add = [&](int e, int b, cdf v) {
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        df_mac(Sx[4 * e + 2 * g], hb[b + g], lb[b + g], v.x);
+        df_mac(Sx[4 * e + 2 * g + 1], hb[b + g], lb[b + g], v.y);
+      }
+    };
+    add(0, 0, W);
+    add(1, 2, W);
+    add(2, 0, Wpp);
+    add(3, 4, W);
+    add(4, 0, Wp);
+    add(5, 4, Wp);
+    Bp = Bj;
+    Aj = An;
+    Bj = Bn;
+  }
+  const cdf omd = {it.oxd, it.oyd};
+  const dflt kap = {S.kaph, S.kapl};
+#pragma unroll
+  for (int e = 0; e < 6; ++e)
+    X[e] = om_comb(omd, kap, {df_add(Sx[4 * e], z), df_add(Sx[4 * e + 1], z)},
+                   {df_add(Sx[4 * e + 2], z), df_add(Sx[4 * e + 3], z)});
+  return true;
+}
+
+__device__ __forceinline__ void lanes_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
+                                           int n_om, const int* __restrict__ count, int* slot_nn, double2* items,
+                                           int* flags, long block) {
+  extern __shared__ double2 sm[];
+  const int warp = threadIdx.x / 32, S_ = a.sys.nspec;
+  PvCols col;
+  const int slots = pvl_slots(a.sys.M_I);
+  col.a = reinterpret_cast<float4*>(sm);
+  col.b = reinterpret_cast<float*>(col.a + slots * RES_WARPS * 32);
+  int* queue = reinterpret_cast<int*>(col.b + slots * RES_WARPS * 32) + warp * 64;
+  const long slot0 = (block * RES_WARPS + warp) * (long)sh.lanes;
+  if (slot0 >= (long)n_om * S_ * a.rcap) return;
+  res_batches(
+      a, sh.lanes, n_om, count, slot0, queue, [](long) { return true; },
+      [&](int nb, long item) {
+        if (item >= 0) {
+          const int u = (int)(item / a.rcap), s = u % S_, w = u / S_;
+          const SpecDev& S = a.sp[s];
+          const int nn = slot_nn[item], n = nn < 0 ? -nn : nn;
+          const double2 o = om[w];
+          double2 res[6];
+          double pref[6];
+          PvItem pv;
+          int lf;
+          int work = res_item(a, S, o, nn, pv, pref, res, lf);
+          cdf X[6];
+          if ((work & 5) == 5 && pv_lane(S, a.sys, pv, o, col, X)) {
+            const double scale = S.Vscale[n] * pv.sm * S.pvc;
+#pragma unroll
+            for (int e = 0; e < 6; ++e) {
+              if (n == 0 && (e == 0 || e == 3 || e == 4)) continue;
+              const double f = scale * pref[e], x = df_val(X[e].x) * f, y = df_val(X[e].y) * f;
+              if (e == 3 || e == 5) res[e] = cadd(res[e], cmk(-y, x));
+              else res[e] = cadd(res[e], cmk(x, y));
+            }
+            work &= ~1;
+          }
+          double2* out = items + item * 6;
+#pragma unroll
+          for (int e = 0; e < 6; ++e) out[e] = res[e];
+          slot_nn[item] = todo_slot(nn, work & 3);
+          if (work & 3) atomicOr(flags, FLAG_TODO);
+        }
+      });
 }
 
 // ---------------------------------------------------------------------------
@@ -2285,7 +2275,7 @@ struct DispJob {
   const DispArgs* a;  // the context's arguments (device copy)
   DispShape sh;
   int n, S;
-  long blk[4];        // first block of the job in classify, pole sums, resonant, finalize
+  long blk[5];        // first block of the job in classify, pole sums, resonant, finalize, resonant lanes
   const double2* om;
   double2* D;
   double2* part;
@@ -2391,8 +2381,16 @@ __global__ void __launch_bounds__(128, 3) k_pole_sums_multi(const DispJob* __res
 __global__ void __launch_bounds__(RES_WARPS * 32, 3) k_resonant_multi(const DispJob* __restrict__ jobs, int nj) {
   __shared__ DispArgs sa;
   const DispJob& J = job_of(jobs, nj, blockIdx.x, 2);
+  if (J.sh.lanes && !(*J.flags & FLAG_TODO)) return;
   const DispArgs& a = stage_args(J.a, sa);
   resonant_body(a, J.sh, J.om, J.n, J.count, J.slot_nn, J.items, (long)blockIdx.x - J.blk[2]);
+}
+
+__global__ void __launch_bounds__(RES_WARPS * 32, 3) k_resonant_lanes(const DispJob* __restrict__ jobs, int nj) {
+  __shared__ DispArgs sa;
+  const DispJob& J = job_of(jobs, nj, blockIdx.x, 4);
+  const DispArgs& a = stage_args(J.a, sa);
+  lanes_body(a, J.sh, J.om, J.n, J.count, J.slot_nn, J.items, J.flags, (long)blockIdx.x - J.blk[4]);
 }
 
 __global__ void k_finalize_multi(const DispJob* __restrict__ jobs, int nj) {
@@ -2400,6 +2398,7 @@ __global__ void k_finalize_multi(const DispJob* __restrict__ jobs, int nj) {
   const DispJob& J = job_of(jobs, nj, blockIdx.x, 3);
   const DispArgs& a = stage_args(J.a, sa);
   const long lb = (long)blockIdx.x - J.blk[3];
+  if (J.sh.lanes && lb == 0 && threadIdx.x == 0) atomicAnd(J.flags, ~FLAG_TODO);
   if (J.sh.fin_warp)
     finalize_warp(a, J.sh, J.om, J.n, J.part, J.count, J.slot_nn, J.items, J.rel, J.bm, J.D, J.ext,
                   lb * (blockDim.x / 32) + threadIdx.x / 32);
@@ -2429,11 +2428,17 @@ void fill_sys_dev(const alps_ctx* c, SysDev* o) {
   o->kperp_norm = c->sys.kperp_norm;
   o->M_I = c->sys.positions_principal;
   o->M_P = c->sys.n_resonance_interval;
+  o->iM_P = 1.0 / c->sys.n_resonance_interval;
   o->Tlim = c->sys.Tlim;
   o->vA = c->sys.vA;
   o->kperp = c->kperp;
   o->kpar = c->kpar;
   o->ikpar = 1.0 / c->kpar;
+  const double k1 = c->sys.kperp_norm ? 1.0 : c->kperp, k2 = c->sys.kperp_norm ? 1.0 : c->kperp * c->kperp;
+  o->k1h = (float)k1;
+  o->k1l = (float)(k1 - (double)o->k1h);
+  o->k2h = (float)k2;
+  o->k2l = (float)(k2 - (double)o->k2h);
 }
 
 void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
@@ -2505,6 +2510,16 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
     o->tpmh = (float)tpm;
     o->tpml = (float)(tpm - (double)o->tpmh);
     o->pvc = 2.0 * ALPS_PI * o->dpperp * 0.25 * (-o->qk * 0.5);
+    auto pair = [](double x, float* h, float* l) {
+      *h = (float)x;
+      *l = (float)(x - (double)*h);
+    };
+    const double z = c->sys.kperp_norm ? c->kperp / S.sp.qs : 1.0 / S.sp.qs;
+    o->iz = 1.0 / z;
+    pair(o->iz, &o->izh, &o->izl);
+    pair(o->dppar_abs, &o->pdh, &o->pdl);
+    pair(c->kpar < 0.0 ? -o->qk : o->qk, &o->qlh, &o->qll);
+    pair(-o->dpperp * ALPS_PI * 2.0 * ALPS_PI, &o->lih, &o->lil);
   }
   o->pcen = bm ? 0.0 : 0.5 * (S.ppar[1] + S.ppar[c->sys.npar - 1]);
   o->prad = bm ? 0.0 : 0.5 * (S.ppar[c->sys.npar - 1] - S.ppar[1]);
@@ -2665,6 +2680,11 @@ void default_shape(long u, bool mixed, int* lanes, long* csize) {
 // context and the table only: the lanes and chunks fix the summation order.
 // tensors: the batch writes chi_low, so every order is a chunk of its own.
 #define FIN_WARP_MAX 4096
+// an item per lane takes 97 us at any size up to some 4096 frequencies (one
+// lane's chain), a warp per item 116 us at 1024 and 208 us at 2999; where a
+// species' Landau terms are left to the warps (no Maxwellian rows) both take
+// 1.06 ms at 2560
+#define RES_LANES_MIN 2560
 #define ALPS_NOALLOC_SCRATCH_BYTES (16u << 20)
 
 // 256-byte aligned carve-out of n bytes from a scratch array
@@ -2748,6 +2768,13 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
   // a node sum
   sh.kmid = (int)(0.8 * (c->sys.npar - 1) / sh.js) + 16;
   sh.ipw = res_items_per_warp((long)b.nslots, ts.warps_per_sm ? ts.warps_per_sm : 12);
+  sh.lanes = 0;
+  if (mixed && !tensors && n >= RES_LANES_MIN && pvl_side(c->sys.positions_principal) <= 8) {
+    // about a third of the slots is occupied: 96 fill a warp's lanes once
+    const long per = ((long)b.nslots / (152 * 12) + 31) / 32 * 32;
+    sh.lanes = (int)std::max(96L, std::min(256L, per));
+    sh.ipw = (int)std::max(256L, ((long)b.nslots / (152 * 12) + 31) / 32 * 32);
+  }
   sh.fin_warp = (n <= FIN_WARP_MAX || tensors || rel_capacity(c) || any_bm(c)) ? 1 : 0;
   return b;
 }
@@ -2762,7 +2789,7 @@ DispJob lone_job(const DispShape& sh, int n, int S_, const double2* om, double2*
   j.sh = sh;
   j.n = n;
   j.S = S_;
-  for (int k = 0; k < 4; ++k) j.blk[k] = 0;
+  for (int k = 0; k < 5; ++k) j.blk[k] = 0;
   j.om = om;
   j.D = D;
   j.part = part;
@@ -2779,18 +2806,24 @@ DispJob lone_job(const DispShape& sh, int n, int S_, const double2* om, double2*
 // dynamic shared memory of k_resonant_multi for a context, and the opt-in
 // above 48 KB (per kernel, once per size)
 size_t res_smem(const alps_ctx* c) {
-  return (size_t)RES_WARPS * res_warp_smem(c->sys.nperp, res_win(c->sys.positions_principal)) * sizeof(double2);
+  return (size_t)RES_WARPS * res_warp_smem(c->sys.nperp, c->sys.positions_principal) * sizeof(double2);
 }
 std::mutex g_res_smem_mu;
-size_t g_res_smem_set = 0;
-int res_smem_optin(size_t smem) {
-  if (smem <= 48 * 1024) return ALPS_OK;
+size_t g_res_smem_set[2] = {0, 0};  // k_resonant_multi, k_resonant_lanes
+int res_smem_optin(size_t smem, size_t lanes_smem) {
+  const size_t want[2] = {smem, lanes_smem};
   std::lock_guard<std::mutex> lk(g_res_smem_mu);
-  if (g_res_smem_set < smem) {
-    ALPS_CUDA_TRY(cudaFuncSetAttribute(k_resonant_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    g_res_smem_set = smem;
-  }
+  for (int q = 0; q < 2; ++q)
+    if (want[q] > 40 * 1024 && g_res_smem_set[q] < want[q]) {
+      ALPS_CUDA_TRY(q ? cudaFuncSetAttribute(k_resonant_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want[q])
+                      : cudaFuncSetAttribute(k_resonant_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want[q]));
+      g_res_smem_set[q] = want[q];
+    }
   return ALPS_OK;
+}
+long lanes_blocks(const BatchGeom& bg) {
+  const long per = (long)RES_WARPS * bg.sh.lanes;
+  return per ? ((long)bg.nslots + per - 1) / per : 0;
 }
 
 }  // namespace
@@ -2859,11 +2892,14 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   if (c->profiling) ALPS_CUDA_TRY(cudaEventRecord(ev[1], st));
   const long g2 = pole_blocks_all(sh, S_);
   const size_t smem = res_smem(c);
-  if ((rcode = res_smem_optin(smem))) return rcode;
+  const size_t lsmem = pvl_smem(c->sys.positions_principal);
+  const long lblocks = lanes_blocks(bg);
+  if ((rcode = res_smem_optin(smem, lblocks ? lsmem : 0))) return rcode;
   long blocks = ((long)nslots + RES_WARPS * sh.ipw - 1) / (RES_WARPS * sh.ipw);
   if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (c->profiling) ALPS_CUDA_TRY(cudaEventRecord(ev[2], st));
+  if (lblocks) k_resonant_lanes<<<(unsigned)lblocks, RES_WARPS * 32, lsmem, st>>>(dj, 1);
   k_resonant_multi<<<(unsigned)blocks, RES_WARPS * 32, smem, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (a.relcap && (rcode = launch_rel_orders(a.sys, a.sp, a.relcap, n, d_om, c->d_rel, c->d_flags, st)))
@@ -2878,7 +2914,8 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   }
   c->stats.n_eval = n;
   c->stats.n_eval_total += n;
-  c->stats.kernels_launched = 5 + (a.relcap ? 1 : 0) + (a.has_bm ? 1 : 0);  // k_stage and the four
+  // k_stage and the four, k_resonant_lanes on lattices
+  c->stats.kernels_launched = 5 + (lblocks ? 1 : 0) + (a.relcap ? 1 : 0) + (a.has_bm ? 1 : 0);
   return ALPS_OK;
 }
 
@@ -2960,8 +2997,8 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
   }
   // shapes, grid offsets and scratch offsets of every job
   std::vector<size_t> o_part(nj), o_count(nj), o_slots(nj);
-  size_t part_n = 0, count_n = 0, slots_n = 0, om_off = 0, smem = 0;
-  long blk[4] = {0, 0, 0, 0};
+  size_t part_n = 0, count_n = 0, slots_n = 0, om_off = 0, smem = 0, lsmem = 0;
+  long blk[5] = {0, 0, 0, 0, 0};
   for (int j = 0; j < nj; ++j) {
     alps_ctx* c = ctx[j];
     const DispArgs* da = nullptr;
@@ -2982,6 +3019,9 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     blk[2] += ((long)bg.nslots + RES_WARPS * bg.sh.ipw - 1) / (RES_WARPS * bg.sh.ipw);
     J.blk[3] = blk[3];
     blk[3] += fin_blocks(bg.sh, n[j]);
+    J.blk[4] = blk[4];
+    blk[4] += lanes_blocks(bg);
+    if (bg.sh.lanes) lsmem = std::max(lsmem, pvl_smem(c->sys.positions_principal));
     J.om = d_om + om_off;
     J.D = d_D + om_off;
     J.flags = d_flags + j;
@@ -3020,11 +3060,12 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     J.items = m->items + o_slots[j] * 6;
   }
   ALPS_CUDA_TRY(cudaMemcpyAsync(m->d_jobs, m->h_jobs, (size_t)nj * sizeof(DispJob), cudaMemcpyHostToDevice, st));
-  if ((rcode = res_smem_optin(smem))) return rcode;
+  if ((rcode = res_smem_optin(smem, lsmem))) return rcode;
   out->jobs = m->d_jobs;
   out->nj = nj;
-  for (int k = 0; k < 4; ++k) out->blocks[k] = blk[k];
+  for (int k = 0; k < 5; ++k) out->blocks[k] = blk[k];
   out->smem = smem;
+  out->lanes_smem = lsmem;
   out->flags = d_flags;
   return ALPS_OK;
 }
@@ -3047,6 +3088,7 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
   ALPS_CUDA_TRY(cudaGetLastError());
   k_pole_sums_multi<<<(unsigned)ml.blocks[1], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
+  if (ml.blocks[4]) k_resonant_lanes<<<(unsigned)ml.blocks[4], RES_WARPS * 32, ml.lanes_smem, st>>>(jobs, ml.nj);
   k_resonant_multi<<<(unsigned)ml.blocks[2], RES_WARPS * 32, ml.smem, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
   k_finalize_multi<<<(unsigned)ml.blocks[3], 128, 0, st>>>(jobs, ml.nj);
@@ -3146,8 +3188,11 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   const size_t smem = res_smem(c);
-  int rcode0 = res_smem_optin(smem);
+  const size_t lsmem = pvl_smem(c->sys.positions_principal);
+  const long lblocks = lanes_blocks(bg);
+  int rcode0 = res_smem_optin(smem, lblocks ? lsmem : 0);
   if (rcode0) return rcode0;
+  if (lblocks) k_resonant_lanes<<<(unsigned)lblocks, RES_WARPS * 32, lsmem, st>>>(dj, 1);
   long blocks = ((long)nslots + RES_WARPS * sh.ipw - 1) / (RES_WARPS * sh.ipw);
   k_resonant_multi<<<(unsigned)blocks, RES_WARPS * 32, smem, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
