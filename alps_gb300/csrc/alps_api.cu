@@ -136,6 +136,7 @@ void alps_destroy(alps_ctx* c) {
     cudaFree(S.d_G);
     cudaFree(S.d_X);
     cudaFree(S.d_mom);
+    cudaFree(S.d_pfac);
     cudaFree(S.d_Vh);  // d_Vl points into it
     cudaFree(S.d_Vscale);
     cudaFree(S.d_Bt);
@@ -284,6 +285,7 @@ int alps_set_species(alps_ctx* c, int is, const alps_species* sp, const double* 
     for (int ip = 0; ip < 5; ++ip)
       for (int f = 0; f < nf; ++f) fit[(0 * 5 + ip) * nf + f] = sp->fit_init[f][ip];
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_pperp, pv.data(), (N + 1) * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  S.grid_ready = false;
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_ppar, qv.data(), (M + 1) * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_f0, S.f0.data(), nn * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   ALPS_CUDA_TRY(cudaMemcpyAsync(S.d_fit, fit.data(), fit.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));

@@ -10,7 +10,7 @@
 //     bessel[(nmax+3)(N+1)]           J_n(k_perp pperp_i / q), n = -1..nmax+1
 //     V[(nmax+1)(M-1)*12]             reduced vectors of the p_perp
 //                                     contraction (k_fold_reduced)
-//     mom[(nmax+1)*ALPS_KFAR*12]      Laurent moments of V about the grid
+//     mom[(nmax+1)*ALPS_KFAR*6]       Laurent moments of V about the grid
 //                                     centre (k_moments)
 //   per omega batch: partial sums, resonant-item slots, results.
 #pragma once
@@ -76,7 +76,8 @@ struct __align__(16) SpecDev {
   const double* fit;
   const double* bessel;
   const double* V;
-  const double* mom;  // Laurent moments [(nmax+1)][ALPS_KFAR][12]
+  const double* mom;  // Laurent moments of the base vectors [(nmax+1)][ALPS_KFAR][6]
+  const double* pfac; // FP64 path: order factors C0 v_e(n), [(nmax+1)][6]
   // V as pairs of floats (hi + lo, ~48 bits) scaled by 2^-e per order, Vscale
   // = 2^e, and ppar as float pairs: the fast path's node sums run on the
   // FP32 pipes in double-float arithmetic
@@ -199,6 +200,7 @@ struct SpeciesHost {
   double* d_G = nullptr;                  // contraction RHS [2][N-1][M-1]
   double* d_X = nullptr;                  // x_j^k, x_j = (ppar_j - pcen)/prad
   double* d_mom = nullptr;                // Laurent moments
+  double* d_pfac = nullptr;               // FP64 path: order factors
   float* d_Bt = nullptr;                  // base tables of the fast pole sums: Bt, mBt, bfac
   size_t Bt_cap = 0;
   double* d_Bd = nullptr;                 // and their FP64 part: Escale[8], Cfull, Pre
@@ -228,7 +230,8 @@ struct SpeciesHost {
   int bm_nrun = 0;
   size_t jrel_cap = 0;
   double int_ee_rel = 0.0;
-  size_t mom_cap = 0;
+  size_t mom_cap = 0, pfac_cap = 0;
+  bool grid_ready = false;                // d_X and the float pairs of ppar are those of d_ppar
   int nmax = 0;
   double int_ee = 0.0;
   double current_int = 0.0;  // n q P_par / m moment of the f0 table

@@ -611,90 +611,163 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
     }
 }
 
-// Plain path: the trapezoid node sum of every order in FP64 over the reduced
-// vectors.  Bound by the FP64 pipe (two lanes a clock and SM): 24 FMA of a
-// node's 32 instructions are the twelve real vectors against R_j.
+// Plain path, all in FP64: the trapezoid node sum over the reduced vectors for
+// orders in or near resonance, the Laurent series about the grid centre to
+// 2^-55 of its bound for the others (rho = prad/|d| < 0.76, K terms for the
+// 12 vectors' sums; the p_par-weighted entries follow from T and U as in
+// pole_fused, without cancellation).  Bound by the FP64 pipe (two lanes a
+// clock and SM): a node takes 33 FP64 instructions (24 are the twelve real
+// vectors against R_j), a term 16, and most orders need 12 to 30 terms
+// instead of 255 nodes: 2867 map frequencies on a 128x256 grid 3180 us by
+// nodes alone, 573 us so.
 __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, double2 o, bool active, int js,
-                                           int chunk, int nch, double* out) {
+                                           int chunk, int nch, int kmid, double* out) {
   const int M = S.M, U_ = 2 * S.nmax + 1;
   const int lane = threadIdx.x & 31, j = lane & (js - 1), gbase = lane - j;
   const unsigned gmask = (js == 32) ? FULL_WARP : (((1u << js) - 1u) << gbase);
   const double kpar = sys.kpar, kappa = S.kappa;
-  const double C0 = 2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25 * S.qs;
-  const double z = sys.kperp_norm ? sys.kperp / S.qs : 1.0 / S.qs;
   const double Di = S.ms * o.y, Di2 = Di * Di;
   const double* __restrict__ pp = S.ppar;
-  const float ikp32 = (float)sys.ikpar;
+  const float ikp32 = (float)sys.ikpar, dy32 = (float)Di * ikp32;
   dbl_val acc[12];
 #pragma unroll
   for (int q = 0; q < 12; ++q) acc[q] = {0.0};
   for (int i0 = 0; chunk + i0 * nch < U_; i0 += js) {
     const int u = chunk + (i0 + j) * nch;
     const bool own = active && u < U_;
-    int nn = 0, lo1 = 1, hi1 = 0, lo2 = 1, hi2 = 0;
+    OrderInfo cur = {0, S.kfar + 1, 0, 1, 0, 1, 0, 0};
     if (own) {
-      nn = u - S.nmax;
-      hi1 = M - 1;
+      cur.nn = u - S.nmax;
+      cur.hi1 = M - 1;
       // the FP32 test of k_classify: an order clearly outside the resonance
       // interval sums every node
-      const float x32 = (float)(S.ms * o.x - (double)nn * S.qs) * ikp32;
+      const float x32 = (float)(S.ms * o.x - (double)cur.nn * S.qs) * ikp32;
       const float mg = 9.5367431640625e-7f * fabsf(x32);
+      bool res = false;
       if (!(x32 < S.qlo - mg || x32 > S.qhi + mg)) {
-        const ResGeom g = res_geometry_of(S, sys, o, nn);
-        lo1 = g.lo1;
-        hi1 = g.hi1;
-        lo2 = g.lo2;
-        hi2 = g.hi2;
+        const ResGeom g = res_geometry_of(S, sys, o, cur.nn);
+        res = g.res;
+        cur.lo1 = g.lo1;
+        cur.hi1 = g.hi1;
+        cur.lo2 = g.lo2;
+        cur.hi2 = g.hi2;
+      }
+      const float dx = x32 - S.pcen32, ddf = fmaf(dx, dx, dy32 * dy32);
+      if (!res && S.prad32 * S.prad32 < 0.58f * ddf && ddf < 1e30f && fabsf(ikp32) < 1e30f) {
+        const float rho = S.prad32 * rsqrtf(ddf);
+        cur.K = (int)ceilf((38.1230949f - log1pf(-rho)) / -__logf(rho)) + 1;  // 55 ln 2
       }
     }
-    unsigned pend = __ballot_sync(FULL_WARP, own) & gmask;
-    while (__any_sync(FULL_WARP, pend != 0)) {
-      const bool go = pend != 0;
-      const int t = go ? __ffs(pend) - 1 : lane;
-      pend &= pend - 1;
-      const int cn = __shfl_sync(FULL_WARP, nn, t);
-      const int b1 = __shfl_sync(FULL_WARP, lo1, t), e1 = __shfl_sync(FULL_WARP, hi1, t);
-      const int b2 = __shfl_sync(FULL_WARP, lo2, t), e2 = __shfl_sync(FULL_WARP, hi2, t);
-      if (!go) continue;
-      const int n = cn < 0 ? -cn : cn;
-      const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
-      const double Ar = S.ms * o.x - (double)cn * S.qs;
-      double2 Sx[12];
-#pragma unroll
-      for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
-      // a range's two ends carry weight 1/2 (a range of a single node none:
-      // integrate(a,a) weighs it fully)
-      for (int r2 = 0; r2 < 2; ++r2) {
-        const int b = r2 ? b2 : b1, e = r2 ? e2 : e1;
-        const int lo = max(1, b), hi = min(M - 1, e);
-        for (int jn = lo + ((j - lo + 1) & (js - 1)); jn <= hi; jn += js) {
-          const double dr = fma(-kpar, pp[jn], Ar);
-          double r = rcp_fast(fma(dr, dr, Di2));
-          if (b < e && (jn == b || jn == e)) r *= 0.5;
-          const double Rr = dr * r, Ri = -Di * r;
-          const double2* v2 = reinterpret_cast<const double2*>(Vn + (size_t)(jn - 1) * 12);
-#pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            const double2 v = __ldg(v2 + q);
-            Sx[2 * q].x = fma(v.x, Rr, Sx[2 * q].x);
-            Sx[2 * q].y = fma(v.x, Ri, Sx[2 * q].y);
-            Sx[2 * q + 1].x = fma(v.y, Rr, Sx[2 * q + 1].x);
-            Sx[2 * q + 1].y = fma(v.y, Ri, Sx[2 * q + 1].y);
+    const bool solo = own && cur.K <= S.kfar && (js == 1 || cur.K <= kmid);
+    unsigned pend = __ballot_sync(FULL_WARP, own && !solo) & gmask;
+    bool go = solo;
+    int jj = 0, jc = 1;
+    const OrderInfo mine = cur;
+    for (;;) {
+      if (go) {
+        const int cn = cur.nn, n = cn < 0 ? -cn : cn, K = cur.K;
+        const double Ar = S.ms * o.x - (double)cn * S.qs;
+        double2 X[6];  // omega S_e1 + kappa S_e2
+        if (K <= S.kfar) {
+          // d = p_res - pcen, t = prad/d, f = 1/(k_par d); U = f sum_{k >= 2}
+          // mom_k t^k over this slice's k, per family and g
+          const double* __restrict__ mn = S.mom + (size_t)n * ALPS_KFAR * 6;
+          const int k0 = (jj >= 2) ? jj : jj + jc * ((2 - jj + jc - 1) / jc);
+          const double2 d = cmk(fma(Ar, sys.ikpar, -S.pcen), Di * sys.ikpar);
+          const double r = rcp_fast(fma(d.x, d.x, d.y * d.y));
+          const double2 iv = cmk(d.x * r, -d.y * r), t1 = cscale(iv, S.prad), f = cscale(iv, sys.ikpar);
+          double2 tp = f, st = t1;
+          {
+            double2 pw = t1;
+            for (int q = k0; q; q >>= 1) {
+              if (q & 1) tp = cmul(tp, pw);
+              pw = cmul(pw, pw);
+            }
+            for (int q = jc; q > 1; q >>= 1) st = cmul(st, st);
           }
+          double2 U[6];
+#pragma unroll
+          for (int b = 0; b < 6; ++b) U[b] = cmk(0.0, 0.0);
+          for (int k = k0; k < K; k += jc) {
+            const double2* m2 = reinterpret_cast<const double2*>(mn + (size_t)k * 6);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+              const double2 m = __ldg(m2 + b);
+              U[2 * b].x = fma(m.x, tp.x, U[2 * b].x);
+              U[2 * b].y = fma(m.x, tp.y, U[2 * b].y);
+              U[2 * b + 1].x = fma(m.y, tp.x, U[2 * b + 1].x);
+              U[2 * b + 1].y = fma(m.y, tp.y, U[2 * b + 1].y);
+            }
+            tp = cmul(tp, st);
+          }
+          double2 Uw[3];
+#pragma unroll
+          for (int F = 0; F < 3; ++F) Uw[F] = cadd(cmul(o, U[2 * F]), cscale(U[2 * F + 1], kappa));
+          // T = f mom_1 t + U, Q = f mom_0 + T on the slices that own k = 1, 0
+          auto mterm = [&](int k, double2 w, double2* to) {
+            const double* m = mn + (size_t)k * 6;
+#pragma unroll
+            for (int F = 0; F < 3; ++F)
+              to[F] = cadd(to[F], cmul(w, cmk(fma(o.x, m[2 * F], kappa * m[2 * F + 1]), o.y * m[2 * F])));
+          };
+          double2 T[3] = {Uw[0], Uw[1], Uw[2]};
+          if (jj == (jc > 1 ? 1 : 0)) mterm(1, cmul(f, t1), T);
+          double2 Q[3] = {T[0], T[1], T[2]};
+          if (jj == 0) mterm(0, f, Q);
+          // sum F p R = pcen Q + d T, sum F p^2 R = pcen (sum F p R) + d (pcen T + d U)
+          X[0] = Q[0];
+          X[1] = Q[1];
+          X[3] = Q[2];
+          X[4] = cadd(cscale(Q[0], S.pcen), cmul(d, T[0]));
+          X[5] = cadd(cscale(Q[2], S.pcen), cmul(d, T[2]));
+          X[2] = cadd(cscale(X[4], S.pcen), cmul(d, cadd(cscale(T[0], S.pcen), cmul(d, Uw[0]))));
+        } else {
+          const double* __restrict__ Vn = S.V + (size_t)n * (M - 1) * 12;
+          double2 Sx[12];
+#pragma unroll
+          for (int q = 0; q < 12; ++q) Sx[q] = cmk(0.0, 0.0);
+          // a range's two ends carry weight 1/2 (a range of a single node none:
+          // integrate(a,a) weighs it fully)
+          for (int r2 = 0; r2 < 2; ++r2) {
+            const int b = r2 ? cur.lo2 : cur.lo1, e = r2 ? cur.hi2 : cur.hi1;
+            const int lo = max(1, b), hi = min(M - 1, e);
+            for (int jn = lo + ((jj - lo + 1) & (jc - 1)); jn <= hi; jn += jc) {
+              const double dr = fma(-kpar, pp[jn], Ar);
+              double r = rcp_fast(fma(dr, dr, Di2));
+              if (b < e && (jn == b || jn == e)) r *= 0.5;
+              const double Rr = dr * r, Ri = -Di * r;
+              const double2* v2 = reinterpret_cast<const double2*>(Vn + (size_t)(jn - 1) * 12);
+#pragma unroll
+              for (int q = 0; q < 6; ++q) {
+                const double2 v = __ldg(v2 + q);
+                Sx[2 * q].x = fma(v.x, Rr, Sx[2 * q].x);
+                Sx[2 * q].y = fma(v.x, Ri, Sx[2 * q].y);
+                Sx[2 * q + 1].x = fma(v.y, Rr, Sx[2 * q + 1].x);
+                Sx[2 * q + 1].y = fma(v.y, Ri, Sx[2 * q + 1].y);
+              }
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 6; ++e) X[e] = cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kappa));
+        }
+        // integrate = C0 pref X (xy and xz odd in n); xy and yz carry the
+        // factor i, applied at the end
+        const double* __restrict__ fac = S.pfac + (size_t)n * 6;
+#pragma unroll
+        for (int e = 0; e < 6; ++e) {
+          if (n == 0 && (e == 0 || e == 3 || e == 4)) continue;
+          const double f = (cn < 0 && (e == 3 || e == 4)) ? -fac[e] : fac[e];
+          acc[2 * e].v = fma(f, X[e].x, acc[2 * e].v);
+          acc[2 * e + 1].v = fma(f, X[e].y, acc[2 * e + 1].v);
         }
       }
-      // integrate = C0 * pref * (omega S_e1 + kappa S_e2); xy and yz carry
-      // the factor i, applied at the end
-      double2 pref[6];
-      t_prefactors(cn, z, sys.kperp, sys.kperp_norm, pref);
-#pragma unroll
-      for (int e = 0; e < 6; ++e) {
-        if (n == 0 && (e == 0 || e == 3 || e == 4)) continue;
-        const double f = C0 * ((e == 3 || e == 5) ? pref[e].y : pref[e].x);
-        const double2 t1 = cadd(cmul(o, Sx[2 * e]), cscale(Sx[2 * e + 1], kappa));
-        acc[2 * e].v = fma(f, t1.x, acc[2 * e].v);
-        acc[2 * e + 1].v = fma(f, t1.y, acc[2 * e + 1].v);
-      }
+      if (!__any_sync(FULL_WARP, pend != 0)) break;
+      go = pend != 0;
+      const int t = go ? __ffs(pend) - 1 : lane;
+      pend &= pend - 1;
+      cur = shfl_info(mine, t);
+      jj = j;
+      jc = js;
     }
   }
   int first, cnt;
@@ -724,7 +797,7 @@ __device__ __forceinline__ void pole_body(const SysDev& sys, const SpecDev& S, c
   if (S.df_sums)
     pole_fused(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, out);
   else
-    pole_plain(sys, S, o, active, js, chunk, sh.nch[s], out);
+    pole_plain(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -1475,6 +1548,65 @@ __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p
   }
 }
 
+__device__ inline double2 crcp(double2 z) {
+  double r = 1.0 / (z.x * z.x + z.y * z.y);
+  return cmk(z.x * r, -z.y * r);
+}
+
+// The same term in FP64 (plain path): false if the neighbours' Gaussians leave
+// exp's range and the rows have to be summed one by one.  Some 350 FP64
+// instructions for 32 items at once, where the rows' two exponentials each
+// take 180 per 32 rows of one item: 2867 map frequencies 1008 us by rows,
+// 321 us so (k_resonant_multi); a single frequency 47 and 33 us.
+__device__ __noinline__ bool landau_lane_fp64(const SpecDev& S, double2 o, double2 p, int lf, int n,
+                                              const double* pref, double2* res) {
+  const double pd = S.dppar_abs, dx = p.x - S.p3r, dy = p.y;
+  const double e0 = -S.p2r * ((dx - dy) * (dx + dy)), ex = S.lcx * dx;
+  if (!(fabs(ex) < 600.0)) return false;
+  // an underflowing Gaussian leaves the term zero (landau_lane's test)
+  const double L2E = 1.4426950408889634;
+  const double k0 = rint(e0 * L2E), akx = fabs(rint(ex * L2E));
+  if (k0 + (double)S.lze < -1072.0 || k0 - akx + (double)(S.lge + S.lze) < -1072.0) return true;
+  const double2 G = cexp_d(cmk(e0, -2.0 * S.p2r * dx * dy));
+  const double2 X = cexp_d(cmk(ex, S.lcx * dy));
+  const double ql = S.qs / fabs(S.kappa * S.ms), lk = S.lgc * S.kappa / (2.0 * pd);
+  const double* __restrict__ lm = S.lmom + (size_t)n * 30;
+  double2 sum[3] = {cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0)};
+#pragma unroll 1
+  for (int u = 0; u < 3; ++u) {
+    double2 z = p, f;
+    if (u == 0) {
+      z.x += pd;
+      f = cscale(X, lk);
+    } else if (u == 1) {
+      z.x -= pd;
+      f = cscale(crcp(X), -lk);
+    } else {
+      f = cmk(fma(-S.kappa, p.x, o.x), fma(-S.kappa, p.y, o.y));
+    }
+    f = cmul(f, G);
+    const double2 z2 = cmul(z, z), z3 = cmul(z2, z), z4 = cmul(z2, z2);
+#pragma unroll
+    for (int F = 0; F < 3; ++F) {
+      const double* c = lm + F * 10 + (u == 2 ? 5 : 0);
+      const double2 q = cmk(fma(c[4], z4.x, fma(c[3], z3.x, fma(c[2], z2.x, fma(c[1], z.x, c[0])))),
+                            fma(c[4], z4.y, fma(c[3], z3.y, fma(c[2], z2.y, c[1] * z.y))));
+      sum[F] = cadd(sum[F], cmul(f, q));
+    }
+  }
+  const double fi = -S.dpperp * ALPS_PI * 2.0 * ALPS_PI * (double)lf * ql;
+#pragma unroll
+  for (int e = 0; e < 6; ++e) {
+    const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
+    double2 v = cscale(sum[fam], pref[e] * fi);
+    if (e == 4 || e == 5) v = cmul(v, p);
+    if (e == 2) v = cmul(cmul(p, p), v);
+    // pref ifac: real pref -> i pref fi; imaginary i pref -> -(pref fi)
+    res[e] = (e == 3 || e == 5) ? cmk(-v.x, -v.y) : cmk(-v.y, v.x);
+  }
+  return true;
+}
+
 // what the warp phase of k_resonant_multi needs of one item
 struct __align__(16) ResItem {
   PvItem pv;
@@ -1533,7 +1665,11 @@ __device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, dou
   }
   if (lf > 0) {
     const double2 p = cmk(g.pr, g.pi);
-    if (landau_factorises(S, p)) {
+    const bool fact = landau_factorises(S, p);
+    if (fact && !S.df_sums) {
+      if (!landau_lane_fp64(S, o, p, lf, n, pref, res)) work |= 2;
+      if (n == 0) res[0] = res[3] = res[4] = cmk(0.0, 0.0);
+    } else if (fact) {
       const dflt izd = {S.izh, S.izl}, dzd = df_mul({(float)nn, 0.0f}, izd);
       const dflt k2d = {a.sys.k2h, a.sys.k2l}, xyd = df_mul({a.sys.k1h, a.sys.k1l}, dzd);
       const dflt prefd[6] = {df_mul(dzd, dzd), k2d, k2d, xyd, xyd, df_neg(k2d)};
@@ -1612,10 +1748,6 @@ inline int res_items_per_warp(long nslots, int warps_per_sm = 12) {
   return (int)(ipw < 1 ? 1 : (ipw > 256 ? 256 : ipw));
 }
 
-__device__ inline double2 crcp(double2 z) {
-  double r = 1.0 / (z.x * z.x + z.y * z.y);
-  return cmk(z.x * r, -z.y * r);
-}
 
 __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
                                               int n_om, const int* __restrict__ count,
@@ -2474,6 +2606,7 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->bessel = S.d_bessel;
   o->V = S.d_V;
   o->mom = S.d_mom;
+  o->pfac = S.d_pfac;
   o->Vh = S.d_Vh;
   o->Vl = S.d_Vl;
   o->Vscale = S.d_Vscale;
@@ -2526,10 +2659,10 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->pcen32 = (float)o->pcen;
   o->prad32 = (float)o->prad;
   // the series is used only where it is cheaper than the node sum
-  o->kfar = (c->precision == ALPS_PREC_FP64) ? 0 : std::min(ALPS_KFAR, (int)(0.8 * (c->sys.npar - 1)));
+  o->kfar = std::min(ALPS_KFAR, (int)(0.8 * (c->sys.npar - 1)));
   o->rcap = S.rcap;
   o->fit_aux = S.d_fit_aux;
-  o->lmom = (S.lfact && c->precision != ALPS_PREC_FP64) ? S.d_lmom : nullptr;
+  o->lmom = S.lfact ? S.d_lmom : nullptr;
   o->p2r = S.p2r;
   o->p3r = S.p3r;
   o->la = S.la;
@@ -2664,15 +2797,20 @@ uint64_t tune_epoch() { return g_tune_epoch.load(); }
 // next form measured faster (us of the pole sums, 128x256 grid, 73 signed
 // orders).  Mixed path: n = 64: 27 with 32 lanes, 30 with 16; 128: 34 with
 // 16, 41 with 32 or 8; 512: 59 with 8, 72 with 16, 80 with 4; 2048: 150 with
-// 8 or 4, 167 with 2; 4096: 256 with 1, 262 with 2, 269 with 4.  FP64 path:
-// 64: 97 with 32, 102 with 16; 512: 622 with 8, 636 with 4; 2867: 3301 with
-// 4, 3452 with 2; 16384: 17760 with 1, 17960 with 2.  At a given number of
-// lanes about one order per lane is best (512 frequencies, 8 lanes: 59 with 8
-// orders, 64 with 4, 81 with 2).
+// 8 or 4, 167 with 2; 4096: 256 with 1, 262 with 2, 269 with 4.  At a given
+// number of lanes about one order per lane is best (512 frequencies, 8 lanes:
+// 59 with 8 orders, 64 with 4, 81 with 2).  FP64 path (lanes/orders): 8: 22
+// with 32/1, 31 with 32/2; 64: 59 with 32/4, 76 with 16/8; 256: 138 with 16/8,
+// 163 with 8/8; 2048: 579 with 8/8, 627 with 16/16, 699 with 4/8; 16384: 3535
+// with 8/64, 4388 with 8/16, 4606 with 1/16.
 void default_shape(long u, bool mixed, int* lanes, long* csize) {
-  *lanes = u < 220 ? 32 : (u < 440 ? 16 : (u < 3000 ? 8 : (u < 7700 ? 4 : 1)));
-  if (mixed) *csize = u < 75 ? 8 : (u < 440 ? 4 : (u < 3000 ? 8 : (u < 7700 ? 4 : 0)));
-  else *csize = u < 440 ? 1 : (u < 3000 ? 2 : (u < 7700 ? 4 : 0));
+  if (mixed) {
+    *lanes = u < 220 ? 32 : (u < 440 ? 16 : (u < 3000 ? 8 : (u < 7700 ? 4 : 1)));
+    *csize = u < 75 ? 8 : (u < 440 ? 4 : (u < 3000 ? 8 : (u < 7700 ? 4 : 0)));
+  } else {
+    *lanes = u < 200 ? 32 : (u < 600 ? 16 : 8);
+    *csize = u < 40 ? 1 : (u < 200 ? 4 : (u < 20000 ? 8 : 64));
+  }
 }
 
 // launch shape of a batch of n omegas on a context (default rule, or the

@@ -740,37 +740,54 @@ __global__ void k_fold_reduced(const double* __restrict__ A, const double* __res
   }
 }
 
-// X[(j-1)*ALPS_KFAR + k] = x_j^k with x_j = (ppar_j - pcen)/prad, j = 1..M-1
+// X[(j-1)*ALPS_KFAR + k] = x_j^k with x_j = (ppar_j - pcen)/prad, j = 1..M-1,
+// each power rounded once (products carried with their error)
 __global__ void k_powers(const double* __restrict__ ppar, int M, double pcen, double prad, double* X) {
   int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (j > M - 1) return;
   double x = (ppar[j] - pcen) / prad;
-  double p = 1.0;
+  double p = 1.0, l = 0.0;
   double* o = X + (size_t)(j - 1) * ALPS_KFAR;
   for (int k = 0; k < ALPS_KFAR; ++k) {
     o[k] = p;
-    p *= x;
+    const double h = p * x, e = fma(p, x, -h) + l * x;
+    p = h + e;
+    l = e - (p - h);
   }
 }
 
-// Laurent moments of the full-range trapezoid pole sum:
-// mom[(n*ALPS_KFAR + k)*12 + q] = sum_j f_j V[n][j][q] x_j^k, f_j = 1/2 at
-// j = 1, M-1 and 1 inside (the reduced vectors carry the interior weight 2).
-// For a pole p far from the grid, sum_j f_j V_j / (p - ppar_j) =
+// the reduced vectors of the Bessel families F1 = J^2, F2 = pperp^2 J'^2,
+// F3 = pperp J J' against g1 and g2 (b = 2 F + g)
+__device__ __forceinline__ int base_q(int b) { return b < 4 ? b : b + 2; }
+
+// Laurent moments of the full-range trapezoid pole sum of the base vectors:
+// mom[(n*ALPS_KFAR + k)*6 + b] = sum_j f_j V[n][j][base_q(b)] x_j^k, f_j = 1/2
+// at j = 1, M-1 and 1 inside (the reduced vectors carry the interior weight
+// 2).  For a pole p far from the grid, sum_j f_j V_j / (p - ppar_j) =
 //   (1/d) sum_k mom_k (prad/d)^k,  d = p - pcen.
-__global__ void k_moments(const double* __restrict__ V, const double* __restrict__ X, int M, int nmax,
-                          double* mom) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int total = (nmax + 1) * ALPS_KFAR * 12;
-  if (t >= total) return;
-  int q = t % 12, k = (t / 12) % ALPS_KFAR, n = t / (12 * ALPS_KFAR);
-  const double* v = V + (size_t)n * (M - 1) * 12 + q;
-  double acc = 0.0;
-  for (int j = 1; j <= M - 1; ++j) {
-    double f = (j == 1 || j == M - 1) ? 0.5 : 1.0;
-    acc = fma(f * v[(size_t)(j - 1) * 12], X[(size_t)(j - 1) * ALPS_KFAR + k], acc);
-  }
-  mom[t] = acc;
+// Bound by the FP64 rate: a warp per 32 powers of one vector, so that the
+// warps spread evenly over the SMs (192x384 grid: 33 us; a thread per (n, k,
+// q) of all twelve vectors, in blocks of 128, took 70).
+__global__ void __launch_bounds__(32) k_moments(const double* __restrict__ V, const double* __restrict__ X, int M,
+                                                double* mom) {
+  const int k = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y, n = blockIdx.z;
+  const double* v = V + (size_t)n * (M - 1) * 12 + base_q(b);
+  const double* x = X + k;
+  // (four partial sums: a shorter chain, and less rounding)
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int j0 = 2; j0 <= M - 2; j0 += 4)
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (j0 + u <= M - 2)
+        acc[u] = fma(__ldg(v + (size_t)(j0 + u - 1) * 12), __ldg(x + (size_t)(j0 + u - 1) * ALPS_KFAR), acc[u]);
+  const double ends = fma(0.5 * v[0], x[0], 0.5 * v[(size_t)(M - 2) * 12] * x[(size_t)(M - 2) * ALPS_KFAR]);
+  mom[((size_t)n * ALPS_KFAR + k) * 6 + b] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ends;
+}
+
+// C0 v_e(n) in FP64
+__global__ void k_plain_fac(int nmax, double z, double kperp, int kperp_norm, double C0, double* pfac) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < (nmax + 1) * 6) pfac[t] = fused_factor(t / 6, t % 6, z, kperp, kperp_norm, C0);
 }
 
 // Base tables of the fast path's pole sums.  The six T-tensor entries use
@@ -785,8 +802,6 @@ __global__ void k_moments(const double* __restrict__ V, const double* __restrict
 // A node or Laurent term then feeds 6 real vectors instead of 12.  The
 // vectors are V's q = 0, 1 (F1), 2, 3 (F2), 6, 7 (F3), scaled by
 // 1/Vscale[n] (a power of two) and split into float pairs.
-__device__ __forceinline__ int base_q(int b) { return b < 4 ? b : b + 2; }
-
 // Bt and mBt: hi parts at [rec*12 + b], lo parts at [rec*12 + 6 + b]
 __global__ void k_base_pairs(const double* __restrict__ V, const double* __restrict__ mom,
                              const double* __restrict__ Vscale, int M, int nmax, float* Bt, float* mBt) {
@@ -798,7 +813,7 @@ __global__ void k_base_pairs(const double* __restrict__ V, const double* __restr
   const size_t rec = u / 6;
   const int b = (int)(u % 6);
   const int n = isv ? (int)(rec / (M - 1)) : (int)(rec / ALPS_KFAR);
-  const double x = (isv ? V[rec * 12 + base_q(b)] : mom[rec * 12 + base_q(b)]) * (1.0 / Vscale[n]);
+  const double x = (isv ? V[rec * 12 + base_q(b)] : mom[rec * 6 + b]) * (1.0 / Vscale[n]);
   const float h = __double2float_rn(x), l = __double2float_rn(x - (double)h);
   float* o = isv ? Bt : mBt;
   o[rec * 12 + b] = h;
@@ -1423,36 +1438,43 @@ int launch_build_bessel_and_reduced(alps_ctx* c, int is, double kperp) {
     S.qlo_in = (float)(rlo + mg);
     S.qhi_in = (float)(rhi - mg);
   }
-  // the plain path sums nodes in FP64 on V alone; the float pairs, Laurent
-  // moments and order-fused tables below serve the mixed path only (a
+  // Laurent moments
+  const double pcen = 0.5 * (S.ppar[1] + S.ppar[M - 1]), prad = 0.5 * (S.ppar[M - 1] - S.ppar[1]);
+  if (!S.grid_ready) {
+    // what depends on the p_par grid alone: powers and float pairs
+    if (!S.d_X) ALPS_CUDA_TRY(cudaMalloc(&S.d_X, (size_t)(M - 1) * ALPS_KFAR * sizeof(double)));
+    if (!S.d_pph) ALPS_CUDA_TRY(cudaMalloc(&S.d_pph, (M + 1) * sizeof(float)));
+    if (!S.d_ppl) ALPS_CUDA_TRY(cudaMalloc(&S.d_ppl, (M + 1) * sizeof(float)));
+    k_powers<<<(M - 1 + 127) / 128, 128, 0, st>>>(S.d_ppar, M, pcen, prad, S.d_X);
+    ALPS_CUDA_TRY(cudaGetLastError());
+    k_split_pp<<<(M + 1 + 127) / 128, 128, 0, st>>>(S.d_ppar, M, S.d_pph, S.d_ppl);
+    ALPS_CUDA_TRY(cudaGetLastError());
+    S.grid_ready = true;
+  }
+  if ((rc = ensure(S.d_mom, S.mom_cap, (size_t)(nmax + 1) * ALPS_KFAR * 6))) return rc;
+  k_moments<<<dim3(ALPS_KFAR / 32, 6, nmax + 1), 32, 0, st>>>(S.d_V, S.d_X, M, S.d_mom);
+  ALPS_CUDA_TRY(cudaGetLastError());
+  const double z = c->sys.kperp_norm ? kperp / S.sp.qs : 1.0 / S.sp.qs;
+  const double dpperp = S.pperp[2] - S.pperp[1], dppar_abs = std::fabs(S.ppar[2] - S.ppar[1]);
+  const double C0 = 2.0 * ALPS_PI * dpperp * dppar_abs * 0.25 * S.sp.qs;
+  // the plain path sums nodes and series in FP64 on V and the moments; the
+  // float pairs and order-fused tables below serve the mixed path only (a
   // change of path rebuilds the k tables)
-  if (c->precision == ALPS_PREC_FP64) return ALPS_OK;
+  if (c->precision == ALPS_PREC_FP64) {
+    if ((rc = ensure(S.d_pfac, S.pfac_cap, (size_t)(nmax + 1) * 6))) return rc;
+    k_plain_fac<<<((nmax + 1) * 6 + 127) / 128, 128, 0, st>>>(nmax, z, kperp, c->sys.kperp_norm, C0, S.d_pfac);
+    ALPS_CUDA_TRY(cudaGetLastError());
+    return ALPS_OK;
+  }
   const size_t nvf = (size_t)(nmax + 1) * (M - 1) * 12;
   if ((rc = ensure(S.d_Vh, S.Vf_cap, 2 * nvf))) return rc;  // hi, then lo
   S.d_Vl = S.d_Vh + nvf;
   if ((rc = ensure(S.d_Vscale, S.Vs_cap, (size_t)(nmax + 1)))) return rc;
   k_split_df<<<nmax + 1, 256, 0, st>>>(S.d_V, M, S.d_Vscale, S.d_Vh, S.d_Vl);
   ALPS_CUDA_TRY(cudaGetLastError());
-  if (!S.d_pph) {
-    ALPS_CUDA_TRY(cudaMalloc(&S.d_pph, (M + 1) * sizeof(float)));
-    ALPS_CUDA_TRY(cudaMalloc(&S.d_ppl, (M + 1) * sizeof(float)));
-  }
-  k_split_pp<<<(M + 1 + 127) / 128, 128, 0, st>>>(S.d_ppar, M, S.d_pph, S.d_ppl);
-  ALPS_CUDA_TRY(cudaGetLastError());
-  double pcen = 0.5 * (S.ppar[1] + S.ppar[M - 1]), prad = 0.5 * (S.ppar[M - 1] - S.ppar[1]);
-  if (!S.d_X) ALPS_CUDA_TRY(cudaMalloc(&S.d_X, (size_t)(M - 1) * ALPS_KFAR * sizeof(double)));
-  if ((rc = ensure(S.d_mom, S.mom_cap, (size_t)(nmax + 1) * ALPS_KFAR * 12))) return rc;
   const size_t nmo = (size_t)(nmax + 1) * ALPS_KFAR * 12;
-  k_powers<<<(M - 1 + 127) / 128, 128, 0, st>>>(S.d_ppar, M, pcen, prad, S.d_X);
-  ALPS_CUDA_TRY(cudaGetLastError());
-  int tot = (nmax + 1) * ALPS_KFAR * 12;
-  k_moments<<<(tot + 127) / 128, 128, 0, st>>>(S.d_V, S.d_X, M, nmax, S.d_mom);
-  ALPS_CUDA_TRY(cudaGetLastError());
   // base tables of the fast path's pole sums
   {
-    const double z = c->sys.kperp_norm ? kperp / S.sp.qs : 1.0 / S.sp.qs;
-    const double dpperp = S.pperp[2] - S.pperp[1], dppar_abs = std::fabs(S.ppar[2] - S.ppar[1]);
-    const double C0 = 2.0 * ALPS_PI * dpperp * dppar_abs * 0.25 * S.sp.qs;
     const size_t nm = (size_t)(nmax + 1);
     if ((rc = ensure(S.d_Bt, S.Bt_cap, nvf + nmo + nm * 12))) return rc;  // Bt, mBt, bfac
     if ((rc = ensure(S.d_Bd, S.Bd_cap, 8 + nm * 6 + nm * (size_t)M * 6))) return rc;  // Escale, Cfull, Pre
@@ -1494,9 +1516,8 @@ int launch_fit_aux(alps_ctx* c, int is) {
 int launch_landau_moments(alps_ctx* c, int is) {
   SpeciesHost& S = c->spec[is];
   if (S.aux_ready) {
-    // the bounds belong to the fit, not to k: only the moments are per k,
-    // and only the mixed path reads them
-    if (!S.lfact || c->precision == ALPS_PREC_FP64) return ALPS_OK;
+    // the bounds belong to the fit, not to k: only the moments are per k
+    if (!S.lfact) return ALPS_OK;
     int rc;
     if ((rc = ensure(S.d_lmom, S.lmom_cap, (size_t)(S.nmax + 1) * (30 + 36)))) return rc;  // FP64, then the pairs
     const int tot = (S.nmax + 1) * 3;
@@ -1530,7 +1551,6 @@ int launch_landau_moments(alps_ctx* c, int is) {
   S.lc = lc;
   S.min_a0 = mina0;
   S.lfact = true;
-  if (c->precision == ALPS_PREC_FP64) return ALPS_OK;
   int rc;
   if ((rc = ensure(S.d_lmom, S.lmom_cap, (size_t)(nmax + 1) * (30 + 36)))) return rc;  // FP64, then the pairs
   int tot = (nmax + 1) * 3;
