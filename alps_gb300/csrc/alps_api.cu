@@ -565,6 +565,10 @@ int alps_set_precision(alps_ctx* c, int precision) {
   return ALPS_OK;
 }
 
+// batches whose frequencies and results the kernels read and write in pinned
+// host memory
+#define DIRECT_MAX 64
+
 int ctx_ensure_batch(alps_ctx* c, int n, bool ext) {
   if ((size_t)n > c->batch_cap) {
     cudaFree(c->d_om);
@@ -577,6 +581,7 @@ int ctx_ensure_batch(alps_ctx* c, int n, bool ext) {
     c->gen++;
   }
   size_t need_pin = (size_t)2 * n;
+  if (ext && n <= DIRECT_MAX) need_pin += (size_t)n * (c->sys.nspec * 36 + 9);
   if (need_pin > c->pinned_cap) {
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
     c->h_pinned = nullptr;
@@ -600,29 +605,38 @@ int ctx_ensure_batch(alps_ctx* c, int n, bool ext) {
   return ALPS_OK;
 }
 
-int ctx_check_flags(alps_ctx* c) {
-  int f = 0;
-  ALPS_CUDA_TRY(cudaMemcpy(&f, c->d_flags, sizeof(int), cudaMemcpyDeviceToHost));
-  if (f & 2) return ALPS_E_SUBLUMINAL;  // resonance window wider than the subluminal cone
-  return f ? ALPS_E_INVALID : ALPS_OK;
-}
-
 // Evaluates n frequencies from host memory through pinned staging.
 static int disp_host(alps_ctx* c, int n, const alps_complex* om, alps_complex* D, alps_complex* ext_out) {
   int st = ctx_ensure_batch(c, n, ext_out != nullptr);
   if (st) return st;
   double2* pin = c->h_pinned;
+  const size_t ne = ext_out ? (size_t)n * (c->sys.nspec * 36 + 9) : 0;
   memcpy(pin, om, (size_t)n * sizeof(double2));
-  ALPS_CUDA_TRY(cudaMemcpyAsync(c->d_om, pin, (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-  st = launch_disp_batch(c, n, c->d_om, c->d_D, ext_out ? c->d_ext : nullptr, c->stream);
+  // a few frequencies: the kernels read them from, and write det D and the
+  // error word to, pinned host memory (three copies and their calls took as
+  // long as the kernels)
+  const bool direct = n <= DIRECT_MAX;
+  if (!direct)
+    ALPS_CUDA_TRY(cudaMemcpyAsync(c->d_om, pin, (size_t)n * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+  bool flag_there = false;
+  *c->h_flag = 0;
+  st = launch_disp_batch(c, n, direct ? pin : c->d_om, direct ? pin + n : c->d_D,
+                         ext_out ? (direct ? pin + 2 * n : c->d_ext) : nullptr, c->stream, c->h_flag, &flag_there);
   if (st) return st;
-  ALPS_CUDA_TRY(cudaMemcpyAsync(pin + n, c->d_D, (size_t)n * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  if (ext_out)
-    ALPS_CUDA_TRY(cudaMemcpyAsync(ext_out, c->d_ext, (size_t)n * (c->sys.nspec * 36 + 9) * sizeof(double2),
-                                  cudaMemcpyDeviceToHost, c->stream));
+  if (!direct) {
+    ALPS_CUDA_TRY(cudaMemcpyAsync(pin + n, c->d_D, (size_t)n * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+    if (ext_out)
+      ALPS_CUDA_TRY(cudaMemcpyAsync(ext_out, c->d_ext, ne * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+  }
+  if (!flag_there)
+    ALPS_CUDA_TRY(cudaMemcpyAsync(c->h_flag, c->d_flags, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   ALPS_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  if ((st = ctx_check_flags(c))) return st;
+  if (*c->h_flag) {
+    c->flags_dirty = true;
+    return (*c->h_flag & 2) ? ALPS_E_SUBLUMINAL : ALPS_E_INVALID;  // (2: window wider than the subluminal cone)
+  }
   memcpy(D, pin + n, (size_t)n * sizeof(double2));
+  if (direct && ext_out) memcpy(ext_out, pin + 2 * n, ne * sizeof(double2));
   return ALPS_OK;
 }
 

@@ -263,7 +263,8 @@ struct alps_ctx {
   double2* d_bm = nullptr;      // [n][S][24] NHDS chi (6) and chi_low (3 x 6)
   size_t bm_cap = 0;
   size_t ext_cap = 0;
-  int* d_flags = nullptr;       // error flags
+  int* d_flags = nullptr;       // two error words (the second of batches that report to the host), counters
+  bool flags_dirty = false;     // the second one may be non-zero
   bool defer_sync = false;      // set_k of a batch (alps_set_k_many): no per-context synchronisation
   // error word of the last asynchronous batch (alps_disp_batch_device: d_flags;
   // alps_disp_batch_noalloc: a word of the static scratch), read by
@@ -304,7 +305,6 @@ int launch_prepare_species(alps_ctx* c, int is);
 // inside the extern "C" block of alps_api.cu and server.cu)
 extern "C" {
 int ctx_ensure_batch(alps_ctx* c, int n, bool ext);  // d_om, d_D, pinned staging for n frequencies
-int ctx_check_flags(alps_ctx* c);                    // device error flags of the last batch
 size_t ctx_device_bytes(const alps_ctx* c);          // device memory a context holds (estimate)
 void map_lattice(const alps_map_params* mp, std::vector<alps_complex>& oms);
 void map_finish(int n, const alps_complex* D, alps_complex* cal, double* val);
@@ -341,8 +341,10 @@ uint64_t tune_epoch();
 // per-order relativistic partials out[(((w*nspec + s)*relcap + n)*2 + sign)*REL_RB + rb][6]
 int launch_rel_orders(const SysDev& sys, const SpecDev* sp, int relcap, int n, const double2* d_om, double2* d_out,
                       int* d_flags, cudaStream_t st);
+// hflag: a host word (pinned, cleared by the caller) for a non-zero error word;
+// flag_there tells whether the batch writes it or leaves c->d_flags to be read
 int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext,
-                      cudaStream_t st);
+                      cudaStream_t st, int* hflag = nullptr, bool* flag_there = nullptr);
 // Fused batches: nj contexts, context j with n[j] frequencies at
 // d_om[o_j ...] (o_j = n[0] + ... + n[j-1]), det D to d_D at the same
 // offsets and the error flags of context j to d_flags[j].  Every context is
@@ -361,7 +363,8 @@ void multi_scratch_free(MultiScratch* m);
 struct MultiLaunch {
   const void* jobs;  // device job table
   int nj;
-  long blocks[5];    // grids of classify, pole sums, resonant, finalize, resonant lanes
+  bool small;        // all in one launch (k_disp_many)
+  long blocks[6];    // grids of classify, pole sums, resonant, finalize, resonant lanes, k_disp_many
   size_t smem;       // dynamic shared memory of k_resonant_multi
   size_t lanes_smem; // and of k_resonant_lanes
   int* flags;        // error words, one per job

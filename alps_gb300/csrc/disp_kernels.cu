@@ -29,6 +29,7 @@
 //   k_finalize_multi    chi, epsilon, wave tensor and det, one thread (or
 //                       warp) per omega; sums in a fixed order, so results
 //                       do not depend on timing or on the other jobs.
+// Small batches run all of it in one launch: k_disp_one, k_disp_many.
 //
 // Double-float (fast path): a value is a pair of floats h + l (about 46-48
 // bits) handled with error-free transformations (device_math.cuh); GB300
@@ -77,6 +78,18 @@ namespace {
 // One warp per (omega, species): the lanes test the orders -nmax..nmax
 // and a ballot prefix gives every resonant order its slot in increasing nn,
 // so the slot order does not depend on the launch shape.
+// whether order nn is resonant: an FP32 estimate of Re p_res settles the
+// orders clearly outside or inside the resonance interval (its bounds carry a
+// margin of 1e-5 of its extent, the estimate's error is below 2^-22 |p|); the
+// FP64 test decides near the interval's ends
+__device__ __forceinline__ bool order_resonant(const SysDev& sys, const SpecDev& S, double2 o, int nn, float ikp32) {
+  const float x32 = (float)(S.ms * o.x - (double)nn * S.qs) * ikp32;
+  const float mg = 9.5367431640625e-7f * fabsf(x32);
+  if (x32 < S.qlo - mg || x32 > S.qhi + mg) return false;
+  if (x32 > S.qlo_in + mg && x32 < S.qhi_in - mg) return true;
+  return res_geometry(S, sys.M_I, o, nn, sys.kpar).res;
+}
+
 __device__ __forceinline__ void classify_body(const DispArgs& a, const double2* __restrict__ om, int n_om,
                                               int* count, int* slot_nn, int* flags, long wid) {
   const int lane = threadIdx.x & 31;
@@ -95,17 +108,7 @@ __device__ __forceinline__ void classify_body(const DispArgs& a, const double2* 
   for (int base = -S.nmax; base <= S.nmax; base += 32) {
     const int nn = base + lane;
     bool res = false;
-    if (nn <= S.nmax) {
-      // an FP32 estimate of Re p_res settles the orders clearly outside or
-      // inside the resonance interval (its bounds carry a margin of 1e-5 of
-      // its extent, the estimate's error is below 2^-22 |p|); the FP64 test
-      // decides near the interval's ends
-      const float x32 = (float)(S.ms * o.x - (double)nn * S.qs) * ikp32;
-      const float mg = 9.5367431640625e-7f * fabsf(x32);
-      if (x32 < S.qlo - mg || x32 > S.qhi + mg) res = false;
-      else if (x32 > S.qlo_in + mg && x32 < S.qhi_in - mg) res = true;
-      else res = res_geometry(S, a.sys.M_I, o, nn, a.sys.kpar).res;
-    }
+    if (nn <= S.nmax) res = order_resonant(a.sys, S, o, nn, ikp32);
     const unsigned m = __ballot_sync(0xffffffffu, res);
     const int at = cnt + __popc(m & ((1u << lane) - 1u));
     if (res && at < a.rcap) slots[at] = nn;
@@ -785,7 +788,7 @@ __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, 
 
 // one warp's unit: an order chunk of species s for a tile of 32 / js
 // frequencies; its entries go to part[(w S + s) nchunk + chunk]
-__device__ __forceinline__ void pole_body(const SysDev& sys, const SpecDev& S, const DispShape& sh,
+__device__ __noinline__ void pole_body(const SysDev& sys, const SpecDev& S, const DispShape& sh,
                                           const double2* __restrict__ om, int n_om, double2* part, int s, long unit) {
   const int chunk = (int)(unit / sh.wt), tile = (int)(unit % sh.wt);
   const int js = sh.js, lane = threadIdx.x & 31;
@@ -1749,33 +1752,26 @@ inline int res_items_per_warp(long nslots, int warps_per_sm = 12) {
 }
 
 
-__device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
-                                              int n_om, const int* __restrict__ count,
-                                              const int* __restrict__ slot_nn, double2* items, long block) {
-  extern __shared__ double2 sm[];
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+// Up to 32 resonant items, one per lane (item < 0: none): the per-lane part,
+// then the principal-value sums and Landau rows item by item over the warp.
+// sv is the item's order (list: what k_resonant_lanes left of it), wk the
+// warp's shared memory.
+__device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __restrict__ om, double2* items,
+                                               double2* wk, long item, int sv, bool list) {
+  const int lane = threadIdx.x % 32;
   const int S_ = a.sys.nspec;
   const int N = a.sp[0].N;  // every species has the same p_perp grid
-  double2* wk = sm + (size_t)warp * res_warp_smem(N, a.sys.M_I);
   double2* frow = wk;                                      // f(i, p_res)
   double2* fpr = frow + (N + 1);                           // f(i, p_res + dppar)
   double2* fmr = fpr + (N + 1);                            // f(i, p_res - dppar)
   ResItem* ri = reinterpret_cast<ResItem*>(wk + res_region(N, a.sys.M_I));
   double2* tb = reinterpret_cast<double2*>(ri + 32);      // values handed to lanes 0-5
-  int* queue = reinterpret_cast<int*>(tb + 3);            // occupied slots, offsets from slot0
-  const long slot0 = (block * RES_WARPS + warp) * (long)sh.ipw;
-  if (slot0 >= (long)n_om * S_ * a.rcap) return;
-  const bool list = sh.lanes;  // only what k_resonant_lanes left
-  res_batches(
-      a, sh.ipw, n_om, count, slot0, queue,
-      [&](long sl) { return !list || (slot_nn[sl] >> 16) != 0; },
-      [&](int nb, long item) {
   // ---- one item per lane ----
   int work = 0;
   if (item >= 0) {
     const int u = (int)(item / a.rcap), s = u % S_, w = u / S_;
     const SpecDev& S = a.sp[s];
-    const int sv = slot_nn[item], nn = list ? (int)(short)(sv & 0xffff) : sv;
+    const int nn = list ? (int)(short)(sv & 0xffff) : sv;
     const double2 o = om[w];
     ResItem& it = ri[lane];
     double2 res[6];
@@ -1914,7 +1910,23 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
     }
     __syncwarp();  // the next item reuses the region
   }
-      });
+}
+
+__device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
+                                              int n_om, const int* __restrict__ count,
+                                              const int* __restrict__ slot_nn, double2* items, long block) {
+  extern __shared__ double2 sm[];
+  const int warp = threadIdx.x / 32;
+  const int N = a.sp[0].N;
+  double2* wk = sm + (size_t)warp * res_warp_smem(N, a.sys.M_I);
+  // occupied slots, offsets from slot0
+  int* queue = reinterpret_cast<int*>(wk + res_region(N, a.sys.M_I) + 32 * (sizeof(ResItem) / sizeof(double2)) + 3);
+  const long slot0 = (block * RES_WARPS + warp) * (long)sh.ipw;
+  if (slot0 >= (long)n_om * a.sys.nspec * a.rcap) return;
+  const bool list = sh.lanes;  // only what k_resonant_lanes left
+  res_batches(
+      a, sh.ipw, n_om, count, slot0, queue, [&](long sl) { return !list || (slot_nn[sl] >> 16) != 0; },
+      [&](int, long item) { resonant_group(a, om, items, wk, item, item >= 0 ? slot_nn[item] : 0, list); });
 }
 
 // ---------------------------------------------------------------------------
@@ -2245,11 +2257,12 @@ __device__ __forceinline__ void finalize_thread(const DispArgs& a, const DispSha
 }
 
 // one warp per omega; all lanes take part.  With ext the order chunks are
-// single orders, from which the n = -1, 0, 1 parts follow.
-__device__ __forceinline__ void finalize_warp(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
-                                              int n_om, const double2* __restrict__ part,
-                                              const int* __restrict__ count, const int* __restrict__ slot_nn,
-                                              const double2* __restrict__ items, const double2* __restrict__ rel,
+// single orders, from which the n = -1, 0, 1 parts follow.  Partial sums and
+// items are read through L2: k_disp_one and k_disp_many write them in the
+// same launch.
+__device__ __noinline__ void finalize_warp(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
+                                              int n_om, const double2* part, const int* count, const int* slot_nn,
+                                              const double2* items, const double2* __restrict__ rel,
                                               const double2* __restrict__ bmres, double2* D, double2* ext, long w) {
   if (w >= n_om) return;
   const int lane = threadIdx.x & 31, h = lane / 12, c = lane % 12, e = c >> 1;
@@ -2269,23 +2282,23 @@ __device__ __forceinline__ void finalize_warp(const DispArgs& a, const DispShape
     double v = 0.0, lw[3] = {0.0, 0.0, 0.0};
     if (h < 2) {
       const int nch = sh.nch[s];
-      const double* __restrict__ pt = reinterpret_cast<const double*>(part + base * 6) + c;
+      const double* pt = reinterpret_cast<const double*>(part + base * 6) + c;
 #pragma unroll 4
       for (int ch = h; ch < nch; ch += 2) {
-        const double x = pt[(size_t)ch * 12];
+        const double x = __ldcg(pt + (size_t)ch * 12);
         v += x;
         if (ext)
           for (int l = 0; l < 3; ++l)
             if (ch - S.nmax == l - 1) lw[l] += x;
       }
-      const int cnt = count[ws];
-      const double* __restrict__ it = reinterpret_cast<const double*>(items + ws * a.rcap * 6) + c;
+      const int cnt = __ldcg(count + ws);
+      const double* it = reinterpret_cast<const double*>(items + ws * a.rcap * 6) + c;
 #pragma unroll 2
       for (int r = h; r < cnt; r += 2) {
-        const double x = it[(size_t)r * 12];
+        const double x = __ldcg(it + (size_t)r * 12);
         v += x;
         if (ext) {
-          const int nn = slot_nn[ws * a.rcap + r];
+          const int nn = __ldcg(slot_nn + ws * a.rcap + r);
           for (int l = 0; l < 3; ++l)
             if (nn == l - 1) lw[l] += x;
         }
@@ -2407,7 +2420,10 @@ struct DispJob {
   const DispArgs* a;  // the context's arguments (device copy)
   DispShape sh;
   int n, S;
-  long blk[5];        // first block of the job in classify, pole sums, resonant, finalize, resonant lanes
+  int nslots;         // resonant slots of the prepared size
+  // first block of the job in classify, pole sums, resonant, finalize,
+  // resonant lanes, and in k_disp_many
+  long blk[6];
   const double2* om;
   double2* D;
   double2* part;
@@ -2415,6 +2431,8 @@ struct DispJob {
   int* slot_nn;
   double2* items;
   int* flags;
+  int* arrive;        // k_disp_one, k_disp_many: units done per frequency, zero between launches
+  int* hflag;         // host word that receives a non-zero error word, or null (k_disp_one)
   double2* ext;       // chi0, chi0_low, wave per omega, or null
   const double2* rel; // relativistic orders, or null
   const double2* bm;  // closed-form species, or null
@@ -2536,6 +2554,119 @@ __global__ void k_finalize_multi(const DispJob* __restrict__ jobs, int nj) {
                   lb * (blockDim.x / 32) + threadIdx.x / 32);
   else
     finalize_thread(a, J.sh, J.om, J.n, J.part, J.count, J.items, J.D, (int)(lb * blockDim.x + threadIdx.x));
+}
+
+// ---------------------------------------------------------------------------
+// Small batches in one launch.  The batches of root searches and scans are a
+// few frequencies: every kernel above is then one chain of dependent
+// instructions, and the sum of the chains and of the gaps between the
+// launches is the time of an evaluation.  Here the pole-sum units and the
+// resonant slots run side by side, a warp each (a slot's warp finds its
+// order itself), and the warp that brings a frequency its last unit goes on
+// to that frequency's det D: nothing waits on anything.  The sums are those of
+// the kernels above, in the same order.  One frequency, mixed path, 60x120
+// grid: 67 us in five kernels, 38 us so; a call from the host 110 and 62 us.
+// pole_body, resonant_group and finalize_warp are compiled once (noinline), so
+// a frequency's det D is the same bit for bit in either form.
+// ---------------------------------------------------------------------------
+// the slot's order (the r-th resonant order of its (omega, species)) and its
+// item; returns the slot's frequency, -1 beyond the batch
+__device__ __forceinline__ int small_slot(const DispArgs& a, const DispJob& J, double2* wk, int slot) {
+  const int lane = threadIdx.x & 31, S_ = a.sys.nspec;
+  const int u = slot / a.rcap, r = slot - u * a.rcap, s = u % S_, w = u / S_;
+  if (w >= J.n) return -1;
+  const SpecDev& S = a.sp[s];
+  const double2 o = J.om[w];
+  const float ikp32 = (float)a.sys.ikpar;
+  int cnt = 0, nn = 0;
+  bool found = false;
+  for (int base = -S.nmax; base <= S.nmax; base += 32) {
+    const bool res = base + lane <= S.nmax && order_resonant(a.sys, S, o, base + lane, ikp32);
+    const unsigned m = __ballot_sync(FULL_WARP, res);
+    const unsigned hit = __ballot_sync(FULL_WARP, res && cnt + __popc(m & ((1u << lane) - 1u)) == r);
+    if (hit) {
+      found = true;
+      nn = base + __ffs(hit) - 1;
+    }
+    cnt += __popc(m);
+  }
+  if (r == 0 && lane == 0) {
+    if (cnt > a.rcap) atomicOr(J.flags, 1);
+    J.count[u] = min(cnt, a.rcap);
+  }
+  if (found) {
+    if (lane == 0) J.slot_nn[slot] = nn;
+    resonant_group(a, J.om, J.items, wk, lane == 0 ? slot : -1, nn, false);
+  }
+  return w;
+}
+
+// A lane with has brings frequency w one unit; whoever brings the last one
+// finishes it.
+__device__ __forceinline__ void small_arrive(const DispArgs& a, const DispJob& J, int w, bool has) {
+  const int lane = threadIdx.x & 31;
+  int need = a.sys.nspec * a.rcap;
+  for (int s = 0; s < a.sys.nspec; ++s) need += J.sh.nch[s];
+  __threadfence();
+  __syncwarp();
+  const bool last = has && atomicAdd(J.arrive + w, 1) == need - 1;
+  unsigned m = __ballot_sync(FULL_WARP, last);
+  if (m) __threadfence();
+  while (m) {
+    const int t = __ffs(m) - 1;
+    m &= m - 1;
+    const int wt = __shfl_sync(FULL_WARP, w, t);
+    finalize_warp(a, J.sh, J.om, J.n, J.part, J.count, J.slot_nn, J.items, nullptr, nullptr, J.D, J.ext, wt);
+    if (lane == 0) {
+      J.arrive[wt] = 0;
+      if (J.hflag) {
+        const int f = atomicOr(J.flags, 0);
+        if (f) *J.hflag = f;
+      }
+    }
+  }
+}
+
+__host__ __device__ inline int small_slot_blocks(int nslots) { return (nslots + RES_WARPS - 1) / RES_WARPS; }
+
+__device__ __forceinline__ void small_body(const DispArgs& a, const DispJob& J, long lb) {
+  extern __shared__ double2 sm[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int nsb = small_slot_blocks(J.nslots);
+  if (lb < nsb) {
+    const int slot = (int)lb * RES_WARPS + warp;
+    if (slot >= J.nslots) return;
+    const int w = small_slot(a, J, sm + (size_t)warp * res_warp_smem(a.sp[0].N, a.sys.M_I), slot);
+    if (w >= 0) small_arrive(a, J, w, lane == 0);
+    return;
+  }
+  lb -= nsb;
+  int s = 0;
+  for (; s + 1 < J.S; ++s) {
+    const long nb = pole_blocks(J.sh, s);
+    if (lb < nb) break;
+    lb -= nb;
+  }
+  const long unit = lb * 4 + warp;
+  if (unit >= (long)J.sh.nch[s] * J.sh.wt) return;
+  pole_body(a.sys, a.sp[s], J.sh, J.om, J.n, J.part, s, unit);
+  const int js = J.sh.js, w = (int)(unit % J.sh.wt) * (32 / js) + lane / js;
+  __syncwarp();
+  small_arrive(a, J, w, w < J.n && (lane & (js - 1)) == 0);
+}
+
+static_assert(RES_WARPS == 4, "pole sums and slots share blocks of 128 threads");
+__global__ void __launch_bounds__(128, 3) k_disp_one(const __grid_constant__ DispArgs pa,
+                                                     const __grid_constant__ DispJob pj) {
+  __shared__ DispArgs sa;
+  const DispArgs& a = stage_args(&pa, sa);
+  small_body(a, pj, blockIdx.x);
+}
+__global__ void __launch_bounds__(128, 3) k_disp_many(const DispJob* __restrict__ jobs, int nj) {
+  __shared__ DispArgs sa;
+  const DispJob& J = job_of(jobs, nj, blockIdx.x, 5);
+  const DispArgs& a = stage_args(J.a, sa);
+  small_body(a, J, (long)blockIdx.x - J.blk[5]);
 }
 
 template <typename T>
@@ -2927,7 +3058,10 @@ DispJob lone_job(const DispShape& sh, int n, int S_, const double2* om, double2*
   j.sh = sh;
   j.n = n;
   j.S = S_;
-  for (int k = 0; k < 5; ++k) j.blk[k] = 0;
+  j.nslots = 0;
+  for (int k = 0; k < 6; ++k) j.blk[k] = 0;
+  j.arrive = nullptr;
+  j.hflag = nullptr;
   j.om = om;
   j.D = D;
   j.part = part;
@@ -2947,16 +3081,43 @@ size_t res_smem(const alps_ctx* c) {
   return (size_t)RES_WARPS * res_warp_smem(c->sys.nperp, c->sys.positions_principal) * sizeof(double2);
 }
 std::mutex g_res_smem_mu;
-size_t g_res_smem_set[2] = {0, 0};  // k_resonant_multi, k_resonant_lanes
-int res_smem_optin(size_t smem, size_t lanes_smem) {
-  const size_t want[2] = {smem, lanes_smem};
+size_t g_res_smem_set[4] = {0, 0, 0, 0};  // k_resonant_multi, k_resonant_lanes, k_disp_one, k_disp_many
+int res_smem_optin(size_t smem, size_t lanes_smem, bool small = false) {
+  const size_t want[4] = {small ? 0 : smem, lanes_smem, small ? smem : 0, small ? smem : 0};
+  auto set = [](int q, int bytes) {
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    return q == 0 ? cudaFuncSetAttribute(k_resonant_multi, at, bytes)
+                  : (q == 1 ? cudaFuncSetAttribute(k_resonant_lanes, at, bytes)
+                            : (q == 2 ? cudaFuncSetAttribute(k_disp_one, at, bytes)
+                                      : cudaFuncSetAttribute(k_disp_many, at, bytes)));
+  };
   std::lock_guard<std::mutex> lk(g_res_smem_mu);
-  for (int q = 0; q < 2; ++q)
+  for (int q = 0; q < 4; ++q)
     if (want[q] > 40 * 1024 && g_res_smem_set[q] < want[q]) {
-      ALPS_CUDA_TRY(q ? cudaFuncSetAttribute(k_resonant_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want[q])
-                      : cudaFuncSetAttribute(k_resonant_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want[q]));
+      ALPS_CUDA_TRY(set(q, (int)want[q]));
       g_res_smem_set[q] = want[q];
     }
+  return ALPS_OK;
+}
+// Batches that run in one launch (k_disp_one, k_disp_many): as many warps as
+// the chip holds twice over at most.  Beyond, the warps of empty slots and
+// the kernel's larger frame cost more than the gaps between the launches (60x120
+// grid, us in one launch and apart: 31 frequencies 53 and 82, 128: 100 and
+// 113, 256: 141 and 125).
+#define SMALL_WARPS (152 * 12 * 2)
+#define MANY_WARPS (152 * 12 * 4)
+long pole_warps(const DispShape& sh, int S_) { return 4 * pole_blocks_all(sh, S_); }
+bool small_batch(const alps_ctx* c, const BatchGeom& bg) {
+  return !c->profiling && !rel_capacity(c) && !any_bm(c) && bg.sh.fin_warp && !bg.sh.lanes &&
+         (long)bg.nslots + pole_warps(bg.sh, c->sys.nspec) <= SMALL_WARPS;
+}
+int launch_one(const alps_ctx* c, const DispArgs& a, const DispShape& sh, const DispJob& job, cudaStream_t st) {
+  const size_t smem = res_smem(c);
+  int rc = res_smem_optin(smem, 0, true);
+  if (rc) return rc;
+  const long blocks = small_slot_blocks(job.nslots) + pole_blocks_all(sh, c->sys.nspec);
+  k_disp_one<<<(unsigned)blocks, 128, smem, st>>>(a, job);
+  ALPS_CUDA_TRY(cudaGetLastError());
   return ALPS_OK;
 }
 long lanes_blocks(const BatchGeom& bg) {
@@ -2966,7 +3127,9 @@ long lanes_blocks(const BatchGeom& bg) {
 
 }  // namespace
 
-int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext, cudaStream_t st) {
+int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext, cudaStream_t st,
+                      int* hflag, bool* flag_there) {
+  if (flag_there) *flag_there = false;
   if (n <= 0) return ALPS_OK;
   const int S_ = c->sys.nspec;
   DispArgs a;
@@ -2990,11 +3153,39 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     if ((rcode = ensure_buf(c->d_rel, c->rel_cap, (size_t)n * S_ * a.relcap * 2 * REL_RB * 6))) return rcode;
   if (a.has_bm)
     if ((rcode = ensure_buf(c->d_bm, c->bm_cap, (size_t)n * S_ * 24))) return rcode;
-  if (!c->d_flags) ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, sizeof(int)));
+  if (!c->d_flags) {
+    // the error word, the error word of batches that report to hflag, and a
+    // counter per frequency of a small batch (zero between launches)
+    ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, (2 + SMALL_WARPS) * sizeof(int)));
+    ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, (2 + SMALL_WARPS) * sizeof(int), st));
+    c->flags_dirty = false;
+  }
   const void* after[7] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_rel, c->d_bm, c->d_flags};
   for (int q = 0; q < 7; ++q)
     if (before[q] != after[q]) c->gen++;  // buffer addresses changed: cached graphs are stale
-  ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, sizeof(int), st));
+  const bool small = small_batch(c, bg);
+  // (the word of batches that report to hflag is zero while none reported)
+  int* flags = c->d_flags;
+  if (small && hflag) {
+    flags = c->d_flags + 1;
+    if (c->flags_dirty) ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
+    c->flags_dirty = false;
+  } else {
+    ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
+  }
+  if (small) {
+    DispJob job = lone_job(sh, n, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, flags);
+    job.ext = d_ext;
+    job.nslots = (int)nslots;
+    job.arrive = c->d_flags + 2;
+    job.hflag = hflag;
+    if ((rcode = launch_one(c, a, sh, job, st))) return rcode;
+    if (flag_there) *flag_there = hflag != nullptr;
+    c->stats.n_eval = n;
+    c->stats.n_eval_total += n;
+    c->stats.kernels_launched = 1;
+    return ALPS_OK;
+  }
 
   std::vector<cudaEvent_t> ev;
   if (c->profiling) {
@@ -3072,6 +3263,8 @@ struct MultiScratch {
   size_t slots_cap = 0;
   double2* items = nullptr;
   size_t items_cap = 0;
+  int* arrive = nullptr;  // units done per frequency, zero between launches
+  size_t arrive_cap = 0;
 };
 
 void multi_scratch_free(MultiScratch* m) {
@@ -3082,6 +3275,7 @@ void multi_scratch_free(MultiScratch* m) {
   cudaFree(m->count);
   cudaFree(m->slots);
   cudaFree(m->items);
+  cudaFree(m->arrive);
   delete m;
 }
 
@@ -3136,7 +3330,8 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
   // shapes, grid offsets and scratch offsets of every job
   std::vector<size_t> o_part(nj), o_count(nj), o_slots(nj);
   size_t part_n = 0, count_n = 0, slots_n = 0, om_off = 0, smem = 0, lsmem = 0;
-  long blk[5] = {0, 0, 0, 0, 0};
+  long blk[6] = {0, 0, 0, 0, 0, 0}, warps = 0;
+  bool small = true;
   for (int j = 0; j < nj; ++j) {
     alps_ctx* c = ctx[j];
     const DispArgs* da = nullptr;
@@ -3159,6 +3354,12 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     blk[3] += fin_blocks(bg.sh, n[j]);
     J.blk[4] = blk[4];
     blk[4] += lanes_blocks(bg);
+    J.nslots = (int)bg.nslots;
+    J.blk[5] = blk[5];
+    blk[5] += small_slot_blocks(J.nslots) + pole_blocks_all(bg.sh, S_);
+    small = small && small_batch(c, bg);
+    warps += (long)bg.nslots + pole_warps(bg.sh, S_);
+    J.hflag = nullptr;
     if (bg.sh.lanes) lsmem = std::max(lsmem, pvl_smem(c->sys.positions_principal));
     J.om = d_om + om_off;
     J.D = d_D + om_off;
@@ -3186,6 +3387,10 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     blk[2] += (nsl + RES_WARPS * ipw - 1) / (RES_WARPS * ipw);
   }
   int rcode;
+  if (om_off > m->arrive_cap) {
+    if ((rcode = ensure_buf(m->arrive, m->arrive_cap, om_off))) return rcode;
+    ALPS_CUDA_TRY(cudaMemsetAsync(m->arrive, 0, m->arrive_cap * sizeof(int), st));
+  }
   if ((rcode = ensure_buf(m->part, m->part_cap, part_n))) return rcode;
   if ((rcode = ensure_buf(m->count, m->count_cap, count_n))) return rcode;
   if ((rcode = ensure_buf(m->slots, m->slots_cap, slots_n))) return rcode;
@@ -3196,12 +3401,15 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
     J.count = m->count + o_count[j];
     J.slot_nn = m->slots + o_slots[j];
     J.items = m->items + o_slots[j] * 6;
+    J.arrive = m->arrive + (J.om - d_om);
   }
   ALPS_CUDA_TRY(cudaMemcpyAsync(m->d_jobs, m->h_jobs, (size_t)nj * sizeof(DispJob), cudaMemcpyHostToDevice, st));
-  if ((rcode = res_smem_optin(smem, lsmem))) return rcode;
+  small = small && warps <= MANY_WARPS;
+  if ((rcode = res_smem_optin(smem, lsmem, small))) return rcode;
+  out->small = small;
   out->jobs = m->d_jobs;
   out->nj = nj;
-  for (int k = 0; k < 5; ++k) out->blocks[k] = blk[k];
+  for (int k = 0; k < 6; ++k) out->blocks[k] = blk[k];
   out->smem = smem;
   out->lanes_smem = lsmem;
   out->flags = d_flags;
@@ -3222,6 +3430,11 @@ void disp_job_layout(size_t* stride, size_t* n_offset) {
 int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
   const DispJob* jobs = static_cast<const DispJob*>(ml.jobs);
   ALPS_CUDA_TRY(cudaMemsetAsync(ml.flags, 0, (size_t)ml.nj * sizeof(int), st));
+  if (ml.small) {
+    k_disp_many<<<(unsigned)ml.blocks[5], 128, ml.smem, st>>>(jobs, ml.nj);
+    ALPS_CUDA_TRY(cudaGetLastError());
+    return ALPS_OK;
+  }
   k_classify_multi<<<(unsigned)ml.blocks[0], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
   k_pole_sums_multi<<<(unsigned)ml.blocks[1], 128, 0, st>>>(jobs, ml.nj);
@@ -3254,7 +3467,8 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 // stream capture.  Every call shares the one array: two calls whose kernels
 // overlap on the GPU (different streams, or different host threads) race on
 // it and must be ordered by the caller.  The error flag is cleared at the
-// start of every call; every other word a call reads it writes first.  The
+// start of every call and the counters of a small batch are zero between
+// calls; every other word a call reads it writes first.  The
 // flag word's device address is recorded in the context, so
 // alps_batch_status reports the call's device errors (read it before the
 // next call on the device clears the word).
@@ -3262,10 +3476,12 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 #define ALPS_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[ALPS_NOALLOC_SCRATCH_BYTES];
+static __device__ int g_noalloc_arrive[SMALL_WARPS];  // counters of a small batch, zero between launches
 
 namespace {
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[ALPS_NOALLOC_MAX_DEVICES] = {nullptr};
+void* g_noalloc_cnt[ALPS_NOALLOC_MAX_DEVICES] = {nullptr};
 }  // namespace
 
 extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d_om, alps_complex* d_D,
@@ -3276,12 +3492,13 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   int dev = -1;
   ALPS_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= ALPS_NOALLOC_MAX_DEVICES) return ALPS_E_INVALID;
-  void* base = nullptr;
+  void *base = nullptr, *cnt = nullptr;
   {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_addr[dev]) {
       void* p = nullptr;
-      cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+      cudaError_t e = cudaGetSymbolAddress(&g_noalloc_cnt[dev], g_noalloc_arrive);
+      if (e == cudaSuccess) e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
       if (e != cudaSuccess || !p) {
         alps_set_last_cuda_error(e, "cudaGetSymbolAddress(g_noalloc_scratch)", __FILE__, __LINE__);
         return ALPS_E_CUDA;
@@ -3289,6 +3506,7 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
       g_noalloc_addr[dev] = p;
     }
     base = g_noalloc_addr[dev];
+    cnt = g_noalloc_cnt[dev];
   }
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   const int S_ = c->sys.nspec;
@@ -3316,6 +3534,14 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   DispJob job = lone_job(sh, n, S_, om, D, part, count, slots, items, flags);
   job.rel = a.relcap ? relb : nullptr;
   job.bm = a.has_bm ? bmb : nullptr;
+  if (small_batch(c, bg)) {
+    job.nslots = (int)nslots;
+    job.arrive = static_cast<int*>(cnt);
+    const int rc = launch_one(c, a, sh, job, st);
+    if (rc) return rc;
+    c->async_flags = flags;
+    return ALPS_OK;
+  }
   DispArgs* da = reinterpret_cast<DispArgs*>(b + off[SC_ARGS]);
   DispJob* dj = reinterpret_cast<DispJob*>(b + off[SC_JOB]);
   k_stage<<<1, 128, 0, st>>>(a, job, da, dj);
