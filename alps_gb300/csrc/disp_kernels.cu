@@ -1458,8 +1458,16 @@ __device__ __forceinline__ double scale_exp(double m, int e) {
   const int e1 = max(-1000, min(1000, e / 2)), e2 = max(-1000, min(1000, e - e1));
   return m * __hiloint2double((1023 + e1) << 20, 0) * __hiloint2double((1023 + e2) << 20, 0);
 }
+// WARP: every lane has the same item; the exponentials, the three points and
+// the entries go over the lanes, and res[0] receives entry min(lane, 5).
+__device__ __forceinline__ dflt df_from(dflt v, int src) {
+  return {__shfl_sync(FULL_WARP, v.h, src), __shfl_sync(FULL_WARP, v.l, src)};
+}
+__device__ __forceinline__ cdf cdf_from(cdf v, int src) { return {df_from(v.x, src), df_from(v.y, src)}; }
+template <bool WARP>
 __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p, int lf, int n, const dflt* prefd,
                                             double2* res) {
+  const int lane = threadIdx.x & 31;
   // Row Gaussian G(x) = exp(-p2r (x - p3r)^2) at x = p, p +- dppar:
   // G(p +- pd) = lgc G(p) X^{+-1}, X = exp(-2 p2r pd (p - p3r)).  In
   // double-float with powers of two kept apart: G(p) = 2^k0 g0,
@@ -1470,9 +1478,9 @@ __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p
   //   sum_F = (q/|k_par|) (kappa Spar + (omega - kappa p) Sperp).
   const double dx = p.x - S.p3r, dy = p.y;
   int k0 = 0, kx = 0;
-  cdf g0, xm, xi;
+  cdf g0 = {{0.0f, 0.0f}, {0.0f, 0.0f}}, xm = g0, xi = g0;
 #pragma unroll 1
-  for (int u = 0; u < 2; ++u) {
+  for (int u = WARP ? (lane & 1) : 0; u < 2; u += WARP ? 2 : 1) {
     int e;
     dflt cs, sn;
     const dflt m = df_exp_scaled(u ? S.lcx * dx : -S.p2r * ((dx - dy) * (dx + dy)), e);
@@ -1487,6 +1495,13 @@ __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p
       g0 = v;
       k0 = e;
     }
+  }
+  if (WARP) {
+    g0 = cdf_from(g0, 0);
+    xm = cdf_from(xm, 1);
+    xi = cdf_from(xi, 1);
+    k0 = __shfl_sync(FULL_WARP, k0, 0);
+    kx = __shfl_sync(FULL_WARP, kx, 1);
   }
   // an underflowing Gaussian (|G| min_a0 below the FP64 range at any of the
   // three points) leaves the term zero, as in FP64
@@ -1505,7 +1520,7 @@ __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p
   const dflt z = {0.0f, 0.0f};
   cdf sum[3] = {{z, z}, {z, z}, {z, z}};  // per family: kappa Spar + (omega - kappa p) Sperp over G
 #pragma unroll 1
-  for (int u = 0; u < 3; ++u) {
+  for (int u = WARP ? min(lane, 2) : 0; u < 3; u += WARP ? 3 : 1) {
     // the moment polynomials at p + pd, p - pd (P_F) and p (Q_F), each times
     // its factor
     cdf zu = pz, f;
@@ -1531,23 +1546,27 @@ __device__ __forceinline__ void landau_lane(const SpecDev& S, cdf omd, double2 p
       sum[F] = cdf_add(sum[F], cdf_mul(f, q));
     }
   }
+  if (WARP)
+    for (int F = 0; F < 3; ++F)
+      sum[F] = cdf_add(cdf_add(cdf_from(sum[F], 0), cdf_from(sum[F], 1)), cdf_from(sum[F], 2));
   // res_e = pref_e c_e sum_F(e) ifac, c_e = 1, p or p^2; ifac =
   // -i dpperp 2 pi^2 lf, pref_e real (imaginary for xy, yz); with q / |k_par|
   const cdf gq = cdf_rmul(g0, df_mul({S.qlh, S.qll}, df_scale({S.lih, S.lil}, (float)lf)));
-  cdf v[6];
-  v[0] = cdf_mul(gq, sum[0]);
-  v[1] = cdf_mul(gq, sum[1]);
-  v[3] = cdf_mul(gq, sum[2]);
-  v[4] = cdf_mul(v[0], pz);
-  v[2] = cdf_mul(v[4], pz);
-  v[5] = cdf_mul(v[3], pz);
 #pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0), ex = k0 + akx + (int)lm0[fam * 24 + 20];
+  for (int t = 0; t < (WARP ? 1 : 6); ++t) {
+    const int e = WARP ? min(lane, 5) : t, fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
+    const int ex = k0 + akx + (int)lm0[fam * 24 + 20];
+    cdf v = cdf_mul(gq, fam == 0 ? sum[0] : (fam == 1 ? sum[1] : sum[2]));
+    if (e == 2 || e == 4 || e == 5) v = cdf_mul(v, pz);
+    if (e == 2) v = cdf_mul(v, pz);
     // pref ifac: real pref -> i pref fi; imaginary i pref -> -(pref fi)
     const bool im = (e == 3 || e == 5);
-    const double vx = scale_exp(df_val(df_mul(v[e].x, prefd[e])), ex), vy = scale_exp(df_val(df_mul(v[e].y, prefd[e])), ex);
-    res[e] = im ? cmk(-vx, -vy) : cmk(-vy, vx);
+    dflt pf = prefd[0];
+#pragma unroll
+    for (int q = 1; q < 6; ++q)
+      if (e == q) pf = prefd[q];
+    const double vx = scale_exp(df_val(df_mul(v.x, pf)), ex), vy = scale_exp(df_val(df_mul(v.y, pf)), ex);
+    res[t] = im ? cmk(-vx, -vy) : cmk(-vy, vx);
   }
 }
 
@@ -1561,51 +1580,83 @@ __device__ inline double2 crcp(double2 z) {
 // instructions for 32 items at once, where the rows' two exponentials each
 // take 180 per 32 rows of one item: 2867 map frequencies 1008 us by rows,
 // 321 us so (k_resonant_multi); a single frequency 47 and 33 us.
+__device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
+  return cmk(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ double2 c_from(double2 v, int src) {
+  return cmk(__shfl_sync(FULL_WARP, v.x, src), __shfl_sync(FULL_WARP, v.y, src));
+}
+// (operations rounded one by one: both forms give the same bits)
+template <bool WARP>
 __device__ __noinline__ bool landau_lane_fp64(const SpecDev& S, double2 o, double2 p, int lf, int n,
                                               const double* pref, double2* res) {
+  const int lane = threadIdx.x & 31;
   const double pd = S.dppar_abs, dx = p.x - S.p3r, dy = p.y;
-  const double e0 = -S.p2r * ((dx - dy) * (dx + dy)), ex = S.lcx * dx;
+  const double e0 = __dmul_rn(-S.p2r, __dmul_rn(dx - dy, dx + dy)), ex = __dmul_rn(S.lcx, dx);
   if (!(fabs(ex) < 600.0)) return false;
   // an underflowing Gaussian leaves the term zero (landau_lane's test)
   const double L2E = 1.4426950408889634;
   const double k0 = rint(e0 * L2E), akx = fabs(rint(ex * L2E));
   if (k0 + (double)S.lze < -1072.0 || k0 - akx + (double)(S.lge + S.lze) < -1072.0) return true;
-  const double2 G = cexp_d(cmk(e0, -2.0 * S.p2r * dx * dy));
-  const double2 X = cexp_d(cmk(ex, S.lcx * dy));
+  double2 G = cmk(0.0, 0.0), X = G;
+#pragma unroll 1
+  for (int u = WARP ? (lane & 1) : 0; u < 2; u += WARP ? 2 : 1) {
+    const double2 v = cexp_d(u ? cmk(ex, __dmul_rn(S.lcx, dy)) : cmk(e0, __dmul_rn(__dmul_rn(-2.0 * S.p2r, dx), dy)));
+    if (u) X = v;
+    else G = v;
+  }
+  if (WARP) {
+    G = c_from(G, 0);
+    X = c_from(X, 1);
+  }
   const double ql = S.qs / fabs(S.kappa * S.ms), lk = S.lgc * S.kappa / (2.0 * pd);
   const double* __restrict__ lm = S.lmom + (size_t)n * 30;
   double2 sum[3] = {cmk(0.0, 0.0), cmk(0.0, 0.0), cmk(0.0, 0.0)};
 #pragma unroll 1
-  for (int u = 0; u < 3; ++u) {
+  for (int u = WARP ? min(lane, 2) : 0; u < 3; u += WARP ? 3 : 1) {
     double2 z = p, f;
     if (u == 0) {
-      z.x += pd;
-      f = cscale(X, lk);
+      z.x = __dadd_rn(z.x, pd);
+      f = cmk(__dmul_rn(X.x, lk), __dmul_rn(X.y, lk));
     } else if (u == 1) {
-      z.x -= pd;
-      f = cscale(crcp(X), -lk);
+      z.x = __dadd_rn(z.x, -pd);
+      const double r = __ddiv_rn(-lk, __fma_rn(X.x, X.x, __dmul_rn(X.y, X.y)));
+      f = cmk(__dmul_rn(X.x, r), __dmul_rn(-X.y, r));
     } else {
-      f = cmk(fma(-S.kappa, p.x, o.x), fma(-S.kappa, p.y, o.y));
+      f = cmk(__fma_rn(-S.kappa, p.x, o.x), __fma_rn(-S.kappa, p.y, o.y));
     }
-    f = cmul(f, G);
-    const double2 z2 = cmul(z, z), z3 = cmul(z2, z), z4 = cmul(z2, z2);
+    f = cmul_rn(f, G);
+    const double2 z2 = cmul_rn(z, z), z3 = cmul_rn(z2, z), z4 = cmul_rn(z2, z2);
 #pragma unroll
     for (int F = 0; F < 3; ++F) {
       const double* c = lm + F * 10 + (u == 2 ? 5 : 0);
-      const double2 q = cmk(fma(c[4], z4.x, fma(c[3], z3.x, fma(c[2], z2.x, fma(c[1], z.x, c[0])))),
-                            fma(c[4], z4.y, fma(c[3], z3.y, fma(c[2], z2.y, c[1] * z.y))));
-      sum[F] = cadd(sum[F], cmul(f, q));
+      const double2 q =
+          cmk(__fma_rn(c[4], z4.x, __fma_rn(c[3], z3.x, __fma_rn(c[2], z2.x, __fma_rn(c[1], z.x, c[0])))),
+              __fma_rn(c[4], z4.y, __fma_rn(c[3], z3.y, __fma_rn(c[2], z2.y, __dmul_rn(c[1], z.y)))));
+      const double2 t = cmul_rn(f, q);
+      sum[F] = cmk(__dadd_rn(sum[F].x, t.x), __dadd_rn(sum[F].y, t.y));
     }
   }
+  if (WARP)
+    for (int F = 0; F < 3; ++F) {
+      const double2 t0 = c_from(sum[F], 0), t1 = c_from(sum[F], 1), t2 = c_from(sum[F], 2);
+      sum[F] = cmk(__dadd_rn(__dadd_rn(t0.x, t1.x), t2.x), __dadd_rn(__dadd_rn(t0.y, t1.y), t2.y));
+    }
   const double fi = -S.dpperp * ALPS_PI * 2.0 * ALPS_PI * (double)lf * ql;
 #pragma unroll
-  for (int e = 0; e < 6; ++e) {
-    const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
-    double2 v = cscale(sum[fam], pref[e] * fi);
-    if (e == 4 || e == 5) v = cmul(v, p);
-    if (e == 2) v = cmul(cmul(p, p), v);
+  for (int t = 0; t < (WARP ? 1 : 6); ++t) {
+    const int e = WARP ? min(lane, 5) : t, fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
+    double pf = pref[0];
+#pragma unroll
+    for (int q = 1; q < 6; ++q)
+      if (e == q) pf = pref[q];
+    pf = __dmul_rn(pf, fi);
+    const double2 sf = fam == 0 ? sum[0] : (fam == 1 ? sum[1] : sum[2]);
+    double2 v = cmk(__dmul_rn(sf.x, pf), __dmul_rn(sf.y, pf));
+    if (e == 2 || e == 4 || e == 5) v = cmul_rn(v, p);
+    if (e == 2) v = cmul_rn(v, p);
     // pref ifac: real pref -> i pref fi; imaginary i pref -> -(pref fi)
-    res[e] = (e == 3 || e == 5) ? cmk(-v.x, -v.y) : cmk(-v.y, v.x);
+    res[t] = (e == 3 || e == 5) ? cmk(-v.x, -v.y) : cmk(-v.y, v.x);
   }
   return true;
 }
@@ -1618,16 +1669,10 @@ struct __align__(16) ResItem {
   int w, s, pad;      // omega, species
   long long slot;     // the item's slot (its output row)
 };
-// prefactor e of an item as the complex number t_prefactors gives
-__device__ __forceinline__ double2 item_pref(const ResItem& it, int e) {
-  return (e == 3 || e == 5) ? cmk(0.0, it.pref[e]) : cmk(it.pref[e], 0.0);
-}
-
-// An item's per-lane part: geometry, prefactors, principal-value constants,
-// Landau term where it factorises (in res).  Returns the work left (ResItem).
-__device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, double2 o, int nn, PvItem& pv,
-                                        double pref[6], double2 res[6], int& lf) {
-  const int n = nn < 0 ? -nn : nn;
+// An item's geometry, prefactors and principal-value constants.  Returns the
+// work left (ResItem; 8: a Landau term that factorises).
+__device__ __forceinline__ int res_core(const DispArgs& a, const SpecDev& S, double2 o, int nn, PvItem& pv,
+                                        double pref[6], int& lf) {
   {
     // t_prefactors' nonzero parts, with 1/z
     const double dz = (double)nn * S.iz;
@@ -1637,8 +1682,6 @@ __device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, dou
     pref[3] = pref[4] = k1 * dz;
     pref[5] = -k2;
   }
-#pragma unroll
-  for (int e = 0; e < 6; ++e) res[e] = cmk(0.0, 0.0);
   const ResGeom g = res_geometry_of(S, a.sys, o, nn);
   lf = (o.y < 0.0) ? 2 : ((o.y == 0.0) ? 1 : 0);
   int work = 0;
@@ -1666,23 +1709,48 @@ __device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, dou
     pv.oxd = df_of(o.x);
     pv.oyd = df_of(o.y);
   }
-  if (lf > 0) {
-    const double2 p = cmk(g.pr, g.pi);
-    const bool fact = landau_factorises(S, p);
-    if (fact && !S.df_sums) {
-      if (!landau_lane_fp64(S, o, p, lf, n, pref, res)) work |= 2;
-      if (n == 0) res[0] = res[3] = res[4] = cmk(0.0, 0.0);
-    } else if (fact) {
-      const dflt izd = {S.izh, S.izl}, dzd = df_mul({(float)nn, 0.0f}, izd);
-      const dflt k2d = {a.sys.k2h, a.sys.k2l}, xyd = df_mul({a.sys.k1h, a.sys.k1l}, dzd);
-      const dflt prefd[6] = {df_mul(dzd, dzd), k2d, k2d, xyd, xyd, df_neg(k2d)};
-      landau_lane(S, {pv.oxd, pv.oyd}, p, lf, n, prefd, res);
-      if (n == 0) res[0] = res[3] = res[4] = cmk(0.0, 0.0);
-    } else {
-      work |= 2;
+  if (lf > 0) work |= landau_factorises(S, cmk(g.pr, g.pi)) ? 8 : 2;
+  return work;
+}
+// compiled once for the forms that have to agree bit for bit
+__device__ __noinline__ int res_core_call(const DispArgs& a, const SpecDev& S, double2 o, int nn, PvItem& pv,
+                                          double pref[6], int& lf) {
+  return res_core(a, S, o, nn, pv, pref, lf);
+}
+// the factorised Landau term of an item (landau_lane); false: by rows
+template <bool WARP>
+__device__ __forceinline__ bool res_landau(const DispArgs& a, const SpecDev& S, double2 o, const PvItem& pv, int lf,
+                                           const double pref[6], double2* res) {
+  const int nn = pv.nn, n = nn < 0 ? -nn : nn;
+  const double2 p = cmk(pv.pr, pv.pim);
+  if (S.df_sums) {
+    const dflt izd = {S.izh, S.izl}, dzd = df_mul({(float)nn, 0.0f}, izd);
+    const dflt k2d = {a.sys.k2h, a.sys.k2l}, xyd = df_mul({a.sys.k1h, a.sys.k1l}, dzd);
+    const dflt prefd[6] = {df_mul(dzd, dzd), k2d, k2d, xyd, xyd, df_neg(k2d)};
+    landau_lane<WARP>(S, {pv.oxd, pv.oyd}, p, lf, n, prefd, res);
+  } else if (!landau_lane_fp64<WARP>(S, o, p, lf, n, pref, res)) {
+    return false;
+  }
+  if (n == 0) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int t = 0; t < (WARP ? 1 : 6); ++t) {
+      const int e = WARP ? min(lane, 5) : t;
+      if (e == 0 || e == 3 || e == 4) res[t] = cmk(0.0, 0.0);
     }
   }
-  return work;
+  return true;
+}
+// an item's per-lane part: the above and the Landau term where it factorises
+// (in res).  Returns the work left.
+template <bool ONCE>
+__device__ __forceinline__ int res_item(const DispArgs& a, const SpecDev& S, double2 o, int nn, PvItem& pv,
+                                        double pref[6], double2 res[6], int& lf) {
+#pragma unroll
+  for (int e = 0; e < 6; ++e) res[e] = cmk(0.0, 0.0);
+  const int work = ONCE ? res_core_call(a, S, o, nn, pv, pref, lf) : res_core(a, S, o, nn, pv, pref, lf);
+  const bool rows = (work & 8) && !res_landau<false>(a, S, o, pv, lf, pref, res);
+  return (work & 7) | (rows ? 2 : 0);
 }
 
 // a slot's order in k_resonant_multi's list mode: the order and the work that
@@ -1752,6 +1820,111 @@ inline int res_items_per_warp(long nslots, int warps_per_sm = 12) {
 }
 
 
+// The Landau term of one item by its rows, over the warp: added to out
+__device__ __noinline__ void landau_rows(const DispArgs& a, const SpecDev& S, double2 o, double2 p, int nn, int lf,
+                                         const double* pref, double2* wk, double2* out) {
+  const int lane = threadIdx.x % 32, N = S.N, n = nn < 0 ? -nn : nn;
+  const double kpar = a.sys.kpar;
+  double2* frow = wk;                  // f(i, p_res)
+  double2* fpr = frow + (N + 1);       // f(i, p_res + dppar)
+  double2* fmr = fpr + (N + 1);        // f(i, p_res - dppar)
+  double2* tb = wk + res_region(N, a.sys.M_I) + 32 * (sizeof(ResItem) / sizeof(double2));  // values handed to lanes 0-5
+    const double pd = S.dppar_abs, dpp = S.dpperp;
+    const double vA = a.sys.vA;
+    if (S.fit_aux) {
+      // Maxwellian terms: f = sum_f a0 exp(-p2 (p - p3)^2)
+      const int nf = S.nf;
+      for (int i = lane; i <= N; i += 32) {
+        double2 f0 = cmk(0, 0), fp = cmk(0, 0), fm = cmk(0, 0);
+        for (int f = 0; f < nf; ++f) {
+          const double* aux = S.fit_aux + ((size_t)i * nf + f) * 4;  // a0, p2, p3, exp(-p2 D^2)
+          double p2 = aux[1];
+          double2 d = cmk(p.x - aux[2], p.y);
+          double2 E0 = cexp_d(cscale(cmul(d, d), -p2));
+          double2 G = cscale(E0, aux[0]);
+          double2 ax = cscale(d, -2.0 * p2 * pd);
+          double2 X, Xi;
+          if (fabs(ax.x) < 600.0) {
+            X = cexp_d(ax);
+            Xi = crcp(X);
+            double2 Gc = cscale(G, aux[3]);
+            fp = cadd(fp, cmul(Gc, X));
+            fm = cadd(fm, cmul(Gc, Xi));
+          } else {
+            double2 dp = cadd(d, cmk(pd, 0.0)), dm = csub(d, cmk(pd, 0.0));
+            fp = cadd(fp, cscale(cexp_d(cscale(cmul(dp, dp), -p2)), aux[0]));
+            fm = cadd(fm, cscale(cexp_d(cscale(cmul(dm, dm), -p2)), aux[0]));
+          }
+          f0 = cadd(f0, G);
+        }
+        frow[i] = f0;
+        fpr[i] = fp;
+        fmr[i] = fm;
+      }
+    } else {
+      for (int i = lane; i <= N; i += 32) {
+        frow[i] = eval_fit_d(S, vA, i, p);
+        fpr[i] = eval_fit_d(S, vA, i, cadd(p, cmk(pd, 0.0)));
+        fmr[i] = eval_fit_d(S, vA, i, csub(p, cmk(pd, 0.0)));
+      }
+    }
+    __syncwarp();
+    bool zero = false;
+    double2 sums[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+    const double ql = S.qs / fabs(kpar);
+    const int L = N + 1;
+    for (int i = lane; i <= N; i += 32) {
+      double2 fpi = fpr[i], fpf = fmr[i];
+      double2 dfperp, dfpar;
+      double h;
+      if (i == 0) {
+        dfperp = cscale(csub(frow[1], frow[0]), 1.0 / dpp);
+        h = 0.5;
+      } else if (i == N) {
+        dfperp = cscale(csub(frow[N], frow[N - 1]), 1.0 / dpp);
+        h = 0.5;
+      } else {
+        // |f| = 0 exactly when both parts are
+        auto nil = [](double2 x) { return x.x == 0.0 && x.y == 0.0; };
+        if (nil(fpi) || nil(fpf) || nil(frow[i + 1])) zero = true;
+        dfperp = cscale(csub(frow[i + 1], frow[i - 1]), 1.0 / (2.0 * dpp));
+        h = (i == N - 1) ? 0.5 : 1.0;
+      }
+      dfpar = cscale(csub(fpi, fpf), 1.0 / (2.0 * pd));
+      double pp_i = S.pperp[i];
+      // (q/|kpar|) ((pperp dfpar - p dfperp) kpar/m + omega dfperp)
+      double2 Lv = cscale(cadd(cscale(csub(cscale(dfpar, pp_i), cmul(p, dfperp)), kpar / S.ms), cmul(o, dfperp)),
+                          ql);
+      double J = S.bessel[(size_t)(n + 1) * L + i];
+      double Jp = (n == 0) ? -S.bessel[(size_t)2 * L + i]
+                           : 0.5 * (S.bessel[(size_t)n * L + i] - S.bessel[(size_t)(n + 2) * L + i]);
+      sums[0] = cadd(sums[0], cscale(Lv, h * (J * J)));
+      sums[1] = cadd(sums[1], cscale(Lv, h * ((pp_i * pp_i) * Jp * Jp)));
+      sums[2] = cadd(sums[2], cscale(Lv, h * (pp_i * J * Jp)));
+    }
+    zero = __any_sync(0xffffffffu, zero);
+    for (int F = 0; F < 3; ++F)
+      for (int off = 16; off > 0; off >>= 1) {
+        sums[F].x += __shfl_xor_sync(0xffffffffu, sums[F].x, off);
+        sums[F].y += __shfl_xor_sync(0xffffffffu, sums[F].y, off);
+      }
+    if (!zero) {
+      // landau_e = -pref_e c_e(p) Sigma_F(e) * i dpperp 2 pi^2, lanes 0-5
+      if (lane == 0)
+        for (int F = 0; F < 3; ++F) tb[F] = sums[F];
+      __syncwarp();
+      if (lane < 6 && !(n == 0 && (lane == 0 || lane == 3 || lane == 4))) {
+        const int e = lane;
+        const double2 ce = (e == 2) ? cmul(p, p) : ((e == 4 || e == 5) ? p : cmk(1.0, 0.0));
+        const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
+        const double2 ifac = cmk(0.0, -dpp * ALPS_PI * 2.0 * ALPS_PI * (double)lf);
+        const double2 land = cmul(cmul((e == 3 || e == 5 ? cmk(0.0, pref[e]) : cmk(pref[e], 0.0)), ce), tb[fam]);
+        out[e] = cadd(out[e], cmul(land, ifac));
+      }
+      __syncwarp();
+    }
+}
+
 // Up to 32 resonant items, one per lane (item < 0: none): the per-lane part,
 // then the principal-value sums and Landau rows item by item over the warp.
 // sv is the item's order (list: what k_resonant_lanes left of it), wk the
@@ -1761,11 +1934,7 @@ __device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __
   const int lane = threadIdx.x % 32;
   const int S_ = a.sys.nspec;
   const int N = a.sp[0].N;  // every species has the same p_perp grid
-  double2* frow = wk;                                      // f(i, p_res)
-  double2* fpr = frow + (N + 1);                           // f(i, p_res + dppar)
-  double2* fmr = fpr + (N + 1);                            // f(i, p_res - dppar)
   ResItem* ri = reinterpret_cast<ResItem*>(wk + res_region(N, a.sys.M_I));
-  double2* tb = reinterpret_cast<double2*>(ri + 32);      // values handed to lanes 0-5
   // ---- one item per lane ----
   int work = 0;
   if (item >= 0) {
@@ -1778,7 +1947,7 @@ __device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __
     double pref[6];
     PvItem pv;
     int lf;
-    work = res_item(a, S, o, nn, pv, pref, res, lf);
+    work = res_item<true>(a, S, o, nn, pv, pref, res, lf);
     double2* out = items + item * 6;
     if (list) work &= (sv >> 16) & 3;  // the FP64 sums and the rows (never the double-float sums)
     else
@@ -1799,11 +1968,9 @@ __device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __
     pend &= pend - 1;
     const ResItem& it = ri[il];
     const int s = it.s, w = it.w, nn = it.pv.nn;
-    const int n = nn < 0 ? -nn : nn;
     const int wkk = it.work & 7, lf = it.work >> 3;
     const SpecDev& S = a.sp[s];
     const double2 o = om[w];
-    const double kpar = a.sys.kpar;
     double2* out = items + it.slot * 6;
 
     if (wkk & 1) {
@@ -1811,105 +1978,29 @@ __device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __
       else pv_warp<double>(S, a.sys, it.pv, o, it.pref, wk, out);
     }
 
-    if (wkk & 2) {
-      const double2 p = cmk(it.pv.pr, it.pv.pim);
-      const double pd = S.dppar_abs, dpp = S.dpperp;
-      const double vA = a.sys.vA;
-      if (S.fit_aux) {
-        // Maxwellian terms: f = sum_f a0 exp(-p2 (p - p3)^2)
-        const int nf = S.nf;
-        for (int i = lane; i <= N; i += 32) {
-          double2 f0 = cmk(0, 0), fp = cmk(0, 0), fm = cmk(0, 0);
-          for (int f = 0; f < nf; ++f) {
-            const double* aux = S.fit_aux + ((size_t)i * nf + f) * 4;  // a0, p2, p3, exp(-p2 D^2)
-            double p2 = aux[1];
-            double2 d = cmk(p.x - aux[2], p.y);
-            double2 E0 = cexp_d(cscale(cmul(d, d), -p2));
-            double2 G = cscale(E0, aux[0]);
-            double2 ax = cscale(d, -2.0 * p2 * pd);
-            double2 X, Xi;
-            if (fabs(ax.x) < 600.0) {
-              X = cexp_d(ax);
-              Xi = crcp(X);
-              double2 Gc = cscale(G, aux[3]);
-              fp = cadd(fp, cmul(Gc, X));
-              fm = cadd(fm, cmul(Gc, Xi));
-            } else {
-              double2 dp = cadd(d, cmk(pd, 0.0)), dm = csub(d, cmk(pd, 0.0));
-              fp = cadd(fp, cscale(cexp_d(cscale(cmul(dp, dp), -p2)), aux[0]));
-              fm = cadd(fm, cscale(cexp_d(cscale(cmul(dm, dm), -p2)), aux[0]));
-            }
-            f0 = cadd(f0, G);
-          }
-          frow[i] = f0;
-          fpr[i] = fp;
-          fmr[i] = fm;
-        }
-      } else {
-        for (int i = lane; i <= N; i += 32) {
-          frow[i] = eval_fit_d(S, vA, i, p);
-          fpr[i] = eval_fit_d(S, vA, i, cadd(p, cmk(pd, 0.0)));
-          fmr[i] = eval_fit_d(S, vA, i, csub(p, cmk(pd, 0.0)));
-        }
-      }
-      __syncwarp();
-      bool zero = false;
-      double2 sums[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-      const double ql = S.qs / fabs(kpar);
-      const int L = N + 1;
-      for (int i = lane; i <= N; i += 32) {
-        double2 fpi = fpr[i], fpf = fmr[i];
-        double2 dfperp, dfpar;
-        double h;
-        if (i == 0) {
-          dfperp = cscale(csub(frow[1], frow[0]), 1.0 / dpp);
-          h = 0.5;
-        } else if (i == N) {
-          dfperp = cscale(csub(frow[N], frow[N - 1]), 1.0 / dpp);
-          h = 0.5;
-        } else {
-          // |f| = 0 exactly when both parts are
-          auto nil = [](double2 x) { return x.x == 0.0 && x.y == 0.0; };
-          if (nil(fpi) || nil(fpf) || nil(frow[i + 1])) zero = true;
-          dfperp = cscale(csub(frow[i + 1], frow[i - 1]), 1.0 / (2.0 * dpp));
-          h = (i == N - 1) ? 0.5 : 1.0;
-        }
-        dfpar = cscale(csub(fpi, fpf), 1.0 / (2.0 * pd));
-        double pp_i = S.pperp[i];
-        // (q/|kpar|) ((pperp dfpar - p dfperp) kpar/m + omega dfperp)
-        double2 Lv = cscale(cadd(cscale(csub(cscale(dfpar, pp_i), cmul(p, dfperp)), kpar / S.ms), cmul(o, dfperp)),
-                            ql);
-        double J = S.bessel[(size_t)(n + 1) * L + i];
-        double Jp = (n == 0) ? -S.bessel[(size_t)2 * L + i]
-                             : 0.5 * (S.bessel[(size_t)n * L + i] - S.bessel[(size_t)(n + 2) * L + i]);
-        sums[0] = cadd(sums[0], cscale(Lv, h * (J * J)));
-        sums[1] = cadd(sums[1], cscale(Lv, h * ((pp_i * pp_i) * Jp * Jp)));
-        sums[2] = cadd(sums[2], cscale(Lv, h * (pp_i * J * Jp)));
-      }
-      zero = __any_sync(0xffffffffu, zero);
-      for (int F = 0; F < 3; ++F)
-        for (int off = 16; off > 0; off >>= 1) {
-          sums[F].x += __shfl_xor_sync(0xffffffffu, sums[F].x, off);
-          sums[F].y += __shfl_xor_sync(0xffffffffu, sums[F].y, off);
-        }
-      if (!zero) {
-        // landau_e = -pref_e c_e(p) Sigma_F(e) * i dpperp 2 pi^2, lanes 0-5
-        if (lane == 0)
-          for (int F = 0; F < 3; ++F) tb[F] = sums[F];
-        __syncwarp();
-        if (lane < 6 && !(n == 0 && (lane == 0 || lane == 3 || lane == 4))) {
-          const int e = lane;
-          const double2 ce = (e == 2) ? cmul(p, p) : ((e == 4 || e == 5) ? p : cmk(1.0, 0.0));
-          const int fam = (e == 1) ? 1 : ((e == 3 || e == 5) ? 2 : 0);
-          const double2 ifac = cmk(0.0, -dpp * ALPS_PI * 2.0 * ALPS_PI * (double)lf);
-          const double2 land = cmul(cmul(item_pref(it, e), ce), tb[fam]);
-          out[e] = cadd(out[e], cmul(land, ifac));
-        }
-        __syncwarp();
-      }
-    }
+    if (wkk & 2) landau_rows(a, S, o, cmk(it.pv.pr, it.pv.pim), nn, lf, it.pref, wk, out);
     __syncwarp();  // the next item reuses the region
   }
+}
+
+// One item by a warp of its own (small batches): what resonant_group does for
+// it, with the factorised Landau term's parts over the lanes too.
+__device__ __noinline__ void resonant_one(const DispArgs& a, const SpecDev& S, double2 o, int nn, double2* wk,
+                                          double2* out) {
+  const int lane = threadIdx.x & 31;
+  PvItem pv;
+  double pref[6];
+  int lf;
+  int work = res_core_call(a, S, o, nn, pv, pref, lf);
+  double2 res = cmk(0.0, 0.0);
+  if ((work & 8) && !res_landau<true>(a, S, o, pv, lf, pref, &res)) work |= 2;
+  if (lane < 6) out[lane] = res;
+  __syncwarp();
+  if (work & 1) {
+    if (work & 4) pv_warp<dflt>(S, a.sys, pv, o, pref, wk, out);
+    else pv_warp<double>(S, a.sys, pv, o, pref, wk, out);
+  }
+  if (work & 2) landau_rows(a, S, o, cmk(pv.pr, pv.pim), nn, lf, pref, wk, out);
 }
 
 __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape& sh, const double2* __restrict__ om,
@@ -2169,7 +2260,7 @@ __device__ __forceinline__ void lanes_body(const DispArgs& a, const DispShape& s
           double pref[6];
           PvItem pv;
           int lf;
-          int work = res_item(a, S, o, nn, pv, pref, res, lf);
+          int work = res_item<false>(a, S, o, nn, pv, pref, res, lf);
           cdf X[6];
           if ((work & 5) == 5 && pv_lane(S, a.sys, pv, o, col, X)) {
             const double scale = S.Vscale[n] * pv.sm * S.pvc;
@@ -2276,31 +2367,40 @@ __device__ __noinline__ void finalize_warp(const DispArgs& a, const DispShape& s
                              : cscale(cscale(cscale(cscale(denom, vA), vA), kperp), kperp);
   }
   double eps = 0.0;  // component c of the sum over species (lanes 0..11)
+  const int cnts = lane < S_ ? __ldcg(count + (size_t)w * S_ + lane) : 0;
   for (int s = 0; s < S_; ++s) {
     const SpecDev& S = a.sp[s];
     const size_t ws = (size_t)w * S_ + s, base = ws * sh.nchunk;
     double v = 0.0, lw[3] = {0.0, 0.0, 0.0};
     if (h < 2) {
-      const int nch = sh.nch[s];
+      const int nch = sh.nch[s], cnt = __shfl_sync(0xffffffu, cnts, s);
       const double* pt = reinterpret_cast<const double*>(part + base * 6) + c;
-#pragma unroll 4
-      for (int ch = h; ch < nch; ch += 2) {
-        const double x = __ldcg(pt + (size_t)ch * 12);
-        v += x;
-        if (ext)
-          for (int l = 0; l < 3; ++l)
-            if (ch - S.nmax == l - 1) lw[l] += x;
-      }
-      const int cnt = __ldcg(count + ws);
       const double* it = reinterpret_cast<const double*>(items + ws * a.rcap * 6) + c;
-#pragma unroll 2
-      for (int r = h; r < cnt; r += 2) {
-        const double x = __ldcg(it + (size_t)r * 12);
-        v += x;
-        if (ext) {
-          const int nn = __ldcg(slot_nn + ws * a.rcap + r);
-          for (int l = 0; l < 3; ++l)
-            if (nn == l - 1) lw[l] += x;
+      // up to eight chunks and four items of a lane are in flight together
+      for (int ch = h; ch < nch; ch += 16) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = ch + 2 * u < nch ? __ldcg(pt + (size_t)(ch + 2 * u) * 12) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          v += x[u];
+          if (ext)
+            for (int l = 0; l < 3; ++l)
+              if (ch + 2 * u - S.nmax == l - 1) lw[l] += x[u];
+        }
+      }
+      for (int r = h; r < cnt; r += 8) {
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = r + 2 * u < cnt ? __ldcg(it + (size_t)(r + 2 * u) * 12) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          v += x[u];
+          if (ext && r + 2 * u < cnt) {
+            const int nn = __ldcg(slot_nn + ws * a.rcap + r + 2 * u);
+            for (int l = 0; l < 3; ++l)
+              if (nn == l - 1) lw[l] += x[u];
+          }
         }
       }
       if (S.relat) {
@@ -2596,7 +2696,7 @@ __device__ __forceinline__ int small_slot(const DispArgs& a, const DispJob& J, d
   }
   if (found) {
     if (lane == 0) J.slot_nn[slot] = nn;
-    resonant_group(a, J.om, J.items, wk, lane == 0 ? slot : -1, nn, false);
+    resonant_one(a, S, o, nn, wk, J.items + (size_t)slot * 6);
   }
   return w;
 }
@@ -2925,22 +3025,25 @@ uint64_t tune_epoch() { return g_tune_epoch.load(); }
 // lanes' own set-up counts.  Within a class the shape is the same for every
 // n, and so are a frequency's sums (csize 0: as many orders as leave twice 32
 // warps per SM, where a batch has warps to spare).  The lines lie where the
-// next form measured faster (us of the pole sums, 128x256 grid, 73 signed
-// orders).  Mixed path: n = 64: 27 with 32 lanes, 30 with 16; 128: 34 with
-// 16, 41 with 32 or 8; 512: 59 with 8, 72 with 16, 80 with 4; 2048: 150 with
-// 8 or 4, 167 with 2; 4096: 256 with 1, 262 with 2, 269 with 4.  At a given
-// number of lanes about one order per lane is best (512 frequencies, 8 lanes:
-// 59 with 8 orders, 64 with 4, 81 with 2).  FP64 path (lanes/orders): 8: 22
-// with 32/1, 31 with 32/2; 64: 59 with 32/4, 76 with 16/8; 256: 138 with 16/8,
-// 163 with 8/8; 2048: 579 with 8/8, 627 with 16/16, 699 with 4/8; 16384: 3535
-// with 8/64, 4388 with 8/16, 4606 with 1/16.
+// next form measured faster.  Small batches, the one launch in us (lanes/
+// orders): mixed 128x256 grid, 73 signed orders, n = 1: 33 with 32/4, 38 with
+// 32/8; 31: 39 with 32/4, 45 with 32/8; 60x120 grid, 113 orders, 31: 41 with
+// 32/8, 45 with 32/4; 64: 52 with 32/8, 68 with 32/4; FP64, 120x240 grid, 138
+// orders, n = 1: 38 with 32/1, 44 with 32/2; 8: 42 with 32/4, 69 with 32/1;
+// 31: 64 with 32/8, 78 with 32/4; 64: 87 with 32/16, 97 with 16/8.  Larger
+// ones, the pole sums in us, 128x256 grid: mixed n = 512: 59 with 8 lanes, 72
+// with 16, 80 with 4; 2048: 150 with 8 or 4, 167 with 2; 4096: 256 with 1, 262
+// with 2, 269 with 4; about one order per lane is best (512, 8 lanes: 59 with
+// 8 orders, 64 with 4, 81 with 2).  FP64 n = 256: 138 with 16/8, 163 with 8/8;
+// 2048: 579 with 8/8, 627 with 16/16, 699 with 4/8; 16384: 3535 with 8/64,
+// 4388 with 8/16, 4606 with 1/16.
 void default_shape(long u, bool mixed, int* lanes, long* csize) {
   if (mixed) {
-    *lanes = u < 220 ? 32 : (u < 440 ? 16 : (u < 3000 ? 8 : (u < 7700 ? 4 : 1)));
-    *csize = u < 75 ? 8 : (u < 440 ? 4 : (u < 3000 ? 8 : (u < 7700 ? 4 : 0)));
+    *lanes = u < 300 ? 32 : (u < 440 ? 16 : (u < 3000 ? 8 : (u < 7700 ? 4 : 1)));
+    *csize = u < 100 ? 4 : (u < 3000 ? 8 : (u < 7700 ? 4 : 0));
   } else {
-    *lanes = u < 200 ? 32 : (u < 600 ? 16 : 8);
-    *csize = u < 40 ? 1 : (u < 200 ? 4 : (u < 20000 ? 8 : 64));
+    *lanes = u < 400 ? 32 : (u < 600 ? 16 : 8);
+    *csize = u < 8 ? 1 : (u < 50 ? 4 : (u < 180 ? 8 : (u < 400 ? 16 : (u < 20000 ? 8 : 64))));
   }
 }
 
