@@ -541,35 +541,56 @@ int fit_smem_optin() {
 // determine_nmax for one species: the smallest n >= 1 with
 // max_i |J_n(z_i)| <= Bessel_zero, z_i = k_perp pperp_i / q, or n = limit.
 // The maximum exceeds the cutoff exactly when some node's |J_n| does.  The
-// orders go in chunks of NMAX_CHUNK: first one thread per order tests the
-// node nearest J_n's largest maximum (z = n + 0.81 n^(1/3); for orders past
-// the grid's last z that is the last node, where |J_n| is largest), which
-// settles nearly every order below the answer with one alps_bessj call;
-// then the unsettled orders, in increasing order, test every node with the
-// whole block, and the first with none above the cutoff is the answer.
-// Each order's decision is the reference's: the same alps_bessj values
-// against the same cutoff.  (The FP64 pipe is narrow on this part: one
-// call of order n costs about 5 (n + sqrt(40 n)) FP64 operations.)
+// orders go in chunks of NMAX_CHUNK, one thread each:
+//   * orders whose n lies above the grid's last z (z < 0.95 n): J_n rises on
+//     (0, n), so the last node decides.  Debye's leading term exp(n (tanh a -
+//     a))/sqrt(2 pi n tanh a), z = n / cosh a, is an upper bound of J_n(z) and
+//     within a third of it there, so where it is a factor 8 off the cutoff
+//     either way, it decides; one alps_bessj call at the last node otherwise.
+//   * the others test the node nearest J_n's largest maximum (z = n + 0.81
+//     n^(1/3)) with one alps_bessj call, which settles nearly all of them.
+// Then the orders still open, in increasing order, test every node with the
+// whole block, and the first with none above the cutoff is the answer.  Each
+// order's decision is the reference's, alps_bessj's values against the cutoff.
+// One call of order n costs about 5 (n + sqrt(40 n)) dependent FP64
+// operations, and the chain of calls is the time: without the estimate, over
+// chunks of 128 orders, 103 us for an answer of 20 to 30 (96 rows), 32 us so.
 #define NMAX_CHUNK 128
 __device__ void nmax_body(const double* __restrict__ pperp, int N, double kperp, double qs, double bzero, int limit,
                           int* nmax_out, unsigned* settled) {
   const int t = threadIdx.x;
   const double zs = fabs(qs) / kperp, dp = pperp[1] - pperp[0];
-  auto above = [&](int nn, int i) {
-    const double z = __ddiv_rn(__dmul_rn(kperp, pperp[i]), qs);
-    return fabs(alps_bessj(nn, z)) > bzero;
-  };
+  auto zat = [&](int i) { return __ddiv_rn(__dmul_rn(kperp, pperp[i]), qs); };
+  auto above = [&](int nn, int i) { return fabs(alps_bessj(nn, zat(i))) > bzero; };
+  const float zlast = fabsf((float)zat(N));
+  const bool rising = pperp[0] >= 0.0 && dp > 0.0;  // |z| grows with the node
+  const float lcut = (bzero >= 1e-290 && bzero <= 1.0) ? (float)log(bzero) : nanf("");
+  unsigned* below = settled + NMAX_CHUNK / 32;
   for (int base = 1;; base += NMAX_CHUNK) {
     if (t < NMAX_CHUNK) {  // whole warps (NMAX_CHUNK is a multiple of 32)
       const int nn = base + t;
-      bool hit = false;
+      bool hit = false, none = false;  // some node above the cutoff; certainly no node
       if (nn < limit) {
-        const double u = ((nn + 0.81 * cbrt((double)nn)) * zs - pperp[0]) / dp;
-        const int i0 = (u >= 0.0 && u <= (double)N) ? (int)rint(u) : ((u > 0.0 || u != u) ? N : 0);
-        hit = above(nn, i0);
+        const float x = zlast / (float)nn;
+        if (rising && x < 0.95f && x > 1e-30f) {
+          const float ta = sqrtf((1.0f - x) * (1.0f + x));
+          // n (tanh a - a): a = log((1 + ta)/x)
+          const float d = (float)nn * (ta - logf((1.0f + ta) / x)) - 0.5f * logf(6.2831853f * (float)nn * ta) - lcut;
+          const float tol = 2.08f + 1e-6f * (float)nn * (1.0f + fabsf(logf(x)));
+          if (d > tol) hit = true;
+          else if (d < -tol) none = true;
+          else hit = above(nn, N), none = !hit;
+        } else {
+          const double u = ((nn + 0.81 * cbrt((double)nn)) * zs - pperp[0]) / dp;
+          const int i0 = (u >= 0.0 && u <= (double)N) ? (int)rint(u) : ((u > 0.0 || u != u) ? N : 0);
+          hit = above(nn, i0);
+        }
       }
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if ((t & 31) == 0) settled[t >> 5] = m;
+      const unsigned m = __ballot_sync(0xffffffffu, hit), q = __ballot_sync(0xffffffffu, none);
+      if ((t & 31) == 0) {
+        settled[t >> 5] = m;
+        below[t >> 5] = q;
+      }
     }
     __syncthreads();
     for (int k = 0; k < NMAX_CHUNK; ++k) {
@@ -580,8 +601,11 @@ __device__ void nmax_body(const double* __restrict__ pperp, int N, double kperp,
       }
       if ((settled[k >> 5] >> (k & 31)) & 1u) continue;
       bool hit = false;
-      for (int i = t; i <= N && !hit; i += blockDim.x) hit = above(nn, i);
-      if (!__syncthreads_or(hit)) {
+      if (!((below[k >> 5] >> (k & 31)) & 1u)) {
+        for (int i = t; i <= N && !hit; i += blockDim.x) hit = above(nn, i);
+        hit = __syncthreads_or(hit);
+      }
+      if (!hit) {
         if (t == 0) *nmax_out = nn;
         return;
       }
@@ -592,7 +616,7 @@ __device__ void nmax_body(const double* __restrict__ pperp, int N, double kperp,
 
 __global__ void k_nmax(const double* __restrict__ pperp, int N, double kperp, double qs, double bzero,
                        int limit, int* nmax_out) {
-  __shared__ unsigned settled[NMAX_CHUNK / 32];
+  __shared__ unsigned settled[2 * (NMAX_CHUNK / 32)];
   nmax_body(pperp, N, kperp, qs, bzero, limit, nmax_out, settled);
 }
 
@@ -609,7 +633,7 @@ struct NmaxJob {
 namespace {
 
 __global__ void k_nmax_many(const NmaxJob* __restrict__ jobs, int n, int limit) {
-  __shared__ unsigned settled[NMAX_CHUNK / 32];
+  __shared__ unsigned settled[2 * (NMAX_CHUNK / 32)];
   if ((int)blockIdx.x >= n) return;
   const NmaxJob& J = jobs[blockIdx.x];
   nmax_body(J.pperp, J.N, J.kperp, J.qs, J.bzero, limit, J.out, settled);
