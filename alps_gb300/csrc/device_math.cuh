@@ -191,6 +191,59 @@ __device__ __forceinline__ void df_mac(dflt& acc, float vh, float vl, dflt r) {
   acc.l = __fadd_rn(acc.l, __fadd_rn(s.l, pl));
 }
 
+// Two double-float values at a time in packed FP32 instructions: the same
+// operations in the same order, so each half has the scalar form's bits.  A
+// packed instruction issues once for both halves and reads its three operands
+// at full rate (FMA chains: 112 lane operations a clock and SM packed, 74
+// scalar).  Pole sums of a 512x512 map: 5850 us scalar, 5150 packed, a third
+// fewer instructions and the FMA pipe busy 73 % of the time; one frequency in
+// one launch 36 and 31 us.
+struct dflt2 {
+  float2 h, l;
+};
+__device__ __forceinline__ float2 f2_all(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 f2_neg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 f2_sub(float2 a, float2 b) { return __fadd2_rn(a, f2_neg(b)); }
+__device__ __forceinline__ dflt2 d2_all(dflt a) { return {f2_all(a.h), f2_all(a.l)}; }
+__device__ __forceinline__ dflt2 d2_of(dflt a, dflt b) { return {make_float2(a.h, b.h), make_float2(a.l, b.l)}; }
+__device__ __forceinline__ dflt d2_x(const dflt2& a) { return {a.h.x, a.l.x}; }
+__device__ __forceinline__ dflt d2_y(const dflt2& a) { return {a.h.y, a.l.y}; }
+__device__ __forceinline__ dflt2 d2_neg(const dflt2& a) { return {f2_neg(a.h), f2_neg(a.l)}; }
+__device__ __forceinline__ void f2_two_sum(float2 a, float2 b, float2& s, float2& e) {
+  s = __fadd2_rn(a, b);
+  const float2 bb = f2_sub(s, a);
+  e = __fadd2_rn(f2_sub(a, f2_sub(s, bb)), f2_sub(b, bb));
+}
+__device__ __forceinline__ dflt2 d2_add(const dflt2& a, const dflt2& b) {
+  float2 s, e;
+  f2_two_sum(a.h, b.h, s, e);
+  e = __fadd2_rn(e, __fadd2_rn(a.l, b.l));
+  const float2 t = __fadd2_rn(s, e);
+  return {t, f2_sub(e, f2_sub(t, s))};
+}
+__device__ __forceinline__ dflt2 d2_mul(const dflt2& a, const dflt2& b) {
+  const float2 p = __fmul2_rn(a.h, b.h);
+  const float2 e = __ffma2_rn(a.h, b.l, __ffma2_rn(a.l, b.h, __ffma2_rn(a.h, b.h, f2_neg(p))));
+  const float2 t = __fadd2_rn(p, e);
+  return {t, f2_sub(e, f2_sub(t, p))};
+}
+// df_mac of both halves: acc += (vh + vl)(rh + rl)
+__device__ __forceinline__ void d2_mac(dflt2& acc, float2 vh, float2 vl, float2 rh, float2 rl) {
+  const float2 p = __fmul2_rn(vh, rh);
+  const float2 pl = __ffma2_rn(vh, rl, __ffma2_rn(vl, rh, __ffma2_rn(vh, rh, f2_neg(p))));
+  float2 e;
+  f2_two_sum(acc.h, p, acc.h, e);
+  acc.l = __fadd2_rn(acc.l, __fadd2_rn(e, pl));
+}
+// df_rcp_approx of both halves
+__device__ __forceinline__ dflt2 d2_rcp_approx(const dflt2& a) {
+  float2 r0;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.x) : "f"(a.h.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0.y) : "f"(a.h.y));
+  const float2 d = __ffma2_rn(f2_neg(a.l), r0, __ffma2_rn(f2_neg(a.h), r0, f2_all(1.0f)));
+  return {r0, __fmul2_rn(r0, __ffma2_rn(d, d, d))};
+}
+
 // 1/j! as float pairs (hi, lo), j = 0..18: the Taylor coefficients of
 // df_exp_scaled and df_cis
 __constant__ float c_inv_fact[19][2] = {

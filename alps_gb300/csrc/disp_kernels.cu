@@ -421,38 +421,63 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
             }
             for (int q = jc; q > 1; q >>= 1) st = cdf_mul(st, st);
           }
-          dflt U[12];
-          float Uf[12];
+          // sums over (g1, g2) side by side, real and imaginary parts; two
+          // terms' powers side by side, steps of t^2jc
+          dflt2 Ur[3], Ui[3];
+          float2 Fr[3], Fi[3];
 #pragma unroll
-          for (int q = 0; q < 12; ++q) {
-            U[q] = {0.0f, 0.0f};
-            Uf[q] = 0.0f;
+          for (int q = 0; q < 3; ++q) {
+            Ur[q] = Ui[q] = d2_all({0.0f, 0.0f});
+            Fr[q] = Fi[q] = f2_all(0.0f);
           }
-          int k = k0;
-          for (; k < K32; k += jc) {
+          auto term = [&](int k, dflt tx, dflt ty) {
             const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
             const float4 a0 = __ldg(m4), a1 = __ldg(m4 + 1), a2 = __ldg(m4 + 2);
-            const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+            const float2 h[3] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}};
+            const float2 l[3] = {{a1.z, a1.w}, {a2.x, a2.y}, {a2.z, a2.w}};
+            const dflt2 x2 = d2_all(tx), y2 = d2_all(ty);
 #pragma unroll
-            for (int b = 0; b < 6; ++b) {
-              df_mac(U[2 * b], hb[b], lb[b], tp.x);
-              df_mac(U[2 * b + 1], hb[b], lb[b], tp.y);
+            for (int q = 0; q < 3; ++q) {
+              d2_mac(Ur[q], h[q], l[q], x2.h, x2.l);
+              d2_mac(Ui[q], h[q], l[q], y2.h, y2.l);
             }
-            tp = cdf_mul(tp, st);
+          };
+          int k = k0;
+          cdf tl = tp;  // the first power left to the tail
+          if (k < K32) {
+            const cdf tb = cdf_mul(tp, st), s2 = cdf_mul(st, st);
+            dflt2 px = d2_of(tp.x, tb.x), py = d2_of(tp.y, tb.y);
+            const dflt2 sx = d2_all(s2.x), sy = d2_all(s2.y);
+            for (;;) {
+              if (k >= K32) {
+                tl = {d2_x(px), d2_x(py)};
+                break;
+              }
+              term(k, d2_x(px), d2_x(py));
+              k += jc;
+              if (k >= K32) {
+                tl = {d2_y(px), d2_y(py)};
+                break;
+              }
+              term(k, d2_y(px), d2_y(py));
+              k += jc;
+              const dflt2 nx = d2_add(d2_mul(px, sx), d2_neg(d2_mul(py, sy)));
+              py = d2_add(d2_mul(px, sy), d2_mul(py, sx));
+              px = nx;
+            }
           }
           if (k < K) {
             // the tail: terms below 2^-33 of the bound, in FP32
-            float fx = tp.x.h + tp.x.l, fy = tp.y.h + tp.y.l;
+            float fx = tl.x.h + tl.x.l, fy = tl.y.h + tl.y.l;
             const float gx = st.x.h + st.x.l, gy = st.y.h + st.y.l;
             for (; k < K; k += jc) {
               const float4* m4 = reinterpret_cast<const float4*>(mBn + (size_t)k * 12);
               const float4 a0 = __ldg(m4);
-              const float2 a1 = __ldg(reinterpret_cast<const float2*>(m4 + 1));
-              const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
+              const float2 h[3] = {{a0.x, a0.y}, {a0.z, a0.w}, __ldg(reinterpret_cast<const float2*>(m4 + 1))};
 #pragma unroll
-              for (int b = 0; b < 6; ++b) {
-                Uf[2 * b] = fmaf(hb[b], fx, Uf[2 * b]);
-                Uf[2 * b + 1] = fmaf(hb[b], fy, Uf[2 * b + 1]);
+              for (int q = 0; q < 3; ++q) {
+                Fr[q] = __ffma2_rn(h[q], f2_all(fx), Fr[q]);
+                Fi[q] = __ffma2_rn(h[q], f2_all(fy), Fi[q]);
               }
               const float nx = fx * gx - fy * gy;
               fy = fx * gy + fy * gx;
@@ -463,9 +488,8 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
           cdf Uw[3];
 #pragma unroll
           for (int fm = 0; fm < 3; ++fm) {
-            const int b1 = 2 * fm, b2 = 2 * fm + 1;
-            const cdf u1 = {df_add(U[2 * b1], {Uf[2 * b1], 0.0f}), df_add(U[2 * b1 + 1], {Uf[2 * b1 + 1], 0.0f})};
-            const cdf u2 = {df_add(U[2 * b2], {Uf[2 * b2], 0.0f}), df_add(U[2 * b2 + 1], {Uf[2 * b2 + 1], 0.0f})};
+            const cdf u1 = {df_add(d2_x(Ur[fm]), {Fr[fm].x, 0.0f}), df_add(d2_x(Ui[fm]), {Fi[fm].x, 0.0f})};
+            const cdf u2 = {df_add(d2_y(Ur[fm]), {Fr[fm].y, 0.0f}), df_add(d2_y(Ui[fm]), {Fi[fm].y, 0.0f})};
             Uw[fm] = om_comb(omd, kap, u1, u2);
           }
           // T = f mom_1 t + U, Q = f mom_0 + T on the slices that own k = 1, 0
@@ -496,41 +520,53 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
           }
         } else {
           // node sum in double-float: Q_b = sum_j w_j B_b(j) / (A - k_par p_j + i D)
-          dflt Qs[12];
+          // (g1, g2 side by side; two nodes' R side by side)
+          dflt2 Qr[3], Qi[3];
 #pragma unroll
-          for (int q = 0; q < 12; ++q) Qs[q] = {0.0f, 0.0f};
-          // the summed ranges (disjoint), each over this slice's nodes
-          // jn = 1 + jj (mod jc), then their ends again at weight -1/2
-          auto node = [&](int jn, bool end) {
-            const dflt dr = df_add(Ad, df_neg(df_mul(kd, {S.pph[jn], S.ppl[jn]})));
-            const dflt r = df_rcp_approx(df_add(df_mul(dr, dr), D2));
-            dflt Rr = df_mul(dr, r), Ri = df_neg(df_mul(Dd, r));
-            if (end) {
-              Rr = df_scale(Rr, -0.5f);
-              Ri = df_scale(Ri, -0.5f);
-            }
+          for (int q = 0; q < 3; ++q) Qr[q] = Qi[q] = d2_all({0.0f, 0.0f});
+          auto mac = [&](int jn, dflt Rr, dflt Ri) {
             const float4* b4 = reinterpret_cast<const float4*>(Bn + (size_t)(jn - 1) * 12);
             const float4 a0 = __ldg(b4), a1 = __ldg(b4 + 1), a2 = __ldg(b4 + 2);
-            const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+            const float2 h[3] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}};
+            const float2 l[3] = {{a1.z, a1.w}, {a2.x, a2.y}, {a2.z, a2.w}};
+            const dflt2 r2 = d2_all(Rr), i2 = d2_all(Ri);
 #pragma unroll
-            for (int b2 = 0; b2 < 6; ++b2) {
-              df_mac(Qs[2 * b2], hb[b2], lb[b2], Rr);
-              df_mac(Qs[2 * b2 + 1], hb[b2], lb[b2], Ri);
+            for (int q = 0; q < 3; ++q) {
+              d2_mac(Qr[q], h[q], l[q], r2.h, r2.l);
+              d2_mac(Qi[q], h[q], l[q], i2.h, i2.l);
             }
           };
+          const dflt2 Ad2 = d2_all(Ad), kd2 = d2_all(df_neg(kd)), DD2 = d2_all(D2), nD2 = d2_all(df_neg(Dd));
+          // nodes ja and jb (jb < 0: ja alone), weight -1/2 for range ends
+          auto nodes = [&](int ja, int jb, bool end) {
+            const int jq = jb < 0 ? ja : jb;
+            const dflt2 pp = {make_float2(S.pph[ja], S.pph[jq]), make_float2(S.ppl[ja], S.ppl[jq])};
+            const dflt2 dr = d2_add(Ad2, d2_mul(kd2, pp));
+            const dflt2 r = d2_rcp_approx(d2_add(d2_mul(dr, dr), DD2));
+            dflt2 Rr = d2_mul(dr, r), Ri = d2_mul(nD2, r);
+            if (end) {
+              Rr = {__fmul2_rn(Rr.h, f2_all(-0.5f)), __fmul2_rn(Rr.l, f2_all(-0.5f))};
+              Ri = {__fmul2_rn(Ri.h, f2_all(-0.5f)), __fmul2_rn(Ri.l, f2_all(-0.5f))};
+            }
+            mac(ja, d2_x(Rr), d2_x(Ri));
+            if (jb >= 0) mac(jb, d2_y(Rr), d2_y(Ri));
+          };
+          // the summed ranges (disjoint), each over this slice's nodes
+          // jn = 1 + jj (mod jc), then their ends again at weight -1/2
           for (int r2 = 0; r2 < 2; ++r2) {
             const int b = r2 ? cur.lo2 : cur.lo1, e = r2 ? cur.hi2 : cur.hi1;
             const int lo = max(1, b), hi = min(M - 1, e);
-            for (int jn = lo + ((jj - lo + 1) & (jc - 1)); jn <= hi; jn += jc) node(jn, false);
+            for (int jn = lo + ((jj - lo + 1) & (jc - 1)); jn <= hi; jn += 2 * jc)
+              nodes(jn, jn + jc <= hi ? jn + jc : -1, false);
           }
           for (int q = 0; q < 4; ++q) {
             const int b = (q & 2) ? cur.lo2 : cur.lo1, e = (q & 2) ? cur.hi2 : cur.hi1, jn = (q & 1) ? e : b;
-            if (b < e && jn >= 1 && jn <= M - 1 && ((jn - 1 - jj) & (jc - 1)) == 0) node(jn, true);
+            if (b < e && jn >= 1 && jn <= M - 1 && ((jn - 1 - jj) & (jc - 1)) == 0) nodes(jn, -1, true);
           }
           cdf P[3];
 #pragma unroll
           for (int fm = 0; fm < 3; ++fm)
-            P[fm] = om_comb(omd, kap, {Qs[4 * fm], Qs[4 * fm + 1]}, {Qs[4 * fm + 2], Qs[4 * fm + 3]});
+            P[fm] = om_comb(omd, kap, {d2_x(Qr[fm]), d2_x(Qi[fm])}, {d2_y(Qr[fm]), d2_y(Qi[fm])});
           const cdf zeta = {df_mul(Ad, ikd), dyd};
           // (1/k_par) times the omega-combined sums of F1, F3 and p_par F1
           // over the summed ranges: six real sums C_c, added once; lane c
@@ -2193,9 +2229,9 @@ __device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, con
     const dflt del = df_add(c.cap, df_add(plo, df_neg({S.pph[j], S.ppl[j]})));
     B = cdf_add(C, cdf_rmul(A, del));
   };
-  dflt Sx[24];
+  dflt2 Sr[6], Si[6];  // per entry, (g1, g2) side by side
 #pragma unroll
-  for (int q = 0; q < 24; ++q) Sx[q] = z;
+  for (int q = 0; q < 6; ++q) Sr[q] = Si[q] = d2_all(z);
   const dflt hid = {S.hidh, S.hidl};
   cdf Aj = {z, z}, Bp = {z, z}, Bj = {z, z};
 #pragma unroll 1
@@ -2208,21 +2244,19 @@ __device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, con
     const cdf Wp = cdf_rmul(W, pj), Wpp = cdf_rmul(Wp, pj);
     const float4* b4 = reinterpret_cast<const float4*>(S.Bt + ((size_t)n * (M - 1) + (j - 1)) * 12);
     const float4 a0 = __ldg(b4), a1 = __ldg(b4 + 1), a2 = __ldg(b4 + 2);
-    const float hb[6] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y}, lb[6] = {a1.z, a1.w, a2.x, a2.y, a2.z, a2.w};
+    const float2 hb[3] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}}, lb[3] = {{a1.z, a1.w}, {a2.x, a2.y}, {a2.z, a2.w}};
     // entries xx yy zz xy xz yz: vectors (F1, F2, F1 p^2, F3, F1 p, F3 p)
-    auto add = [&](int e, int b, cdf v) {
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        df_mac(Sx[4 * e + 2 * g], hb[b + g], lb[b + g], v.x);
-        df_mac(Sx[4 * e + 2 * g + 1], hb[b + g], lb[b + g], v.y);
-      }
+    auto add = [&](int e, int f, cdf v) {
+      const dflt2 x2 = d2_all(v.x), y2 = d2_all(v.y);
+      d2_mac(Sr[e], hb[f], lb[f], x2.h, x2.l);
+      d2_mac(Si[e], hb[f], lb[f], y2.h, y2.l);
     };
     add(0, 0, W);
-    add(1, 2, W);
+    add(1, 1, W);
     add(2, 0, Wpp);
-    add(3, 4, W);
+    add(3, 2, W);
     add(4, 0, Wp);
-    add(5, 4, Wp);
+    add(5, 2, Wp);
     Bp = Bj;
     Aj = An;
     Bj = Bn;
@@ -2231,8 +2265,8 @@ __device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, con
   const dflt kap = {S.kaph, S.kapl};
 #pragma unroll
   for (int e = 0; e < 6; ++e)
-    X[e] = om_comb(omd, kap, {df_add(Sx[4 * e], z), df_add(Sx[4 * e + 1], z)},
-                   {df_add(Sx[4 * e + 2], z), df_add(Sx[4 * e + 3], z)});
+    X[e] = om_comb(omd, kap, {df_add(d2_x(Sr[e]), z), df_add(d2_x(Si[e]), z)},
+                   {df_add(d2_y(Sr[e]), z), df_add(d2_y(Si[e]), z)});
   return true;
 }
 
