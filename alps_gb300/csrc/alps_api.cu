@@ -138,6 +138,8 @@ void alps_destroy(alps_ctx* c) {
     cudaFree(S.d_X);
     cudaFree(S.d_mom);
     cudaFree(S.d_pfac);
+    cudaFree(S.d_far);
+    cudaFree(S.d_farc);
     cudaFree(S.d_Vh);  // d_Vl points into it
     cudaFree(S.d_Vscale);
     cudaFree(S.d_Bt);

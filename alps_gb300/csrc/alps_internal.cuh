@@ -27,6 +27,9 @@
 #define ALPS_MAX_SPECIES 8
 // Laurent terms kept per order for poles far from the p_par grid
 #define ALPS_KFAR 128
+// far-order series (k_far_levels): levels (first orders summed) and terms
+#define FAR_LEVELS 24
+#define FAR_K 44
 #define ALPS_PI 3.141592653589793115997963468544185161590576171875
 
 // ---------------------------------------------------------------------------
@@ -118,6 +121,9 @@ struct __align__(16) SpecDev {
   double pcen, prad;  // centre and half-width of ppar[1..M-1]
   float pcen32, prad32;  // the same rounded to FP32
   int kfar;           // max Laurent terms used (<= ALPS_KFAR)
+  int farn;           // first order of the far-order series, 0: none
+  void* far;          // its coefficients by level (k_far_levels)
+  double* farc;       // and by order (k_far_orders)
   int rcap;           // resonant-item slots per (omega, species)
   // [(N+1)][nf][4] = {p1 exp(-pc pperp^2), p2, p3, exp(-p2 dppar^2)} when
   // every fit term is a Maxwellian (ACmethod 1, type 1); else null
@@ -201,6 +207,9 @@ struct SpeciesHost {
   double* d_X = nullptr;                  // x_j^k, x_j = (ppar_j - pcen)/prad
   double* d_mom = nullptr;                // Laurent moments
   double* d_pfac = nullptr;               // FP64 path: order factors
+  double* d_far = nullptr;                // far-order series: FP64, or float pairs in the same bytes
+  double* d_farc = nullptr;               // its coefficients order by order
+  size_t farc_cap = 0;
   float* d_Bt = nullptr;                  // base tables of the fast pole sums: Bt, mBt, bfac
   size_t Bt_cap = 0;
   double* d_Bd = nullptr;                 // and their FP64 part: Escale[8], Cfull, Pre
@@ -364,6 +373,7 @@ struct MultiLaunch {
   const void* jobs;  // device job table
   int nj;
   bool small;        // all in one launch (k_disp_many)
+  int far;           // most groups of eight orders of a job with far orders, 0 if none (k_far_orders)
   long blocks[6];    // grids of classify, pole sums, resonant, finalize, resonant lanes, k_disp_many
   size_t smem;       // dynamic shared memory of k_resonant_multi
   size_t lanes_smem; // and of k_resonant_lanes

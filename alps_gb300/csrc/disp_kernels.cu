@@ -68,6 +68,7 @@ struct DispShape {
   int nch[ALPS_MAX_SPECIES];  // order chunks of each species (0: no pole sums)
   int ipw;       // resonant-item slots per warp of k_resonant (1..256)
   int fin_warp;  // k_finalize takes a warp per omega (else a thread)
+  int far;       // orders beyond the frequency's reach through the far-order series
   int lanes;     // slots per warp of k_resonant_lanes, which takes the items, k_resonant_multi
                  // what it leaves (0: k_resonant_multi takes all)
 };
@@ -241,11 +242,38 @@ __device__ __forceinline__ void lane_sum12(T v[12], int js, int lane, int& first
   if (lane & off) cnt = 0;
 }
 
+// The far-order series (k_far_orders, k_far_levels) at a frequency: with s = m omega and P the
+// largest |k_par p| on the grid, the orders |n| >= n0 have poles |n q| - P or
+// more away, and their sum is a power series in s / r, r = n0 |q| - P.  n0 is
+// the first with |s| <= 0.4 r.  Returns n0, or INT_MAX where fewer than ten
+// orders would be left to the series.
+struct FarLevel {
+  int n0, K, K32;
+  double r;
+};
+__device__ __forceinline__ FarLevel far_level(const SysDev& sys, const SpecDev& S, double2 o, bool on) {
+  FarLevel f = {0x7fffffff, 0, 0, 1.0};
+  if (!on || !S.farn) return f;
+  const float q = fabsf((float)S.qs), P = fabsf((float)sys.kpar) * (fabsf(S.pcen32) + S.prad32);
+  const float sx = (float)(S.ms * o.x), sy = (float)(S.ms * o.y), sa = sqrtf(fmaf(sx, sx, sy * sy));
+  const float t = (2.5f * sa + P) / q * 1.00001f;
+  if (!(t < 1e6f)) return f;
+  const int n0 = max(S.farn, (int)ceilf(t));
+  if (n0 - S.farn >= FAR_LEVELS || n0 + 4 > S.nmax) return f;
+  f.n0 = n0;
+  f.r = (double)n0 * fabs(S.qs) - fabs(sys.kpar) * (fabs(S.pcen) + S.prad);
+  // rho <= 0.4: terms to 2^-55 of the bound, 2^-33 in double-float
+  const float rho = sa / (float)f.r, lr = -__logf(fmaxf(rho, 1e-30f)), l1 = log1pf(-rho);
+  f.K = min(FAR_K, (int)ceilf((38.1230949f - l1) / lr) + 1);
+  f.K32 = min(f.K, (int)ceilf((22.8738570f - l1) / lr) + 1);
+  return f;
+}
+
 // what the lanes of a frequency need of one signed order
 struct OrderInfo {
   int nn, K, K32;         // K > kfar: node sum; else the Laurent terms (K32 of them in double-float)
   int lo1, hi1, lo2, hi2; // summed node ranges
-  int flags;              // 1 resonant, 2 the double-float node sum applies
+  int flags;              // 1 resonant, 2 the double-float node sum applies, 4 the far orders
 };
 __device__ __forceinline__ OrderInfo shfl_info(const OrderInfo& a, int src) {
   OrderInfo r;
@@ -284,8 +312,9 @@ __device__ __forceinline__ OrderInfo shfl_info(const OrderInfo& a, int src) {
 // code in the instruction cache.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, double2 o, bool active, int js,
-                                           int chunk, int nch, int kmid, double* out) {
+                                           int chunk, int nch, int kmid, bool far, double* out) {
   const int M = S.M, U_ = 2 * S.nmax + 1;
+  const FarLevel fl = far_level(sys, S, o, active && far);
   const int lane = threadIdx.x & 31, j = lane & (js - 1), gbase = lane - j;
   const unsigned gmask = (js == 32) ? FULL_WARP : (((1u << js) - 1u) << gbase);
   const double kpar = sys.kpar;
@@ -301,12 +330,18 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
   const dflt dyd = df_mul(Dd, ikd);  // Im p_res
   const dflt mox = df_mul(msd, oxd);
   const float ikp32 = (float)sys.ikpar;
-  for (int i0 = 0; chunk + i0 * nch < U_; i0 += js) {
+  for (int i0 = 0; chunk + i0 * nch < U_ + (far ? 1 : 0); i0 += js) {
     // ---- this lane's own order: resonance geometry, series or nodes ----
     const int u = chunk + (i0 + j) * nch;
-    const bool own = active && u < U_;
+    // (unit U_ is the far orders')
+    const bool isfar = fl.n0 != 0x7fffffff && u == U_;
+    const bool own = isfar || (active && u < U_ && abs(u - S.nmax) < fl.n0);
     OrderInfo cur = {0, S.kfar + 1, S.kfar + 1, 1, 0, 1, 0, 0};
-    if (own) {
+    if (isfar) {
+      cur.K = fl.K;
+      cur.K32 = fl.K32;
+      cur.flags = 4;
+    } else if (own) {
       const int nn = u - S.nmax;
       // A = m omega_r - nn q, the pole's real part times k_par
       const dflt Ad = df_add(mox, df_neg(df_mul({(float)nn, 0.0f}, qsd)));
@@ -369,7 +404,57 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
     int jj = 0, jc = 1;
     const OrderInfo mine = cur;
     for (;;) {
-      if (go) {
+      if (go && (cur.flags & 4)) {
+        // the far orders: entries (xx yy zz xy xz yz) against g1, g2 as power
+        // series in t = m omega / r, this slice's terms
+        const float* __restrict__ cf = reinterpret_cast<const float*>(S.far) + (size_t)(fl.n0 - S.farn) * FAR_K * 24;
+        const double ir = 1.0 / fl.r;
+        const cdf t1 = {df_of(S.ms * o.x * ir), df_of(S.ms * o.y * ir)};
+        cdf tp = {{1.0f, 0.0f}, {0.0f, 0.0f}}, st = t1;
+        for (int q = 0; q < jj; ++q) tp = cdf_mul(tp, t1);
+        for (int q = jc; q > 1; q >>= 1) st = cdf_mul(st, st);
+        dflt2 Xr[6], Xi[6];
+#pragma unroll
+        for (int e = 0; e < 6; ++e) Xr[e] = Xi[e] = d2_all({0.0f, 0.0f});
+        int k = jj;
+        for (; k < cur.K32; k += jc) {
+          const float4* c4 = reinterpret_cast<const float4*>(cf + (size_t)k * 24);
+          const dflt2 x2 = d2_all(tp.x), y2 = d2_all(tp.y);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const float4 h = __ldg(c4 + e), l = __ldg(c4 + 3 + e);
+            d2_mac(Xr[2 * e], make_float2(h.x, h.y), make_float2(l.x, l.y), x2.h, x2.l);
+            d2_mac(Xi[2 * e], make_float2(h.x, h.y), make_float2(l.x, l.y), y2.h, y2.l);
+            d2_mac(Xr[2 * e + 1], make_float2(h.z, h.w), make_float2(l.z, l.w), x2.h, x2.l);
+            d2_mac(Xi[2 * e + 1], make_float2(h.z, h.w), make_float2(l.z, l.w), y2.h, y2.l);
+          }
+          tp = cdf_mul(tp, st);
+        }
+        float fx = tp.x.h + tp.x.l, fy = tp.y.h + tp.y.l;
+        const float gx = st.x.h + st.x.l, gy = st.y.h + st.y.l;
+        for (; k < cur.K; k += jc) {
+          const float4* c4 = reinterpret_cast<const float4*>(cf + (size_t)k * 24);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            const float4 h = __ldg(c4 + e);
+            Xr[2 * e].l = __ffma2_rn(make_float2(h.x, h.y), f2_all(fx), Xr[2 * e].l);
+            Xi[2 * e].l = __ffma2_rn(make_float2(h.x, h.y), f2_all(fy), Xi[2 * e].l);
+            Xr[2 * e + 1].l = __ffma2_rn(make_float2(h.z, h.w), f2_all(fx), Xr[2 * e + 1].l);
+            Xi[2 * e + 1].l = __ffma2_rn(make_float2(h.z, h.w), f2_all(fy), Xi[2 * e + 1].l);
+          }
+          const float nx = fx * gx - fy * gy;
+          fy = fx * gy + fy * gx;
+          fx = nx;
+        }
+        const dflt z = {0.0f, 0.0f};
+#pragma unroll
+        for (int e = 0; e < 6; ++e) {
+          const cdf x = om_comb(omd, kap, {df_add(d2_x(Xr[e]), z), df_add(d2_x(Xi[e]), z)},
+                                {df_add(d2_y(Xr[e]), z), df_add(d2_y(Xi[e]), z)});
+          df_acc(acc[2 * e], x.x);
+          df_acc(acc[2 * e + 1], x.y);
+        }
+      } else if (go) {
         const int nn = cur.nn, n = nn < 0 ? -nn : nn, K = cur.K, K32 = cur.K32;
         const dflt Ad = df_add(mox, df_neg(df_mul({(float)nn, 0.0f}, qsd)));
         const float* __restrict__ Bn = S.Bt + (size_t)n * (M - 1) * 12;
@@ -660,8 +745,9 @@ __device__ __forceinline__ void pole_fused(const SysDev& sys, const SpecDev& S, 
 // instead of 255 nodes: 2867 map frequencies on a 128x256 grid 3180 us by
 // nodes alone, 573 us so.
 __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, double2 o, bool active, int js,
-                                           int chunk, int nch, int kmid, double* out) {
+                                           int chunk, int nch, int kmid, bool far, double* out) {
   const int M = S.M, U_ = 2 * S.nmax + 1;
+  const FarLevel fl = far_level(sys, S, o, active && far);
   const int lane = threadIdx.x & 31, j = lane & (js - 1), gbase = lane - j;
   const unsigned gmask = (js == 32) ? FULL_WARP : (((1u << js) - 1u) << gbase);
   const double kpar = sys.kpar, kappa = S.kappa;
@@ -671,11 +757,15 @@ __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, 
   dbl_val acc[12];
 #pragma unroll
   for (int q = 0; q < 12; ++q) acc[q] = {0.0};
-  for (int i0 = 0; chunk + i0 * nch < U_; i0 += js) {
+  for (int i0 = 0; chunk + i0 * nch < U_ + (far ? 1 : 0); i0 += js) {
     const int u = chunk + (i0 + j) * nch;
-    const bool own = active && u < U_;
+    const bool isfar = fl.n0 != 0x7fffffff && u == U_;
+    const bool own = isfar || (active && u < U_ && abs(u - S.nmax) < fl.n0);
     OrderInfo cur = {0, S.kfar + 1, 0, 1, 0, 1, 0, 0};
-    if (own) {
+    if (isfar) {
+      cur.K = fl.K;
+      cur.flags = 4;
+    } else if (own) {
       cur.nn = u - S.nmax;
       cur.hi1 = M - 1;
       // the FP32 test of k_classify: an order clearly outside the resonance
@@ -697,13 +787,42 @@ __device__ __forceinline__ void pole_plain(const SysDev& sys, const SpecDev& S, 
         cur.K = (int)ceilf((38.1230949f - log1pf(-rho)) / -__logf(rho)) + 1;  // 55 ln 2
       }
     }
-    const bool solo = own && cur.K <= S.kfar && (js == 1 || cur.K <= kmid);
+    const bool solo = own && (isfar || cur.K <= S.kfar) && (js == 1 || cur.K <= kmid);
     unsigned pend = __ballot_sync(FULL_WARP, own && !solo) & gmask;
     bool go = solo;
     int jj = 0, jc = 1;
     const OrderInfo mine = cur;
     for (;;) {
-      if (go) {
+      if (go && (cur.flags & 4)) {
+        // the far orders as in pole_fused
+        const double* __restrict__ cf = reinterpret_cast<const double*>(S.far) + (size_t)(fl.n0 - S.farn) * FAR_K * 12;
+        const double ir = 1.0 / fl.r;
+        const double2 t1 = cmk(S.ms * o.x * ir, S.ms * o.y * ir);
+        double2 tp = cmk(1.0, 0.0), st = t1;
+        for (int q = 0; q < jj; ++q) tp = cmul(tp, t1);
+        for (int q = jc; q > 1; q >>= 1) st = cmul(st, st);
+        double2 X[12];
+#pragma unroll
+        for (int e = 0; e < 12; ++e) X[e] = cmk(0.0, 0.0);
+        for (int k = jj; k < cur.K; k += jc) {
+          const double2* c2 = reinterpret_cast<const double2*>(cf + (size_t)k * 12);
+#pragma unroll
+          for (int e = 0; e < 6; ++e) {
+            const double2 c = __ldg(c2 + e);
+            X[2 * e].x = fma(c.x, tp.x, X[2 * e].x);
+            X[2 * e].y = fma(c.x, tp.y, X[2 * e].y);
+            X[2 * e + 1].x = fma(c.y, tp.x, X[2 * e + 1].x);
+            X[2 * e + 1].y = fma(c.y, tp.y, X[2 * e + 1].y);
+          }
+          tp = cmul(tp, st);
+        }
+#pragma unroll
+        for (int e = 0; e < 6; ++e) {
+          const double2 x = cadd(cmul(o, X[2 * e]), cscale(X[2 * e + 1], kappa));
+          acc[2 * e].v += x.x;
+          acc[2 * e + 1].v += x.y;
+        }
+      } else if (go) {
         const int cn = cur.nn, n = cn < 0 ? -cn : cn, K = cur.K;
         const double Ar = S.ms * o.x - (double)cn * S.qs;
         double2 X[6];  // omega S_e1 + kappa S_e2
@@ -834,9 +953,9 @@ __device__ __noinline__ void pole_body(const SysDev& sys, const SpecDev& S, cons
   const double2 o = active ? om[w] : cmk(0.0, 0.0);
   double* out = active ? reinterpret_cast<double*>(part + (((size_t)w * sys.nspec + s) * sh.nchunk + chunk) * 6) : nullptr;
   if (S.df_sums)
-    pole_fused(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, out);
+    pole_fused(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, sh.far != 0, out);
   else
-    pole_plain(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, out);
+    pole_plain(sys, S, o, active, js, chunk, sh.nch[s], sh.kmid, sh.far != 0, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -2641,10 +2760,139 @@ __device__ __forceinline__ void stage_bytes(const void* src, void* dst, int n) {
   for (int q = threadIdx.x; q < n / 16; q += blockDim.x) d4[q] = s4[q];
 }
 
+// Coefficients of the far-order series.  For the orders nn = +-n with n |q| >=
+// 2.5 P (P the largest |k_par p| on the grid) and s = m omega,
+//   sum_j w_j F_j / (s - nn q - k_par p_j) = sum_l s^l c_l(nn),
+//   c_l = -sum_k binom(l + k, k) (-k_par prad)^k A^-(l+k+1) mom_k,  A = nn q +
+//   k_par pcen,
+// with the Laurent moments mom_k of the family vectors (k_moments); the
+// p_par-weighted entries take the moments of p F = pcen F + prad x F.  Times
+// the order factors: farc[(n - farn) FAR_K + l][entry][g], the two orders +-n
+// together.  A warp per term l and eight n, four lanes per n over quarters of
+// the k; bound by the FP64 pipe (some 35 instructions a term k).
+__global__ void __launch_bounds__(32) k_far_orders(const DispJob* __restrict__ jobs) {
+  __shared__ double ratio[ALPS_KFAR];
+  const DispJob& J = jobs[blockIdx.z];
+  const int l = blockIdx.x % FAR_K, grp = blockIdx.x / FAR_K, s = blockIdx.y, lane = threadIdx.x;
+  if (!J.sh.far || s >= J.S) return;
+  const SpecDev& S = J.a->sp[s];
+  const SysDev& sys = J.a->sys;
+  const int n1 = S.farn, n = n1 + grp * 8 + (lane & 7), k0 = (lane >> 3) * (ALPS_KFAR / 4);
+  if (!n1 || n1 + grp * 8 > S.nmax) return;
+  for (int k = lane; k < ALPS_KFAR; k += 32) ratio[k] = (double)(l + k + 1) * rcp_fast((double)(k + 1));
+  __syncwarp();
+  // binom(l + k0, k0) at the quarters' starts: products of four, then over the lanes
+  double bin = ratio[4 * lane] * ratio[4 * lane + 1] * ratio[4 * lane + 2] * ratio[4 * lane + 3];
+  for (int off = 1; off < 32; off <<= 1) {
+    const double t = __shfl_up_sync(FULL_WARP, bin, off);
+    if (lane >= off) bin *= t;
+  }
+  bin = __shfl_sync(FULL_WARP, bin, max(0, k0 / 4 - 1));
+  if (k0 == 0) bin = 1.0;
+  const double kpar = sys.kpar, pc = S.pcen, pr = S.prad;
+  auto power = [](double x, int e) {
+    double y = 1.0;
+    for (; e; e >>= 1) {
+      if (e & 1) y *= x;
+      x *= x;
+    }
+    return y;
+  };
+  double2 v[6];  // entries xx yy zz xy xz yz, (g1, g2)
+#pragma unroll
+  for (int e = 0; e < 6; ++e) v[e] = cmk(0.0, 0.0);
+  if (n <= S.nmax) {
+    const double r1 = (double)n1 * fabs(S.qs) - fabs(kpar) * (fabs(pc) + pr);
+    const double ip = 1.0 / ((double)n * S.qs + kpar * pc), im = 1.0 / (-(double)n * S.qs + kpar * pc);
+    const double cp = -kpar * pr * ip, cm = -kpar * pr * im;
+    double wp = -ip * power(r1 * ip, l) * power(cp, k0) * bin, wm = -im * power(r1 * im, l) * power(cm, k0) * bin;
+    const double2* __restrict__ m = reinterpret_cast<const double2*>(S.mom + ((size_t)n * ALPS_KFAR + k0) * 6);
+    double2 a0 = __ldg(m), a1 = __ldg(m + 3), b0 = __ldg(m + 2), b1 = __ldg(m + 5);
+    const int ke = min(k0 + ALPS_KFAR / 4, ALPS_KFAR - 2);
+#pragma unroll 4
+    for (int k = k0; k < ke; ++k, m += 3) {
+      const double2 a2 = __ldg(m + 6), b2 = __ldg(m + 8), f2 = __ldg(m + 1);
+      const double we = wp + wm, wo = wp - wm;
+      const double2 ap = cmk(fma(pc, a0.x, pr * a1.x), fma(pc, a0.y, pr * a1.y));
+      const double2 aq = cmk(fma(pc, a1.x, pr * a2.x), fma(pc, a1.y, pr * a2.y));
+      v[0] = cmk(fma(we, a0.x, v[0].x), fma(we, a0.y, v[0].y));
+      v[1] = cmk(fma(we, f2.x, v[1].x), fma(we, f2.y, v[1].y));
+      v[2] = cmk(fma(we, fma(pc, ap.x, pr * aq.x), v[2].x), fma(we, fma(pc, ap.y, pr * aq.y), v[2].y));
+      v[3] = cmk(fma(wo, b0.x, v[3].x), fma(wo, b0.y, v[3].y));
+      v[4] = cmk(fma(wo, ap.x, v[4].x), fma(wo, ap.y, v[4].y));
+      v[5] = cmk(fma(we, fma(pc, b0.x, pr * b1.x), v[5].x), fma(we, fma(pc, b0.y, pr * b1.y), v[5].y));
+      wp *= cp * ratio[k];
+      wm *= cm * ratio[k];
+      a0 = a1;
+      a1 = a2;
+      b0 = b1;
+      b1 = b2;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 6; ++e)
+    for (int off = 8; off < 32; off <<= 1) {
+      v[e].x += __shfl_xor_sync(FULL_WARP, v[e].x, off);
+      v[e].y += __shfl_xor_sync(FULL_WARP, v[e].y, off);
+    }
+  if (lane < 8 && n <= S.nmax) {
+    const double C0 = 2.0 * ALPS_PI * S.dpperp * S.dppar_abs * 0.25 * S.qs;
+    const double z = sys.kperp_norm ? sys.kperp / S.qs : 1.0 / S.qs;
+    double2* o = reinterpret_cast<double2*>(S.farc + ((size_t)(n - n1) * FAR_K + l) * 12);
+    double2 pref[6];
+    t_prefactors(n, z, sys.kperp, sys.kperp_norm, pref);
+#pragma unroll
+    for (int e = 0; e < 6; ++e) o[e] = cscale(v[e], C0 * ((e == 3 || e == 5) ? pref[e].y : pref[e].x));
+  }
+}
+
+// Summed from the highest order down and scaled to t = s / r: the series of all
+// orders |n| >= n0 for the levels n0 = farn .. farn + FAR_LEVELS - 1, FP64 or
+// float pairs.  A block per term and species, a thread per entry and g for
+// the running sums, then one per coefficient.  Both kernels together take 58 us for 30 + 7 orders.
+__global__ void __launch_bounds__(96) k_far_levels(const DispJob* __restrict__ jobs) {
+  __shared__ double sum[FAR_LEVELS][12];
+  const DispJob& J = jobs[blockIdx.z];
+  const int l = blockIdx.x, s = blockIdx.y;
+  if (!J.sh.far || s >= J.S) return;
+  const SpecDev& S = J.a->sp[s];
+  const int n1 = S.farn, nl = min(FAR_LEVELS, S.nmax - n1 + 1);
+  if (!n1) return;
+  if (threadIdx.x < 12) {
+    const double* c = S.farc + (size_t)l * 12 + threadIdx.x;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int n = S.nmax - n1; n >= 0; --n) {
+      acc += __ldg(c + (size_t)n * FAR_K * 12);
+      if (n < FAR_LEVELS) sum[n][threadIdx.x] = acc;
+    }
+  }
+  __syncthreads();
+  const double qa = fabs(S.qs), P = fabs(J.a->sys.kpar) * (fabs(S.pcen) + S.prad), i1 = 1.0 / ((double)n1 * qa - P);
+  for (int t = threadIdx.x; t < nl * 12; t += blockDim.x) {
+    const int n = t / 12, q = t % 12;
+    double y = sum[n][q], x = ((double)(n + n1) * qa - P) * i1;
+    if (S.df_sums) y *= 1.0 / S.Escale[q >> 1];
+    for (int e = l; e; e >>= 1) {
+      if (e & 1) y *= x;
+      x *= x;
+    }
+    const size_t at = (size_t)n * FAR_K + l;
+    if (S.df_sums) {
+      float* o = reinterpret_cast<float*>(S.far) + at * 24 + q;
+      const float h = __double2float_rn(y);
+      o[0] = h;
+      o[12] = __double2float_rn(y - (double)h);
+    } else {
+      reinterpret_cast<double*>(S.far)[at * 12 + q] = y;
+    }
+  }
+}
+
 // A pole-sums block works on one species: it stages the system constants
 // and that species' constants only (an eighth of DispArgs), which matters
 // when a fused round has many small jobs, each of many small blocks.
-__global__ void __launch_bounds__(128, 3) k_pole_sums_multi(const DispJob* __restrict__ jobs, int nj) {
+__global__ void __launch_bounds__(128, 4) k_pole_sums_multi(const DispJob* __restrict__ jobs, int nj) {
   __shared__ __align__(16) SysDev ssys;
   __shared__ __align__(16) SpecDev sspec;
   const DispJob& J = job_of(jobs, nj, blockIdx.x, 1);
@@ -2925,6 +3173,17 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->prad32 = (float)o->prad;
   // the series is used only where it is cheaper than the node sum
   o->kfar = std::min(ALPS_KFAR, (int)(0.8 * (c->sys.npar - 1)));
+  o->far = S.d_far;
+  o->farc = S.d_farc;
+  {
+    // far orders: n |q| >= 2.5 P; the window beyond the grid's ends lies well
+    // inside their distance on grids of a few windows
+    const double P = std::fabs(c->kpar) * (std::fabs(o->pcen) + o->prad), n1 = std::ceil(2.5 * P / std::fabs(S.sp.qs));
+    o->farn = (!bm && S.d_far && S.sp.qs != 0.0 && n1 + 4.0 <= (double)S.nmax &&
+               c->sys.npar >= 4 * (c->sys.positions_principal + 2))
+                  ? std::max(1, (int)n1)
+                  : 0;
+  }
   o->rcap = S.rcap;
   o->fit_aux = S.d_fit_aux;
   o->lmom = S.lfact ? S.d_lmom : nullptr;
@@ -3091,6 +3350,12 @@ void default_shape(long u, bool mixed, int* lanes, long* csize) {
 // species' Landau terms are left to the warps (no Maxwellian rows) both take
 // 1.06 ms at 2560
 #define RES_LANES_MIN 2560
+// The far-order series takes the orders |n| >= n0 of a frequency (some two
+// thirds of them) in 44 terms; its coefficients are built for each batch.
+// Pole sums by single orders and so, with the 58 us of the coefficients (128x256
+// grid, 73 signed orders): 12000 frequencies 481 and 465 us, 16384: 636 and
+// 546, 32768: 1141 and 926, 262144: 5145 and 3140; FP64, 16384: 3643 and 3317.
+#define FAR_MIN 25000
 #define ALPS_NOALLOC_SCRATCH_BYTES (16u << 20)
 
 // 256-byte aligned carve-out of n bytes from a scratch array
@@ -3181,6 +3446,7 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
     sh.lanes = (int)std::max(96L, std::min(256L, per));
     sh.ipw = (int)std::max(256L, ((long)b.nslots / (152 * 12) + 31) / 32 * 32);
   }
+  sh.far = (!tensors && (long)n * orders / 32 >= FAR_MIN) ? 1 : 0;
   sh.fin_warp = (n <= FIN_WARP_MAX || tensors || rel_capacity(c) || any_bm(c)) ? 1 : 0;
   return b;
 }
@@ -3245,7 +3511,7 @@ int res_smem_optin(size_t smem, size_t lanes_smem, bool small = false) {
 #define MANY_WARPS (152 * 12 * 4)
 long pole_warps(const DispShape& sh, int S_) { return 4 * pole_blocks_all(sh, S_); }
 bool small_batch(const alps_ctx* c, const BatchGeom& bg) {
-  return !c->profiling && !rel_capacity(c) && !any_bm(c) && bg.sh.fin_warp && !bg.sh.lanes &&
+  return !c->profiling && !rel_capacity(c) && !any_bm(c) && bg.sh.fin_warp && !bg.sh.lanes && !bg.sh.far &&
          (long)bg.nslots + pole_warps(bg.sh, c->sys.nspec) <= SMALL_WARPS;
 }
 int launch_one(const alps_ctx* c, const DispArgs& a, const DispShape& sh, const DispJob& job, cudaStream_t st) {
@@ -3256,6 +3522,11 @@ int launch_one(const alps_ctx* c, const DispArgs& a, const DispShape& sh, const 
   k_disp_one<<<(unsigned)blocks, 128, smem, st>>>(a, job);
   ALPS_CUDA_TRY(cudaGetLastError());
   return ALPS_OK;
+}
+int far_groups(int maxn) { return (maxn + 7) / 8; }
+void launch_far(const DispJob* jobs, int groups, int species, int nj, cudaStream_t st) {
+  k_far_orders<<<dim3(FAR_K * groups, species, nj), 32, 0, st>>>(jobs);
+  k_far_levels<<<dim3(FAR_K, species, nj), 32, 0, st>>>(jobs);
 }
 long lanes_blocks(const BatchGeom& bg) {
   const long per = (long)RES_WARPS * bg.sh.lanes;
@@ -3362,6 +3633,7 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   const long lblocks = lanes_blocks(bg);
   if ((rcode = res_smem_optin(smem, lblocks ? lsmem : 0))) return rcode;
   long blocks = ((long)nslots + RES_WARPS * sh.ipw - 1) / (RES_WARPS * sh.ipw);
+  if (sh.far) launch_far(dj, far_groups(maxn), S_, 1, st);
   if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (c->profiling) ALPS_CUDA_TRY(cudaEventRecord(ev[2], st));
@@ -3380,8 +3652,8 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   }
   c->stats.n_eval = n;
   c->stats.n_eval_total += n;
-  // k_stage and the four, k_resonant_lanes on lattices
-  c->stats.kernels_launched = 5 + (lblocks ? 1 : 0) + (a.relcap ? 1 : 0) + (a.has_bm ? 1 : 0);
+  // k_stage and the four; the far orders' two and k_resonant_lanes for large batches
+  c->stats.kernels_launched = 5 + (sh.far ? 2 : 0) + (lblocks ? 1 : 0) + (a.relcap ? 1 : 0) + (a.has_bm ? 1 : 0);
   return ALPS_OK;
 }
 
@@ -3544,6 +3816,9 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
   small = small && warps <= MANY_WARPS;
   if ((rcode = res_smem_optin(smem, lsmem, small))) return rcode;
   out->small = small;
+  out->far = 0;
+  for (int j = 0; j < nj; ++j)
+    if (m->h_jobs[j].sh.far) out->far = std::max(out->far, far_groups(ctx[j]->args_maxn));
   out->jobs = m->d_jobs;
   out->nj = nj;
   for (int k = 0; k < 6; ++k) out->blocks[k] = blk[k];
@@ -3574,6 +3849,7 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
   }
   k_classify_multi<<<(unsigned)ml.blocks[0], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
+  if (ml.far) launch_far(jobs, ml.far, ALPS_MAX_SPECIES, ml.nj, st);
   k_pole_sums_multi<<<(unsigned)ml.blocks[1], 128, 0, st>>>(jobs, ml.nj);
   ALPS_CUDA_TRY(cudaGetLastError());
   if (ml.blocks[4]) k_resonant_lanes<<<(unsigned)ml.blocks[4], RES_WARPS * 32, ml.lanes_smem, st>>>(jobs, ml.nj);
@@ -3686,6 +3962,7 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   k_classify_multi<<<(unsigned)cls_blocks(n, S_), 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   const long g2 = pole_blocks_all(sh, S_);
+  if (sh.far) launch_far(dj, far_groups(maxn), S_, 1, st);
   if (g2 > 0) k_pole_sums_multi<<<(unsigned)g2, 128, 0, st>>>(dj, 1);
   ALPS_CUDA_TRY(cudaGetLastError());
   const size_t smem = res_smem(c);

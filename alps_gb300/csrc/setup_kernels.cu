@@ -1462,6 +1462,8 @@ int launch_build_bessel_and_reduced(alps_ctx* c, int is, double kperp) {
     S.qlo_in = (float)(rlo + mg);
     S.qhi_in = (float)(rhi - mg);
   }
+  if (!S.d_far) ALPS_CUDA_TRY(cudaMalloc(&S.d_far, (size_t)FAR_LEVELS * FAR_K * 12 * sizeof(double)));
+  if ((rc = ensure(S.d_farc, S.farc_cap, (size_t)nmax * FAR_K * 12))) return rc;
   // Laurent moments
   const double pcen = 0.5 * (S.ppar[1] + S.ppar[M - 1]), prad = 0.5 * (S.ppar[M - 1] - S.ppar[1]);
   if (!S.grid_ready) {

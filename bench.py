@@ -144,11 +144,12 @@ def pole_sum_flops(nmax, npar):
     return sum(150.0 * (n + 1) * (npar - 1) for n in nmax)
 
 
-def pole_sum_flops_issued(nmax, npar):
-    """FP64 flops the pole-sum kernel issues per evaluation (FMA = 2): per
-    (signed order, p_par node) 1 add, 1 FMA for |D|^2, reciprocal = rcp seed +
-    2 Newton steps (4 FMA), 2 multiplies and 24 FMA: 61 flops."""
-    return sum(61.0 * (2 * n + 1) * (npar - 1) for n in nmax)
+# FP64 flops (FMA = 2) of the plain path's pole sums, counted from the kernel's
+# code (disp_kernels.cu pole_plain).  A node: 1 add, 1 FMA for |D|^2, reciprocal
+# (seed and 2 Newton steps, 4 FMA), 2 multiplies, 24 FMA.  A Laurent term: 12
+# FMA and a complex product.  A far-order term: 24 FMA and a complex product.
+# An order summed by its series: powers, T, U, Q and the six entries.
+FP64_NODE_FLOPS, FP64_TERM_FLOPS, FP64_FAR_FLOPS, FP64_ORDER_FLOPS = 61, 30, 54, 250
 
 
 # FP32-pipe flops (FMA = 2) of the fast path's pole sums, counted from the
@@ -175,29 +176,50 @@ DF_ORDER_NODE_FLOPS = 1000
 DF_ORDER_SERIES_FLOPS = 2100
 
 
-def pole_sum_work_fast(system, species, kpar, oms, nmax):
-    """Work of the fast path's pole sums over a lattice, with the kernel's own
+# one double-float term of the far-order series: 24 multiply-accumulates and
+# the power's complex product; in FP32, 24 FMA and a complex product
+DF_FAR_FLOPS = 24 * 15 + 4 * 9 + 2 * 10
+FP32_FAR_FLOPS = 24 * 2 + 6
+
+
+def pole_sum_work(system, species, kpar, oms, nmax):
+    """Work of the pole sums over a lattice, with the kernels' own
     decisions per (omega, signed order): a pole far from the grid (not
     resonant, rho = prad/|p_res - pcen| with rho^2 < 0.58) takes K Laurent
     terms, rho^K <= 2^-53 (1 - rho), of which those from K32 on
     (rho^K32 <= 2^-33 (1 - rho)) run in FP32 and the ones before in
-    double-float; any other order sums its nodes (a resonant one outside the
-    principal-value window) in double-float.  The series' k = 0, 1 terms
-    are part of the order's combination.  Returns counts: nodes (signed
-    order x node pairs summed), series terms in double-float and in FP32,
-    orders summed over nodes and by series, and resonant items (omega,
-    species, signed order)."""
+    double-float (the plain path: all of them in FP64, to 2^-55); any other
+    order sums its nodes (a resonant one outside the principal-value window).
+    Large batches sum the orders |n| >= n0(omega) in one series of omega.  The
+    Laurent series' k = 0, 1 terms are part of the order's combination.
+    Returns counts: nodes (signed order x node pairs summed), series terms in
+    double-float, in FP32 and in the plain path, the far-order series' terms
+    likewise, orders summed over nodes and by series, and resonant items
+    (omega, species, signed order)."""
     ns, npar, M_I = system.nspec, system.npar, system.positions_principal
     M = npar
     kfar = min(128, int(0.8 * (M - 1)))
-    out = {"nodes": 0.0, "series_df": 0.0, "series_fp32": 0.0, "node_orders": 0.0, "series_orders": 0.0,
-           "items": 0.0}
+    out = {"nodes": 0.0, "series_df": 0.0, "series_fp32": 0.0, "series_plain": 0.0, "far_df": 0.0, "far_fp32": 0.0,
+           "node_orders": 0.0, "series_orders": 0.0, "items": 0.0}
+    orders = sum(2 * n + 1 for n in nmax)
+    use_far = len(oms) * orders // 32 >= 25000 and npar >= 4 * (M_I + 2)
     for si in range(ns):
         spc, pl = species[si][0], np.asarray(species[si][2])
         ppar = pl.reshape(-1, M + 1)[0]
         pcen, prad = 0.5 * (ppar[1] + ppar[M - 1]), 0.5 * (ppar[M - 1] - ppar[1])
         dpp = ppar[2] - ppar[1]
+        P, qa, sa = abs(kpar) * (abs(pcen) + prad), abs(spc.qs), np.abs(spc.ms * oms)
+        n1 = max(1, int(np.ceil(2.5 * P / qa)))
+        n0 = np.maximum(n1, np.ceil((2.5 * sa + P) / qa * 1.00001))
+        on = (n0 - n1 < 24) & (n0 + 4 <= nmax[si]) & bool(use_far and n1 + 4 <= nmax[si])
+        n0 = np.where(on, n0, 1 << 30)
+        rho = np.maximum(sa / np.where(on, n0 * qa - P, 1e300), 1e-30)
+        Kf = np.minimum(44, np.ceil((38.1230949 - np.log1p(-rho)) / -np.log(rho)) + 1)
+        Kf32 = np.minimum(Kf, np.ceil((22.873857 - np.log1p(-rho)) / -np.log(rho)) + 1)
+        out["far_df"] += Kf32[on].sum()
+        out["far_fp32"] += (Kf - Kf32)[on].sum()
         for nn in range(-nmax[si], nmax[si] + 1):
+            own = abs(nn) < n0
             x = (spc.ms * oms.real - nn * spc.qs) / kpar
             y = spc.ms * oms.imag / kpar
             res = ((ppar[1] <= x) & (x < ppar[M])) | ((x < ppar[1]) & (x >= ppar[1] - M_I * dpp)) | \
@@ -208,13 +230,14 @@ def pole_sum_work_fast(system, species, kpar, oms, nmax):
             # the kernel adds one term to each count for the rounding of its FP32 logarithms
             K = np.where(far, np.ceil((36.7368005696771 - np.log1p(-rho)) / -np.log(rho)) + 1, kfar + 1)
             K32 = np.where(far, np.ceil((22.8738569584782 - np.log1p(-rho)) / -np.log(rho)) + 1, kfar + 1)
-            lau = K <= kfar
+            lau = (K <= kfar) & own
             out["series_df"] += np.maximum(np.minimum(K32, K) - 2, 0)[lau].sum()
             out["series_fp32"] += np.maximum(K - np.maximum(K32, 2), 0)[lau].sum()
+            out["series_plain"] += np.maximum(K, 2)[lau].sum()
             out["series_orders"] += lau.sum()
             nodes = np.where(res, (M - 1) - (2 * M_I + 2), M - 1)
-            out["nodes"] += nodes[~lau].sum()
-            out["node_orders"] += (~lau).sum()
+            out["nodes"] += nodes[own & ~lau].sum()
+            out["node_orders"] += (own & ~lau).sum()
             out["items"] += res.sum()
     return {k: float(v) for k, v in out.items()}
 
@@ -822,7 +845,7 @@ def main():
             t0 = time.perf_counter()
             tune[precision] = G.autotune(n, om_dev.data_ptr())
             tune[precision]["tuning_s"] = time.perf_counter() - t0
-    # plain FP64 path (node sums everywhere): the baseline of the fast path
+    # plain FP64 path: the baseline of the fast path
     t_plain, prof_plain, D_plain = timed("fp64")
     peak64 = fp64_peak_tflops(torch)
     peak32 = fp32_peak_tflops(torch)
@@ -841,22 +864,23 @@ def main():
     pm_plain, nb_plain = prof_plain
     per_fast = [x / max(nb, 1) for x in prof_ms]
     fast_pole_ms, res_ms = per_fast[1], per_fast[2]
-    work = pole_sum_work_fast(system, species, kpar, oms, nmax)
+    work = pole_sum_work(system, species, kpar, oms, nmax)
     # pole sums: double-float node sums and series terms, FP32 series tails
     # and the per-order combinations, all on the FP32 pipes
     f32 = (work["nodes"] * DF_NODE_FLOPS + work["series_df"] * DF_TERM_FLOPS + work["series_fp32"] * FP32_TERM_FLOPS +
-           work["node_orders"] * DF_ORDER_NODE_FLOPS + work["series_orders"] * DF_ORDER_SERIES_FLOPS)
-    pole = {"kernel": "k_pole_sums_multi<false> (fast path)", "bound": "fp32", "kernel_ms": fast_pole_ms,
+           work["node_orders"] * DF_ORDER_NODE_FLOPS + work["series_orders"] * DF_ORDER_SERIES_FLOPS +
+           work["far_df"] * DF_FAR_FLOPS + work["far_fp32"] * FP32_FAR_FLOPS)
+    pole = {"kernel": "k_pole_sums_multi (fast path)", "bound": "fp32", "kernel_ms": fast_pole_ms,
             "achieved": f32 / (fast_pole_ms / 1e3) / 1e12, "peak": peak32, "unit": "TFLOP/s",
             "frac": f32 / (fast_pole_ms / 1e3) / 1e12 / peak32, "fp32_flop_per_step": f32,
             "double_float_nodes_per_step": work["nodes"], "df_node_flops": DF_NODE_FLOPS,
             "series_terms_df": work["series_df"], "df_term_flops": DF_TERM_FLOPS,
-            "series_terms_fp32": work["series_fp32"], "node_orders": work["node_orders"],
+            "series_terms_fp32": work["series_fp32"], "far_terms_df": work["far_df"], "node_orders": work["node_orders"],
             "series_orders": work["series_orders"], "order_flops": [DF_ORDER_NODE_FLOPS, DF_ORDER_SERIES_FLOPS]}
     # resonant items: the algorithmic count per item, 24 M_P flops of
     # principal-value sums and 60 (N_perp + 1) of Landau rows, FP64
     f_res = work["items"] * (24.0 * system.n_resonance_interval + 60.0 * (system.nperp + 1))
-    res = {"kernel": "k_resonant_multi (fast path)", "bound": "fp64-equivalent", "kernel_ms": res_ms,
+    res = {"kernel": "k_resonant_lanes (fast path)", "bound": "fp64-equivalent", "kernel_ms": res_ms,
            "achieved": f_res / (res_ms / 1e3) / 1e12, "peak": peak64, "unit": "TFLOP/s",
            "frac": f_res / (res_ms / 1e3) / 1e12 / peak64, "items_per_step": work["items"],
            "fp64_flop_per_step": f_res,
@@ -864,10 +888,12 @@ def main():
                     "principal-value sums in double-float on the FP32 pipes and factorises the Landau rows, "
                     "so the figure can read above 1")}
     dom = pole if fast_pole_ms >= res_ms else res
-    # the plain path's pole sums: every order sums its nodes in FP64
+    # the plain path's pole sums, by the all-node convention and as issued
     pole_ms = pm_plain[1] / max(nb_plain, 1)
     plain_achieved = pole_sum_flops(nmax, s.npar) * n / (pole_ms / 1e3) / 1e12
-    plain_issued = pole_sum_flops_issued(nmax, s.npar) * n / (pole_ms / 1e3) / 1e12
+    f64 = (work["nodes"] * FP64_NODE_FLOPS + work["series_plain"] * FP64_TERM_FLOPS +
+           work["series_orders"] * FP64_ORDER_FLOPS + (work["far_df"] + work["far_fp32"]) * FP64_FAR_FLOPS)
+    plain_issued = f64 / (pole_ms / 1e3) / 1e12
     roofline = {"bound": dom["bound"], "achieved": dom["achieved"], "peak": dom["peak"], "unit": "TFLOP/s",
                 "frac": dom["frac"], "traffic": None,
                 "peak_source": ("cuBLAS DGEMM 4096^3 (fp64) and SGEMM 8192^3 with TF32 off (fp32), measured in "
@@ -876,7 +902,7 @@ def main():
                 "kernel_share": dom["kernel_ms"] / max(sum(per_fast), 1e-30),
                 "fp64_peak": peak64, "fp32_peak": peak32,
                 "kernels": {"pole_sums": pole, "resonant": res},
-                "plain_path": {"kernel": "k_pole_sums_multi<false> (plain FP64 path)", "kernel_ms": pole_ms,
+                "plain_path": {"kernel": "k_pole_sums_multi (plain FP64 path)", "kernel_ms": pole_ms,
                                "achieved": plain_achieved, "frac": plain_achieved / peak64,
                                "achieved_issued": plain_issued, "frac_issued": plain_issued / peak64},
                 "per_kernel_ms_plain": dict(zip(names, [x / max(nb_plain, 1) for x in pm_plain])),
