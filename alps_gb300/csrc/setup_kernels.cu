@@ -10,6 +10,8 @@
 //   k_bessel_rows     weighted Bessel-product rows of the p_perp contraction
 //   k_dgemm           FP64 tiled GEMM for the contraction
 //   k_fold_reduced    reduced vectors V[n][j][12] of the omega pass
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstring>
 #include <cstdio>
@@ -40,26 +42,39 @@ __global__ void k_derivatives(const double* __restrict__ f0, const double* __res
   G[row + (M - 1) + (j - 1)] = gg2;
 }
 
-// ee term; weights w_perp(i) * w_par(j) of the reference's trapezoid.
-__global__ void k_int_ee(const double* __restrict__ g2, const double* __restrict__ ppar, int N, int M,
-                         double scale, double* out) {
-  __shared__ double red[256];
+// ee term; weights w_perp(i) * w_par(j) of the reference's trapezoid.  Bound by
+// the FP64 pipe of the SMs that take part: a cluster of eight blocks, rows over
+// the warps, the blocks' sums through distributed shared memory (192x384 grid:
+// 116 us in one block, 15 us so).
+#define EE_BLOCKS 8
+__global__ void __cluster_dims__(EE_BLOCKS, 1, 1) __launch_bounds__(256)
+    k_int_ee(const double* __restrict__ g2, const double* __restrict__ ppar, int N, int M, double scale, double* out) {
+  __shared__ double red[8];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, L = M + 1;
   double acc = 0.0;
-  int L = M + 1;
-  long total = (long)(N - 1) * (M - 1);
-  for (long t = threadIdx.x; t < total; t += blockDim.x) {
-    int i = (int)(t / (M - 1)) + 1, j = (int)(t % (M - 1)) + 1;
-    double wperp = (i <= N - 2) ? 2.0 : 1.0;
-    double wpar = (j == 1 || j == M - 1) ? 1.0 : 2.0;
-    acc += wperp * wpar * (ppar[j] * g2[i * L + j]);
+  for (int i = 1 + (int)cl.block_rank() * 8 + warp; i <= N - 1; i += EE_BLOCKS * 8) {
+    const double* row = g2 + (size_t)i * L;
+    double r = 0.0;
+    for (int j = 1 + lane; j <= M - 1; j += 32) {
+      const double x = ppar[j] * row[j];
+      r += (j == 1 || j == M - 1) ? x : x + x;
+    }
+    acc += (i <= N - 2) ? r + r : r;
   }
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) red[warp] = acc;
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+    double t = 0.0;
+    for (unsigned b = 0; b < EE_BLOCKS; ++b) {
+      const double* p = cl.map_shared_rank(red, b);
+      for (int w = 0; w < 8; ++w) t += p[w];
+    }
+    *out = t * scale;
   }
-  if (threadIdx.x == 0) *out = red[0] * scale;
+  cl.sync();  // the other blocks' sums stay until they are read
 }
 
 // ---------------------------------------------------------------------------
@@ -847,45 +862,77 @@ __global__ void k_base_pairs(const double* __restrict__ V, const double* __restr
 // Pre[(n*M + j)*6 + c] = sum_{i=1..j} X_c(i), X = V[q]/Vscale[n] for
 // q = 0, 1 (F1), 6, 7 (F3), 8, 9 (p_par F1), compensated (two-sum) so that
 // each stored prefix is the exact sum rounded once; Cfull[n*6 + c] = the
-// trapezoid sum over j = 1..M-1 (ends at weight 1/2).  One thread per (n, c).
-__global__ void k_base_consts(const double* __restrict__ V, const double* __restrict__ Vscale, int M, int nmax,
-                              double* Pre, double* Cfull) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// trapezoid sum over j = 1..M-1 (ends at weight 1/2).  One warp per (n, c): a
+// lane sums a run of nodes with its error, the runs' totals are scanned as
+// pairs, and each lane goes over its run again from there (192x384 grid: 119
+// us by one thread per (n, c), 12 us so).
+__device__ __forceinline__ void comp_add(double& s, double& e, double x) {
+  const double y = s + x, b = y - s;
+  e += (s - (y - b)) + (x - b);
+  s = y;
+}
+__global__ void __launch_bounds__(64) k_base_consts(const double* __restrict__ V, const double* __restrict__ Vscale,
+                                                    int M, int nmax, double* Pre, double* Cfull) {
+  const int t = blockIdx.x * 2 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= (nmax + 1) * 6) return;
   const int n = t / 6, c = t % 6;
   const int q = (c < 2) ? c : c + 4;
   const double sc = 1.0 / Vscale[n];
   const double* v = V + (size_t)n * (M - 1) * 12 + q;
   double* P = Pre + (size_t)n * M * 6 + c;
+  const int per = (M - 1 + 31) / 32, j0 = 1 + lane * per, j1 = min(M - 1, j0 + per - 1);
   double s = 0.0, e = 0.0;
-  P[0] = 0.0;
-  for (int j = 1; j <= M - 1; ++j) {
-    const double x = v[(size_t)(j - 1) * 12] * sc;
-    const double y = s + x, bb = y - s;
-    e += (s - (y - bb)) + (x - bb);
-    s = y;
+#pragma unroll 4
+  for (int j = j0; j <= j1; ++j) comp_add(s, e, v[(size_t)(j - 1) * 12] * sc);
+  for (int off = 1; off < 32; off <<= 1) {
+    const double ps = __shfl_up_sync(0xffffffffu, s, off), pe = __shfl_up_sync(0xffffffffu, e, off);
+    if (lane >= off) {
+      e += pe;
+      comp_add(s, e, ps);
+    }
+  }
+  const double ts = __shfl_sync(0xffffffffu, s, 31), te = __shfl_sync(0xffffffffu, e, 31);
+  s = __shfl_up_sync(0xffffffffu, s, 1);
+  e = __shfl_up_sync(0xffffffffu, e, 1);
+  if (lane == 0) {
+    s = e = 0.0;
+    P[0] = 0.0;
+  }
+#pragma unroll 4
+  for (int j = j0; j <= j1; ++j) {
+    comp_add(s, e, v[(size_t)(j - 1) * 12] * sc);
     P[(size_t)j * 6] = s + e;
   }
-  const double x1 = v[0] * sc, xe = v[(size_t)(M - 2) * 12] * sc;
-  Cfull[t] = (s + e) - 0.5 * (x1 + xe);
+  if (lane == 0) {
+    const double x1 = v[0] * sc, xe = v[(size_t)(M - 2) * 12] * sc;
+    Cfull[t] = (ts + te) - 0.5 * (x1 + xe);
+  }
 }
 
-// Escale[e] = 2^E, E the exponent of max_n |C0 v_e(n) Vscale[n]|, and
-// bfac[(n*6 + e)*2 + {0,1}] = C0 v_e(n) Vscale[n] / Escale[e] as a float
-// pair (v_e of order n >= 0; xy and xz flip sign for -n).  One warp.
-__global__ void k_base_fac(int nmax, double z, double kperp, int kperp_norm, double C0,
-                           const double* __restrict__ Vscale, double* Escale, float* bfac) {
-  const int e = threadIdx.x;
-  if (e >= 6) return;
-  double mx = 0.0;
-  for (int n = 0; n <= nmax; ++n) mx = fmax(mx, fabs(fused_factor(n, e, z, kperp, kperp_norm, C0) * Vscale[n]));
-  const double sc = (mx > 0.0 && isfinite(mx)) ? ldexp(1.0, ilogb(mx)) : 1.0;
-  Escale[e] = sc;
-  for (int n = 0; n <= nmax; ++n) {
-    const double x = fused_factor(n, e, z, kperp, kperp_norm, C0) * Vscale[n] * (1.0 / sc);
+// bfac and Escale: the order factors C0 v_e(n) Vscale[n] over the power of two
+// Escale[e] of the largest, as float pairs.  One block, a thread per (n, e) in
+// turn (30 orders: 45 us by a thread per entry, under 12 us so).
+__global__ void __launch_bounds__(192) k_base_fac(int nmax, double z, double kperp, int kperp_norm, double C0,
+                                                  const double* __restrict__ Vscale, double* Escale, float* bfac) {
+  __shared__ unsigned long long mx[6];  // bits of the largest finite-or-not magnitude (ordered as integers)
+  if (threadIdx.x < 6) mx[threadIdx.x] = 0;
+  __syncthreads();
+  const int total = (nmax + 1) * 6;
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const double x = fabs(fused_factor(t / 6, t % 6, z, kperp, kperp_norm, C0) * Vscale[t / 6]);
+    if (x == x) atomicMax(&mx[t % 6], (unsigned long long)__double_as_longlong(x));
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const double m = __longlong_as_double((long long)mx[threadIdx.x]);
+    Escale[threadIdx.x] = (m > 0.0 && isfinite(m)) ? ldexp(1.0, ilogb(m)) : 1.0;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const double x = fused_factor(t / 6, t % 6, z, kperp, kperp_norm, C0) * Vscale[t / 6] * (1.0 / Escale[t % 6]);
     const float h = __double2float_rn(x);
-    bfac[((size_t)n * 6 + e) * 2] = h;
-    bfac[((size_t)n * 6 + e) * 2 + 1] = __double2float_rn(x - (double)h);
+    bfac[(size_t)t * 2] = h;
+    bfac[(size_t)t * 2 + 1] = __double2float_rn(x - (double)h);
   }
 }
 
@@ -1138,7 +1185,7 @@ int launch_prepare_species(alps_ctx* c, int is) {
   if (!S.d_words) ALPS_CUDA_TRY(cudaMalloc(&S.d_words, 2 * sizeof(double)));
   double* d_ee = S.d_words;
   int* d_status = reinterpret_cast<int*>(S.d_words + 1);
-  k_int_ee<<<1, 256, 0, st>>>(S.d_g2, S.d_ppar, N, M, scale, d_ee);
+  k_int_ee<<<EE_BLOCKS, 256, 0, st>>>(S.d_g2, S.d_ppar, N, M, scale, d_ee);
   ALPS_CUDA_TRY(cudaGetLastError());
   // relativistic species: (Gamma, pparbar) grid, f0_rel and its derivatives
   int st_fit = ALPS_OK;
@@ -1263,7 +1310,7 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
       k_derivatives<<<grid, 128, 0, s>>>(S.d_f0, S.d_pperp, S.d_ppar, N, M, S.d_g1, S.d_g2, S.d_G);
       const double dpperp = S.pperp[2] - S.pperp[1], dppar = std::fabs(S.ppar[2] - S.ppar[1]);
       const double scale = 2.0 * ALPS_PI * S.sp.qs / S.sp.ms * dpperp * dppar * 0.25;
-      k_int_ee<<<1, 256, 0, s>>>(S.d_g2, S.d_ppar, N, M, scale, S.d_words);
+      k_int_ee<<<EE_BLOCKS, 256, 0, s>>>(S.d_g2, S.d_ppar, N, M, scale, S.d_words);
       fail(cudaGetLastError());
       FitJob j;
       j.a = fa;
@@ -1508,10 +1555,10 @@ int launch_build_bessel_and_reduced(alps_ctx* c, int is, double kperp) {
     k_base_pairs<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(S.d_V, S.d_mom, S.d_Vscale, M, nmax, S.d_Bt,
                                                               S.d_Bt + nvf);
     ALPS_CUDA_TRY(cudaGetLastError());
-    k_base_consts<<<(unsigned)((nm * 6 + 127) / 128), 128, 0, st>>>(S.d_V, S.d_Vscale, M, nmax,
+    k_base_consts<<<(unsigned)((nm * 6 + 1) / 2), 64, 0, st>>>(S.d_V, S.d_Vscale, M, nmax,
                                                                       S.d_Bd + 8 + nm * 6, S.d_Bd + 8);
     ALPS_CUDA_TRY(cudaGetLastError());
-    k_base_fac<<<1, 32, 0, st>>>(nmax, z, kperp, c->sys.kperp_norm, C0, S.d_Vscale, S.d_Bd, S.d_Bt + nvf + nmo);
+    k_base_fac<<<1, 192, 0, st>>>(nmax, z, kperp, c->sys.kperp_norm, C0, S.d_Vscale, S.d_Bd, S.d_Bt + nvf + nmo);
     ALPS_CUDA_TRY(cudaGetLastError());
   }
   return ALPS_OK;
