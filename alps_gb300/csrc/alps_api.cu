@@ -133,6 +133,7 @@ void alps_destroy(alps_ctx* c) {
     cudaFree(S.d_nmax);
     cudaFree(S.d_words);
     cudaFree(S.d_fit_scratch);
+    cudaFree(S.d_flog);
     cudaFree(S.d_Rw);
     cudaFree(S.d_G);
     cudaFree(S.d_X);

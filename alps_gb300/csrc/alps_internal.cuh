@@ -200,6 +200,8 @@ struct SpeciesHost {
   int* d_nmax = nullptr;                  // determine_nmax's result word
   double* d_words = nullptr;              // ee term and fit status words of prepare
   double* d_fit_scratch = nullptr;        // Levenberg-Marquardt scratch
+  double* d_flog = nullptr;               // log f0 of a log-space fit
+  size_t flog_cap = 0;
   size_t fit_scratch_cap = 0;
   double* d_Rw = nullptr;                 // weighted Bessel rows scratch
   size_t Rw_cap = 0;

@@ -81,7 +81,13 @@ __global__ void __cluster_dims__(EE_BLOCKS, 1, 1) __launch_bounds__(256)
 // Levenberg-Marquardt fit of the analytic continuation.  One block walks the
 // iperp rows of one species in order (each row starts from the previous
 // result, src/ALPS_analyt.f90:518); within a row the threads share the
-// points, the warps the entries of J^T J, and one warp solves.
+// points, the warps the entries of J^T J, and one warp solves.  Bound by the
+// FP64 pipe of one SM (16 clocks an instruction of any warp): the table's
+// logarithms come from the whole chip (k_fit_logs), one warp prepares what all
+// need of the parameters, and four warps share what each repeats; one
+// Maxwellian in log space takes its normal equations from seven sums of the
+// residual pass, and its three unknowns in registers.  193 rows of 385 points,
+// one Maxwellian: 3690 us before, 2840 us so (28 thousand clocks a row).
 // ---------------------------------------------------------------------------
 struct FitArgs {
   int N, M, nf, log_fit;
@@ -92,6 +98,7 @@ struct FitArgs {
   double lambda0, lambdafac, eps;
   // relativistic species: rows of the (Gamma, pparbar) grid
   int rel, ng, np;
+  const double* flog;   // log f0 [(N+1)*(M+1)], log fits of a non-relativistic species
   const double* f0rel;  // [(ng+1)*(np+1)]
   const double* grel;   // [ng+1]
   const double* prel;   // [np+1]
@@ -222,12 +229,14 @@ __device__ void fit_jacobian(const FitArgs& a, const double* params, int iperp, 
 // same partial-pivot elimination without forming the inverse.
 // On a 192x384 grid, two species: 35.7 ms as one warp with the sums in
 // series, 3.7 ms so.
-#define FIT_THREADS 256
+#define FIT_THREADS 128
 struct FitShared {
   double a[FIT_MAXP * (FIT_MAXP + 1)];  // normal matrix, right-hand side in the last column
   double params[FIT_MAXP], delta[FIT_MAXP];
   double red[FIT_THREADS / 32];
-  int lower, upper, singular;
+  double logp, ip0, lp;  // one Maxwellian in log space: log p0 and 1/p0 of the parameters, log amplitude on the row
+  double acc[2][FIT_THREADS / 32][8];  // one Maxwellian: the pass's sums per warp, two passes in turn
+  int lower, upper, singular, plain;
 };
 // doubles of point storage per point: two rows of table values, residual,
 // value, Jacobian
@@ -270,8 +279,12 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
   auto load_row = [&](int row, int off, int npts, int t0, int nt) {
     double* g = pts + (size_t)(row & 1) * P;
     for (int j = t0; j <= npts; j += nt) {
-      const double v = a.rel ? a.f0rel[(size_t)row * (a.np + 1) + off + j] : f0[row * (a.M + 1) + j];
-      g[j] = a.log_fit ? log(v) : v;
+      if (a.flog) {
+        g[j] = a.flog[(size_t)row * (a.M + 1) + j];
+      } else {
+        const double v = a.rel ? a.f0rel[(size_t)row * (a.np + 1) + off + j] : f0[row * (a.M + 1) + j];
+        g[j] = a.log_fit ? log(v) : v;
+      }
     }
   };
   if (!a.rel) load_row(0, 0, a.M, tid, FIT_THREADS);
@@ -332,25 +345,69 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
     const double* xp = a.rel ? a.prel + off : ppar;
     bool ahead = a.rel || iperp == N;  // the next row's table values are there (or are not wanted)
     if (npts >= 0) {
-      // residuals (and values) at the current parameters; returns their sum
-      // of squares.  maxw without exponentials, where the value is a normal
-      // number on the whole row.
+      // What every thread needs of the current parameters, by warp 0 (the
+      // logarithm on one lane, the reciprocal on another; each warp that
+      // repeated them took its share of the SM's FP64 pipe).  Unmoved
+      // parameters keep both.
+      auto settle = [&](bool moved) {
+        if (maxw) {
+          const double p0 = sh.params[0], p1 = sh.params[1], p2 = sh.params[2];
+          if (moved) {
+            if (lane == 0) sh.logp = log(p0);
+            if (lane == 1) sh.ip0 = 1.0 / p0;
+            __syncwarp();
+          }
+          if (lane == 0) {
+            const double lp = sh.logp - a.pc[0] * (xperp * xperp);
+            const double d0 = xp[0] - p2, d1 = xp[npts] - p2, dm = fmax(d0 * d0, d1 * d1);
+            sh.plain = p0 > 0.0 && p1 >= 0.0 && fabs(lp) < 600.0 && lp - p1 * dm > -690.0;
+            sh.lp = lp;
+          }
+        } else if (lane == 0) {
+          sh.plain = 0;
+        }
+      };
+      // residuals (and values) at the current, settled parameters; returns
+      // their sum of squares.  maxw without exponentials, where the value is a
+      // normal number on the whole row.
+      int buf = 0;
       auto residuals = [&](bool& plain) {
         double s = 0.0;
-        plain = false;
-        double lp = 0.0;
-        const double p0 = sh.params[0], p1 = sh.params[1], p2 = sh.params[2];
-        if (maxw && p0 > 0.0) {
-          lp = log(p0) - a.pc[0] * (xperp * xperp);
-          const double d0 = xp[0] - p2, d1 = xp[npts] - p2, dm = fmax(d0 * d0, d1 * d1);
-          plain = p1 >= 0.0 && fabs(lp) < 600.0 && lp - p1 * dm > -690.0;
-        }
+        plain = sh.plain != 0;
         if (plain) {
+          // sums of r^2, r, r d, r d^2 and d, d^2, d^3, d^4, d = x - p2: all
+          // that J^T J and J^T r need (columns 1/p0, -d^2, 2 p1 d)
+          const double lp = sh.lp, p1 = sh.params[1], p2 = sh.params[2];
+          double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
           for (int j = tid; j <= npts; j += FIT_THREADS) {
-            const double d = xp[j] - p2, r = (g[j] - lp) + p1 * (d * d);
-            resid[j] = r;
-            s = fma(r, r, s);
+            const double d = xp[j] - p2, d2 = d * d, r = (g[j] - lp) + p1 * d2;
+            v[0] = fma(r, r, v[0]);
+            v[1] += r;
+            v[2] = fma(r, d, v[2]);
+            v[3] = fma(r, d2, v[3]);
+            v[4] += d;
+            v[5] += d2;
+            v[6] = fma(d2, d, v[6]);
+            v[7] = fma(d2, d2, v[7]);
           }
+          // eight sums over the lanes by halving
+#pragma unroll
+          for (int h = 4; h >= 1; h >>= 1) {
+            const int off = 4 * h;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (i < h) {
+                const double keep = (lane & off) ? v[i + h] : v[i], give = (lane & off) ? v[i] : v[i + h];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+              }
+          }
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+          buf ^= 1;
+          if ((lane & 3) == 0) sh.acc[buf][warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = v[0];
+          __syncthreads();
+          for (int w = 0; w < FIT_THREADS / 32; ++w) s += sh.acc[buf][w][0];
+          return s;
         } else {
           for (int j = tid; j <= npts; j += FIT_THREADS) {
             const double fv = fit_value_real(a, sh.params, xperp, xp[j]);
@@ -365,53 +422,94 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
       double lambda_fit = a.lambda0;
       int counter = 0;
       bool converged = false, plain;
+      if (warp == 0) settle(iperp == 0);
+      __syncthreads();
       double LSQ = residuals(plain);
       while (!converged) {
         counter++;
-        if (plain) {
-          const double ip0 = 1.0 / sh.params[0], p1 = sh.params[1], p2 = sh.params[2];
-          for (int j = tid; j <= npts; j += FIT_THREADS) {
-            const double d = xp[j] - p2;
-            JT[j] = ip0;
-            JT[P + j] = -(d * d);
-            JT[2 * P + j] = 2.0 * p1 * d;
-          }
-        } else {
+        const int ld = nJT + 1;
+        if (!plain) {
           for (int j = tid; j <= npts; j += FIT_THREADS) {
             double J[FIT_MAXP];
             fit_jacobian(a, sh.params, iperp, xperp, xp[j], J);
             const double iv = a.log_fit ? 1.0 / fval[j] : 1.0;
             for (int k = 0; k < nJT; ++k) JT[(size_t)k * P + j] = J[k] * iv;
           }
-        }
-        __syncthreads();
-        // J^T J (upper triangle) and J^T r: a warp per entry
-        const int nq = nJT * (nJT + 1) / 2 + nJT, ld = nJT + 1;
-        for (int t = warp; t < nq; t += FIT_THREADS / 32) {
-          int k, l;
-          if (t < nJT) {
-            k = t;
-            l = nJT;
-          } else {
-            int u = t - nJT;
-            for (k = 0; u >= nJT - k; ++k) u -= nJT - k;
-            l = k + u;
+          __syncthreads();
+          // J^T J (upper triangle) and J^T r: a warp per entry
+          const int nq = nJT * (nJT + 1) / 2 + nJT;
+          for (int t = warp; t < nq; t += FIT_THREADS / 32) {
+            int k, l;
+            if (t < nJT) {
+              k = t;
+              l = nJT;
+            } else {
+              int u = t - nJT;
+              for (k = 0; u >= nJT - k; ++k) u -= nJT - k;
+              l = k + u;
+            }
+            const double *x = JT + (size_t)k * P, *y = l == nJT ? resid : JT + (size_t)l * P;
+            double acc = 0.0;
+            for (int j = lane; j <= npts; j += 32) acc = fma(x[j], y[j], acc);
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane == 0) {
+              if (l == k) acc = acc + lambda_fit * acc;
+              sh.a[k * ld + l] = acc;
+              if (l < nJT) sh.a[l * ld + k] = acc;
+            }
           }
-          const double *x = JT + (size_t)k * P, *y = l == nJT ? resid : JT + (size_t)l * P;
-          double acc = 0.0;
-          for (int j = lane; j <= npts; j += 32) acc = fma(x[j], y[j], acc);
-          for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          if (lane == 0) {
-            if (l == k) acc = acc + lambda_fit * acc;
-            sh.a[k * ld + l] = acc;
-            if (l < nJT) sh.a[l * ld + k] = acc;
-          }
+          __syncthreads();
         }
-        __syncthreads();
         if (warp == 0) {
           // elimination with partial pivoting on the augmented matrix
           bool singular = false;
-          for (int k = 0; k < nJT; ++k) {
+          if (plain) {
+            // three unknowns, in registers on every lane
+            double t[8];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) {
+              t[q] = 0.0;
+              for (int w = 0; w < FIT_THREADS / 32; ++w) t[q] += sh.acc[buf][w][q];
+            }
+            const double i0 = sh.ip0, tp = 2.0 * sh.params[1];
+            double m[3][4] = {{(double)(npts + 1) * (i0 * i0), -i0 * t[5], i0 * (tp * t[4]), i0 * t[1]},
+                              {-i0 * t[5], t[7], -tp * t[6], -t[3]},
+                              {i0 * (tp * t[4]), -tp * t[6], tp * (tp * t[5]), tp * t[2]}};
+            double x[3], rp[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) m[k][k] = m[k][k] + lambda_fit * m[k][k];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+#pragma unroll
+              for (int i = k + 1; i < 3; ++i)
+                if (fabs(m[i][k]) > fabs(m[k][k])) {
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) {
+                    const double u = m[k][c];
+                    m[k][c] = m[i][c];
+                    m[i][c] = u;
+                  }
+                }
+              if (m[k][k] == 0.0) singular = true;
+              rp[k] = 1.0 / m[k][k];
+#pragma unroll
+              for (int i = k + 1; i < 3; ++i) {
+                const double f = m[i][k] * rp[k];
+#pragma unroll
+                for (int c = k + 1; c < 4; ++c) m[i][c] -= f * m[k][c];
+              }
+            }
+            x[2] = m[2][3] * rp[2];
+            x[1] = (m[1][3] - m[1][2] * x[2]) * rp[1];
+            x[0] = ((m[0][3] - m[0][1] * x[1]) - m[0][2] * x[2]) * rp[0];
+            if (lane == 0 && !singular) {
+              sh.delta[0] = x[0];
+              sh.delta[1] = x[1];
+              sh.delta[2] = x[2];
+            }
+            __syncwarp();
+          }
+          for (int k = 0; k < (plain ? 0 : nJT); ++k) {
             int p = k;
             double mx = fabs(sh.a[k * ld + k]);
             for (int i = k + 1; i < nJT; ++i)
@@ -437,7 +535,7 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
             }
             __syncwarp();
           }
-          if (!singular)
+          if (!singular && !plain)
             for (int i = nJT - 1; i >= 0; --i) {
               const double x = sh.a[i * ld + nJT] / sh.a[i * ld + i];
               __syncwarp();
@@ -451,6 +549,8 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
               for (int k = 0, l = 0; k < n_params; ++k)
                 if ((mask >> k) & 1u) sh.params[k] = sh.params[k] + sh.delta[l++];
           }
+          __syncwarp();
+          if (!singular) settle(true);
         } else if (!ahead) {
           load_row(iperp + 1, 0, a.M, tid - 32, FIT_THREADS - 32);
         }
@@ -463,9 +563,13 @@ __device__ void lm_fit_body(const FitArgs& a, const double* __restrict__ f0, con
         const double LSQnew = residuals(plain);
         const double diff = fabs(LSQnew - LSQ);
         if (LSQnew > LSQ) {
-          if (tid == 0)
-            for (int k = 0, l = 0; k < n_params; ++k)
-              if ((mask >> k) & 1u) sh.params[k] = sh.params[k] - sh.delta[l++];
+          if (warp == 0) {
+            if (lane == 0)
+              for (int k = 0, l = 0; k < n_params; ++k)
+                if ((mask >> k) & 1u) sh.params[k] = sh.params[k] - sh.delta[l++];
+            __syncwarp();
+            settle(true);
+          }
           __syncthreads();
           lambda_fit = lambda_fit * a.lambdafac;
         } else {
@@ -543,6 +647,12 @@ __global__ void __launch_bounds__(FIT_THREADS) k_lm_fit_many(const FitJob* __res
   if (threadIdx.x == 0) J = jobs[j];
   __syncthreads();
   lm_fit_body(J.a, J.f0, J.pperp, J.ppar, J.fit, fit_points(J.a, J.scratch, fit_smem, smem_words), J.status, sh);
+}
+
+// log f0 of a whole table, over the chip
+__global__ void k_fit_logs(const double* __restrict__ f0, size_t n, double* flog) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) flog[t] = log(f0[t]);
 }
 
 // both fit kernels may take FIT_SMEM_WORDS doubles
@@ -1222,6 +1332,14 @@ int launch_prepare_species(alps_ctx* c, int is) {
     if (!words && (rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(maxpts + 1) * fit_point_words(FIT_MAXP))))
       return rc;
     ALPS_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));
+    a.flog = nullptr;
+    if (a.log_fit && !a.rel) {
+      const size_t nn = (size_t)(N + 1) * (M + 1);
+      if ((rc = ensure(S.d_flog, S.flog_cap, nn))) return rc;
+      k_fit_logs<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(S.d_f0, nn, S.d_flog);
+      ALPS_CUDA_TRY(cudaGetLastError());
+      a.flog = S.d_flog;
+    }
     k_lm_fit<<<1, FIT_THREADS, words * sizeof(double), st>>>(a, S.d_f0, S.d_pperp, S.d_ppar, S.d_fit, S.d_fit_scratch,
                                                              d_status, words);
     ALPS_CUDA_TRY(cudaGetLastError());
@@ -1264,6 +1382,7 @@ static FitArgs fit_args_of(const alps_ctx* c, const SpeciesHost& S) {
   a.f0rel = S.d_f0rel;
   a.grel = S.d_grel;
   a.prel = S.d_prel;
+  a.flog = nullptr;
   return a;
 }
 
@@ -1297,12 +1416,13 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
       if (!S.d_G && !rc) fail(cudaMalloc(&S.d_G, (size_t)(N - 1) * 2 * (M - 1) * sizeof(double)));
       if (!S.d_words && !rc) fail(cudaMalloc(&S.d_words, 2 * sizeof(double)));
       if (rc) break;
-      const FitArgs fa = fit_args_of(c, S);
+      FitArgs fa = fit_args_of(c, S);
       const int words = fit_smem_words(fa);
       fit_words = std::max(fit_words, words);
       if (!words &&
           (rc = ensure(S.d_fit_scratch, S.fit_scratch_cap, (size_t)(M + 1) * fit_point_words(FIT_MAXP))))
         break;
+      if (fa.log_fit && (rc = ensure(S.d_flog, S.flog_cap, nn))) break;
       fail(cudaMemsetAsync(S.d_g1, 0, nn * sizeof(double), s));
       fail(cudaMemsetAsync(S.d_g2, 0, nn * sizeof(double), s));
       fail(cudaMemsetAsync(S.d_words + 1, 0, sizeof(double), s));
@@ -1311,6 +1431,10 @@ int prepare_contexts(alps_ctx* const* ctx, int n, int* status) {
       const double dpperp = S.pperp[2] - S.pperp[1], dppar = std::fabs(S.ppar[2] - S.ppar[1]);
       const double scale = 2.0 * ALPS_PI * S.sp.qs / S.sp.ms * dpperp * dppar * 0.25;
       k_int_ee<<<EE_BLOCKS, 256, 0, s>>>(S.d_g2, S.d_ppar, N, M, scale, S.d_words);
+      if (fa.log_fit) {
+        fa.flog = S.d_flog;
+        k_fit_logs<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(S.d_f0, nn, S.d_flog);
+      }
       fail(cudaGetLastError());
       FitJob j;
       j.a = fa;
