@@ -15,10 +15,12 @@
 //   k_stage             a lone batch's arguments and job to device memory
 //   k_classify_multi    resonant orders of each (omega, species) into
 //                       fixed slots, one warp per (omega, species)
+//   k_far_orders, k_far_levels  (large batches) coefficients of the power
+//                       series in omega that sums a frequency's far orders
 //   k_pole_sums_multi   the pole sums over all orders: order chunks x omega
-//                       tiles x node slices.  Plain path in FP64; fast path
-//                       (pole_fused) in double-float on the FP32 pipes, all
-//                       orders of a chunk in one set of sums
+//                       tiles x lanes of a frequency.  Plain path in FP64; fast
+//                       path (pole_fused) in double-float on the FP32 pipes,
+//                       all orders of a chunk in one set of sums
 //   k_resonant_lanes    (mixed batches of 2560 and more) principal value +
 //                       Landau per resonant (omega, species, n), an item per
 //                       lane; marks the few items it leaves
@@ -299,8 +301,10 @@ __device__ __forceinline__ OrderInfo shfl_info(const OrderInfo& a, int src) {
 //   * far poles: the Laurent series Q = f sum_k mom_k t^k, d = p_res - pcen,
 //     t = prad/d, f = 1/(k_par d); with T = f sum_{k>=1}, U = f sum_{k>=2}:
 //     sum F p R = pcen Q + d T, sum F p^2 R = pcen^2 Q + 2 pcen d T + d^2 U
-//     (no cancellation for far poles); the terms from K32 on in FP32.
-// An FP32 test settles orders far from resonance (the FP64 geometry decides
+//     (no cancellation for far poles); the terms from K32 on in FP32;
+//   * in large batches, the orders |n| >= n0 in one series of omega (far_level).
+// g1 and g2, two nodes' R and two powers of t go side by side through packed
+// instructions.  An FP32 test settles orders far from resonance (the FP64 geometry decides
 // the rest).  Each order's entries X_e = omega S_{e,1} + kappa S_{e,2} are
 // added, times the order factor C0 v_e(n) (sign of -n for xy, xz), to one
 // double-float sum per entry; the phase (i for xy, yz) and the entry scale

@@ -186,17 +186,19 @@ int alps_set_k_many(alps_ctx* const* ctx, int n, const double* kperp,
                     const double* kpar, int* status);
 
 /* Evaluation mode of the omega pass.
- * ALPS_PREC_FP64 (plain): every p_par pole sum is the trapezoid node sum of
- *   the reference, in FP64 (the parity path).
- * ALPS_PREC_MIXED (fast): for non-resonant orders whose pole lies well
- *   outside the p_par grid the node sum is replaced by its Laurent series
- *   about the grid centre, truncated where the remainder is below FP64
- *   rounding (rho^K <= 2^-53 (1-rho)); one-Maxwellian Landau rows are
- *   factorised where their deviation bound is below 1e-5; the node sums,
- *   series terms and principal-value sums run in double-float arithmetic
- *   (float pairs, about 46-48 bits).  Resonance decisions, windows and
- *   sample points are the reference's in both modes; results agree with the
- *   plain mode to about 1e-10 in det D on the benchmark map. */
+ * ALPS_PREC_FP64 (plain): FP64 throughout (the parity path).  Orders in or
+ *   near resonance sum the reference's trapezoid nodes; for a pole well
+ *   outside the p_par grid the node sum is replaced by its Laurent series about
+ *   the grid centre, truncated below FP64 rounding (rho^K <= 2^-55 (1-rho));
+ *   large batches sum the orders far beyond a frequency in one power series of
+ *   omega, to the same remainder; one-Maxwellian Landau rows are factorised
+ *   where their deviation bound is below 1e-5 (a relative error of 2e-16).
+ * ALPS_PREC_MIXED (fast): the same sums with the node sums, series terms,
+ *   principal-value sums and factorised Landau terms in double-float
+ *   arithmetic (float pairs, about 46-48 bits), and the series' terms below
+ *   2^-33 in FP32.  Resonance decisions, windows and sample points are the
+ *   reference's in both modes; results agree with the plain mode to about
+ *   2e-11 in det D on the benchmark map. */
 enum { ALPS_PREC_FP64 = 0, ALPS_PREC_MIXED = 1 };
 int alps_set_precision(alps_ctx* ctx, int precision);
 
@@ -522,7 +524,7 @@ int alps_tc_product(const double* d_A, const double* d_B, double* d_C, int M,
 
 /* Autotuner of the batch kernels' launch shapes.  Times the candidate
  * shapes of a batch of n frequencies on this context (its k and precision
- * path): j slices per frequency of the pole sums (1, 2, 4, 8, 16, 32) x
+ * path): lanes per frequency of the pole sums (1, 2, 4, 8, 16, 32) x
  * pole-sum blocks per SM (2, 4, 8) x resonant-item warps per SM (6, 12, 24),
  * each the best of two launches after a warm-up.  The fastest (if 3 % faster
  * than the default rule) is kept for every batch of the same bucket: N_perp,
