@@ -3649,7 +3649,9 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     if (c->flags_dirty) ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
     c->flags_dirty = false;
   } else {
-    ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
+    // (with the counters: calls that a caller let overlap, against the
+    // contract, leave nothing behind)
+    ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, (small ? 2 + n : 1) * sizeof(int), st));
   }
   if (small) {
     DispJob job = lone_job(sh, n, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, flags);
@@ -3949,9 +3951,9 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 // that device (with that device current); make that first call before any
 // stream capture.  Every call shares the one array: two calls whose kernels
 // overlap on the GPU (different streams, or different host threads) race on
-// it and must be ordered by the caller.  The error flag is cleared at the
-// start of every call and the counters of a small batch are zero between
-// calls; every other word a call reads it writes first.  The
+// it and must be ordered by the caller.  The error flag and a small batch's
+// counters are cleared at the start of every call; every other word a call
+// reads it writes first.  The
 // flag word's device address is recorded in the context, so
 // alps_batch_status reports the call's device errors (read it before the
 // next call on the device clears the word).
@@ -3959,7 +3961,7 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 #define ALPS_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[ALPS_NOALLOC_SCRATCH_BYTES];
-static __device__ int g_noalloc_arrive[SMALL_WARPS];  // counters of a small batch, zero between launches
+static __device__ int g_noalloc_arrive[SMALL_WARPS];  // counters of a small batch
 
 namespace {
 std::mutex g_noalloc_mu;
@@ -4018,6 +4020,7 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   job.rel = a.relcap ? relb : nullptr;
   job.bm = a.has_bm ? bmb : nullptr;
   if (small_batch(c, bg)) {
+    ALPS_CUDA_TRY(cudaMemsetAsync(cnt, 0, n * sizeof(int), st));
     job.nslots = (int)nslots;
     job.arrive = static_cast<int*>(cnt);
     const int rc = launch_one(c, a, sh, job, st);
