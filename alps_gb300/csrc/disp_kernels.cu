@@ -3271,7 +3271,8 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->lgch = (float)o->lgc;
   o->lgcl = (float)(o->lgc - (double)o->lgch);
   o->lcx = -2.0 * S.p2r * o->dppar_abs;
-  o->lze = (S.min_a0 > 0.0 && std::isfinite(S.min_a0)) ? std::ilogb(S.min_a0) : 0;
+  // (a row of amplitude zero leaves the Landau term zero at every frequency)
+  o->lze = S.min_a0 > 0.0 ? std::ilogb(S.min_a0) : -1000000;
   o->lge = (o->lgc > 0.0) ? std::ilogb(o->lgc) : -2000;
   o->relat = S.sp.relat ? 1 : 0;
   o->ng = c->sys.ngamma;
