@@ -3436,12 +3436,18 @@ inline size_t carve(size_t& off, size_t bytes) {
   return at;
 }
 
+// doubles of a species' far-order tables: by level (far), then by order (farc)
+size_t far_words(const SpeciesHost& S) { return (size_t)(FAR_LEVELS + S.nmax) * FAR_K * 12; }
+
 // the scratch of a batch in one array: error word, counts, slots, items,
-// relativistic and closed-form results, arguments, job, and last the
-// partial sums (part_bytes of them); off[] receives the offsets
-enum { SC_FLAGS, SC_COUNT, SC_SLOTS, SC_ITEMS, SC_REL, SC_BM, SC_ARGS, SC_JOB, SC_PART, SC_N };
-size_t scratch_layout(const alps_ctx* c, size_t n, size_t nslots, size_t part_bytes, size_t* off) {
+// relativistic and closed-form results, arguments, job, far-order tables
+// (far: the batch takes that series), and last the partial sums (part_bytes
+// of them); off[] receives the offsets
+enum { SC_FLAGS, SC_COUNT, SC_SLOTS, SC_ITEMS, SC_REL, SC_BM, SC_ARGS, SC_JOB, SC_FAR, SC_PART, SC_N };
+size_t scratch_layout(const alps_ctx* c, size_t n, size_t nslots, size_t part_bytes, bool far, size_t* off) {
   const size_t S_ = c->sys.nspec;
+  size_t farw = 0;
+  for (size_t s = 0; s < S_ && far; ++s) farw += far_words(c->spec[s]);
   size_t end = 0;
   off[SC_FLAGS] = carve(end, sizeof(int));
   off[SC_COUNT] = carve(end, n * S_ * sizeof(int));
@@ -3451,6 +3457,7 @@ size_t scratch_layout(const alps_ctx* c, size_t n, size_t nslots, size_t part_by
   off[SC_BM] = carve(end, n * S_ * (any_bm(c) ? 24 : 0) * sizeof(double2));
   off[SC_ARGS] = carve(end, sizeof(DispArgs));
   off[SC_JOB] = carve(end, DISP_JOB_BYTES);
+  off[SC_FAR] = carve(end, farw * sizeof(double));
   off[SC_PART] = carve(end, part_bytes);
   return end;
 }
@@ -3492,10 +3499,15 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
   if (tensors) csize = 1;
   csize = std::max(csize, 1L);
   b.nslots = (size_t)n * S_ * rcap;
+  sh.far = (!tensors && (long)n * orders / 32 >= FAR_MIN) ? 1 : 0;
   if (!tensors) {
     size_t off[SC_N];
-    const size_t row = (size_t)n * S_ * 6 * sizeof(double2);
-    if (scratch_layout(c, n, b.nslots, row * noalloc_chunks(n, S_, maxn), off) <= ALPS_NOALLOC_SCRATCH_BYTES) {
+    const size_t row = (size_t)n * S_ * 6 * sizeof(double2), part = row * noalloc_chunks(n, S_, maxn);
+    if (scratch_layout(c, n, b.nslots, part, false, off) <= ALPS_NOALLOC_SCRATCH_BYTES) {
+      // (a batch that fits without the far-order tables alone does without
+      // the series, through every entry point)
+      if (sh.far && scratch_layout(c, n, b.nslots, part, true, off) > ALPS_NOALLOC_SCRATCH_BYTES) sh.far = 0;
+      scratch_layout(c, n, b.nslots, part, sh.far != 0, off);
       const long room = (long)((ALPS_NOALLOC_SCRATCH_BYTES - off[SC_PART]) / row);
       csize = std::max(csize, (2L * maxn + room) / room);
     }
@@ -3517,7 +3529,6 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
     sh.lanes = (int)std::max(96L, std::min(256L, per));
     sh.ipw = (int)std::max(256L, ((long)b.nslots / (152 * 12) + 31) / 32 * 32);
   }
-  sh.far = (!tensors && (long)n * orders / 32 >= FAR_MIN) ? 1 : 0;
   sh.fin_warp = (n <= FIN_WARP_MAX || tensors || rel_capacity(c) || any_bm(c)) ? 1 : 0;
   return b;
 }
@@ -3943,8 +3954,9 @@ int run_disp_multi(const MultiLaunch& ml, cudaStream_t st) {
 // forbids plugins from creating allocations behind its back.  For them,
 // alps_disp_batch_noalloc runs the same kernels as
 // alps_disp_batch_device with all of their scratch (partial sums,
-// resonant-order slots, resonant results, error flag) carved from the
-// file-scope device array below instead of context buffers.
+// resonant-order slots, resonant results, far-order tables, error flag)
+// carved from the file-scope device array below instead of context buffers:
+// a call may overlap the context's other batches.
 //
 // The array is ALPS_NOALLOC_SCRATCH_BYTES (16 MiB) and lives on every device
 // that loads this library until the process exits.  Its device address is
@@ -4003,7 +4015,7 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   const DispShape sh = bg.sh;
   size_t off[SC_N];
   const size_t nslots = bg.nslots;
-  const size_t total = scratch_layout(c, n, nslots, (size_t)n * S_ * sh.nchunk * 6 * sizeof(double2), off);
+  const size_t total = scratch_layout(c, n, nslots, (size_t)n * S_ * sh.nchunk * 6 * sizeof(double2), sh.far != 0, off);
   if (scratch_bytes) *scratch_bytes = total;
   if (total > ALPS_NOALLOC_SCRATCH_BYTES) return ALPS_E_INVALID;  // batch too large for the static scratch
   unsigned char* b = static_cast<unsigned char*>(base);
@@ -4031,6 +4043,16 @@ extern "C" int alps_disp_batch_noalloc(alps_ctx* c, int n, const alps_complex* d
   }
   DispArgs* da = reinterpret_cast<DispArgs*>(b + off[SC_ARGS]);
   DispJob* dj = reinterpret_cast<DispJob*>(b + off[SC_JOB]);
+  if (sh.far) {
+    // the coefficients belong to this batch's k_par: the context's own tables
+    // may serve another batch of it at another k_par meanwhile
+    double* f = reinterpret_cast<double*>(b + off[SC_FAR]);
+    for (int s = 0; s < S_; ++s) {
+      a.sp[s].far = f;
+      a.sp[s].farc = f + (size_t)FAR_LEVELS * FAR_K * 12;
+      f += far_words(c->spec[s]);
+    }
+  }
   k_stage<<<1, 128, 0, st>>>(a, job, da, dj);
   ALPS_CUDA_TRY(cudaGetLastError());
   k_classify_multi<<<(unsigned)cls_blocks(n, S_), 128, 0, st>>>(dj, 1);

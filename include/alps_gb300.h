@@ -229,7 +229,8 @@ int alps_disp_batch_device(alps_ctx* ctx, int n, const alps_complex* d_om,
  * call on a device looks up that array's address (cudaGetSymbolAddress) with
  * the device current; make it before any stream capture.  All calls share
  * the array: calls that overlap on the GPU race and must be serialised by the
- * caller.  Batches whose scratch would exceed 16 MiB return ALPS_E_INVALID
+ * caller; a call may overlap the context's other batches (also at another
+ * k_par, as its k tables stay).  Batches whose scratch would exceed 16 MiB return ALPS_E_INVALID
  * without launching; *scratch_bytes (may be NULL) receives the bytes the
  * batch needs.  stream: cudaStream_t, NULL = the context's stream. */
 int alps_disp_batch_noalloc(alps_ctx* ctx, int n, const alps_complex* d_om,
