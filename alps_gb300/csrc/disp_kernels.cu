@@ -3645,9 +3645,13 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     if ((rcode = ensure_buf(c->d_bm, c->bm_cap, (size_t)n * S_ * 24))) return rcode;
   if (!c->d_flags) {
     // the error word, the error word of batches that report to hflag, and a
-    // counter per frequency of a small batch (zero between launches)
-    ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, (2 + SMALL_WARPS) * sizeof(int)));
-    ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, (2 + SMALL_WARPS) * sizeof(int), st));
+    // counter per frequency of a small batch (zero between launches), once
+    // for the batches without hflag and once for those with it: the latter
+    // are over when their call returns, so nothing that a caller leaves
+    // running reaches their counters
+    ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, (2 + 2 * SMALL_WARPS) * sizeof(int)));
+    ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, (2 + 2 * SMALL_WARPS) * sizeof(int), st));
+    ALPS_CUDA_TRY(cudaStreamSynchronize(st));
     c->flags_dirty = false;
   }
   const void* after[7] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_rel, c->d_bm, c->d_flags};
@@ -3669,7 +3673,7 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     DispJob job = lone_job(sh, n, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, flags);
     job.ext = d_ext;
     job.nslots = (int)nslots;
-    job.arrive = c->d_flags + 2;
+    job.arrive = c->d_flags + 2 + (hflag ? SMALL_WARPS : 0);
     job.hflag = hflag;
     if ((rcode = launch_one(c, a, sh, job, st))) return rcode;
     if (flag_there) *flag_there = hflag != nullptr;

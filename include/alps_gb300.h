@@ -214,7 +214,10 @@ int alps_disp_batch(alps_ctx* ctx, int n, const alps_complex* om,
                     alps_complex* D);
 
 /* det D for n frequencies already in device memory; stream is a
- * cudaStream_t (NULL = the context's stream).  Asynchronous. */
+ * cudaStream_t (NULL = the context's stream).  Asynchronous.  The batches of
+ * a context share its workspace: order a call on another stream, or a call
+ * from host memory, after the batches still running, or their det D is
+ * undefined (later calls are not touched). */
 int alps_disp_batch_device(alps_ctx* ctx, int n, const alps_complex* d_om,
                            alps_complex* d_D, void* stream);
 
