@@ -1388,12 +1388,21 @@ struct __align__(16) PvPiece {
   T Ax, Ay, Bx, By;
   int a, pad[3];
 };
+// Windows of more than PV_WIDE nodes to a side are summed sample by sample
+// (pv_direct): a piece then holds two samples or fewer of the usual 100, the
+// weights of a window's nodes cost its square, and past 354 nodes they would
+// not fit a block's shared memory.  Mixed and FP64, 64x256 grid, 700
+// frequencies, us by pieces and by samples: 24 nodes 333 and 388, 633 and 621;
+// 48: 461 and 334, 771 and 555; 100: 517 and 272, 774 and 423; 4096
+// frequencies: 24: 871 and 1446, 2160 and 2357; 48: 1114 and 1156, 2504 and
+// 1992; 100: 1181 and 705, 2278 and 1429.
+#define PV_WIDE 48
 // pieces at most: both sides of the window, the tiny rest
-__host__ __device__ inline int pv_max_pieces(int M_I) { return 2 * (M_I + 4) + 8; }
-// double2 words per warp: prefix sums of a chunk, pieces, node weights
+__host__ __device__ inline int pv_max_pieces(int M_I) { return 2 * ((M_I < PV_WIDE ? M_I : PV_WIDE) + 4) + 8; }
+// double2 words per warp: prefix sums of a chunk, pieces, node weights (as many as pieces)
 __host__ __device__ inline size_t pv_warp_words(int M_I) {
   const size_t np = (size_t)pv_max_pieces(M_I);
-  return (PV_CHUNK * 24 + 15) / 16 + np * (sizeof(PvPiece<double>) / 16) + (2 * (M_I + 4) + 8);
+  return (PV_CHUNK * 24 + 15) / 16 + np * (sizeof(PvPiece<double>) / 16) + np;
 }
 
 // prefix sums at the lane's cut kc (see pv_sample); pre: PV_CHUNK PvSums
@@ -1535,7 +1544,7 @@ __device__ bool pv_warp_weights(const SpecDev& S, const SysDev& sys, const PvIte
     hi = max(hi, rec[t].a);
   }
   a0 = __reduce_min_sync(FULL_WARP, lo) - 1;
-  cnt = min(__reduce_max_sync(FULL_WARP, hi) + 1 - a0 + 1, 2 * (sys.M_I + 4) + 8);
+  cnt = min(__reduce_max_sync(FULL_WARP, hi) + 1 - a0 + 1, cap_rec);
   const T hid = SS::hid(S);
   for (int t = lane; t < cnt; t += 32) {
     T Wx = z, Wy = z, Dx = z, Dy = z;
@@ -1567,7 +1576,8 @@ __device__ __forceinline__ void pv_add_out(double2* out, const double* pref, int
 }
 
 // The same sum sample by sample over the reference's own points, in FP64: for
-// items with a sample that funct_g's search finds no node for.
+// items with a sample that funct_g's search finds no node for, and for
+// windows of more than PV_WIDE nodes to a side.
 __device__ __noinline__ void pv_direct(const SpecDev& S, const SysDev& sys, const PvItem& it, double2 o,
                                        const double* pref, double2* out) {
   const int lane = threadIdx.x & 31, M = S.M, M_P = sys.M_P, n = it.nn < 0 ? -it.nn : it.nn;
@@ -1639,7 +1649,7 @@ __device__ __noinline__ void pv_warp(const SpecDev& S, const SysDev& sys, const 
   PvPiece<T>* rec = reinterpret_cast<PvPiece<T>*>(wk + (PV_CHUNK * 24 + 15) / 16);
   T* wts = reinterpret_cast<T*>(wk + (PV_CHUNK * 24 + 15) / 16 + pv_max_pieces(sys.M_I) * (sizeof(PvPiece<double>) / 16));
   int a0, cnt;
-  if (!pv_warp_weights<T>(S, sys, it, o.x, pre, rec, wts, lane, a0, cnt)) {
+  if (sys.M_I > PV_WIDE || !pv_warp_weights<T>(S, sys, it, o.x, pre, rec, wts, lane, a0, cnt)) {
     pv_direct(S, sys, it, o, pref, out);
     return;
   }

@@ -849,8 +849,12 @@ struct RelPiece {
 
 #define REL_PRE_WORDS (3 * (REL_CHUNK + 1) + 1)  // even: the pieces after them are 16-byte aligned
 
-// pieces of a row at most: both sides of the window, the tiny rest
-__host__ __device__ inline int rel_max_pieces(int M_I) { return 2 * (M_I + 4) + 8; }
+// pieces of a row held at a time: both sides of the window and the tiny rest,
+// for windows of more than REL_WIDE nodes to a side REL_PART of the former (the
+// pieces' node weights add up, so a row may take them part by part)
+#define REL_WIDE 128
+#define REL_PART 256
+__host__ __device__ inline int rel_max_pieces(int M_I) { return 2 * ((M_I < REL_WIDE ? M_I : REL_WIDE) + 4) + 8; }
 // shared memory per warp in doubles: prefix sums of a chunk of samples, pieces
 __host__ __device__ inline size_t rel_warp_words(int M_I) {
   return REL_PRE_WORDS + (size_t)rel_max_pieces(M_I) * (sizeof(RelPiece) / sizeof(double));
@@ -926,9 +930,10 @@ __device__ RelSums rel_cut_sums(const RelSamples& q, double dI2, bool from0, int
 // of one node and linear in p, so each piece needs only the sums of its
 // samples' weights and of their first moments; the samples are summed once,
 // as prefix sums, for both sides of the window, and each lane cuts them at
-// the ends of its piece.  Returns the number of pieces left in rec.
-__device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, int ig, double* pre, RelPiece* rec,
-                          int lane) {
+// the ends of its piece.  Returns the number of pieces left in rec; more: there
+// are further parts.
+__device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, int ig, int part, double* pre,
+                          RelPiece* rec, int lane, bool& more) {
   const double* pb = S.prel;
   const int np = S.np, M_P = sy.M_P;
   const double dpb = pb[2] - pb[1];
@@ -938,12 +943,14 @@ __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, i
   const int cap_rec = rel_max_pieces(sy.M_I);
   int nrec = 0;
   RelSamples q = {dR, cap, sm, 1.0, M_P, false};
+  more = false;
   if (sym) {
     const int jc = rel_piece(S, dR);  // the pole's own interval (the window lies inside the grid)
     const int nu = max(0, rel_piece(S, dR + cap) - jc) + 1, nd = max(0, jc - rel_piece(S, 2.0 * dR - (dR + cap))) + 1;
-    for (int t0 = 0; t0 < nu + nd; t0 += 32) {
+    const int first = part * REL_PART, last = min(nu + nd, sy.M_I > REL_WIDE ? first + REL_PART : cap_rec);
+    for (int t0 = first; t0 < last; t0 += 32) {
       const int t = t0 + lane;
-      const bool has = t < nu + nd && t < cap_rec, down = t >= nu;
+      const bool has = t < last, down = t >= nu;
       const int i = down ? t - nu : t, j = down ? jc - i : jc + i;
       // first sample beyond the piece: up p_k >= pb[j+1], down 2 dR - p_k < pb[j]
       int kc = M_P + 1;
@@ -988,10 +995,15 @@ __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, i
         // up: w/(dx - i dI) = w r (dx + i dI); down: -w/(dx + i dI) at -dx
         pc.A = down ? cmk(-s1, s2) : cmk(s1, s2);
         pc.B = cmk(fma(del, pc.A.x, s3), fma(del, pc.A.y, down ? -dI * s1 : dI * s1));
-        rec[t] = pc;
+        rec[t - first] = pc;
       }
     }
-    nrec = min(nu + nd, cap_rec);
+    nrec = last - first;
+    if (sy.M_I > REL_WIDE && last < nu + nd) {
+      more = true;
+      __syncwarp();
+      return nrec;
+    }
   } else {
     // g' sum_k w_k dx^2/(dx^2 + dI^2), and +- i pi G(p_res)/smdelta
     const RelSums s = rel_cut_sums(q, dI2, false, M_P + 1, pre, lane);
@@ -1250,8 +1262,9 @@ __global__ void __launch_bounds__(REL_THREADS) k_rel_orders(RelArgs a, const dou
             node(ig, ip, cmk(dx * x, r.dI * x));
           }
         }
-        if (r.pv) {
-          const int nrec = rel_pieces(S, sy, r, ig, wsm, rec, lane);
+        bool more = r.pv;
+        for (int part = 0; more; ++part) {
+          const int nrec = rel_pieces(S, sy, r, ig, part, wsm, rec, lane, more);
           int a0 = np, a1 = 0;
           for (int t = lane; t < nrec; t += 32) {
             a0 = min(a0, rec[t].a);
