@@ -1134,8 +1134,10 @@ __device__ void eval_fit3_d(const SpecDev& S, double vA, int iperp, double2 p, d
 //
 // Two kernels:
 //   k_resonant_lanes  an item per lane: lattices on the mixed path.  No
-//     exchange between lanes; items that need the FP64 sums or the Landau
-//     rows are left to the other kernel.
+//     exchange between lanes; items that need the FP64 sums, the Landau
+//     rows, or a shape that a lane does not take (PVL_SAMPLES samples, pieces
+//     at the grid's ends) are left to the other kernel, which sums them as in
+//     a smaller batch.
 //   k_resonant_multi  an item per warp (the per-item set-up still one per
 //     lane): everything else.
 // ---------------------------------------------------------------------------
@@ -2184,7 +2186,7 @@ __device__ __noinline__ void resonant_group(const DispArgs& a, const double2* __
     int lf;
     work = res_item<true>(a, S, o, nn, pv, pref, res, lf);
     double2* out = items + item * 6;
-    if (list) work &= (sv >> 16) & 3;  // the FP64 sums and the rows (never the double-float sums)
+    if (list) work &= sv >> 16;
     else
       for (int e = 0; e < 6; ++e) out[e] = res[e];
     it.pv = pv;
@@ -2268,6 +2270,7 @@ __device__ __forceinline__ void resonant_body(const DispArgs& a, const DispShape
 // 1539 us so; 8192 frequencies 384 and 119 us.
 // ---------------------------------------------------------------------------
 #define PVL_TINY 4  // cuts of the tiny rest at most
+#define PVL_SAMPLES 128  // samples of a run below this (a cut is a byte); more go by warps
 __host__ __device__ inline int pvl_side(int M_I) { return M_I + 3; }  // cuts of a side at most (eight)
 __host__ __device__ inline int pvl_slots(int M_I) { return 2 * pvl_side(M_I) + PVL_TINY; }
 // bytes per block: two float pairs and a weight per cut and lane, the warps' queues
@@ -2320,7 +2323,7 @@ __device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, con
   const bool sym = fabs(it.pim) > sys.Tlim;
   // the cuts of the three runs of samples (up, down, tiny rest), a byte each
   unsigned long long cu = ~0ull, cd = ~0ull, ct = ~0ull;
-  bool ok = M_P < 128 && it.ntiny < 128, lost = it.direct;
+  bool ok = M_P < PVL_SAMPLES && it.ntiny < PVL_SAMPLES, lost = it.direct;
   int nu = 2, nd = 2, nt = 0;  // pieces (without sym: H at p_res and a spacing to either side)
 #pragma unroll 1
   for (int sd = 0; sd < 3; ++sd) {
@@ -2509,7 +2512,7 @@ __device__ __forceinline__ void lanes_body(const DispArgs& a, const DispShape& s
           double2* out = items + item * 6;
 #pragma unroll
           for (int e = 0; e < 6; ++e) out[e] = res[e];
-          slot_nn[item] = todo_slot(nn, work & 3);
+          slot_nn[item] = todo_slot(nn, (work & 3) ? work : 0);
           if (work & 3) atomicOr(flags, FLAG_TODO);
         }
       });
@@ -3533,7 +3536,8 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
   sh.kmid = (int)(0.8 * (c->sys.npar - 1) / sh.js) + 16;
   sh.ipw = res_items_per_warp((long)b.nslots, ts.warps_per_sm ? ts.warps_per_sm : 12);
   sh.lanes = 0;
-  if (mixed && !tensors && n >= RES_LANES_MIN && pvl_side(c->sys.positions_principal) <= 8) {
+  if (mixed && !tensors && n >= RES_LANES_MIN && pvl_side(c->sys.positions_principal) <= 8 &&
+      c->sys.n_resonance_interval < PVL_SAMPLES) {
     // about a third of the slots is occupied: 96 fill a warp's lanes once
     const long per = ((long)b.nslots / (152 * 12) + 31) / 32 * 32;
     sh.lanes = (int)std::max(96L, std::min(256L, per));
