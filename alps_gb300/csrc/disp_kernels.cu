@@ -3424,6 +3424,17 @@ void default_shape(long u, bool mixed, int* lanes, long* csize) {
   }
 }
 
+// Lanes per frequency of a batch with tensors (u as above), whose chunks are
+// single orders: one lane of a frequency takes its order's series, so more of
+// them pay only where the batch leaves the chip idle and the node sums are the
+// longest chain.  calc_eigen on a 96x192 grid, mixed, us with 32/16/8/4/2/1
+// lanes: u = 80: 113, 121, 170, 282, 491, 874; 208: 196, 175, 216, 350, 631,
+// 1123; 832: 345, 273, 235, 255, 701, 1225; 1181: 622, 537, 488, 463, 479, 509;
+// 2418: 851, 660, 547, 512, 487, 539; 24187: 6911, 4929, 3872, 3293, 3009,
+// 2874; FP64: 80: 141, 145, 229, ..; 832: 710, 480, 386, 427, ..; 2418: 1891,
+// 1303, 1000, 886, 870, 1130; 8062: 5841, 3903, 2835, 2265, 2126, 2079.
+int tensor_lanes(long u) { return u < 100 ? 32 : (u < 300 ? 16 : (u < 900 ? 8 : (u < 1500 ? 4 : (u < 7000 ? 2 : 1)))); }
+
 // launch shape of a batch of n omegas on a context (default rule, or the
 // autotuner's shape for the batch's bucket).  The shape depends on n, the
 // context and the table only: the lanes and chunks fix the summation order.
@@ -3510,7 +3521,7 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
     if (!c->spec[s].sp.relat && !c->spec[s].sp.use_bM) orders += 2 * c->spec[s].nmax + 1;
   long csize = 0;
   default_shape((long)n * orders / 32, mixed, &sh.js, &csize);
-  if (tensors) sh.js = 32;
+  if (tensors) sh.js = tensor_lanes((long)n * orders / 32);
   else if (ts.js) sh.js = ts.js;
   sh.wt = (int)(((long)n * sh.js + 31) / 32);
   if (ts.blocks_per_sm || csize == 0) {
