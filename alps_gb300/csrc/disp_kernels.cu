@@ -3650,10 +3650,9 @@ long lanes_blocks(const BatchGeom& bg) {
 
 }  // namespace
 
-int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext, cudaStream_t st,
-                      int* hflag, bool* flag_there) {
-  if (flag_there) *flag_there = false;
-  if (n <= 0) return ALPS_OK;
+// first: the first part of a batch, which clears its error word
+static int launch_disp_part(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext, cudaStream_t st,
+                            int* hflag, bool* flag_there, bool first) {
   const int S_ = c->sys.nspec;
   DispArgs a;
   int maxn = 0;
@@ -3697,7 +3696,7 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
     flags = c->d_flags + 1;
     if (c->flags_dirty) ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
     c->flags_dirty = false;
-  } else {
+  } else if (first) {
     // (with the counters: calls that a caller let overlap, against the
     // contract, leave nothing behind)
     ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, (small ? 2 + n : 1) * sizeof(int), st));
@@ -3775,6 +3774,40 @@ int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, dou
   c->stats.n_eval_total += n;
   // k_stage and the four; the far orders' two and k_resonant_lanes for large batches
   c->stats.kernels_launched = 5 + (sh.far ? 2 : 0) + (lblocks ? 1 : 0) + (a.relcap ? 1 : 0) + (a.has_bm ? 1 : 0);
+  return ALPS_OK;
+}
+
+// The partial sums of a batch with tensors, one per order, are held for at most
+// so many bytes of frequencies at a time: each part still has some 22 000 warps
+// of orders, twelve times what the chip holds.
+#define TENSOR_PART_BYTES (64L << 20)
+
+int launch_disp_batch(alps_ctx* c, int n, const double2* d_om, double2* d_D, double2* d_ext, cudaStream_t st,
+                      int* hflag, bool* flag_there) {
+  if (flag_there) *flag_there = false;
+  if (n <= 0) return ALPS_OK;
+  long parts = 1;
+  if (d_ext) {
+    long orders = 1;
+    for (const SpeciesHost& S : c->spec)
+      if (!S.sp.relat && !S.sp.use_bM) orders = std::max(orders, 2L * S.nmax + 1);
+    const long bytes = orders * c->sys.nspec * 6 * (long)sizeof(double2);
+    parts = std::min((long)n, (n * bytes + TENSOR_PART_BYTES - 1) / TENSOR_PART_BYTES);
+  }
+  if (parts <= 1) return launch_disp_part(c, n, d_om, d_D, d_ext, st, hflag, flag_there, true);
+  // (even parts: one launch shape for all)
+  auto launched = c->stats.kernels_launched;
+  launched = 0;
+  for (int p = 0, o = 0; p < (int)parts; ++p) {
+    const int m = n / (int)parts + (p < n % (int)parts ? 1 : 0);
+    const int rc = launch_disp_part(c, m, d_om + o, d_D + o, d_ext + (size_t)o * (c->sys.nspec * 36 + 9), st, nullptr,
+                                    nullptr, p == 0);
+    if (rc) return rc;
+    launched += c->stats.kernels_launched;
+    o += m;
+  }
+  c->stats.n_eval = n;
+  c->stats.kernels_launched = launched;
   return ALPS_OK;
 }
 
