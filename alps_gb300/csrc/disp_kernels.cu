@@ -2744,13 +2744,13 @@ __device__ __noinline__ void finalize_warp(const DispArgs& a, const DispShape& s
 }
 
 // ---------------------------------------------------------------------------
-// Jobs.  Every batch, of one context or fused over many, runs the same four
+// Jobs.  Every batch, of one context or fused over many, runs the same
 // kernels over a table of jobs in device memory: each kernel's grid is the
 // concatenation of the jobs' own grids, and a block finds its job by the
 // first block of each job.  A job's arguments (the context at its k) and its
-// launch shape are those of a lone batch of its size, and one compiled
-// kernel serves every case, so a context's results do not depend on what it
-// was batched with, bit for bit.
+// launch shape are those of a lone batch of its size, and small batches in
+// one launch give the bits of the kernels apart (k_disp_one), so a context's
+// results do not depend on what it was batched with, bit for bit.
 // ---------------------------------------------------------------------------
 struct DispJob {
   const DispArgs* a;  // the context's arguments (device copy)
@@ -3031,8 +3031,11 @@ __global__ void k_finalize_multi(const DispJob* __restrict__ jobs, int nj) {
 // to that frequency's det D: nothing waits on anything.  The sums are those of
 // the kernels above, in the same order.  One frequency, mixed path, 60x120
 // grid: 67 us in five kernels, 38 us so; a call from the host 110 and 62 us.
-// pole_body, resonant_group and finalize_warp are compiled once (noinline), so
-// a frequency's det D is the same bit for bit in either form.
+// The bodies both forms share (pole_body, res_core_call, pv_warp, pv_direct,
+// landau_rows, finalize_warp) are compiled once (noinline), and the factorised
+// Landau terms, of which resonant_one spreads one over the lanes, round every
+// operation by itself, so a frequency's det D is the same bit for bit in
+// either form.
 // ---------------------------------------------------------------------------
 // the slot's order (the r-th resonant order of its (omega, species)) and its
 // item; returns the slot's frequency, -1 beyond the batch
