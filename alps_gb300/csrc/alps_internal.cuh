@@ -120,6 +120,7 @@ struct __align__(16) SpecDev {
   double pvc;         // 2 pi dpperp/4 (-q/(2 k_par)): the principal-value scale over smdelta
   double pcen, prad;  // centre and half-width of ppar[1..M-1]
   float pcen32, prad32;  // the same rounded to FP32
+  float gtol, ptol;   // places in spacings nearer than this to a node or a half-way point are not estimated
   int kfar;           // max Laurent terms used (<= ALPS_KFAR)
   int farn;           // first order of the far-order series, 0: none
   void* far;          // its coefficients by level (k_far_levels)
@@ -130,14 +131,15 @@ struct __align__(16) SpecDev {
   const double* fit_aux;
   // factorised Landau sums (one Maxwellian term): moments
   // lmom[((n*3 + F)*2 + w)*5 + m], reference row Gaussian exp(-p2r (p-p3r)^2),
-  // bounds of the row deviation delta_i(p) = la p^2 + lb p + lc, smallest a0
+  // bounds of the row deviation delta_i(p) = la p^2 + lb p + lc
   const double* lmom;
-  double p2r, p3r, la, lb, lc, min_a0;
+  double p2r, p3r, la, lb, lc;
   double lgc;  // exp(-p2r dppar^2)
   // the fast path's copy of the moments: per (n, F) ten float pairs scaled
   // by 2^-e (hi 0..9, lo 10..19, e at 20, 24 floats); the bound's
   // coefficients in FP32, lgc as a float pair, -2 p2r dppar, and the
-  // exponents of min_a0 and lgc (the underflow test of the row Gaussians)
+  // exponents of the smallest row amplitude and of lgc (the underflow test of
+  // the row Gaussians)
   const float* lmomf;
   float la32, lb32, lc32, lgch, lgcl;
   double lcx;

@@ -396,9 +396,10 @@ __device__ inline ResGeom res_geometry(const SpecDev& S, int M_I, double2 om, in
 
 // The same geometry without the reference's roundings where they cannot
 // matter: the resonance momentum's place in node units, to some 1e-13, settles
-// every index unless it lies within 1e-5 of a node or of a half-way point
-// (nodes are within 1e-6 of a spacing of their uniform positions).  Returns
-// false where res_geometry has to decide.  About 10 FP64 operations for some
+// every index unless it lies within gtol of a node or of a half-way point (1e-5,
+// and twice what the nodes may be off their uniform positions: accepted grids
+// have spacings within 1e-9 of one another, which adds up).  Returns false
+// where res_geometry has to decide.  About 10 FP64 operations for some
 // 150, on a part with two FP64 lanes per SM and clock.
 __device__ __forceinline__ bool res_geometry_fast(const SpecDev& S, int M_I, double2 om, int nn, double ikpar,
                                                   ResGeom& g) {
@@ -410,7 +411,7 @@ __device__ __forceinline__ bool res_geometry_fast(const SpecDev& S, int M_I, dou
   const double fv = floor(v);
   const int i = (int)fv;
   const float fr = (float)(v - fv);
-  if (!(fr > 1e-5f && fr < 0.99999f && fabsf(fr - 0.5f) > 1e-5f)) return false;
+  if (!(fr > S.gtol && fr < 1.0f - S.gtol && fabsf(fr - 0.5f) > S.gtol)) return false;
   g.res = i >= 1 - M_I && i < M - 1 + (M_I > 1 ? M_I : 1);
   g.ipar_res = i;
   g.lower = g.upper = 0;

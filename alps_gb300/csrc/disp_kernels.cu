@@ -1122,7 +1122,8 @@ __device__ void eval_fit3_d(const SpecDev& S, double vA, int iperp, double2 p, d
 //
 // The cuts are the reference's decisions.  An FP32 estimate in units of a
 // spacing, measured from the node next to p_res, settles each to 5e-6 of a
-// spacing; nearer, the search over the reference's own sample points does.
+// spacing (more where it is far from p_res, or the grid long: pv_cut); nearer,
+// the search over the reference's own sample points does.
 // Exactly half-way its rounded distances may exceed half a spacing to both
 // nodes: funct_g then falls back to the grid's second node, and such an item
 // is summed sample by sample (pv_direct).
@@ -1143,7 +1144,9 @@ __device__ void eval_fit3_d(const SpecDev& S, double vA, int iperp, double2 p, d
 // ---------------------------------------------------------------------------
 #define RES_WARPS 4
 #define PV_CHUNK 128   // samples a warp sums between two looks at the cuts
-#define PV_TOL 5e-6f   // a cut nearer than this (in spacings) to a sample is decided by the search
+#define PV_TOL 5e-6f   // a cut nearer than this (in spacings; SpecDev::ptol on long grids) to a sample is
+                       // decided by the search, and a distance's rounding more
+#define PV_DIST 4e-7f  // of a cut far from p_res, per spacing
 
 // scalar arithmetic of the principal-value sums: FP64 or double-float
 __device__ __forceinline__ double sc_add(double a, double b) { return a + b; }
@@ -1293,7 +1296,7 @@ __device__ __forceinline__ void pv_setup(const SpecDev& S, const SysDev& sys, co
   it.ft0 = (float)(ut - (double)it.jt0);
   it.dut = it.du * (float)it.cor;
   it.direct = 0;
-  if (fabsf(it.f0) > 0.5f - PV_TOL || (nt > 0 && fabsf(it.ft0) > 0.5f - PV_TOL)) {
+  if (fabsf(it.f0) > 0.5f - S.ptol || (nt > 0 && fabsf(it.ft0) > 0.5f - S.ptol)) {
     // the sample at p_res (or the tiny rest's first) half-way between nodes
     const PvExact x = pv_exact(S, sys, it, omr);
     const int j = pv_search(S, x.sym(0)), jt = pv_search(S, x.tiny(0));
@@ -1322,7 +1325,7 @@ __device__ __forceinline__ int pv_cut(const SpecDev& S, const SysDev& sys, const
   if (!(t < (float)K + 1.0f)) return K + 1;
   const float tr = rintf(t);
   int k = (side == 1) ? (int)floorf(t) + 1 : (int)ceilf(t);
-  if (fabsf(t - tr) * du < PV_TOL) {
+  if (fabsf(t - tr) * du < fmaf(PV_DIST, dist, S.ptol)) {
     k = (int)tr;
     const PvExact x = pv_exact(S, sys, it, omr);
     const int j = pv_search(S, side == 0 ? x.sym(k) : (side == 1 ? 2.0 * x.pr - x.sym(k) : x.tiny(k)));
@@ -3257,6 +3260,9 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->prad = bm ? 0.0 : 0.5 * (S.ppar[c->sys.npar - 1] - S.ppar[1]);
   o->pcen32 = (float)o->pcen;
   o->prad32 = (float)o->prad;
+  const float drift = 4e-9f * (float)c->sys.npar;
+  o->gtol = std::max(1e-5f, drift);
+  o->ptol = std::max(PV_TOL, drift);
   // the series is used only where it is cheaper than the node sum
   o->kfar = std::min(ALPS_KFAR, (int)(0.8 * (c->sys.npar - 1)));
   o->far = S.d_far;
@@ -3278,7 +3284,6 @@ void fill_spec_dev(const alps_ctx* c, int is, SpecDev* o) {
   o->la = S.la;
   o->lb = S.lb;
   o->lc = S.lc;
-  o->min_a0 = S.min_a0;
   o->lgc = std::exp(-S.p2r * o->dppar * o->dppar);  // dppar is 0 for closed-form species (no grid)
   o->lmomf = o->lmom ? reinterpret_cast<const float*>(S.d_lmom + (size_t)(S.nmax + 1) * 30) : nullptr;
   o->la32 = (float)S.la;
