@@ -169,6 +169,7 @@ void alps_destroy(alps_ctx* c) {
   cudaFree(c->d_rel);
   cudaFree(c->d_bm);
   cudaFree(c->d_flags);
+  cudaFree(c->d_hflags);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
   if (c->h_flag) cudaFreeHost(c->h_flag);
   if (c->ev_done) cudaEventDestroy(c->ev_done);

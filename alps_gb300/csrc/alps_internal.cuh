@@ -276,8 +276,9 @@ struct alps_ctx {
   double2* d_bm = nullptr;      // [n][S][24] NHDS chi (6) and chi_low (3 x 6)
   size_t bm_cap = 0;
   size_t ext_cap = 0;
-  int* d_flags = nullptr;       // two error words (the second of batches that report to the host), their counters
-  bool flags_dirty = false;     // the second one may be non-zero
+  int* d_flags = nullptr;       // error word and counters of small batches
+  int* d_hflags = nullptr;      // the same of batches that report to the host
+  bool flags_dirty = false;     // the latter's word may be non-zero
   bool defer_sync = false;      // set_k of a batch (alps_set_k_many): no per-context synchronisation
   // error word of the last asynchronous batch (alps_disp_batch_device: d_flags;
   // alps_disp_batch_noalloc: a word of the static scratch), read by

@@ -3684,36 +3684,38 @@ static int launch_disp_part(alps_ctx* c, int n, const double2* d_om, double2* d_
   if (a.has_bm)
     if ((rcode = ensure_buf(c->d_bm, c->bm_cap, (size_t)n * S_ * 24))) return rcode;
   if (!c->d_flags) {
-    // the error word, the error word of batches that report to hflag, and a
-    // counter per frequency of a small batch (zero between launches), once
-    // for the batches without hflag and once for those with it: the latter
-    // are over when their call returns, so nothing that a caller leaves
-    // running reaches their counters
-    ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, (2 + 2 * SMALL_WARPS) * sizeof(int)));
-    ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, (2 + 2 * SMALL_WARPS) * sizeof(int), st));
-    ALPS_CUDA_TRY(cudaStreamSynchronize(st));
-    c->flags_dirty = false;
+    // the error word, and a counter per frequency of a small batch (zero
+    // between launches)
+    ALPS_CUDA_TRY(cudaMalloc(&c->d_flags, (1 + SMALL_WARPS) * sizeof(int)));
+    ALPS_CUDA_TRY(cudaMemsetAsync(c->d_flags, 0, (1 + SMALL_WARPS) * sizeof(int), st));
   }
   const void* after[7] = {c->d_part, c->d_count, c->d_slot_nn, c->d_items, c->d_rel, c->d_bm, c->d_flags};
   for (int q = 0; q < 7; ++q)
     if (before[q] != after[q]) c->gen++;  // buffer addresses changed: cached graphs are stale
   const bool small = small_batch(c, bg);
-  // (the word of batches that report to hflag is zero while none reported)
   int* flags = c->d_flags;
   if (small && hflag) {
-    flags = c->d_flags + 1;
+    // a word and counters of their own: these batches are over when their call
+    // returns, so nothing that a caller leaves running reaches them, and the
+    // word is zero while none reported
+    if (!c->d_hflags) {
+      ALPS_CUDA_TRY(cudaMalloc(&c->d_hflags, (1 + SMALL_WARPS) * sizeof(int)));
+      ALPS_CUDA_TRY(cudaMemsetAsync(c->d_hflags, 0, (1 + SMALL_WARPS) * sizeof(int), st));
+      c->flags_dirty = false;
+    }
+    flags = c->d_hflags;
     if (c->flags_dirty) ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(int), st));
     c->flags_dirty = false;
   } else if (first) {
     // (with the counters: calls that a caller let overlap, against the
     // contract, leave nothing behind)
-    ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, (small ? 2 + n : 1) * sizeof(int), st));
+    ALPS_CUDA_TRY(cudaMemsetAsync(flags, 0, (small ? 1 + n : 1) * sizeof(int), st));
   }
   if (small) {
     DispJob job = lone_job(sh, n, S_, d_om, d_D, c->d_part, c->d_count, c->d_slot_nn, c->d_items, flags);
     job.ext = d_ext;
     job.nslots = (int)nslots;
-    job.arrive = c->d_flags + 2 + (hflag ? SMALL_WARPS : 0);
+    job.arrive = flags + 1;
     job.hflag = hflag;
     if ((rcode = launch_one(c, a, sh, job, st))) return rcode;
     if (flag_there) *flag_there = hflag != nullptr;
