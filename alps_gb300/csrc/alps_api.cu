@@ -315,7 +315,7 @@ int alps_prepare(alps_ctx* c) {
   if (!c) return ALPS_E_INVALID;
   for (int is = 0; is < c->sys.nspec; ++is)
     if (!c->spec[is].loaded) return ALPS_E_INVALID;
-  // the batched setup: every species' fit in one launch, one warp each
+  // the batched setup: every species' fit in one launch, one block each
   // (the reference's warm start orders the rows of a fit, not the species)
   if (ctx_batch_preparable(c)) return alps_prepare_many(&c, 1, nullptr);
   c->gen++;

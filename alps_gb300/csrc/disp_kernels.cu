@@ -2934,9 +2934,10 @@ __global__ void __launch_bounds__(32) k_far_orders(const DispJob* __restrict__ j
 
 // Summed from the highest order down and scaled to t = s / r: the series of all
 // orders |n| >= n0 for the levels n0 = farn .. farn + FAR_LEVELS - 1, FP64 or
-// float pairs.  A block per term and species, a thread per entry and g for
-// the running sums, then one per coefficient.  Both kernels together take 58 us for 30 + 7 orders.
-__global__ void __launch_bounds__(96) k_far_levels(const DispJob* __restrict__ jobs) {
+// float pairs.  A warp per term and species, a lane per entry and g for the
+// running sums, then one per coefficient in turn.  Both kernels together take
+// 58 us for 30 + 7 orders.
+__global__ void __launch_bounds__(32) k_far_levels(const DispJob* __restrict__ jobs) {
   __shared__ double sum[FAR_LEVELS][12];
   const DispJob& J = jobs[blockIdx.z];
   const int l = blockIdx.x, s = blockIdx.y;
@@ -4255,6 +4256,7 @@ extern "C" int alps_autotune(alps_ctx* c, int n, const alps_complex* d_om_in, al
     g_tune_epoch++;
     const BatchGeom bg = batch_geom(c, n, c->sys.nspec, maxn, a.rcap, false);
     out->js = bg.sh.js;
+    // (the default rule has no fixed number of either: nominal figures)
     out->blocks_per_sm = best.blocks_per_sm ? best.blocks_per_sm : 4;
     out->warps_per_sm = best.warps_per_sm ? best.warps_per_sm : 12;
     out->tuned = best.js != 0;

@@ -228,7 +228,7 @@ __device__ void fit_jacobian(const FitArgs& a, const double* params, int iperp, 
 // running sums; the step solves (J^T J + lambda diag) delta = J^T r by the
 // same partial-pivot elimination without forming the inverse.
 // On a 192x384 grid, two species: 35.7 ms as one warp with the sums in
-// series, 3.7 ms so.
+// series, 2.84 ms so.
 #define FIT_THREADS 128
 struct FitShared {
   double a[FIT_MAXP * (FIT_MAXP + 1)];  // normal matrix, right-hand side in the last column

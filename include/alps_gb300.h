@@ -155,7 +155,7 @@ int alps_get_f0_rel(alps_ctx* ctx, int is, double* gamma, double* pparbar, doubl
 /* alps_prepare for n contexts at once (the per-run setup of many plasmas,
  * e.g. of an uneven batch or a request server's pool).  The
  * Levenberg-Marquardt continuation fits of every (context, species) run in
- * one launch, one warp each: the reference's warm start over the p_perp
+ * one launch, one block each: the reference's warm start over the p_perp
  * rows orders a fit (src/ALPS_analyt.f90:518), but the fits of different
  * plasmas and species are independent.  Derivatives and ee terms of all
  * contexts run on a few streams; one synchronisation in all.  Contexts
@@ -539,7 +539,8 @@ int alps_tc_product(const double* d_A, const double* d_B, double* d_C, int M,
  * fused and no-allocation batches of a bucket use the same shape.  No
  * reference counterpart: ALPS has one fixed loop order. */
 typedef struct alps_tune_result {
-  int js, blocks_per_sm, warps_per_sm; /* the shape the bucket now uses          */
+  int js, blocks_per_sm, warps_per_sm; /* the shape the bucket now uses (tuned 0: */
+                                       /* the default's lanes, nominally 4 and 12) */
   int tuned;                           /* 1: a candidate beat the default rule   */
   int candidates;                      /* shapes timed                           */
   double ms_default, ms_best;          /* per batch: default rule, chosen shape  */
@@ -571,7 +572,8 @@ int alps_get_stats(alps_ctx* ctx, alps_stats* st);
 /* Measurement support: when on, every disp batch records CUDA events around
  * its four kernels (classify, pole sums, resonant items, finalize) on the
  * stream it runs on; alps_get_profile returns the summed device milliseconds
- * per kernel and the number of batches since profiling was switched on. */
+ * per kernel and the number of batches since profiling was switched on (of a
+ * large batch with tensors, which runs in parts, the number of parts). */
 int alps_set_profiling(alps_ctx* ctx, int on);
 int alps_get_profile(alps_ctx* ctx, double* ms /* [4] */, int64_t* batches);
 
