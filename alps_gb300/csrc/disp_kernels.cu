@@ -3547,8 +3547,10 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
     if (scratch_layout(c, n, b.nslots, part, false, off) <= ALPS_NOALLOC_SCRATCH_BYTES) {
       // (a batch that fits without the far-order tables alone does without
       // the series, through every entry point)
-      if (sh.far && scratch_layout(c, n, b.nslots, part, true, off) > ALPS_NOALLOC_SCRATCH_BYTES) sh.far = 0;
-      scratch_layout(c, n, b.nslots, part, sh.far != 0, off);
+      if (sh.far && scratch_layout(c, n, b.nslots, part, true, off) > ALPS_NOALLOC_SCRATCH_BYTES) {
+        sh.far = 0;
+        scratch_layout(c, n, b.nslots, part, false, off);
+      }
       const long room = (long)((ALPS_NOALLOC_SCRATCH_BYTES - off[SC_PART]) / row);
       csize = std::max(csize, (2L * maxn + room) / room);
     }

@@ -930,8 +930,9 @@ __device__ RelSums rel_cut_sums(const RelSamples& q, double dI2, bool from0, int
 // of one node and linear in p, so each piece needs only the sums of its
 // samples' weights and of their first moments; the samples are summed once,
 // as prefix sums, for both sides of the window, and each lane cuts them at
-// the ends of its piece.  Returns the number of pieces left in rec; more: there
-// are further parts.
+// the ends of its piece.  Returns the number of pieces left in rec.  WIDE: those
+// of one part; more: there are further parts.
+template <bool WIDE>
 __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, int ig, int part, double* pre,
                           RelPiece* rec, int lane, bool& more) {
   const double* pb = S.prel;
@@ -947,7 +948,7 @@ __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, i
   if (sym) {
     const int jc = rel_piece(S, dR);  // the pole's own interval (the window lies inside the grid)
     const int nu = max(0, rel_piece(S, dR + cap) - jc) + 1, nd = max(0, jc - rel_piece(S, 2.0 * dR - (dR + cap))) + 1;
-    const int first = part * REL_PART, last = min(nu + nd, sy.M_I > REL_WIDE ? first + REL_PART : cap_rec);
+    const int first = WIDE ? part * REL_PART : 0, last = min(nu + nd, WIDE ? first + REL_PART : cap_rec);
     for (int t0 = first; t0 < last; t0 += 32) {
       const int t = t0 + lane;
       const bool has = t < last, down = t >= nu;
@@ -999,7 +1000,7 @@ __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, i
       }
     }
     nrec = last - first;
-    if (sy.M_I > REL_WIDE && last < nu + nd) {
+    if (WIDE && last < nu + nd) {
       more = true;
       __syncwarp();
       return nrec;
@@ -1131,7 +1132,9 @@ __device__ bool rel_resonant(const SpecDev& S, const SysDev& sy, double2 om, int
 // more nodes with complex weights.  Rows' decisions are taken a row per lane,
 // and so are the Landau rows, by one warp beside the others.
 // 8 frequencies, 41 signed orders, 100x200 (Gamma, pparbar): 5340 us before,
-// 304 us so.
+// 304 us so.  WIDE: windows of more than REL_WIDE nodes to a side (a loop over
+// the parts costs the others 7 us of those).
+template <bool WIDE>
 __global__ void __launch_bounds__(REL_THREADS) k_rel_orders(RelArgs a, const double2* __restrict__ om, int n_om,
                                                             double2* __restrict__ out, int* flags) {
   extern __shared__ __align__(16) double rel_smem[];
@@ -1264,7 +1267,8 @@ __global__ void __launch_bounds__(REL_THREADS) k_rel_orders(RelArgs a, const dou
         }
         bool more = r.pv;
         for (int part = 0; more; ++part) {
-          const int nrec = rel_pieces(S, sy, r, ig, part, wsm, rec, lane, more);
+          const int nrec = rel_pieces<WIDE>(S, sy, r, ig, part, wsm, rec, lane, more);
+          more = WIDE && more;
           int a0 = np, a1 = 0;
           for (int t = lane; t < nrec; t += 32) {
             a0 = min(a0, rec[t].a);
@@ -1381,9 +1385,10 @@ int launch_rel_orders(const SysDev& sys, const SpecDev* sp, int relcap, int n, c
   a.relcap = relcap;
   if (!any || n <= 0) return ALPS_OK;
   const size_t smem = REL_WARPS * rel_warp_words(sys.M_I) * sizeof(double);
+  auto kernel = sys.M_I > REL_WIDE ? k_rel_orders<true> : k_rel_orders<false>;
   if (smem > 40 * 1024)
-    ALPS_CUDA_TRY(cudaFuncSetAttribute(k_rel_orders, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_rel_orders<<<dim3(n, 2 * relcap * REL_RB, sys.nspec), REL_THREADS, smem, st>>>(a, d_om, n, d_out, d_flags);
+    ALPS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<dim3(n, 2 * relcap * REL_RB, sys.nspec), REL_THREADS, smem, st>>>(a, d_om, n, d_out, d_flags);
   ALPS_CUDA_TRY(cudaGetLastError());
   return ALPS_OK;
 }
