@@ -3457,11 +3457,11 @@ int tensor_lanes(long u) { return u < 100 ? 32 : (u < 300 ? 16 : (u < 900 ? 8 : 
 // Slots per warp of k_resonant_multi at most where it only takes what the lanes
 // left.  Where the Landau terms do not factorise that is every damped order by
 // its rows, and the warps' times differ: two Maxwellians on a 64x128 grid,
-// 2600, 16384 and 50000 frequencies, us in all: 32 slots 1093, 5221, 13789;
-// 64: 1093, 5438, 14232; 128: 1090, 5944, 15369; 256 and more 3969, 7154, 14845.
-// With nothing left the blocks end at once: 150000 frequencies 4316 us with 32
-// slots, 4315 with 1824 warps in all.
-const int RES_LEFT_IPW = 32;
+// 2600, 16384 and 150000 frequencies, us in all: 32 slots 1093, 5221, 39396;
+// 64: 1093, 5438, 39746; 128: 1090, 5944, 40635; 256 and more 3969, 7154, 40521.
+// With nothing left the blocks end at once, which very many of them feel: sixteen
+// times what the chip holds at most.
+inline int res_left_per_warp(long nslots) { return (int)std::max(32L, std::min(256L, nslots / (152L * 12 * 16))); }
 // The far-order series takes the orders |n| >= n0 of a frequency (some two
 // thirds of them) in 44 terms; its coefficients are built for each batch.
 // Pole sums by single orders and so, with the 58 us of the coefficients (128x256
@@ -3571,7 +3571,7 @@ BatchGeom batch_geom(const alps_ctx* c, int n, int S_, int maxn, int rcap, bool 
     // about a third of the slots is occupied: 96 fill a warp's lanes once
     const long per = ((long)b.nslots / (152 * 12) + 31) / 32 * 32;
     sh.lanes = (int)std::max(96L, std::min(256L, per));
-    sh.ipw = std::min(sh.ipw, RES_LEFT_IPW);
+    sh.ipw = std::min(sh.ipw, res_left_per_warp((long)b.nslots));
   }
   sh.fin_warp = (n <= FIN_WARP_MAX || tensors || rel_capacity(c) || any_bm(c)) ? 1 : 0;
   return b;
@@ -3957,9 +3957,9 @@ int prepare_disp_multi(alps_ctx* const* ctx, const int* n, int nj, const double2
   blk[2] = 0;
   for (int j = 0; j < nj; ++j) {
     DispJob& J = m->h_jobs[j];
-    J.sh.ipw = J.sh.lanes ? std::min(ipw, RES_LEFT_IPW) : ipw;
-    J.blk[2] = blk[2];
     const long nsl = (long)((j + 1 < nj ? o_slots[j + 1] : slots_n) - o_slots[j]);
+    J.sh.ipw = J.sh.lanes ? std::min(ipw, res_left_per_warp(nsl)) : ipw;
+    J.blk[2] = blk[2];
     blk[2] += (nsl + RES_WARPS * J.sh.ipw - 1) / (RES_WARPS * J.sh.ipw);
   }
   int rcode;
