@@ -439,6 +439,12 @@ __device__ __forceinline__ bool res_geometry_fast(const SpecDev& S, int M_I, dou
   return true;
 }
 
+// The samples of a principal-value window's rest: the quotient's whole part.
+// One that no int holds (a window of no width: no principal positions and the
+// pole on a node) counts none, as the reference's conversion gives on x86, where
+// it is the least int.
+__device__ __forceinline__ int rest_samples(double q) { return q < 2147483647.0 ? (int)q : 0; }
+
 // the fast form, and the exact one (out of line: it is seldom needed) where
 // it does not settle the geometry
 static __device__ __noinline__ void res_geometry_exact(const SpecDev& S, int M_I, double2 om, int nn, double kpar, ResGeom& g) {

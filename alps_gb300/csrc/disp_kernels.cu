@@ -1279,11 +1279,11 @@ __device__ __forceinline__ void pv_setup(const SpecDev& S, const SysDev& sys, co
   it.sm = cap * sys.iM_P;
   // ntiny = floor(rest / smdelta); the reference's own quotient near integers
   const double rest = S.ppar[g.upper] - g.pr - cap, q = rest * rcp_fast(it.sm);
-  int nt = (int)q;
+  int nt = rest_samples(q);
   if (!(fabs(q - rint(q)) > 1e-6)) {
     it.ntiny = 0;
     const PvExact x = pv_exact(S, sys, it, omr);
-    nt = (int)((S.ppar[g.upper] - x.pr - x.cap) / x.sm);
+    nt = rest_samples((S.ppar[g.upper] - x.pr - x.cap) / x.sm);
   }
   it.ntiny = nt;
   it.cor = nt > 0 ? q * rcp_fast((double)nt) : 0.0;
@@ -1410,19 +1410,21 @@ __host__ __device__ inline size_t pv_warp_words(int M_I) {
   return (PV_CHUNK * 24 + 15) / 16 + np * (sizeof(PvPiece<double>) / 16) + np;
 }
 
-// prefix sums at the lane's cut kc (see pv_sample); pre: PV_CHUNK PvSums
+// prefix sums at the lane's cut kc (see pv_sample); pre: PV_CHUNK PvSums (a
+// chunk's first sample is unsigned: the last chunk of the most samples ends
+// past the largest int)
 template <typename T>
 __device__ __forceinline__ PvSums<T> pv_cut_sums(const PvScal<T>& c, int K, bool tiny, bool sym, int kc,
                                                  PvSums<T>* pre, int lane) {
   const T z = sc_of<T>(0.0);
   PvSums<T> out = {z, z, z}, carry = {z, z, z};
-  for (int k0 = 0; k0 <= K; k0 += PV_CHUNK) {
-    const int n = min(PV_CHUNK, K + 1 - k0), per = (n + 31) / 32;
+  for (unsigned k0 = 0; k0 <= (unsigned)K; k0 += PV_CHUNK) {
+    const int n = (int)min((unsigned)PV_CHUNK, (unsigned)K + 1u - k0), per = (n + 31) / 32;
     const int b = min(n, lane * per), e = min(n, b + per);
     PvSums<T> loc = {z, z, z};
     for (int j = b; j < e; ++j) {
       pre[j] = loc;
-      pv_sample(loc, c, k0 + j, K, tiny, sym);
+      pv_sample(loc, c, (int)k0 + j, K, tiny, sym);
     }
     PvSums<T> inc = loc;
     for (int o = 1; o < 32; o <<= 1) {
@@ -1444,7 +1446,8 @@ __device__ __forceinline__ PvSums<T> pv_cut_sums(const PvScal<T>& c, int K, bool
     carry = {sc_add(carry.s1, sc_shfl(inc.s1, 31)), sc_add(carry.s2, sc_shfl(inc.s2, 31)),
              sc_add(carry.s3, sc_shfl(inc.s3, 31))};
     __syncwarp();
-    if (kc >= k0 && kc < k0 + n) out = pre[kc - k0];
+    const int at = kc - (int)k0;
+    if (at >= 0 && at < n) out = pre[at];
     __syncwarp();
   }
   if (kc > K) out = carry;
@@ -1606,17 +1609,17 @@ __device__ __noinline__ void pv_direct(const SpecDev& S, const SysDev& sys, cons
     }
   };
   if (fabs(y) > sys.Tlim) {
-    for (int k = lane; k <= M_P; k += 32) {
-      const double p = x.sym(k), dx = p - x.pr;
-      const double r = ((k == 0 || k == M_P) ? 1.0 : 2.0) * rcp_fast(fma(dx, dx, y2));
+    for (unsigned k = lane; k <= (unsigned)M_P; k += 32) {
+      const double p = x.sym((int)k), dx = p - x.pr;
+      const double r = ((k == 0 || k == (unsigned)M_P) ? 1.0 : 2.0) * rcp_fast(fma(dx, dx, y2));
       add(p, cmk(dx * r, y * r));
       add(2.0 * x.pr - p, cmk(-dx * r, y * r));
     }
   } else {
     double fr = 0.0;
-    for (int k = 1 + lane; k <= M_P; k += 32) {
-      const double d = x.sym(k) - x.pr;
-      fr += (k == M_P ? 1.0 : 2.0) * ((d * d) / (d * d + y2));
+    for (unsigned k = 1 + lane; k <= (unsigned)M_P; k += 32) {
+      const double d = x.sym((int)k) - x.pr;
+      fr += (k == (unsigned)M_P ? 1.0 : 2.0) * ((d * d) / (d * d + y2));
     }
     for (int off = 16; off > 0; off >>= 1) fr += __shfl_xor_sync(FULL_WARP, fr, off);
     const double c = fr * S.idppar;
@@ -1624,9 +1627,9 @@ __device__ __noinline__ void pv_direct(const SpecDev& S, const SysDev& sys, cons
     if (lane == 1) add(x.pr - S.dppar, cmk(-c, 0.0));
     if (lane == 2 && y != 0.0) add(x.pr, cmk(0.0, (y > 0.0 ? 2.0 : -2.0) * ALPS_PI / x.sm));
   }
-  for (int k = lane; k <= it.ntiny && it.ntiny > 0; k += 32) {
-    const double p = x.tiny(k), dx = p - x.pr;
-    const double r = ((k == 0 || k == it.ntiny) ? 1.0 : 2.0) * x.cor * rcp_fast(fma(dx, dx, y2));
+  for (unsigned k = lane; k <= (unsigned)it.ntiny && it.ntiny > 0; k += 32) {
+    const double p = x.tiny((int)k), dx = p - x.pr;
+    const double r = ((k == 0 || k == (unsigned)it.ntiny) ? 1.0 : 2.0) * x.cor * rcp_fast(fma(dx, dx, y2));
     add(p, cmk(dx * r, y * r));
   }
   int first, cnt;

@@ -888,12 +888,12 @@ struct RelSamples {
 };
 __device__ RelSums rel_cut_sums(const RelSamples& q, double dI2, bool from0, int kc, double* pre, int lane) {
   RelSums out = {0.0, 0.0, 0.0}, carry = {0.0, 0.0, 0.0};
-  for (int k0 = 0; k0 <= q.K; k0 += REL_CHUNK) {
-    const int n = min(REL_CHUNK, q.K + 1 - k0), per = (n + 31) / 32;
+  for (unsigned k0 = 0; k0 <= (unsigned)q.K; k0 += REL_CHUNK) {
+    const int n = (int)min((unsigned)REL_CHUNK, (unsigned)q.K + 1u - k0), per = (n + 31) / 32;
     const int b = min(n, lane * per), e = min(n, b + per);
     RelSums loc = {0.0, 0.0, 0.0};
     for (int j = b; j < e; ++j) {
-      const int k = k0 + j;
+      const int k = (int)k0 + j;
       pre[3 * j] = loc.s1;
       pre[3 * j + 1] = loc.s2;
       pre[3 * j + 2] = loc.s3;
@@ -917,7 +917,7 @@ __device__ RelSums rel_cut_sums(const RelSamples& q, double dI2, bool from0, int
     carry.s2 = __shfl_sync(0xffffffffu, bef.s2 + loc.s2, 31);
     carry.s3 = __shfl_sync(0xffffffffu, bef.s3 + loc.s3, 31);
     __syncwarp();
-    const int at = kc - k0;
+    const int at = kc - (int)k0;
     if (at >= 0 && at < n) out = {pre[3 * at], pre[3 * at + 1], pre[3 * at + 2]};
     __syncwarp();
   }
@@ -1022,9 +1022,7 @@ __device__ int rel_pieces(const SpecDev& S, const SysDev& sy, const RelRow& r, i
     nrec = 3;
   }
   // the tiny rest between dR + capDelta and the upper limit
-  // (bounded: a window of no width, possible only with no principal positions, would ask for 2^31)
-  const double rest = (pb[r.up] - dR - cap) / sm;
-  const int ntiny = rest < 4194304.0 ? (int)rest : (rest >= 4194304.0 ? 4194304 : 0);
+  const int ntiny = rest_samples((pb[r.up] - dR - cap) / sm);
   if (ntiny > 0) {
     q.corr = ((pb[r.up] - dR - cap) / (1.0 * ntiny)) / sm;
     q.K = ntiny;
