@@ -1315,7 +1315,8 @@ __device__ __forceinline__ void pv_setup(const SpecDev& S, const SysDev& sys, co
 // First sample k beyond piece i of a side (0: p_k upwards from p_res, 1: the
 // mirrored points downwards, 2: the tiny rest upwards): i + 1/2 spacings from
 // the side's first node.  A point half-way belongs to the upper node; lost: to
-// none.
+// none.  FAR: a cut may lie more than a dozen spacings from p_res.
+template <bool FAR>
 __device__ __forceinline__ int pv_cut(const SpecDev& S, const SysDev& sys, const PvItem& it, double omr, int side,
                                       int i, bool& lost) {
   const int K = side == 2 ? it.ntiny : sys.M_P;
@@ -1325,7 +1326,7 @@ __device__ __forceinline__ int pv_cut(const SpecDev& S, const SysDev& sys, const
   if (!(t < (float)K + 1.0f)) return K + 1;
   const float tr = rintf(t);
   int k = (side == 1) ? (int)floorf(t) + 1 : (int)ceilf(t);
-  if (fabsf(t - tr) * du < fmaf(PV_DIST, dist, S.ptol)) {
+  if (fabsf(t - tr) * du < (FAR ? fmaf(PV_DIST, dist, S.ptol) : S.ptol)) {
     k = (int)tr;
     const PvExact x = pv_exact(S, sys, it, omr);
     const int j = pv_search(S, side == 0 ? x.sym(k) : (side == 1 ? 2.0 * x.pr - x.sym(k) : x.tiny(k)));
@@ -1483,8 +1484,8 @@ __device__ bool pv_warp_weights(const SpecDev& S, const SysDev& sys, const PvIte
     const int most = 2 * (sys.M_I + 4);
     for (int t0 = 0; t0 < most; t0 += 32) {
       const int t = t0 + lane, side = t & 1, i = t >> 1;
-      const int kb = i == 0 ? 0 : pv_cut(S, sys, it, omr, side, i - 1, lost);
-      const int ke = pv_cut(S, sys, it, omr, side, i, lost);
+      const int kb = i == 0 ? 0 : pv_cut<true>(S, sys, it, omr, side, i - 1, lost);
+      const int ke = pv_cut<true>(S, sys, it, omr, side, i, lost);
       const bool has = t < most && kb <= M_P;
       const PvSums<T> se = pv_cut_sums(c, M_P, false, true, has ? ke : 0, pre, lane);
       PvSums<T> sb;
@@ -1527,7 +1528,7 @@ __device__ bool pv_warp_weights(const SpecDev& S, const SysDev& sys, const PvIte
   }
   if (it.ntiny > 0) {
     const int i = lane;
-    const int ke = pv_cut(S, sys, it, omr, 2, i, lost), kb = i == 0 ? 0 : pv_cut(S, sys, it, omr, 2, i - 1, lost);
+    const int ke = pv_cut<true>(S, sys, it, omr, 2, i, lost), kb = i == 0 ? 0 : pv_cut<true>(S, sys, it, omr, 2, i - 1, lost);
     const bool has = i < 6 && kb <= it.ntiny;
     const PvSums<T> se = pv_cut_sums(c, it.ntiny, true, true, has ? ke : 0, pre, lane);
     PvSums<T> sb;
@@ -2339,7 +2340,7 @@ __device__ __forceinline__ bool pv_lane(const SpecDev& S, const SysDev& sys, con
     unsigned long long pk = ~0ull;
 #pragma unroll 1
     for (int i = 0; i <= most; ++i) {
-      const int k = pv_cut(S, sys, it, o.x, sd, i, lost);
+      const int k = pv_cut<false>(S, sys, it, o.x, sd, i, lost);  // (at most pvl_side's eight spacings)
       if (k > K) break;
       ok = ok && k > last && i < most;
       last = k;
